@@ -99,7 +99,6 @@ struct NodeSet {
 };
 
 enum { D_NONE = 0, D_REFINE = 1, D_COARSEN = 2 };
-enum { PF_LEAF = 1, PF_DELETED = 2, PF_VISITED = 4 };
 
 __device__ __forceinline__ int64_t find_key(const uint64_t *__restrict__ keys, int64_t n, uint64_t k) {
     int64_t lo = 0, hi = n;
@@ -130,7 +129,7 @@ __device__ __forceinline__ int64_t find_key_set(const NodeSet &A, uint64_t k) {
 // find_key on the leaf table, within k's background cell (T.rfirst)
 __device__ __forceinline__ int64_t find_key_t(const Tables &T, uint64_t k) {
     const int64_t r = (int64_t)(k >> 34);
-    if (!T.rfirst || r >= T.nroots) return find_key_t(T, k);
+    if (!T.rfirst || r >= T.nroots) return find_key(T.lkey, T.NL, k);
     int64_t lo = __ldg(T.rfirst + r), hi = __ldg(T.rfirst + r + 1);
     while (lo < hi) {
         const int64_t mid = (lo + hi) >> 1;
@@ -279,24 +278,10 @@ __global__ void k_internal_vals(int64_t NInt, const uint64_t *ikey, double4 *iva
     ival[i] = mean4(c[0], c[1], c[2], c[3]);
 }
 
-// ------------------------------------------------------------- sorting
-__global__ void k_iota(int64_t n, int32_t *o) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i < n) o[i] = (int32_t)i;
-}
-__global__ void k_gather_nodes(int64_t n, const int32_t *perm, const uint8_t *leaf_in, const double4 *val_in,
-                               uint8_t *leaf_out, double4 *val_out) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    leaf_out[i] = leaf_in[perm[i]];
-    val_out[i] = val_in[perm[i]];
-}
-
 struct AmrCtx {
     fdm_handle *h;
     NodeSet A, B;          // current / next node set
     int a = 0;             // which buffer triple (amr[0..2] or amr[3..5]) holds A
-    int64_t cap = 0;       // capacity of both triples
 };
 
 static void bind_sets(fdm_handle *h, AmrCtx &X) {
@@ -317,20 +302,12 @@ static void swap_sets(fdm_handle *h, AmrCtx &X) {
     std::swap(X.A.n, X.B.n);
     bind_sets(h, X);
 }
-// room for n nodes in both triples; the contents of both are dropped when
-// they have to grow (callers grow only before writing into B, after A's last
-// reader has finished)
-static int grow_nodes(fdm_handle *h, AmrCtx &X, int64_t n) {
-    if (n <= X.cap) return FDM_OK;
-    FDM_CK(h, cudaStreamSynchronize(h->s));
-    int64_t c = n + n / 2 + 1024;
-    if (c < 2 * X.cap) c = 2 * X.cap;   // geometric growth while a run refines from its background mesh
-    for (int s = 0; s < 2; ++s) {
-        FDM_CK(h, h->amr[3 * s + 0].ensure(c * 8));
-        FDM_CK(h, h->amr[3 * s + 1].ensure(c));
-        FDM_CK(h, h->amr[3 * s + 2].ensure(c * 32));
-    }
-    X.cap = c;
+// room for n nodes in the next set; the current one stays as it is
+static int grow_next(fdm_handle *h, AmrCtx &X, int64_t n) {
+    const int b = 1 - X.a;
+    FDM_CK(h, h->amr[3 * b + 0].ensure(n * 8));
+    FDM_CK(h, h->amr[3 * b + 1].ensure(n));
+    FDM_CK(h, h->amr[3 * b + 2].ensure(n * 32));
     bind_sets(h, X);
     return FDM_OK;
 }
@@ -365,18 +342,6 @@ static void merge_into(fdm_handle *h, const uint64_t *keys, const uint8_t *leaf,
         k_merge_runs<<<nblk(n, 256), 256, 0, h->s>>>(keys, leaf, val, m, keys + m, leaf + m, val + m, n - m, out);
     out.n = n;
 }
-// (keys, leaf, val) of length n, already in key order, into out
-static int copy_into(fdm_handle *h, int64_t n, const uint64_t *keys, const uint8_t *leaf, const double4 *val,
-                     NodeSet &out) {
-    if (n > 0) {
-        FDM_CK(h, cudaMemcpyAsync(out.key, keys, n * 8, cudaMemcpyDeviceToDevice, h->s));
-        FDM_CK(h, cudaMemcpyAsync(out.leaf, leaf, n, cudaMemcpyDeviceToDevice, h->s));
-        FDM_CK(h, cudaMemcpyAsync(out.val, val, n * 32, cudaMemcpyDeviceToDevice, h->s));
-    }
-    out.n = n;
-    return FDM_OK;
-}
-
 // per-cell index of A's keys (amr[22]) for the root-confined searches
 static int index_set(fdm_handle *h, NodeSet &A) {
     const int64_t nroots = (int64_t)h->G.m * h->G.n;
@@ -636,8 +601,10 @@ __global__ void k_gm1_count(int64_t n, Links L, const int8_t *d, int32_t *cnt) {
     if (x >= n) return;
     cnt[x] = ancestor_coarsened(L, d, (int32_t)x) ? 0 : (d[x] == D_REFINE ? 5 : 1);
 }
-__global__ void k_gm1_emit(NodeSet A, Links L, const int8_t *d, const int32_t *off, uint64_t *okey, uint8_t *oleaf,
-                           double4 *oval) {
+__global__ void k_gm1_emit(NodeSet A, Links L, const int8_t *d, const int32_t *off, NodeSet out) {
+    uint64_t *okey = out.key;
+    uint8_t *oleaf = out.leaf;
+    double4 *oval = out.val;
     const int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (x >= A.n || ancestor_coarsened(L, d, (int32_t)x)) return;
     const int64_t o = off[x];
@@ -656,439 +623,52 @@ __global__ void k_gm1_emit(NodeSet A, Links L, const int8_t *d, const int32_t *o
 }
 
 // ----------------------------------------------------------- gridmodify4
-// live neighbour (src/neighbor.F90:65-196) on a sorted node set: the
-// same-level node, else the deepest existing ancestor of it (a leaf)
-__device__ int64_t live_nb_set(const NodeSet &A, const Geometry &G, uint64_t k, int dir) {
-    uint64_t t;
-    if (!shift_key(G, k, dir, t)) return -1;
-    for (;;) {
-        const int64_t i = find_key_set(A, t);
-        if (i >= 0) return i;
-        if ((t & 15u) == 0) return -1;
-        t = parent_key(t);
-    }
-}
-// leaves that can act in gridmodify4 (a neighbour, or the neighbour's
-// neighbour, two or more levels coarser).  Later refinements of leaves only
-// make neighbours finer; the one way a region gets coarser during the pass
-// (a non-leaf refinement dropping a deep subtree) queues the leaves around
-// it (push_ring)
-__global__ void k_gm4_triggers(NodeSet A, Geometry G, int32_t *flag, uint64_t *rank, int32_t *idx) {
-    const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (c >= A.n) return;
-    int f = 0;
-    if (A.leaf[c]) {
-        const uint64_t k = A.key[c];
-        const int lc = (int)(k & 15u);
-        const int dirs[4] = {DIR_RIGHT, DIR_LEFT, DIR_UP, DIR_DOWN};
-        for (int t = 0; t < 4 && !f; ++t) {
-            const int64_t nb = live_nb_set(A, G, k, dirs[t]);
-            if (nb < 0) continue;
-            if ((int)(A.key[nb] & 15u) <= lc - 2) { f = 1; break; }
-            const int64_t nn = live_nb_set(A, G, A.key[nb], dirs[t]);
-            if (nn >= 0 && (int)(A.key[nn] & 15u) <= lc - 2) f = 1;
-        }
-    }
-    flag[c] = f;
-    rank[c] = visit_rank(A.key[c]);
-    idx[c] = (int32_t)c;
-}
+// gridmodify4 (src/mesh.F90:355-395) visits the leaves in traversal order
+// (sons 1,2,3,4), those created ahead of the traversal included.  A leaf c
+// looks right, left, up, down: it refines a neighbour two or more levels
+// coarser, then that neighbour's neighbour in the same direction when that
+// one is.  Every Refine_cell therefore has a time of its own, (visit rank of
+// c, direction, neighbour or neighbour's neighbour), and the whole pass is
+// the map t: node -> time of its Refine_cell (GM4_NEVER if none), which
+// obeys, for every leaf c that is still a leaf when its turn comes,
+//
+//     t(N) = min over the looks that find N two levels coarser of their time,
+//
+// where a look at time T sees the node set as it is then: a node exists at T
+// when its father was refined before T.  So a look depends on earlier times
+// only; t is the unique fixpoint, and iterating "all looks from the current
+// estimate of t" reaches it: after k sweeps every Refine_cell whose chain of
+// causes has at most k links is final, and a sweep that changes nothing
+// proves the rest.  A chain has a link per level of a cascade and per leaf
+// whose look an earlier refinement answers differently, 4 to 9 sweeps on the
+// developed four-quadrant and double Mach meshes.
+//
+// The one effect outside the map is the Refine_cell of a node that has sons
+// (:389-392), which drops its subtree.  Its time is known at the fixpoint
+// (the earliest look that finds such a node); the node set up to and
+// including it is then written out and the pass goes on from that time on
+// the new set.  It happens about once in 1300 refinements.
 
-// An item of the replay: mk = visit rank * 2, + 1 for a leaf queued ahead of
-// the traversal (so that on equal rank the initial trigger comes first), its
-// pool index and the generation it was queued with.
-struct __align__(16) HEnt {
-    uint64_t mk;
-    int32_t idx, gen;
-};
-// Hash table of the pool: open addressing over buckets of 8 entries, one
-// 128-byte line each (8 keys, then 8 slot words).  A key's probe sequence is
-// its home bucket's entries in order, then the next buckets' (linear
-// probing from a bucket boundary), so at the table's load (a quarter or
-// less) one bucket read settles a lookup but about once in a thousand.
-constexpr int HB = 8;
-struct __align__(128) HBucket {
-    uint64_t key[HB];
-    int32_t slot[HB];    // pool index (| SLOT_DEL when deleted), -1 empty
-    int32_t pad[HB];
-};
-constexpr int HB_COPY = 96;   // the bytes of a bucket that a probe reads (keys and slots)
-struct Pool {
-    uint64_t *key;
-    uint8_t *flags;
-    int32_t *gen;
-    double4 *val;
-    HBucket *tab;
-    uint64_t bmask;      // buckets - 1
-    int64_t cap;         // pool capacity
-    int64_t *n;          // pool size (device counter)
-    HEnt *heap;          // heap of leaves to visit ahead of the traversal (spill)
-    int64_t hcap;
-    int32_t *err;        // [0] capacity exceeded, [1] visits, [2] non-leaf refines, [3] step limit,
-                         // [4] refines, [5] replay steps
-};
-constexpr int32_t SLOT_DEL = 0x40000000;
-// Home bucket hash: the key folded to 32 bits, then MurmurHash3's 32-bit
-// finaliser (A. Appleby, public domain); 32-bit multiplies only
-__device__ __forceinline__ uint64_t hmix(uint64_t k) {
-    uint32_t x = (uint32_t)k ^ ((uint32_t)(k >> 32) * 0x9E3779B1u);
-    x ^= x >> 16; x *= 0x85EBCA6Bu; x ^= x >> 13; x *= 0xC2B2AE35u; x ^= x >> 16;
-    return x;
-}
-__device__ __forceinline__ uint64_t hhome(const Pool &P, uint64_t k) { return hmix(k) & P.bmask; }
-__device__ __forceinline__ int32_t *hslot(const Pool &P, uint64_t pos) { return &P.tab[pos >> 3].slot[pos & 7]; }
-__device__ __forceinline__ uint64_t *hkey(const Pool &P, uint64_t pos) { return &P.tab[pos >> 3].key[pos & 7]; }
-// the entry after pos in every probe sequence through it
-__device__ __forceinline__ uint64_t hnext(const Pool &P, uint64_t pos) {
-    return (pos & 7) == 7 ? (((pos >> 3) + 1) & P.bmask) << 3 : pos + 1;
-}
-// key k in bucket b, read from memory: 1 found at entry e (slot word s),
-// 0 absent (e = the first empty entry), -1 every entry holds another key
-__device__ __forceinline__ int hscan_mem(const Pool &P, uint64_t b, uint64_t k, int &e, int32_t &s) {
-    for (int j = 0; j < HB; ++j) {
-        s = P.tab[b].slot[j];
-        if (s == -1) { e = j; return 0; }
-        if (P.tab[b].key[j] == k) { e = j; return 1; }
-    }
-    return -1;
-}
-// the same on the copy of a bucket in shared memory, without branches: bit
-// masks of the empty entries and of the entries holding k, then the first of
-// each
-__device__ __forceinline__ int hscan_copy(const unsigned char *c, uint64_t k, int &e, int32_t &s) {
-    const ulonglong2 *kp = reinterpret_cast<const ulonglong2 *>(c);
-    const int4 *sp = reinterpret_cast<const int4 *>(c + HB * 8);
-    unsigned em = 0, mm = 0;
-#pragma unroll
-    for (int j = 0; j < HB / 2; ++j) {
-        const ulonglong2 v = kp[j];
-        mm |= (v.x == k ? 1u : 0u) << (2 * j);
-        mm |= (v.y == k ? 1u : 0u) << (2 * j + 1);
-    }
-#pragma unroll
-    for (int j = 0; j < HB / 4; ++j) {
-        const int4 v = sp[j];
-        em |= (v.x == -1 ? 1u : 0u) << (4 * j);
-        em |= (v.y == -1 ? 1u : 0u) << (4 * j + 1);
-        em |= (v.z == -1 ? 1u : 0u) << (4 * j + 2);
-        em |= (v.w == -1 ? 1u : 0u) << (4 * j + 3);
-    }
-    // entries fill in order, so the key can only sit before the first empty one
-    const unsigned live = em ? (em & (0u - em)) - 1u : 0xFFu;   // entries before the first empty
-    mm &= live;
-    const int fe = em ? __ffs(em) - 1 : HB, fm = mm ? __ffs(mm) - 1 : HB;
-    e = mm ? fm : fe;
-    s = mm ? reinterpret_cast<const int32_t *>(c + HB * 8)[fm] : -1;
-    return mm ? 1 : (em ? 0 : -1);
-}
-// key k's entry from bucket b on: 1 found at pos (slot word s), 0 absent
-// (pos = the first empty entry of its sequence), -1 the table is full
-__device__ __forceinline__ int hlocate_from(const Pool &P, uint64_t k, uint64_t b, uint64_t &pos, int32_t &s) {
-    for (uint64_t probe = 0; probe <= P.bmask; ++probe) {
-        int e = 0;
-        const int r = hscan_mem(P, b, k, e, s);
-        if (r >= 0) { pos = b * HB + (uint64_t)e; return r; }
-        b = (b + 1) & P.bmask;
-    }
-    return -1;
-}
-__device__ __forceinline__ int hlocate(const Pool &P, uint64_t k, uint64_t &pos, int32_t &s) {
-    return hlocate_from(P, k, hhome(P, k), pos, s);
-}
-// asynchronous copy of a bucket's keys and slot words into shared memory
-__device__ __forceinline__ void hfetch(const Pool &P, uint64_t b, unsigned char *dst) {
-    const unsigned char *src = reinterpret_cast<const unsigned char *>(&P.tab[b]);
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-#pragma unroll
-    for (int q = 0; q < HB_COPY / 16; ++q)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(d + 16 * q), "l"(src + 16 * q) : "memory");
-}
-__device__ __forceinline__ void hfetch_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+constexpr uint64_t GM4_NEVER = ~0ull;
+// time of look s (0..7: direction, then neighbour / neighbour's neighbour) of
+// the leaf with visit rank r: below 2^57, above 0
+FDM_HD uint64_t gm4_time(uint64_t r, int s) { return ((r << 3) | (uint64_t)s) + 1u; }
+// the reference's direction order: right, left, up, down
+__device__ __forceinline__ int gm4_dir(int t) { return (t + DIR_RIGHT) & 3; }
 
-__global__ void k_pool_init(NodeSet A, Pool P) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= A.n) return;
-    const uint64_t k = A.key[i];
-    P.key[i] = k;
-    P.flags[i] = A.leaf[i] ? PF_LEAF : 0;
-    P.gen[i] = 0;
-    P.val[i] = A.val[i];
-    // claim the first free entry of the sequence (entries only fill up here)
-    uint64_t b = hhome(P, k);
-    for (uint64_t probe = 0; probe <= P.bmask; ++probe) {
-        for (int j = 0; j < HB; ++j) {
-            if (P.tab[b].slot[j] != -1) continue;
-            if (atomicCAS(&P.tab[b].slot[j], -1, (int32_t)i) == -1) {
-                P.tab[b].key[j] = k;
-                return;
-            }
-        }
-        b = (b + 1) & P.bmask;
+// The node of A that holds position key_pos(k): the last one that starts at
+// or before it, always a leaf (an internal node's first son starts where it
+// does and comes after it).
+__device__ __forceinline__ int64_t holder(const NodeSet &A, uint64_t k) {
+    const uint64_t pos = key_pos(k);
+    const int64_t r = (int64_t)(k >> 34);
+    int64_t lo = __ldg(A.rf + r), hi = (int64_t)__ldg(A.rf + r + 1) - 1;
+    while (lo < hi) {
+        const int64_t mid = (lo + hi + 1) >> 1;
+        if (key_pos(__ldg(A.key + mid)) <= pos) lo = mid;
+        else hi = mid - 1;
     }
-}
-// entry position of key k (live or deleted), or -1
-__device__ __forceinline__ int64_t hpos(const Pool &P, uint64_t k, int32_t &s) {
-    uint64_t pos = 0;
-    s = -1;
-    return hlocate(P, k, pos, s) == 1 ? (int64_t)pos : -1;
-}
-// pool index of the live node with key k, or -1
-__device__ __forceinline__ int32_t hfind(const Pool &P, uint64_t k) {
-    int32_t s;
-    if (hpos(P, k, s) < 0) return -1;
-    return (s & SLOT_DEL) ? -1 : s;
-}
-// insert or revive a leaf with value v (one lane); pn is the pool size.
-// Returns its pool index or -1
-__device__ int32_t hinsert(const Pool &P, uint64_t k, const double4 &v, int64_t &pn) {
-    int32_t s;
-    uint64_t pos;
-    const int r = hlocate(P, k, pos, s);
-    if (r < 0) return -1;
-    if (r == 1) {
-        const int32_t i = s & ~SLOT_DEL;
-        *hslot(P, pos) = i;
-        P.flags[i] = PF_LEAF;
-        P.gen[i] = P.gen[i] + 1;
-        P.val[i] = v;
-        return i;
-    }
-    const int64_t i = pn;
-    if (i >= P.cap) return -1;
-    pn = i + 1;
-    P.key[i] = k; P.flags[i] = PF_LEAF; P.gen[i] = 0; P.val[i] = v;
-    *hslot(P, pos) = (int32_t)i;
-    *hkey(P, pos) = k;
-    return (int32_t)i;
-}
-
-constexpr int GM4_BATCH = 8;      // items looked at together
-constexpr int GM4_TWIN = 64;      // trigger window in shared memory
-constexpr int GM4_SQ = 4096;      // sorted queue in shared memory (16 B entries)
-
-// Leaves to visit ahead of the traversal, ordered by mk: a sorted array
-// q[head, tail) in shared memory that the warp inserts into and consumes
-// from the front, and a binary min-heap in global memory for what does not
-// fit there and for the (rare) entries that one lane queues alone.  The
-// sizes are kept uniform across the warp.
-struct Heap {
-    HEnt *e;
-    int64_t cap, n;
-};
-struct Queue {
-    HEnt *q;
-    int head, tail;
-    Heap g;
-};
-__device__ __forceinline__ bool hpush(Heap &H, const HEnt &x) {
-    if (H.n >= H.cap) return false;
-    int64_t i = H.n++;
-    while (i > 0) {
-        const int64_t pa = (i - 1) >> 1;
-        const HEnt p = H.e[pa];
-        if (p.mk <= x.mk) break;
-        H.e[i] = p;
-        i = pa;
-    }
-    H.e[i] = x;
-    return true;
-}
-__device__ __forceinline__ HEnt hpop(Heap &H) {
-    const HEnt top = H.e[0];
-    const int64_t hn = --H.n;
-    const HEnt last = H.e[hn];
-    int64_t i = 0;
-    for (;;) {
-        int64_t c = 2 * i + 1;
-        if (c >= hn) break;
-        HEnt a = H.e[c];
-        if (c + 1 < hn) {
-            const HEnt b = H.e[c + 1];
-            if (b.mk < a.mk) { a = b; ++c; }
-        }
-        if (a.mk >= last.mk) break;
-        H.e[i] = a;
-        i = c;
-    }
-    if (hn > 0) H.e[i] = last;
-    return top;
-}
-__device__ __forceinline__ HEnt queued_leaf(uint64_t key, int32_t idx, int32_t gen) {
-    HEnt x;
-    x.mk = visit_rank(key) * 2 + 1;
-    x.idx = idx;
-    x.gen = gen;
-    return x;
-}
-// one lane: into the global heap
-__device__ __forceinline__ bool gpush_leaf(Heap &H, uint64_t key, int32_t idx, int32_t gen) {
-    return hpush(H, queued_leaf(key, idx, gen));
-}
-
-// The warp inserts the entries x of the lanes with has (at most 4, lanes
-// 0..3) into the sorted array: entries at or above each new one move up by
-// the number of new ones below them, top chunk first; each new entry lands
-// after the old entries with mk not above its own.  When the array is full
-// its upper half moves to the global heap first.  Returns false when the
-// global heap overflowed.
-__device__ __forceinline__ bool sq_insert(Queue &Q, const HEnt &x, bool has) {
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const unsigned hm = __ballot_sync(FULL, has);
-    const int k = __popc(hm);
-    if (k == 0) return true;
-    bool ok = true;
-    if (Q.tail + k > GM4_SQ) {
-        // move [head, tail) down to 0, ascending chunks (the target lies below the source)
-        const int n = Q.tail - Q.head;
-        if (Q.head > 0) {
-            for (int b = 0; b < n; b += 32) {
-                HEnt y;
-                if (b + lane < n) y = Q.q[Q.head + b + lane];
-                __syncwarp();
-                if (b + lane < n) Q.q[b + lane] = y;
-                __syncwarp();
-            }
-            Q.head = 0;
-            Q.tail = n;
-        }
-        if (Q.tail + k > GM4_SQ) {   // the upper half goes to the global heap
-            int e = 0;
-            if (lane == 0)
-                for (int j = n / 2; j < n; ++j)
-                    if (!hpush(Q.g, Q.q[j])) e = 1;
-            Q.tail = n / 2;
-            Q.g.n = __shfl_sync(FULL, Q.g.n, 0);
-            ok = __shfl_sync(FULL, e, 0) == 0;
-            __syncwarp();
-        }
-    }
-    uint64_t m[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) m[j] = __shfl_sync(FULL, x.mk, j);
-    // rank among the new entries (equal keys by lane) and place among the old ones
-    int rank = 0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-        rank += ((hm >> j) & 1u) && (m[j] < x.mk || (m[j] == x.mk && j < lane)) ? 1 : 0;
-    int ub = Q.head;
-    if (has) {
-        int hi = Q.tail;
-        while (ub < hi) {
-            const int mid = (ub + hi) >> 1;
-            if (Q.q[mid].mk <= x.mk) ub = mid + 1;
-            else hi = mid;
-        }
-    }
-    for (int b = Q.tail - 32;; b -= 32) {
-        const int p = b + lane;
-        const bool in = p >= Q.head;
-        HEnt y;
-        int s = 0;
-        if (in) {
-            y = Q.q[p];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) s += ((hm >> j) & 1u) && m[j] < y.mk ? 1 : 0;
-        }
-        __syncwarp();
-        if (in && s > 0) Q.q[p + s] = y;
-        __syncwarp();
-        if (b <= Q.head || __any_sync(FULL, in && s == 0)) break;
-    }
-    if (has) Q.q[ub + rank] = x;
-    Q.tail += k;
-    __syncwarp();
-    return ok;
-}
-// Entries of the global heap that belong among the first GM4_BATCH come
-// into the sorted array before a merge
-__device__ __forceinline__ bool sq_pull(Queue &Q) {
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    bool ok = true;
-    while (Q.g.n > 0 && ok) {
-        const uint64_t kth = Q.tail - Q.head >= GM4_BATCH ? Q.q[Q.head + GM4_BATCH - 1].mk : ~0ull;
-        if (Q.g.e[0].mk >= kth) break;
-        HEnt x;
-        if (lane == 0) x = hpop(Q.g);
-        Q.g.n = __shfl_sync(FULL, Q.g.n, 0);
-        __syncwarp();
-        ok = sq_insert(Q, x, lane == 0);
-    }
-    return ok;
-}
-
-// After a non-leaf Refine_cell dropped a subtree two or more levels deep,
-// the region of pk (level l0) is coarser than before: leaves at level
-// >= l0 + 3 in the four edge-adjacent level-l0 cells can now find one of the
-// new sons as a neighbour (or neighbour's neighbour) two levels coarser.  The
-// reference visits every leaf, so those ahead of the traversal are queued.
-__device__ __noinline__ bool push_ring(const Pool &P, const Geometry &G, Heap &H, uint64_t pk, uint64_t cur_rank) {
-    const int l0 = (int)(pk & 15u);
-    const int dirs[4] = {DIR_RIGHT, DIR_LEFT, DIR_UP, DIR_DOWN};
-    bool ok = true;
-    for (int d = 0; d < 4; ++d) {
-        uint64_t t;
-        if (!shift_key(G, pk, dirs[d], t)) continue;
-        const int32_t s0 = hfind(P, t);
-        if (s0 < 0 || (P.flags[s0] & PF_LEAF)) continue;
-        uint64_t st[64];
-        int sp = 0;
-        st[sp++] = t;
-        while (sp > 0) {
-            const uint64_t k = st[--sp];
-            for (int q = 0; q < 4; ++q) {
-                const uint64_t ck = child_key(k, q);
-                const int32_t c = hfind(P, ck);
-                if (c < 0) continue;
-                if (P.flags[c] & PF_LEAF) {
-                    if ((int)(ck & 15u) >= l0 + 3 && visit_rank(ck) > cur_rank) ok = gpush_leaf(H, ck, c, P.gen[c]) && ok;
-                } else if (sp < 64) {
-                    st[sp++] = ck;
-                } else {
-                    ok = false;
-                }
-            }
-        }
-    }
-    return ok;
-}
-// Refine_cell (src/mesh.F90:199-260) of a non-leaf whose old subtree is
-// dropped and whose new sons copy its stale value (counted in nl); one lane.
-// cur_rank is the visit rank of the leaf being visited.
-__device__ __noinline__ bool refine_nonleaf(const Pool &P, const Geometry &G, Heap &H, int32_t p, uint64_t cur_rank,
-                                            int32_t &nl, int64_t &pn) {
-    const uint64_t pk = P.key[p];
-    bool deep = false, ok = true;
-    nl += 1;
-    uint64_t st[64];
-    int sp = 0;
-    st[sp++] = pk;
-    while (sp > 0) {
-        const uint64_t k = st[--sp];
-        for (int q = 0; q < 4; ++q) {
-            int32_t s;
-            const int64_t pos = hpos(P, child_key(k, q), s);
-            if (pos < 0 || (s & SLOT_DEL)) continue;
-            if (!(P.flags[s] & PF_LEAF)) {
-                if (k != pk) deep = true;
-                if (sp < 64) st[sp++] = P.key[s];
-                else ok = false;
-            }
-            P.flags[s] |= PF_DELETED;
-            *hslot(P, (uint64_t)pos) = s | SLOT_DEL;
-        }
-    }
-    P.flags[p] = 0;   // internal, value kept
-    const double4 v = P.val[p];
-    for (int q = 0; q < 4; ++q) {
-        const uint64_t ck = child_key(pk, q);
-        const int32_t c = hinsert(P, ck, v, pn);
-        if (c < 0) return false;
-        if (visit_rank(ck) > cur_rank) ok = gpush_leaf(H, ck, c, P.gen[c]) && ok;
-    }
-    if (deep) ok = push_ring(P, G, H, pk, cur_rank) && ok;
-    return ok;
+    return lo;
 }
 // Is the node with key s (or the position s stands for) inside node r?
 __device__ __forceinline__ bool key_inside(uint64_t r, uint64_t s) {
@@ -1099,400 +679,299 @@ __device__ __forceinline__ bool key_inside(uint64_t r, uint64_t s) {
     return (((s >> 4) & path_mask) & keep) == ((r >> 4) & path_mask);
 }
 
-// A lookup from key k towards d starts at the shifted key S and walks up to
-// the first existing node; refining or dropping node R changes it only when
-// S lies inside R.  sk = S (or ~0 when the shift leaves the grid).  It is
-// made by a group of 4 consecutive lanes (mask gm, first lane g0): lane
-// g0 + j probes the j-th ancestor of the walk's current start, copying its
-// home bucket into the lane's shared-memory area lk (HB_COPY bytes), and
-// the deepest node found ends the walk; otherwise the walk moves up 4
-// levels.  Every lane of the group returns the result.
-__device__ __forceinline__ int32_t group_lookup(const Pool &P, const Geometry &G, uint64_t k, int d, uint64_t &nk,
-                                                uint64_t &sk, unsigned char *lk, unsigned gm, int g0) {
-    const int j = (int)(threadIdx.x & 3);
-    uint64_t t;
-    if (!shift_key(G, k, d, t)) { sk = ~0ull; return -1; }
-    sk = t;
-    for (;;) {
-        const int lt = (int)(t & 15u);
-        const uint64_t c = ancestor_key(t, lt > j ? lt - j : 0);
-        bool found = false;
-        int32_t s = -1;
-        if (j <= lt) {
-            const uint64_t b = hhome(P, c);
-            hfetch(P, b, lk);
-            hfetch_wait();
-            int e = 0;
-            int r = hscan_copy(lk, c, e, s);
-            if (r < 0) {   // a full bucket: the sequence goes on in the next ones
-                uint64_t pos;
-                r = hlocate_from(P, c, (b + 1) & P.bmask, pos, s);
-            }
-            found = r == 1 && !(s & SLOT_DEL);
+// Leaves that can act: a neighbour, or the neighbour's neighbour, two or
+// more levels coarser in the node set at the start.  Refining a leaf only
+// makes neighbours finer, so no other leaf of the set can act later.  Four
+// lanes per node, one per direction; the leaves are appended to list in no
+// particular order.  Only leaves whose looks come after time t0 count.
+__global__ void __launch_bounds__(256) k_gm4_triggers(NodeSet A, Geometry G, uint64_t t0, int32_t *list,
+                                                      int32_t *count) {
+    const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t c = g >> 2;
+    bool acts = false;
+    if (c < A.n && A.leaf[c]) {
+        const uint64_t k = A.key[c];
+        const int lc = (int)(k & 15u), d = gm4_dir((int)(g & 3));
+        uint64_t s;
+        if (lc >= 2 && gm4_time(visit_rank(k), 7) > t0 && shift_key(G, k, d, s)) {
+            const uint64_t nb = __ldg(A.key + holder(A, s));
+            const int ln = min((int)(nb & 15u), lc);   // deeper: the same-level node has sons
+            acts = ln <= lc - 2;
+            if (!acts && shift_key(G, ln < lc ? nb : s, d, s))
+                acts = (int)(__ldg(A.key + holder(A, s)) & 15u) <= lc - 2;
         }
-        const unsigned fm = (__ballot_sync(gm, found) >> g0) & 0xFu;
-        if (fm) {
-            const int w = g0 + __ffs(fm) - 1;
-            nk = __shfl_sync(gm, c, w);
-            return __shfl_sync(gm, s, w);
-        }
-        if (lt < 4) return -1;   // level 0 was probed
-        t = ancestor_key(t, lt - 4);
     }
-}
-// the reference's direction order of gridmodify4: right, left, up, down
-__device__ __forceinline__ int gm4_dir(int t) { return (t + DIR_RIGHT) & 3; }
-// the neighbour of leaf k in direction t of that order and the neighbour's
-// neighbour, by a group of 4 lanes
-struct Look {
-    int32_t nb, nn;
-    uint64_t nbk, nnk, snb, snn;
-};
-__device__ __forceinline__ void group_dir_lookups(const Pool &P, const Geometry &G, uint64_t k, int t, Look &L,
-                                                  unsigned char *lk, unsigned gm, int g0) {
-    L.nn = -1;
-    L.snn = ~0ull;
-    L.nnk = 0;
-    L.nb = group_lookup(P, G, k, gm4_dir(t), L.nbk, L.snb, lk, gm, g0);
-    if (L.nb >= 0) L.nn = group_lookup(P, G, L.nbk, gm4_dir(t), L.nnk, L.snn, lk, gm, g0);
-}
-
-// Refine_cell of pool node p (key pk) by the warp.  Lanes 0..3 read the
-// node's flags and value and make the first probe for their son's key at
-// once.  A leaf's sons are then stored by those lanes: a son found in the
-// table (dropped earlier) is revived, the others take new pool entries and
-// the first empty slot of their probe sequence.  Sons whose sequences share
-// that slot take it one at a time, lowest lane first, the others probing on
-// past it.  A non-leaf (rare) is refined by lane 0 alone.  pn (the pool
-// size) is uniform.  Returns false when the pool or the queue overflowed.
-__device__ __forceinline__ bool refine_warp(Pool &P, const Geometry &G, Queue &Q, int32_t p, uint64_t pk, uint64_t cur_rank,
-                            int32_t &nonleaf, int64_t &pn, unsigned char *lk) {
-    const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const bool son = lane < 4;
-    int fp = 0;
+    const unsigned m = __ballot_sync(0xffffffffu, acts);
+    const bool first = (lane & 3) == 0 && ((m >> lane) & 0xFu) != 0;   // one lane per acting leaf
+    const unsigned fm = __ballot_sync(0xffffffffu, first);
+    int base = 0;
+    if (lane == 0 && fm) base = atomicAdd(count, __popc(fm));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (first) list[base + __popc(fm & ((1u << lane) - 1u))] = (int32_t)c;
+}
+
+// The map t and the nodes made on the way.  Nodes are named by their index
+// in A (below n) or n + the order in which they were made; a node that some
+// sweep refines gets four sons (first one: son), in key order, which stay
+// even when a later sweep takes the refinement back (t = GM4_NEVER again).
+struct Gm4 {
+    uint64_t *t, *tn;      // [n + cap] current estimate, next one
+    int32_t *son;          // [n + cap] first son, -1 none
+    uint64_t *mkey;        // [cap] key of a made node
+    int32_t *mfather;      // [cap] its father
+    int32_t *refd;         // [n + cap] nodes that some sweep refined
+    const int32_t *list;   // the leaves of A that can act
+    int64_t cap;
+    uint64_t *nl;          // [2] earliest refinement of a node with sons, by sweep parity
+    int32_t *w;            // GW_* words
+};
+enum { GW_NLIST = 0, GW_MADE, GW_NREFD, GW_CHG0, GW_CHG1, GW_FULL, GW_STUCK, GW_SWEEPS, GW_VISITS, GW_REFINES,
+       GW_NONLEAF, GW_WORDS };
+struct Gm4Result {         // read back by the host
+    int32_t w[GW_WORDS + 1];
+    uint64_t nl_time, nl_key;
+};
+
+__device__ __forceinline__ uint64_t gm4_key(const NodeSet &A, const Gm4 &M, int32_t id) {
+    return id < A.n ? __ldg(A.key + id) : __ldcg(M.mkey + (id - A.n));
+}
+// What a look from s towards the node at s's level finds at time T: the node
+// itself (same: with its level that of s) or the leaf above it.  id is the
+// node's name, or -1 for a node of A that has sons.
+struct Found {
+    uint64_t key;
+    int32_t id;
+    bool sons;
+};
+__device__ __forceinline__ Found gm4_look(const NodeSet &A, const Gm4 &M, uint64_t s, uint64_t T) {
+    Found f;
+    const int ls = (int)(s & 15u);
+    int32_t id = (int32_t)holder(A, s);
+    uint64_t k = __ldg(A.key + id);
+    int l = (int)(k & 15u);
+    if (l > ls) {
+        f.key = s; f.id = -1; f.sons = true;
+        return f;
+    }
+    bool sons = __ldcg(M.t + id) < T;
+    while (l < ls && sons) {
+        ++l;
+        id = __ldcg(M.son + id) + (int32_t)((s >> key_digit_shift(l)) & 3u);
+        k = ancestor_key(s, l);
+        sons = __ldcg(M.t + id) < T;
+    }
+    f.key = k; f.id = id; f.sons = sons;
+    return f;
+}
+// look s of the leaf with key k and visit rank r: the neighbour (tn.id >= 0
+// when it refines it) and the neighbour's neighbour
+struct Looks {
+    int32_t nb, nn;          // nodes refined, or -1
+    bool nonleaf;            // the neighbour's neighbour is refined and has sons
+    uint64_t nnkey;
+};
+__device__ __forceinline__ Looks gm4_looks(const NodeSet &A, const Geometry &G, const Gm4 &M, uint64_t k, uint64_t r,
+                                           int t) {
+    Looks L;
+    L.nb = L.nn = -1;
+    L.nonleaf = false;
+    L.nnkey = 0;
+    const int lc = (int)(k & 15u), d = gm4_dir(t);
+    uint64_t s;
+    if (!shift_key(G, k, d, s)) return L;
+    const Found b = gm4_look(A, M, s, gm4_time(r, 2 * t));
+    if ((int)(b.key & 15u) <= lc - 2) L.nb = b.id;   // no node at lc: a leaf
+    if (!shift_key(G, b.key, d, s)) return L;
+    const Found n = gm4_look(A, M, s, gm4_time(r, 2 * t + 1));
+    if ((int)(n.key & 15u) <= lc - 2) {
+        L.nnkey = n.key;
+        if (n.sons) L.nonleaf = true;
+        else L.nn = n.id;
+    }
+    return L;
+}
+// is node id a leaf when its turn (rank r) comes, after time t0?
+__device__ __forceinline__ bool gm4_visited(const NodeSet &A, const Gm4 &M, int32_t id, uint64_t r) {
+    const uint64_t T = gm4_time(r, 0);
+    if (__ldcg(M.t + id) < T) return false;
+    return id < A.n || __ldcg(M.t + __ldcg(M.mfather + (id - A.n))) < T;
+}
+__device__ __forceinline__ void gm4_propose(const NodeSet &A, const Gm4 &M, int32_t id, uint64_t T) {
+    atomicMin((unsigned long long *)(M.tn + id), (unsigned long long)T);
+    if (__ldcg(M.son + id) != -1) return;
+    if (atomicCAS(M.son + id, -1, -2) != -1) return;   // the first sweep that refines it makes its sons
+    const int32_t j = atomicAdd(M.w + GW_MADE, 4);
+    if (j + 4 > M.cap) {
+        M.w[GW_FULL] = 1;
+        return;
+    }
+    const uint64_t k = gm4_key(A, M, id);
+    for (int q = 0; q < 4; ++q) {
+        __stcg(M.mkey + j + q, child_key(k, q));
+        __stcg(M.mfather + j + q, id);
+    }
+    __stcg(M.son + id, (int32_t)(A.n + j));
+    M.refd[atomicAdd(M.w + GW_NREFD, 1)] = id;
+}
+
+__device__ __forceinline__ void cluster_barrier() {
+    __syncwarp();   // lanes come here from divergent loops
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+constexpr int GM4_CTAS = 8, GM4_THREADS = 512;
+
+// The fixpoint, by one cluster of blocks: a sweep is all looks (four lanes
+// per leaf, one per direction), a cluster barrier, then the comparison of
+// the two estimates over the nodes ever refined, and another barrier.  The
+// hardware's cluster barrier costs a fraction of a grid-wide one, and a pass
+// has a few thousand looks: it is bound by the latency of a look (two
+// searches in a background cell's nodes, about 20 dependent L2 reads) times
+// the sweeps, not by the number of SMs.  One B200, two regrids of a developed
+// 128^2, 4-level four-quadrant run (82k leaves, 2029 refinements): 0.94 ms in
+// 39 sweeps, against 14.0 ms for visiting the leaves in order by one block;
+// 64 x 16-cell double Mach at 4 levels, four regrids: 1.0 against 10.2 ms.
+__global__ void __cluster_dims__(GM4_CTAS, 1, 1) __launch_bounds__(GM4_THREADS)
+    k_gm4_fixpoint(NodeSet A, Geometry G, Gm4 M, uint64_t t0, int max_sweeps, Gm4Result *out) {
+    const int nthr = GM4_CTAS * GM4_THREADS;
+    const int me = blockIdx.x * GM4_THREADS + threadIdx.x;
+    const int nlist = __ldcg(M.w + GW_NLIST);
+    int made = 0;        // made nodes that this sweep visits
+    int sweep = 0;
+    bool full = false;
+    if (nlist > 0) {
+        for (;; ++sweep) {
+            const int par = sweep & 1;
+            const int64_t looks = 4 * ((int64_t)nlist + made);
+            for (int64_t x = me; x < looks; x += nthr) {
+                const int v = (int)(x >> 2), t = (int)(x & 3);
+                const int32_t id = v < nlist ? __ldg(M.list + v) : (int32_t)(A.n + (v - nlist));
+                const uint64_t k = gm4_key(A, M, id), r = visit_rank(k);
+                if (gm4_time(r, 7) <= t0 || !gm4_visited(A, M, id, r)) continue;
+                const Looks L = gm4_looks(A, G, M, k, r, t);
+                const uint64_t Tb = gm4_time(r, 2 * t), Tn = gm4_time(r, 2 * t + 1);
+                if (L.nb >= 0 && Tb > t0) gm4_propose(A, M, L.nb, Tb);
+                if (Tn > t0) {
+                    if (L.nonleaf) atomicMin((unsigned long long *)(M.nl + par), (unsigned long long)Tn);
+                    else if (L.nn >= 0) gm4_propose(A, M, L.nn, Tn);
+                }
+            }
+            cluster_barrier();
+            const int nrefd = __ldcg(M.w + GW_NREFD);
+            made = __ldcg(M.w + GW_MADE);
+            full = made > M.cap || __ldcg(M.w + GW_FULL) != 0;
+            bool changed = false;
+            for (int x = me; x < nrefd; x += nthr) {
+                const int32_t id = __ldcg(M.refd + x);
+                const uint64_t a = __ldcg(M.t + id), b = __ldcg(M.tn + id);
+                if (a != b) {
+                    __stcg(M.t + id, b);
+                    changed = true;
+                }
+                __stcg(M.tn + id, GM4_NEVER);
+            }
+            if (__any_sync(0xffffffffu, changed) && (threadIdx.x & 31) == 0) __stcg(M.w + GW_CHG0 + par, 1);
+            if (me == 0) {   // last read before this sweep's first barrier
+                __stcg(M.w + GW_CHG0 + (par ^ 1), 0);
+                __stcg(M.nl + (par ^ 1), GM4_NEVER);
+            }
+            cluster_barrier();
+            if (full || __ldcg(M.w + GW_CHG0 + par) == 0 || sweep >= max_sweeps) break;
+        }
+    }
+    const uint64_t nl = nlist > 0 ? __ldcg(M.nl + (sweep & 1)) : GM4_NEVER;
+    if (nlist > 0 && !full) {
+        // counts, of what comes no later than the first refinement of a node
+        // with sons
+        const int nrefd = __ldcg(M.w + GW_NREFD);
+        int refines = 0, visits = 0;
+        for (int x = me; x < nrefd; x += nthr) refines += __ldcg(M.t + __ldcg(M.refd + x)) < nl ? 1 : 0;
+        for (int v = me; v < nlist + made; v += nthr) {
+            const int32_t id = v < nlist ? __ldg(M.list + v) : (int32_t)(A.n + (v - nlist));
+            const uint64_t r = visit_rank(gm4_key(A, M, id)), T = gm4_time(r, 0);
+            visits += T > t0 && T <= nl && gm4_visited(A, M, id, r) ? 1 : 0;
+        }
+        refines = __reduce_add_sync(0xffffffffu, refines);
+        visits = __reduce_add_sync(0xffffffffu, visits);
+        if ((threadIdx.x & 31) == 0) {
+            if (refines) atomicAdd(M.w + GW_REFINES, refines);
+            if (visits) atomicAdd(M.w + GW_VISITS, visits);
+        }
+    }
+    cluster_barrier();
+    if (me == 0) {
+        uint64_t nlkey = 0;
+        if (nl != GM4_NEVER && !full) {   // the look of that time again, for its node
+            const uint64_t r = (nl - 1u) >> 3;
+            nlkey = gm4_looks(A, G, M, key_of_visit_rank(r), r, (int)((nl - 1u) & 7u) >> 1).nnkey;
+        }
+        for (int q = 0; q < GW_WORDS; ++q) out->w[q] = __ldcg(M.w + q);
+        out->w[GW_FULL] = full;
+        out->w[GW_STUCK] = nlist > 0 && !full && __ldcg(M.w + GW_CHG0 + (sweep & 1)) != 0;
+        out->w[GW_SWEEPS] = nlist > 0 ? sweep + 1 : 0;
+        out->w[GW_NONLEAF] = nl != GM4_NEVER;
+        out->nl_time = nl;
+        out->nl_key = nlkey;
+    }
+}
+
+// The nodes of the set after the pass that come from node i of A, in key
+// order: node i itself and, below a leaf that was refined, its made subtree.
+// The node refined although it had sons (res->nl_key) keeps four new leaves
+// and loses what was below it.  All of them carry node i's value
+// (Refine_cell copies U, src/mesh.F90:210-252).  Returns their number;
+// WRITE: stores them from place o on.
+template <bool WRITE>
+__device__ __forceinline__ int gm4_nodes(const NodeSet &A, const Gm4 &M, const Gm4Result *res, int64_t i, int64_t o,
+                                         NodeSet out) {
+    const uint64_t k0 = A.key[i], nl = res->nl_time, nlkey = res->nl_key;
+    const bool hasnl = nl != GM4_NEVER;
     double4 v = make_double4(0.0, 0.0, 0.0, 0.0);
-    uint64_t ck = 0, b = 0;
-    if (son) {
-        ck = child_key(pk, lane);
-        b = hhome(P, ck);
-        hfetch(P, b, lk);
-        fp = P.flags[p];
-        v = P.val[p];
-        hfetch_wait();
+    if (WRITE) v = A.val[i];
+    int n = 0;
+    const auto put = [&](uint64_t k, bool leaf) {
+        if (WRITE) {
+            out.key[o + n] = k;
+            out.leaf[o + n] = leaf ? 1 : 0;
+            out.val[o + n] = v;
+        }
+        ++n;
+    };
+    if (hasnl && key_inside(nlkey, k0)) {
+        if (k0 != nlkey) return 0;   // dropped
+        put(k0, false);
+        for (int q = 0; q < 4; ++q) put(child_key(k0, q), true);
+        return n;
     }
-    fp = __shfl_sync(FULL, fp, 0);
-    bool ok = true;
-    if (!(fp & PF_LEAF)) {
-        int e = 0;
-        if (lane == 0) {
-            // out of line on copies, so that the queue and counters stay in registers
-            Heap g = Q.g;
-            int32_t nl = nonleaf;
-            int64_t pn1 = pn;
-            e = refine_nonleaf(P, G, g, p, cur_rank, nl, pn1) ? 0 : 1;
-            Q.g.n = g.n;
-            nonleaf = nl;
-            pn = pn1;
-        }
-        ok = __shfl_sync(FULL, e, 0) == 0;
-        pn = __shfl_sync(FULL, pn, 0);
-    } else {
-        // the son's own entry (a dropped node), or the first empty entry
-        bool found = false;
-        uint64_t h = 0;
-        int32_t s = -1;
-        int r = 0;
-        if (son) {
-            int e = 0;
-            r = hscan_copy(lk, ck, e, s);
-            if (r >= 0) h = b * HB + (uint64_t)e;
-            else r = hlocate_from(P, ck, (b + 1) & P.bmask, h, s);
-            found = r == 1;
-        }
-        const unsigned nm = __ballot_sync(FULL, son && !found);
-        int32_t i = -1, gen = 0;
-        if (found) {
-            i = s & ~SLOT_DEL;
-            gen = P.gen[i] + 1;
-        } else if (son) {
-            i = (int32_t)(pn + __popc(nm & ((1u << lane) - 1u)));
-        }
-        pn += __popc(nm);
-        ok = pn <= P.cap && !__any_sync(FULL, r < 0);   // the pool, or the table, is full
-        if (ok) {
-            bool need = son && !found;
-            for (;;) {
-                const unsigned pend = __ballot_sync(FULL, need);
-                if (!pend) break;
-                if (need) {
-                    const unsigned peers = __match_any_sync(pend, h);
-                    if (__ffs(peers) - 1 == lane) {
-                        *hslot(P, h) = i;
-                        *hkey(P, h) = ck;
-                        need = false;
-                    }
-                }
-                __syncwarp();
-                bool lost = false;
-                if (need) {   // a lower lane took the entry: probe on to the next empty one
-                    lost = true;
-                    for (uint64_t probe = 0; probe <= P.bmask * HB && lost; ++probe) {
-                        h = hnext(P, h);
-                        lost = *hslot(P, h) != -1;
-                    }
-                }
-                if (__any_sync(FULL, lost)) { ok = false; break; }
-            }
-        }
-        if (ok) {
-            if (son) {
-                if (found) *hslot(P, h) = i;
-                else P.key[i] = ck;
-                P.flags[i] = PF_LEAF;
-                P.gen[i] = gen;
-                P.val[i] = v;
-            }
-            if (lane == 0) P.flags[p] = 0;   // internal, value kept
-            // the sons ahead of the traversal are queued
-            ok = sq_insert(Q, queued_leaf(ck, i, gen), son && visit_rank(ck) > cur_rank);
+    if (!A.leaf[i] || M.t[i] >= nl) {   // nl is GM4_NEVER when there is none
+        put(k0, A.leaf[i] != 0);
+        return n;
+    }
+    int32_t st[3 * LMAX + 4];
+    int sp = 0;
+    st[sp++] = (int32_t)i;
+    while (sp > 0) {
+        const int32_t id = st[--sp];
+        const uint64_t k = id < A.n ? k0 : M.mkey[id - A.n];
+        const bool refined = M.t[id] < nl;
+        put(k, !refined);
+        if (!refined) continue;
+        if (hasnl && k == nlkey) {
+            for (int q = 0; q < 4; ++q) put(child_key(k, q), true);
+        } else {
+            for (int q = 3; q >= 0; --q) st[sp++] = M.son[id] + q;
         }
     }
-    Q.g.n = __shfl_sync(FULL, Q.g.n, 0);
-    if (!ok && lane == 0) P.err[0] = 1;
-    __syncwarp();
-    return ok;
+    return n;
 }
-
-__device__ __forceinline__ Look shfl_look(const Look &L, int src) {
-    const unsigned FULL = 0xffffffffu;
-    Look o;
-    o.nb = __shfl_sync(FULL, L.nb, src);
-    o.nn = __shfl_sync(FULL, L.nn, src);
-    o.nbk = __shfl_sync(FULL, L.nbk, src);
-    o.nnk = __shfl_sync(FULL, L.nnk, src);
-    o.snb = __shfl_sync(FULL, L.snb, src);
-    o.snn = __shfl_sync(FULL, L.snn, src);
-    return o;
-}
-
-constexpr int GM4_THREADS = 128;   // 8 leaves x 4 directions x 4 probing lanes
-
-// gridmodify4 (src/mesh.F90:355-395) over one pass of the tree, by one
-// block.  The leaves that can act (the initial triggers, sorted by visit
-// rank, and every leaf queued ahead of the traversal) are visited in
-// traversal order.  Warp 0 merges the next 8 of them from the sorted queue
-// and the trigger window (its lanes at once); then the whole block looks at
-// them together: 16 threads per leaf find its right/left/up/down neighbour
-// and that neighbour's neighbour, 4 per direction.  Warp 0 then tells which
-// directions would refine something.  The leaves before the first one that
-// refines have no effect but being visited, so they are marked in
-// parallel; the first one that refines is then applied alone, in order, by
-// warp 0, and the batch ends there (the leaves after it stay where they are
-// for the next batch).  Within that leaf a lookup starts at a shifted key
-// and walks up to the first existing node, so a refinement (or a dropped
-// subtree) of node R can change a later lookup only when its start lies
-// inside R: those lookups, and only those, are repeated.  A leaf that is
-// both a trigger and queued is looked at twice; the second look finds it
-// visited.
-__global__ void __launch_bounds__(GM4_THREADS) k_gm4_block(Pool P, Geometry G, const uint64_t *__restrict__ trank,
-                                                           const int32_t *__restrict__ tidx, int64_t ntrig,
-                                                           int64_t max_steps) {
-    extern __shared__ __align__(16) unsigned char gm4_smem[];
-    __shared__ HEnt items[GM4_BATCH];
-    __shared__ uint64_t twr[GM4_TWIN];
-    __shared__ int32_t twx[GM4_TWIN];
-    __shared__ __align__(16) unsigned char lkbuf[GM4_THREADS][HB_COPY];   // each thread's bucket copy
-    __shared__ Look looks[GM4_BATCH][4];
-    __shared__ uint8_t s_fl[GM4_BATCH], s_valid[GM4_BATCH];
-    __shared__ int s_cnt;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    unsigned char *lk = lkbuf[tid];
-    const unsigned FULL = 0xffffffffu;
-    // this thread's part of the block-wide lookups
-    const int bi = tid >> 4, bd = (tid >> 2) & 3, g0 = lane & ~3;
-    const unsigned gmask = 0xFu << g0;
-    // warp 0's state (uniform in warp 0)
-    Queue Q;
-    Q.q = reinterpret_cast<HEnt *>(gm4_smem);
-    Q.head = Q.tail = 0;
-    Q.g.e = P.heap;
-    Q.g.cap = P.hcap;
-    Q.g.n = 0;
-    int64_t pn = *P.n;     // pool size (stored at the end)
-    int64_t tg = 0;        // next trigger to bring into the window
-    int tw_n = 0, tp = 0;  // triggers in the window, next one to merge
-    int64_t step = 0;
-    int32_t visits = 0, nonleaf = 0, refines = 0;   // lane 0's counts, stored at the end
-    bool ok = true;
-    bool take = false;     // warp 0: this lane's merged entry is an item ...
-    int pos = 0;           // ... at this place
-    for (;; ++step) {
-        // warp 0 reaches here from lane-level branches of the refinement;
-        // reconverge it before the lane-parallel merge, or its lanes can run
-        // the merge in separate groups
-        __syncwarp();
-        if (warp == 0) {
-            int c = 0;
-            if (step >= max_steps) {
-                if (lane == 0) P.err[3] = 1;
-            } else if (ok) {
-                // keep at least a batch of triggers in the window
-                if (tw_n - tp < GM4_BATCH && tg < ntrig) {
-                    const int rem = tw_n - tp;
-                    uint64_t rr = 0;
-                    int32_t rx = 0;
-                    if (lane < rem) { rr = twr[tp + lane]; rx = twx[tp + lane]; }
-                    __syncwarp();
-                    if (lane < rem) { twr[lane] = rr; twx[lane] = rx; }
-                    const int nl = (int)min((int64_t)(GM4_TWIN - rem), ntrig - tg);
-                    for (int j = lane; j < nl; j += 32) { twr[rem + j] = trank[tg + j]; twx[rem + j] = tidx[tg + j]; }
-                    tg += nl;
-                    tw_n = rem + nl;
-                    tp = 0;
-                    __syncwarp();
-                }
-                if (Q.g.n > 0 && !sq_pull(Q)) ok = false;
-            }
-            if (step < max_steps && ok) {
-                // the next items in traversal order: lanes 0..7 hold the first
-                // queued leaves, lanes 8..15 the first triggers; each finds its
-                // place among the other list's eight (a trigger's mk is even, a
-                // queued leaf's odd: no ties)
-                HEnt x;
-                x.mk = ~0ull; x.idx = -1; x.gen = 0;
-                if (lane < GM4_BATCH) {
-                    if (Q.head + lane < Q.tail) x = Q.q[Q.head + lane];
-                } else if (lane < 2 * GM4_BATCH) {
-                    const int j = tp + lane - GM4_BATCH;
-                    if (j < tw_n) { x.mk = twr[j] * 2; x.idx = twx[j]; }
-                }
-                pos = lane & (GM4_BATCH - 1);
-                const int other = lane < GM4_BATCH ? GM4_BATCH : 0;
-#pragma unroll
-                for (int j = 0; j < GM4_BATCH; ++j) {
-                    const uint64_t o = __shfl_sync(FULL, x.mk, other + j);
-                    pos += o < x.mk ? 1 : 0;
-                }
-                take = lane < 2 * GM4_BATCH && x.mk != ~0ull && pos < GM4_BATCH;
-                if (take) items[pos] = x;
-                c = __popc(__ballot_sync(FULL, take));
-            }
-            if (lane == 0) s_cnt = c;
-        }
-        __syncthreads();
-        const int cnt = s_cnt;
-        if (cnt == 0) break;
-        // lookups: 16 threads per item, 4 per direction; the item's key comes
-        // from its rank, so its flags and generation load meanwhile
-        if (bi < cnt) {
-            const HEnt it = items[bi];
-            const uint64_t ck = key_of_visit_rank(it.mk >> 1);
-            uint8_t fl = 0;
-            int32_t gc = 0;
-            const bool lead = (tid & 15) == 0;
-            if (lead) { fl = P.flags[it.idx]; gc = P.gen[it.idx]; }
-            Look L;
-            group_dir_lookups(P, G, ck, bd, L, lk, gmask, g0);
-            if ((tid & 3) == 0) looks[bi][bd] = L;
-            if (lead) {
-                s_fl[bi] = fl;
-                s_valid[bi] = gc == it.gen && (fl & (PF_LEAF | PF_DELETED | PF_VISITED)) == PF_LEAF;
-            }
-        }
-        __syncthreads();
-        if (warp != 0) continue;
-        // decisions: lane (grp, tl) tells whether direction tl of item grp refines
-        const int grp = lane >> 2, tl = lane & 3;
-        bool valid = false, acts = false;
-        uint8_t fl = 0;
-        HEnt it;
-        it.mk = 0; it.idx = -1; it.gen = 0;
-        if (grp < cnt) {
-            it = items[grp];
-            valid = s_valid[grp] != 0;
-            fl = s_fl[grp];
-            const Look L = looks[grp][tl];
-            const int lc = (int)(it.mk >> 1) & 15;
-            acts = valid &&
-                   ((L.nb >= 0 && (int)(L.nbk & 15u) <= lc - 2) || (L.nn >= 0 && (int)(L.nnk & 15u) <= lc - 2));
-        }
-        const unsigned am = __ballot_sync(FULL, acts);
-        const int fa = am ? (__ffs(am) - 1) >> 2 : cnt;   // first item that refines
-        // items before it: visited, nothing else
-        const unsigned vm = __ballot_sync(FULL, valid && tl == 0 && grp < fa);
-        if (valid && tl == 0 && grp < fa) P.flags[it.idx] = fl | PF_VISITED;
-        if (lane == 0) visits += __popc(vm);
-        const int consumed = fa < cnt ? fa + 1 : cnt;
-        // the consumed items leave the front of their lists (the sons queued
-        // below all rank after the item being visited)
-        const int cq = __popc(__ballot_sync(FULL, take && lane < GM4_BATCH && pos < consumed));
-        Q.head += cq;
-        tp += consumed - cq;
-        if (fa < cnt) {
-            const HEnt ib = items[fa];
-            const uint64_t rb = ib.mk >> 1;
-            const uint64_t kb = key_of_visit_rank(rb);
-            const int lc = (int)(kb & 15u);
-            if (lane == 0) {
-                P.flags[ib.idx] = s_fl[fa] | PF_VISITED;
-                ++visits;
-            }
-            uint64_t refined[8];   // uniform: nodes refined by this leaf
-            int nref = 0;
-            for (int t = 0; t < 4 && ok; ++t) {
-                Look Lt = looks[fa][t];
-                // repeat the lookups whose start lies inside a node refined earlier
-                bool re_nb = false, re_nn = false;
-                for (int k = 0; k < nref; ++k) {
-                    re_nb = re_nb || key_inside(refined[k], Lt.snb);
-                    re_nn = re_nn || key_inside(refined[k], Lt.snn);
-                }
-                if (re_nb || re_nn) {
-                    if (lane < 4) {
-                        if (re_nb) group_dir_lookups(P, G, kb, t, Lt, lk, 0xFu, 0);
-                        else Lt.nn = group_lookup(P, G, Lt.nbk, gm4_dir(t), Lt.nnk, Lt.snn, lk, 0xFu, 0);
-                    }
-                    Lt = shfl_look(Lt, 0);
-                }
-                if (Lt.nb < 0) continue;
-                // a neighbour two levels coarser is a leaf (every internal node
-                // has four sons), and refining it leaves the lookup of its own
-                // neighbour unchanged (that start lies outside it)
-                if ((int)(Lt.nbk & 15u) <= lc - 2) {
-                    ok = refine_warp(P, G, Q, Lt.nb, Lt.nbk, rb, nonleaf, pn, lk);
-                    refined[nref++] = Lt.nbk;
-                    ++refines;
-                }
-                if (ok && Lt.nn >= 0 && (int)(Lt.nnk & 15u) <= lc - 2) {
-                    ok = refine_warp(P, G, Q, Lt.nn, Lt.nnk, rb, nonleaf, pn, lk);
-                    refined[nref++] = Lt.nnk;
-                    ++refines;
-                }
-            }
-        }
-    }
-    if (tid == 0) {
-        if (!ok) P.err[0] = 1;
-        *P.n = pn;
-        P.err[1] = visits;
-        P.err[2] = nonleaf;
-        P.err[4] = refines;
-        P.err[5] = (int32_t)step;
-    }
-}
-
-__global__ void k_pool_live(int64_t n, const uint8_t *flags, int32_t *live) {
+__global__ void k_gm4_count(NodeSet A, Gm4 M, const Gm4Result *res, int32_t *cnt) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i < n) live[i] = !(flags[i] & PF_DELETED);
+    if (i < A.n) cnt[i] = res->w[GW_FULL] ? 1 : gm4_nodes<false>(A, M, res, i, 0, A);
 }
-__global__ void k_pool_emit(int64_t n, const uint8_t *flags, const uint64_t *key, const double4 *val,
-                            const int32_t *off, uint64_t *okey, uint8_t *oleaf, double4 *oval) {
+__global__ void k_gm4_emit(NodeSet A, Gm4 M, const Gm4Result *res, const int32_t *off, NodeSet out) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n || (flags[i] & PF_DELETED)) return;
-    okey[off[i]] = key[i];
-    oleaf[off[i]] = (flags[i] & PF_LEAF) ? 1 : 0;
-    oval[off[i]] = val[i];
+    if (i < A.n) gm4_nodes<true>(A, M, res, i, off[i], out);
 }
 
 // ------------------------------------------------------------ extraction
@@ -1584,13 +1063,11 @@ static int gridmodify1_pass(fdm_handle *h, AmrCtx &X, bool *did) {
     k_gm1_count<<<nblk(n, TB), TB, 0, h->s>>>(n, L, cur, cnt);
     int64_t total = 0;
     AMR_RC(scan_total32(h, cnt, off, n, total));
-    Emit E;
-    AMR_RC(emit_buffers(h, total, E));
-    k_gm1_emit<<<nblk(n, TB), TB, 0, h->s>>>(X.A, L, cur, off, E.key, E.leaf, E.val);
-    AMR_RC(grow_nodes(h, X, total));
     // the emit keeps key order: a refined leaf's sons follow it directly and
     // lie before every later node (they fill the leaf's own span)
-    AMR_RC(copy_into(h, total, E.key, E.leaf, E.val, X.B));
+    AMR_RC(grow_next(h, X, total));
+    k_gm1_emit<<<nblk(n, TB), TB, 0, h->s>>>(X.A, L, cur, off, X.B);
+    X.B.n = total;
     swap_sets(h, X);
     return FDM_OK;
 }
@@ -1600,118 +1077,58 @@ static int gridmodify1_pass(fdm_handle *h, AmrCtx &X, bool *did) {
 static int gridmodify4_pass(fdm_handle *h, AmrCtx &X, bool *did) {
     Nvtx range("fdm regrid: gridmodify4");
     const int TB = 256;
-    const int64_t n = X.A.n;
-    Carve cv;
-    cv.add(n * 4); cv.add(n * 8); cv.add(n * 4); cv.add(n * 8); cv.add(n * 4); cv.add(n * 4); cv.add(16);
-    FDM_CK(h, h->amr[15].ensure(cv.total));
-    DevBuf &b = h->amr[15];
-    int32_t *flag = cv.at<int32_t>(b, 0), *idx = cv.at<int32_t>(b, 2), *sidx = cv.at<int32_t>(b, 4);
-    uint64_t *rk = cv.at<uint64_t>(b, 1), *srk = cv.at<uint64_t>(b, 3);
-    int32_t *foff = cv.at<int32_t>(b, 5);
-    int64_t *nsel = cv.at<int64_t>(b, 6);
-    AMR_RC(index_set(h, X.A));
-    k_gm4_triggers<<<nblk(n, TB), TB, 0, h->s>>>(X.A, h->G, flag, rk, idx);
-    // keep the triggering leaves, sorted by traversal rank
-    size_t bytes = 0;
-    FDM_CK(h, cub::DeviceSelect::Flagged(nullptr, bytes, rk, flag, srk, nsel, (int)n, h->s));
-    FDM_CK(h, h->cub_tmp.ensure(bytes));
-    FDM_CK(h, cub::DeviceSelect::Flagged(h->cub_tmp.p, bytes, rk, flag, srk, nsel, (int)n, h->s));
-    FDM_CK(h, cub::DeviceSelect::Flagged(nullptr, bytes, idx, flag, sidx, nsel + 1, (int)n, h->s));
-    FDM_CK(h, h->cub_tmp.ensure(bytes));
-    FDM_CK(h, cub::DeviceSelect::Flagged(h->cub_tmp.p, bytes, idx, flag, sidx, nsel + 1, (int)n, h->s));
-    int64_t ntrig = 0;
-    FDM_CK(h, cudaMemcpyAsync(&ntrig, nsel, 8, cudaMemcpyDeviceToHost, h->s));
-    FDM_CK(h, cudaStreamSynchronize(h->s));
     *did = false;
-    if (ntrig == 0) return FDM_OK;
-    // key order is Morton order (son4 before son3); the traversal visits
-    // son3 first, so sort the triggers by traversal rank
-    FDM_CK(h, cub::DeviceRadixSort::SortPairs(nullptr, bytes, srk, rk, sidx, idx, (int)ntrig, 0, 56, h->s));
-    FDM_CK(h, h->cub_tmp.ensure(bytes));
-    FDM_CK(h, cub::DeviceRadixSort::SortPairs(h->cub_tmp.p, bytes, srk, rk, sidx, idx, (int)ntrig, 0, 56, h->s));
-    // pool + hash of all nodes, room for new ones
-    const int64_t cap = 2 * n + 4096;
-    uint64_t slots = 1;
-    while (slots < (uint64_t)(2 * cap)) slots <<= 1;
-    Carve cp;
-    cp.add(cap * 8); cp.add(cap); cp.add(cap * 4); cp.add(cap * 32); cp.add(slots / HB * sizeof(HBucket)); cp.add(16);
-    cp.add(cap * sizeof(HEnt)); cp.add(32);
-    FDM_CK(h, h->amr[16].ensure(cp.total));
-    DevBuf &pb = h->amr[16];
-    Pool P;
-    P.key = cp.at<uint64_t>(pb, 0); P.flags = cp.at<uint8_t>(pb, 1); P.gen = cp.at<int32_t>(pb, 2);
-    P.val = cp.at<double4>(pb, 3); P.tab = cp.at<HBucket>(pb, 4); P.n = cp.at<int64_t>(pb, 5);
-    P.heap = cp.at<HEnt>(pb, 6);
-    P.err = cp.at<int32_t>(pb, 7);
-    P.bmask = slots / HB - 1;
-    P.cap = cap;
-    P.hcap = cap;
-    FDM_CK(h, cudaMemsetAsync(P.tab, 0xff, slots / HB * sizeof(HBucket), h->s));
-    FDM_CK(h, cudaMemsetAsync(P.err, 0, 32, h->s));
-    FDM_CK(h, cudaMemcpyAsync(P.n, &n, 8, cudaMemcpyHostToDevice, h->s));
-    k_pool_init<<<nblk(n, TB), TB, 0, h->s>>>(X.A, P);
-    // every step consumes a trigger or a queued leaf, or ends the pass
-    const size_t gm4_smem = (size_t)GM4_SQ * sizeof(HEnt);
-    FDM_CK(h, cudaFuncSetAttribute(k_gm4_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gm4_smem));
     for (cudaEvent_t &e : h->gm4_ev)
         if (!e) FDM_CK(h, cudaEventCreate(&e));
-    FDM_CK(h, cudaEventRecord(h->gm4_ev[0], h->s));
-    k_gm4_block<<<1, GM4_THREADS, gm4_smem, h->s>>>(P, h->G, rk, idx, ntrig, 2 * ntrig + 2 * P.hcap + 16);
-    FDM_CK(h, cudaEventRecord(h->gm4_ev[1], h->s));
-    int32_t herr[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    int64_t pn = 0;
-    FDM_CK(h, cudaMemcpyAsync(herr, P.err, 32, cudaMemcpyDeviceToHost, h->s));
-    FDM_CK(h, cudaMemcpyAsync(&pn, P.n, 8, cudaMemcpyDeviceToHost, h->s));
-    FDM_CK(h, cudaStreamSynchronize(h->s));
-    float gm4_t = 0.f;
-    if (cudaEventElapsedTime(&gm4_t, h->gm4_ev[0], h->gm4_ev[1]) == cudaSuccess) h->gm4_ms += gm4_t;
-    if (herr[0]) { h->err = "gridmodify4 cascade exceeded its node pool"; return FDM_ERR_UNSUPPORTED; }
-    if (herr[3]) { h->err = "gridmodify4 replay did not finish"; return FDM_ERR_UNSUPPORTED; }
-    h->gm4_visits += herr[1];
-    h->gm4_nonleaf += herr[2];
-    h->gm4_refines += herr[4];
-    h->gm4_steps += herr[5];
-    h->gm4_triggers += ntrig;
-    *did = herr[4] != 0;
-    if (!*did) return FDM_OK;   // no Refine_cell: the pool holds A unchanged
-    // live nodes back into a sorted node set
-    Carve ce;
-    ce.add(pn * 4); ce.add(pn * 4);
-    FDM_CK(h, h->amr[17].ensure(ce.total));
-    int32_t *live = ce.at<int32_t>(h->amr[17], 0), *loff = ce.at<int32_t>(h->amr[17], 1);
-    k_pool_live<<<nblk(pn, TB), TB, 0, h->s>>>(pn, P.flags, live);
-    int64_t total = 0, m = 0;   // m: live nodes of A (pool entries below n, in key order)
-    AMR_RC(scan_total32(h, live, loff, pn, total, n, &m));
-    Emit E;
-    AMR_RC(emit_buffers(h, total, E));
-    k_pool_emit<<<nblk(pn, TB), TB, 0, h->s>>>(pn, P.flags, P.key, P.val, loff, E.key, E.leaf, E.val);
-    // the new nodes (in the order they were made) sorted by key, then merged
-    // with the survivors of A
-    const int64_t nb = total - m;
-    FDM_CK(h, h->amr[23].ensure(nb * 8 + 16));
-    FDM_CK(h, h->amr[24].ensure(nb + 16));
-    FDM_CK(h, h->amr[25].ensure(nb * 32 + 32));
-    uint64_t *bk = h->amr[23].as<uint64_t>();
-    uint8_t *bl = h->amr[24].as<uint8_t>();
-    double4 *bv = h->amr[25].as<double4>();
-    if (nb > 0) {
-        FDM_CK(h, h->amr[6].ensure(nb * 4 + 16));
-        FDM_CK(h, h->amr[7].ensure(nb * 4 + 16));
-        int32_t *iota = h->amr[6].as<int32_t>(), *perm = h->amr[7].as<int32_t>();
-        k_iota<<<nblk(nb, TB), TB, 0, h->s>>>(nb, iota);
-        size_t bytes = 0;
-        const int kb = 34 + root_bits(h);
-        FDM_CK(h, cub::DeviceRadixSort::SortPairs(nullptr, bytes, E.key + m, bk, iota, perm, (int)nb, 0, kb, h->s));
-        FDM_CK(h, h->cub_tmp.ensure(bytes));
-        FDM_CK(h, cub::DeviceRadixSort::SortPairs(h->cub_tmp.p, bytes, E.key + m, bk, iota, perm, (int)nb, 0, kb, h->s));
-        k_gather_nodes<<<nblk(nb, TB), TB, 0, h->s>>>(nb, perm, E.leaf + m, E.val + m, bl, bv);
+    uint64_t t0 = 0;   // everything up to this time is in A already
+    for (;;) {
+        const int64_t n = X.A.n, cap = (n + 4096 + 3) / 4 * 4;   // room for as many new nodes as the set has
+        Carve c;
+        c.add((n + cap) * 8); c.add((n + cap) * 8); c.add((n + cap) * 4); c.add(2 * 8);   // set to all ones
+        c.add(cap * 8); c.add(cap * 4); c.add((n + cap) * 4); c.add(n * 4);
+        c.add(GW_WORDS * 4); c.add(sizeof(Gm4Result)); c.add(n * 4); c.add(n * 4);
+        FDM_CK(h, h->amr[15].ensure(c.total));
+        DevBuf &b = h->amr[15];
+        Gm4 M;
+        M.t = c.at<uint64_t>(b, 0); M.tn = c.at<uint64_t>(b, 1); M.son = c.at<int32_t>(b, 2);
+        M.nl = c.at<uint64_t>(b, 3); M.mkey = c.at<uint64_t>(b, 4); M.mfather = c.at<int32_t>(b, 5);
+        M.refd = c.at<int32_t>(b, 6);
+        int32_t *list = c.at<int32_t>(b, 7);
+        M.list = list;
+        M.w = c.at<int32_t>(b, 8);
+        Gm4Result *res = c.at<Gm4Result>(b, 9);
+        int32_t *cnt = c.at<int32_t>(b, 10), *off = c.at<int32_t>(b, 11);
+        M.cap = cap;
+        AMR_RC(index_set(h, X.A));
+        FDM_CK(h, cudaMemsetAsync(M.t, 0xff, c.off[4], h->s));
+        FDM_CK(h, cudaMemsetAsync(M.w, 0, GW_WORDS * 4, h->s));
+        k_gm4_triggers<<<nblk(4 * n, TB), TB, 0, h->s>>>(X.A, h->G, t0, list, M.w + GW_NLIST);
+        FDM_CK(h, cudaEventRecord(h->gm4_ev[0], h->s));
+        k_gm4_fixpoint<<<GM4_CTAS, GM4_THREADS, 0, h->s>>>(X.A, h->G, M, t0, 1 << 16, res);
+        FDM_CK(h, cudaEventRecord(h->gm4_ev[1], h->s));
+        k_gm4_count<<<nblk(n, TB), TB, 0, h->s>>>(X.A, M, res, cnt);
+        Gm4Result hr;
+        FDM_CK(h, cudaMemcpyAsync(&hr, res, sizeof hr, cudaMemcpyDeviceToHost, h->s));
+        int64_t total = 0;
+        AMR_RC(scan_total32(h, cnt, off, n, total));   // waits
+        float ms = 0.f;
+        if (cudaEventElapsedTime(&ms, h->gm4_ev[0], h->gm4_ev[1]) == cudaSuccess) h->gm4_ms += ms;
+        if (hr.w[GW_FULL]) { h->err = "gridmodify4 cascade exceeded its node pool"; return FDM_ERR_UNSUPPORTED; }
+        if (hr.w[GW_STUCK]) { h->err = "gridmodify4 times did not settle"; return FDM_ERR_UNSUPPORTED; }
+        h->gm4_visits += hr.w[GW_VISITS];
+        h->gm4_nonleaf += hr.w[GW_NONLEAF];
+        h->gm4_refines += hr.w[GW_REFINES] + hr.w[GW_NONLEAF];
+        h->gm4_steps += hr.w[GW_SWEEPS];
+        if (t0 == 0) h->gm4_triggers += hr.w[GW_NLIST];
+        if (hr.w[GW_REFINES] == 0 && !hr.w[GW_NONLEAF]) return FDM_OK;
+        *did = true;
+        AMR_RC(grow_next(h, X, total));
+        k_gm4_emit<<<nblk(n, TB), TB, 0, h->s>>>(X.A, M, res, off, X.B);
+        X.B.n = total;
+        swap_sets(h, X);
+        if (!hr.w[GW_NONLEAF]) return FDM_OK;
+        t0 = hr.nl_time;
     }
-    AMR_RC(grow_nodes(h, X, total));
-    if (total > 0)
-        k_merge_runs<<<nblk(total, TB), TB, 0, h->s>>>(E.key, E.leaf, E.val, m, bk, bl, bv, nb, X.B);
-    X.B.n = total;
-    swap_sets(h, X);
-    return FDM_OK;
 }
 
 // AMR (src/solution.F90:408-421) after the trigger test: indicators,
@@ -1804,8 +1221,7 @@ static int run_amr_impl(fdm_handle *h, fdm_handle *lead) {
                                               h->ival.as<double4>(), NInt, cflag, off, E.key, E.leaf, E.val);
     AmrCtx X;
     X.h = h;
-    AMR_RC(grow_nodes(h, X, total));
-    bind_sets(h, X);
+    AMR_RC(grow_next(h, X, total));
     merge_into(h, E.key, E.leaf, E.val, split, total, X.B);
     swap_sets(h, X);
     FDM_CK(h, cudaEventRecord(h->amr_ev[2], h->s));

@@ -135,8 +135,8 @@ typedef struct fdm_counters {
                                   (src/mesh.F90:389-392)                      */
     int64_t n_gm4_triggers;    /* gridmodify4: leaves marked able to act at pass start */
     int64_t n_gm4_refines;     /* gridmodify4: Refine_cell calls */
-    int64_t n_gm4_steps;       /* gridmodify4: replay iterations (batches and queued leaves) */
-    int64_t gm4_replay_us;     /* gridmodify4: device time of the replay kernel, microseconds */
+    int64_t n_gm4_steps;       /* gridmodify4: fixpoint sweeps (all passes) */
+    int64_t gm4_replay_us;     /* gridmodify4: device time of the fixpoint kernel, microseconds */
 } fdm_counters;
 
 /* ------------------------------------------------------------- lifecycle */
