@@ -58,7 +58,7 @@ struct Member {
     const float *gate_P;
     GateLists GL;
     int64_t nfx, nfy;
-    Den gm1;                 // gama - 1 with its correctly rounded reciprocal (branch-free division)
+    FluxDen den;             // the face flux's constant denominators
 };
 
 struct GridBar {
@@ -80,27 +80,13 @@ struct BatchArgs {
     int32_t *act;                  // member not finished at the start of the step
     const int32_t *skip_j1;        // host: a regrid follows this step (no body_boundary(1) here)
     unsigned long long *stamp;     // [3][16] global-timer stamps at the phase ends of each stage
-    Den d2;                        // d2 of WCNS_Z3 with its correctly rounded reciprocal
 };
 
-// The full WCNS flux of face f of member M: in the reference's operation
-// order (NRF false), or in the split order with the branch-free division
-// (NRF true, the same bits; a face with an operand outside its range is
-// computed again with the compiler's division).
-template <int DIR, bool NRF>
+// The full WCNS flux of face f of member M.
+template <int DIR>
 __device__ __forceinline__ void batch_face(const Member &M, const double4 *__restrict__ cur, double4 *F, double lam,
-                                           const Den &d2, int64_t f) {
-    if constexpr (NRF) {
-        int32_t a, b, c, d;
-        face_slots<DIR>(M.T, f, a, b, c, d);
-        double out[4];
-        DivNR dv(M.gm1, d2);
-        face_flux_slots_d<DIR>(cur, a, b, c, d, M.gama, dv, lam, out);
-        if (!dv.ok) face_flux_slots<DIR>(cur, a, b, c, d, M.gama, lam, out);
-        F[f] = make_double4(out[0], out[1], out[2], out[3]);
-    } else {
-        face_item<DIR, false>(M.T, cur, F, lam, M.gama, f);
-    }
+                                           int64_t f) {
+    face_item<DIR>(M.T, cur, F, lam, M.gama, M.den, f);
 }
 
 __device__ __forceinline__ unsigned long long gtimer() {
@@ -258,7 +244,6 @@ __device__ __forceinline__ void ph_request_tile(const BatchArgs &A, int krk, int
 
 // faces: plain flux, or gate / guard with the linear flux (whole block);
 // s_loaded names the gate weights held in S.gate
-template <bool NRF>
 __device__ __forceinline__ void ph_face_tile(const BatchArgs &A, int krk, int m, int64_t t, BatchSmem &S,
                                              const float *&s_loaded) {
     const Member &M = A.mem[m];
@@ -273,8 +258,8 @@ __device__ __forceinline__ void ph_face_tile(const BatchArgs &A, int krk, int m,
     if (!M.gate_on) {
         const int64_t f = lt * BT + threadIdx.x;
         if (f < nf) {
-            if (dir == 0) batch_face<0, NRF>(M, cur, M.Fx, lam, A.d2, f);
-            else batch_face<1, NRF>(M, cur, M.Fy, lam, A.d2, f);
+            if (dir == 0) batch_face<0>(M, cur, M.Fx, lam, f);
+            else batch_face<1>(M, cur, M.Fy, lam, f);
         }
         return;
     }
@@ -318,17 +303,16 @@ __device__ __forceinline__ void ph_hard_offsets(const BatchArgs &A, int krk) {
 }
 
 // hard faces (full WCNS flux) of tile t of member m
-template <bool NRF>
 __device__ __forceinline__ void ph_hard_tile(const BatchArgs &A, int krk, int m, int64_t t) {
     const Member &M = A.mem[m];
     const double4 *cur = stage_cur(M, krk);
     const int64_t tx = cdiv(M.GL.cnt[0], BT);
     if (t < tx) {
         const int64_t i = t * BT + threadIdx.x;
-        if (i < M.GL.cnt[0]) batch_face<0, NRF>(M, cur, M.Fx, M.sc->lambda_x, A.d2, M.GL.hx[i]);
+        if (i < M.GL.cnt[0]) batch_face<0>(M, cur, M.Fx, M.sc->lambda_x, M.GL.hx[i]);
     } else {
         const int64_t i = (t - tx) * BT + threadIdx.x;
-        if (i < M.GL.cnt[1]) batch_face<1, NRF>(M, cur, M.Fy, M.sc->lambda_y, A.d2, M.GL.hy[i]);
+        if (i < M.GL.cnt[1]) batch_face<1>(M, cur, M.Fy, M.sc->lambda_y, M.GL.hy[i]);
     }
 }
 
@@ -372,7 +356,7 @@ __device__ __forceinline__ void ph_end_member(const BatchArgs &A, int m, double 
 
 // One RK stage (krk) of every member; MINB resident blocks per SM (the
 // register budget follows: 128 per thread at 2, up to 255 at 1).
-template <int MINB, bool NRF>
+template <int MINB>
 __global__ void __launch_bounds__(BT, MINB) k_batch_stage(BatchArgs A, int krk) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BatchSmem &S = *reinterpret_cast<BatchSmem *>(smem_raw);
@@ -399,14 +383,14 @@ __global__ void __launch_bounds__(BT, MINB) k_batch_stage(BatchArgs A, int krk) 
     if (threadIdx.x == 0) s_loaded = nullptr;
     __syncthreads();
     run_tiles(A, PH_FACE, A.off + PH_FACE * np1, &s_t, s_off,
-              [&](int m, int64_t t) { ph_face_tile<NRF>(A, krk, m, t, S, s_loaded); });
+              [&](int m, int64_t t) { ph_face_tile(A, krk, m, t, S, s_loaded); });
     BAR_STAMP(3);
 
     // ---- hard faces of gated members (full WCNS flux)
     if (A.any_gate) {
         if (blockIdx.x == 0 && threadIdx.x == 0) ph_hard_offsets(A, krk);
         BAR_STAMP(4);
-        run_tiles(A, PH_HARD, A.off_hard, &s_t, s_off, [&](int m, int64_t t) { ph_hard_tile<NRF>(A, krk, m, t); });
+        run_tiles(A, PH_HARD, A.off_hard, &s_t, s_off, [&](int m, int64_t t) { ph_hard_tile(A, krk, m, t); });
         BAR_STAMP(5);
     }
 
@@ -464,7 +448,6 @@ __global__ void __launch_bounds__(BT) k_bp_requests(BatchArgs A, int krk) {
     __shared__ int64_t s_off[OFF_CAP];
     flat_tiles(A, A.off + PH_REQ * (A.nmem + 1), s_off, [&](int m, int64_t t) { ph_request_tile(A, krk, m, t, S); });
 }
-template <bool NRF>
 __global__ void __launch_bounds__(BT, 2) k_bp_faces(BatchArgs A, int krk) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BatchSmem &S = *reinterpret_cast<BatchSmem *>(smem_raw);
@@ -473,15 +456,14 @@ __global__ void __launch_bounds__(BT, 2) k_bp_faces(BatchArgs A, int krk) {
     if (threadIdx.x == 0) s_loaded = nullptr;
     __syncthreads();
     flat_tiles(A, A.off + PH_FACE * (A.nmem + 1), s_off,
-               [&](int m, int64_t t) { ph_face_tile<NRF>(A, krk, m, t, S, s_loaded); });
+               [&](int m, int64_t t) { ph_face_tile(A, krk, m, t, S, s_loaded); });
 }
 __global__ void k_bp_hard_offsets(BatchArgs A, int krk) {
     if (threadIdx.x == 0 && blockIdx.x == 0) ph_hard_offsets(A, krk);
 }
-template <bool NRF>
 __global__ void __launch_bounds__(BT, 2) k_bp_hard(BatchArgs A, int krk) {
     __shared__ int64_t s_off[OFF_CAP];
-    flat_tiles(A, A.off_hard, s_off, [&](int m, int64_t t) { ph_hard_tile<NRF>(A, krk, m, t); });
+    flat_tiles(A, A.off_hard, s_off, [&](int m, int64_t t) { ph_hard_tile(A, krk, m, t); });
 }
 __global__ void __launch_bounds__(BT) k_bp_cells(BatchArgs A, int krk) {
     __shared__ CellsSmem s_cells;
@@ -522,7 +504,6 @@ struct fdm_batch {
                                                      // 3: phase kernels (no persistent kernel)
     std::vector<int64_t> h_off;                      // tile offsets per phase (host copy)
     int sms = 0;
-    bool face_nr = false;                            // branch-free division in the face phases
     size_t smem = 0;
     bool any_gate = false;
     cudaGraphExec_t graph = nullptr;
@@ -578,7 +559,7 @@ static int batch_refresh(fdm_batch *b) {
         d.nfx = h->NI + h->nux;
         d.nfy = h->NI + h->nuy;
         d.gate_on = h->gate_on;
-        d.gm1 = Den{h->G.gama - 1.0, 1.0 / (h->G.gama - 1.0)};   // IEEE division on the host
+        d.den = flux_den(h->G.gama);
         if (h->gate_on) {
             b->any_gate = true;
             d.logit_thr = h->gate_logit_thr;
@@ -625,8 +606,7 @@ static bool batch_stale(const fdm_batch *b) {
 
 // the persistent kernel of the batch's launch shape and face flux
 static const void *batch_kernel(const fdm_batch *b) {
-    if (b->want_bps == 1) return b->face_nr ? (const void *)k_batch_stage<1, true> : (const void *)k_batch_stage<1, false>;
-    return b->face_nr ? (const void *)k_batch_stage<2, true> : (const void *)k_batch_stage<2, false>;
+    return b->want_bps == 1 ? (const void *)k_batch_stage<1> : (const void *)k_batch_stage<2>;
 }
 
 static int batch_grid(fdm_batch *b) {
@@ -638,8 +618,7 @@ static int batch_grid(fdm_batch *b) {
         BCK(b, cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, b->device));
         BCK(b, cudaFuncSetAttribute(k_bp_requests, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->smem));
         BCK(b, cudaFuncSetAttribute(k_bp_ghosts, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->smem));
-        BCK(b, cudaFuncSetAttribute(k_bp_faces<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->smem));
-        BCK(b, cudaFuncSetAttribute(k_bp_faces<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->smem));
+        BCK(b, cudaFuncSetAttribute(k_bp_faces, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->smem));
         b->blocks_per_sm = 0;
         b->grid = 0;
         return FDM_OK;
@@ -664,16 +643,12 @@ static int enqueue_phase_kernels(fdm_batch *b, const BatchArgs &A, int krk) {
     auto grid = [](int64_t t) { return (unsigned)std::min<int64_t>(t, 1ll << 30); };
     k_bp_begin<<<1, BT, 0, b->s>>>(A, krk);
     if (total(PH_REQ) > 0) k_bp_requests<<<grid(total(PH_REQ)), BT, b->smem, b->s>>>(A, krk);
-    if (total(PH_FACE) > 0) {
-        if (b->face_nr) k_bp_faces<true><<<grid(total(PH_FACE)), BT, b->smem, b->s>>>(A, krk);
-        else k_bp_faces<false><<<grid(total(PH_FACE)), BT, b->smem, b->s>>>(A, krk);
-    }
+    if (total(PH_FACE) > 0) k_bp_faces<<<grid(total(PH_FACE)), BT, b->smem, b->s>>>(A, krk);
     if (A.any_gate) {
         // hard-face tiles are known on the device only: a grid-stride launch
         k_bp_hard_offsets<<<1, 32, 0, b->s>>>(A, krk);
         const unsigned g = (unsigned)(4 * b->sms);
-        if (b->face_nr) k_bp_hard<true><<<g, BT, 0, b->s>>>(A, krk);
-        else k_bp_hard<false><<<g, BT, 0, b->s>>>(A, krk);
+        k_bp_hard<<<g, BT, 0, b->s>>>(A, krk);
     }
     if (total(PH_CELL) > 0) k_bp_cells<<<grid(total(PH_CELL)), BT, 0, b->s>>>(A, krk);
     if (total(PH_GHOST) > 0) k_bp_ghosts<<<grid(total(PH_GHOST)), BT, b->smem, b->s>>>(A, krk, 3);
@@ -697,7 +672,6 @@ static int enqueue_batch_stage(fdm_batch *b, int krk) {
     A.act = b->d_act.as<int32_t>();
     A.skip_j1 = b->d_skip.as<int32_t>();
     A.stamp = b->d_stamp.as<unsigned long long>();
-    A.d2 = Den{FDM_D2_WCNS, 1.0 / FDM_D2_WCNS};   // IEEE division on the host
     BCK(b, cudaMemsetAsync(A.ctr, 0, sizeof(unsigned long long) * N_PHASE, b->s));
     if (b->want_bps == 3) return enqueue_phase_kernels(b, A, krk);
     cudaLaunchConfig_t cfg = {};
@@ -710,13 +684,8 @@ static int enqueue_batch_stage(fdm_batch *b, int krk) {
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (b->want_bps == 1) {
-        if (b->face_nr) BCK(b, cudaLaunchKernelEx(&cfg, k_batch_stage<1, true>, A, krk));
-        else BCK(b, cudaLaunchKernelEx(&cfg, k_batch_stage<1, false>, A, krk));
-    } else {
-        if (b->face_nr) BCK(b, cudaLaunchKernelEx(&cfg, k_batch_stage<2, true>, A, krk));
-        else BCK(b, cudaLaunchKernelEx(&cfg, k_batch_stage<2, false>, A, krk));
-    }
+    if (b->want_bps == 1) BCK(b, cudaLaunchKernelEx(&cfg, k_batch_stage<1>, A, krk));
+    else BCK(b, cudaLaunchKernelEx(&cfg, k_batch_stage<2>, A, krk));
     return FDM_OK;
 }
 
@@ -1044,16 +1013,10 @@ int fdm_batch_set_blocks_per_sm(fdm_batch *b, int32_t bps) {
     return FDM_OK;
 }
 
-// Face phases of the persistent kernel: the reference's operation order
-// (0) or the split order with the branch-free division (1); the same bits.
+// Kept for its callers: both face fluxes are one kernel path now, with the
+// same bits.
 int fdm_batch_set_face_flux(fdm_batch *b, int32_t branch_free) {
-    if (!b || branch_free < 0 || branch_free > 1) return FDM_ERR_ARG;
-    cudaSetDevice(b->device);
-    b->face_nr = branch_free != 0;
-    int rc = batch_grid(b);
-    if (rc) return rc;
-    drop_batch_graph(b);
-    return FDM_OK;
+    return !b || branch_free < 0 || branch_free > 1 ? FDM_ERR_ARG : FDM_OK;
 }
 
 // Wait limit of one grid barrier of the persistent kernel, in seconds

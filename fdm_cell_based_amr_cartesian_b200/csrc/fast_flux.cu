@@ -203,12 +203,20 @@ __device__ __forceinline__ void face_item(const Tables &T, const double4 *__rest
 
 static inline int nblk(int64_t n, int t) { return (int)((n + t - 1) / t); }
 
-template <int DIR, int TB, int MINB>
-__global__ void __launch_bounds__(TB, MINB) k_faces_fast(Tables T, const double4 *__restrict__ cur, double4 *F,
-                                                         const DevScalars *__restrict__ sc, double g) {
-    const int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (f >= T.NI + (DIR == 0 ? T.nux : T.nuy)) return;
-    fast::face_item<DIR>(T, cur, F, DIR == 0 ? sc->lambda_x : sc->lambda_y, g, 1.0 / (g - 1.0), f);
+// x faces' blocks (nbx), then the y faces', as k_faces of stage.cu
+template <int TB, int MINB>
+__global__ void __launch_bounds__(TB, MINB) k_faces_fast(Tables T, const double4 *__restrict__ cur, double4 *Fx,
+                                                         double4 *Fy, const DevScalars *__restrict__ sc, double g,
+                                                         int nbx) {
+    const int64_t b = blockIdx.x;
+    const double ig1 = 1.0 / (g - 1.0);
+    if (b < nbx) {
+        const int64_t f = b * TB + threadIdx.x;
+        if (f < T.NI + T.nux) fast::face_item<0>(T, cur, Fx, sc->lambda_x, g, ig1, f);
+    } else {
+        const int64_t f = (b - nbx) * TB + threadIdx.x;
+        if (f < T.NI + T.nuy) fast::face_item<1>(T, cur, Fy, sc->lambda_y, g, ig1, f);
+    }
 }
 
 // hard-face list of the learned gate
@@ -225,21 +233,20 @@ __global__ void __launch_bounds__(256, 2) k_faces_list_fast(Tables T, const doub
 
 template <int TB, int MINB>
 static void faces_fast(fdm_handle *h, const double4 *cur) {
-    const Tables T = h->tables();
-    const DevScalars *sc = h->scal.as<DevScalars>();
-    k_faces_fast<0, TB, MINB><<<nblk(h->NI + h->nux, TB), TB, 0, h->s>>>(T, cur, h->Fx.as<double4>(), sc, h->G.gama);
-    k_faces_fast<1, TB, MINB><<<nblk(h->NI + h->nuy, TB), TB, 0, h->s>>>(T, cur, h->Fy.as<double4>(), sc, h->G.gama);
+    const int nbx = nblk(h->NI + h->nux, TB), nby = nblk(h->NI + h->nuy, TB);
+    k_faces_fast<TB, MINB><<<nbx + nby, TB, 0, h->s>>>(h->tables(), cur, h->Fx.as<double4>(), h->Fy.as<double4>(),
+                                                       h->scal.as<DevScalars>(), h->G.gama, nbx);
 }
 
-// the launch shapes of the autotuner, one thread per face
+// the launch shapes of the autotuner (stage.cu)
 void launch_faces_fast(fdm_handle *h, const double4 *cur) {
-    switch (h->face_variant) {
-        case 1: faces_fast<128, 4>(h, cur); break;
-        case 2: faces_fast<64, 7>(h, cur); break;
+    switch (h->face_variant % 6) {
+        case 1: faces_fast<128, 3>(h, cur); break;
+        case 2: faces_fast<64, 8>(h, cur); break;
         case 3: faces_fast<256, 2>(h, cur); break;
-        case 5: faces_fast<128, 5>(h, cur); break;
-        case 6: faces_fast<64, 10>(h, cur); break;
-        default: faces_fast<128, 3>(h, cur); break;
+        case 4: faces_fast<128, 5>(h, cur); break;
+        case 5: faces_fast<64, 10>(h, cur); break;
+        default: faces_fast<128, 4>(h, cur); break;
     }
 }
 

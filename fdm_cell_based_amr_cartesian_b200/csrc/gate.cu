@@ -20,52 +20,66 @@ namespace fdm {
 
 static inline int nblk(int64_t n, int t) { return (int)((n + t - 1) / t); }
 
+// The gate's per-direction arguments of the two kernels below, which take
+// the warps' chunks of 32 x faces and then those of the y faces in one
+// launch (half the launches of a stage, one partial wave instead of two).
+struct GateDir {
+    double4 *F;
+    int32_t *hard;
+    float *jump1;
+};
 // Stage 1, persistent: each warp takes 32 faces at a time.
-template <int DIR>
-__global__ void __launch_bounds__(128, 4) k_gate_linear(Tables T, const double4 *__restrict__ cur, double4 *F,
+__global__ void __launch_bounds__(128, 4) k_gate_linear(Tables T, const double4 *__restrict__ cur,
                                                         const float *__restrict__ P, float logit_thr,
                                                         float jump_thr, const DevScalars *__restrict__ sc, double g,
-                                                        int32_t *hard,
-                                                        uint32_t *count, float *jump1) {
+                                                        GateDir X, GateDir Y, uint32_t *count) {
     __shared__ GateWeights W;
     __shared__ XTile tiles[4];
     load_weights_smem(W, P);
     __syncthreads();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int64_t nf = T.NI + (DIR == 0 ? T.nux : T.nuy);
-    const double lam = DIR == 0 ? sc->lambda_x : sc->lambda_y;
+    const int64_t wx = (T.NI + T.nux + 31) / 32, wy = (T.NI + T.nuy + 31) / 32;
     const double ig1 = 1.0 / (g - 1.0);
     XTile &Tt = tiles[wid];
     for (int k = GF; k < XLD; ++k) Tt.X[lane][k] = __float2bfloat16_rn(0.f);
     const int64_t nwarps = (int64_t)gridDim.x * 4;
-    for (int64_t w = blockIdx.x * 4 + wid; w * 32 < nf; w += nwarps)
-        gate_linear_chunk<DIR>(T, cur, F, W, Tt, logit_thr, jump_thr, lam, ig1, g, hard, count, jump1, w);
+    for (int64_t w = blockIdx.x * 4 + wid; w < wx + wy; w += nwarps) {
+        if (w < wx)
+            gate_linear_chunk<0>(T, cur, X.F, W, Tt, logit_thr, jump_thr, sc->lambda_x, ig1, g, X.hard, count, X.jump1,
+                                 w);
+        else
+            gate_linear_chunk<1>(T, cur, Y.F, W, Tt, logit_thr, jump_thr, sc->lambda_y, ig1, g, Y.hard, count + 1,
+                                 Y.jump1, w - wx);
+    }
 }
 
 // Stages 2 and 3: the guard on the faces that were linear at stage 1.
-template <int DIR>
-__global__ void __launch_bounds__(256) k_guard_linear(Tables T, const double4 *__restrict__ cur, double4 *F,
-                                                      const float *__restrict__ jump1,
-                                                      const DevScalars *__restrict__ sc, double g, int32_t *hard,
-                                                      uint32_t *count) {
-    const int64_t nf = T.NI + (DIR == 0 ? T.nux : T.nuy);
-    const double lam = DIR == 0 ? sc->lambda_x : sc->lambda_y;
+__global__ void __launch_bounds__(256) k_guard_linear(Tables T, const double4 *__restrict__ cur,
+                                                      const DevScalars *__restrict__ sc, double g, GateDir X,
+                                                      GateDir Y, uint32_t *count) {
+    const int64_t wx = (T.NI + T.nux + 31) / 32, wy = (T.NI + T.nuy + 31) / 32;
     const double ig1 = 1.0 / (g - 1.0);
-    const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t w = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); w * 32 < nf; w += nwarps)
-        guard_linear_chunk<DIR>(T, cur, F, jump1, lam, ig1, g, hard, count, w);
+    const int64_t w = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (w < wx) guard_linear_chunk<0>(T, cur, X.F, X.jump1, sc->lambda_x, ig1, g, X.hard, count, w);
+    else if (w < wx + wy)
+        guard_linear_chunk<1>(T, cur, Y.F, Y.jump1, sc->lambda_y, ig1, g, Y.hard, count + 1, w - wx);
 }
 
 // full WCNS flux of the faces on the hard list
-template <int DIR>
-__global__ void __launch_bounds__(256, 2) k_faces_list(Tables T, const double4 *__restrict__ cur, double4 *F,
-                                                       const int32_t *__restrict__ hard,
+__global__ void __launch_bounds__(128, 4) k_faces_list(Tables T, const double4 *__restrict__ cur, double4 *Fx,
+                                                       double4 *Fy, const int32_t *__restrict__ hx,
+                                                       const int32_t *__restrict__ hy,
                                                        const uint32_t *__restrict__ count,
-                                                       const DevScalars *__restrict__ sc, double g) {
-    const int64_t n = *count;
-    const double lam = DIR == 0 ? sc->lambda_x : sc->lambda_y;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        face_item<DIR>(T, cur, F, lam, g, hard[i]);
+                                                       const DevScalars *__restrict__ sc, double g, FluxDen den) {
+    // the x list, then the y list, whole warps to each
+    const int64_t nx = count[0], ny = count[1], px = (nx + 31) / 32 * 32, stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < px + ny; i += stride) {
+        if (i < px) {
+            if (i < nx) face_item<0>(T, cur, Fx, sc->lambda_x, g, den, hx[i]);
+        } else {
+            face_item<1>(T, cur, Fy, sc->lambda_y, g, den, hy[i - px]);
+        }
+    }
 }
 
 // --------------------------------------------------- training samples
@@ -299,25 +313,24 @@ void launch_gated_faces(fdm_handle *h, const double4 *cur, int krk) {
     const float *P = h->gate_params.as<float>();
     const int sms = sm_count();
     const int lx = (int)std::min<int64_t>(nblk(nfx, 256), 2 * sms), ly = (int)std::min<int64_t>(nblk(nfy, 256), 2 * sms);
+    const GateDir X{h->Fx.as<double4>(), hx, jx}, Y{h->Fy.as<double4>(), hy, jy};
+    const int64_t warps = (nfx + 31) / 32 + (nfy + 31) / 32;
     if (krk == 1 || !h->gate_stage1_valid) {
-        const int gx = (int)std::min<int64_t>(nblk(nfx, 128), 4 * sms), gy = (int)std::min<int64_t>(nblk(nfy, 128), 4 * sms);
         cudaMemsetAsync(cnt, 0, 2 * sizeof(uint32_t), h->s);
-        if (gx > 0) k_gate_linear<0><<<gx, 128, 0, h->s>>>(T, cur, h->Fx.as<double4>(), P, h->gate_logit_thr, h->gate_jump_thr, sc, h->G.gama, hx, cnt, jx);
-        if (gy > 0) k_gate_linear<1><<<gy, 128, 0, h->s>>>(T, cur, h->Fy.as<double4>(), P, h->gate_logit_thr, h->gate_jump_thr, sc, h->G.gama, hy, cnt + 1, jy);
+        k_gate_linear<<<(int)std::min<int64_t>(nblk(warps, 4), 4 * sms), 128, 0, h->s>>>(
+            T, cur, P, h->gate_logit_thr, h->gate_jump_thr, sc, h->G.gama, X, Y, cnt);
         cudaMemcpyAsync(cnt + 2, cnt, 2 * sizeof(uint32_t), cudaMemcpyDeviceToDevice, h->s);
         h->gate_stage1_valid = true;
     } else {
-        const int gx = (int)std::min<int64_t>(nblk(nfx, 256), 4 * sms), gy = (int)std::min<int64_t>(nblk(nfy, 256), 4 * sms);
         cudaMemcpyAsync(cnt, cnt + 2, 2 * sizeof(uint32_t), cudaMemcpyDeviceToDevice, h->s);
-        if (gx > 0) k_guard_linear<0><<<gx, 256, 0, h->s>>>(T, cur, h->Fx.as<double4>(), jx, sc, h->G.gama, hx, cnt);
-        if (gy > 0) k_guard_linear<1><<<gy, 256, 0, h->s>>>(T, cur, h->Fy.as<double4>(), jy, sc, h->G.gama, hy, cnt + 1);
+        k_guard_linear<<<nblk(warps, 8), 256, 0, h->s>>>(T, cur, sc, h->G.gama, X, Y, cnt);
     }
     if (h->p.flux_variant == 1) {
         launch_faces_list_fast(h, cur, hx, hy, cnt, lx, ly);
         return;
     }
-    if (lx > 0) k_faces_list<0><<<lx, 256, 0, h->s>>>(T, cur, h->Fx.as<double4>(), hx, cnt, sc, h->G.gama);
-    if (ly > 0) k_faces_list<1><<<ly, 256, 0, h->s>>>(T, cur, h->Fy.as<double4>(), hy, cnt + 1, sc, h->G.gama);
+    k_faces_list<<<(int)std::min<int64_t>(nblk(nfx + nfy, 128), 4 * sms), 128, 0, h->s>>>(
+        T, cur, h->Fx.as<double4>(), h->Fy.as<double4>(), hx, hy, cnt, sc, h->G.gama, flux_den(h->G.gama));
 }
 
 size_t gate_list_bytes(const fdm_handle *h) {

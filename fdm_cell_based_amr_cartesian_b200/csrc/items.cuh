@@ -18,6 +18,7 @@
 
 #include "handle.cuh"
 #include "numerics.cuh"
+#include "numerics_nr.cuh"
 
 namespace fdm {
 
@@ -259,19 +260,12 @@ __device__ __forceinline__ void face_slots(const Tables &T, int64_t f, int32_t &
     }
 }
 
-template <int DIR, bool SPLIT = true>
+template <int DIR>
 __device__ __forceinline__ void face_item(const Tables &T, const double4 *__restrict__ cur, double4 *F, double lam,
-                                          double g, int64_t f) {
+                                          double g, const FluxDen &den, int64_t f) {
     int32_t a, b, c, d;
     face_slots<DIR>(T, f, a, b, c, d);
-    double out[4];
-    if constexpr (SPLIT) {   // the records read again for the flux half: fewer live registers
-        face_flux_slots<DIR>(cur, a, b, c, d, g, lam, out);
-    } else {
-        const Prim p0 = load_prim(cur, a), p1 = load_prim(cur, b), p2 = load_prim(cur, c), p3 = load_prim(cur, d);
-        face_flux<DIR, false>(p0, p1, p2, p3, g, lam, out);
-    }
-    F[f] = make_double4(out[0], out[1], out[2], out[3]);
+    F[f] = face_flux_of<DIR>(cur, a, b, c, d, g, den, lam);
 }
 
 // Residual + forward-Euler candidate (LXL) fused with updateRK for leaf i.

@@ -14,8 +14,6 @@
 #include "handle.cuh"
 #include "items.cuh"
 #include "numerics.cuh"
-#include "numerics_nr.cuh"
-#include "numerics_sm.cuh"
 
 namespace fdm {
 
@@ -38,112 +36,28 @@ __global__ void __launch_bounds__(128) k_requests_restrict(Tables T, double4 *cu
 }
 
 // One thread per face; TB threads per block, at least MINB blocks per SM
-// (the register budget follows from both).
-template <int DIR, int TB, int MINB>
-__global__ void __launch_bounds__(TB, MINB) k_faces(Tables T, const double4 *__restrict__ cur, double4 *F,
-                                                    const DevScalars *__restrict__ sc, double g) {
-    const int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t nu = DIR == 0 ? T.nux : T.nuy;
-    if (f >= T.NI + nu) return;
-    face_item<DIR>(T, cur, F, DIR == 0 ? sc->lambda_x : sc->lambda_y, g, f);
-}
-
-// The same faces with every division formed by DivNR (numerics_nr.cuh):
-// identical quotients without the branches of the compiler's division, so
-// the reconstructions of a face can be interleaved.  A face with an operand
-// outside DivNR's range is computed again with the compiler's division.
-template <int DIR, int TB, int MINB>
-__global__ void __launch_bounds__(TB, MINB) k_faces_nr(Tables T, const double4 *__restrict__ cur, double4 *F,
-                                                       const DevScalars *__restrict__ sc, double g, Den gm1,
-                                                       Den d2) {
-    const int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t nu = DIR == 0 ? T.nux : T.nuy;
-    if (f >= T.NI + nu) return;
-    int32_t a, b, c, d;
-    face_slots<DIR>(T, f, a, b, c, d);
-    const double lam = DIR == 0 ? sc->lambda_x : sc->lambda_y;
-    double out[4];
-    DivNR dv(gm1, d2);
-    face_flux_slots_d<DIR>(cur, a, b, c, d, g, dv, lam, out);
-    if (!dv.ok) face_flux_slots<DIR>(cur, a, b, c, d, g, lam, out);
-    F[f] = make_double4(out[0], out[1], out[2], out[3]);
-}
-
-// One thread per face in the reference's operation order (the four states
-// and fluxes formed first), with the compiler's division (NR false) or the
-// branch-free one (NR true; a face with an operand outside its range is
-// computed again with the compiler's division).
-template <int DIR, int TB, int MINB, bool NR>
-__global__ void __launch_bounds__(TB, MINB) k_faces_ref(Tables T, const double4 *__restrict__ cur, double4 *F,
-                                                        const DevScalars *__restrict__ sc, double g, Den gm1,
-                                                        Den d2) {
-    const int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t nu = DIR == 0 ? T.nux : T.nuy;
-    if (f >= T.NI + nu) return;
-    int32_t a, b, c, d;
-    face_slots<DIR>(T, f, a, b, c, d);
-    const double lam = DIR == 0 ? sc->lambda_x : sc->lambda_y;
-    const Prim p0 = load_prim(cur, a), p1 = load_prim(cur, b), p2 = load_prim(cur, c), p3 = load_prim(cur, d);
-    double out[4];
-    if constexpr (NR) {
-        DivNR dv(gm1, d2);
-        face_flux_ref_d<DIR>(p0, p1, p2, p3, g, dv, lam, out);
-        if (!dv.ok) face_flux<DIR, false>(p0, p1, p2, p3, g, lam, out);
+// (the register budget follows from both).  One launch covers the x faces
+// and then the y faces (nbx blocks of x), so both share the last wave.
+//
+// Bound by the FP64 pipe: about 2000 FP64 instructions per face, two cycles
+// each on a quarter of an SM.  What it took to keep the pipe busy was
+// straight-line code (numerics_nr.cuh), not occupancy: 16 warps at 128
+// registers or 12 at 168 or 20 at 96 are within 2 %.  One B200, x+y pair, ms,
+// beside the compiler's division in one launch per direction (its best
+// shape): 1.03M leaves 0.213 (0.432), 260k 0.060 (0.113), 148k 0.037 (0.077),
+// 17k 0.0104 (0.0309), 3k 0.0067 (0.0247).
+template <int TB, int MINB>
+__global__ void __launch_bounds__(TB, MINB) k_faces(Tables T, const double4 *__restrict__ cur, double4 *Fx,
+                                                    double4 *Fy, const DevScalars *__restrict__ sc, double g,
+                                                    FluxDen den, int nbx) {
+    const int64_t b = blockIdx.x;
+    if (b < nbx) {
+        const int64_t f = b * TB + threadIdx.x;
+        if (f < T.NI + T.nux) face_item<0>(T, cur, Fx, sc->lambda_x, g, den, f);
     } else {
-        face_flux<DIR, false>(p0, p1, p2, p3, g, lam, out);
+        const int64_t f = (b - nbx) * TB + threadIdx.x;
+        if (f < T.NI + T.nuy) face_item<1>(T, cur, Fy, sc->lambda_y, g, den, f);
     }
-    F[f] = make_double4(out[0], out[1], out[2], out[3]);
-}
-
-// The faces with the constant denominators divided by one correction
-// (DivConst, numerics_nr.cuh), every other division as the compiler forms
-// it; SPLIT: the split order (state half, then flux half), else the
-// reference's order.  A face with an operand outside the range is computed
-// again with the compiler's division.
-template <int DIR, int TB, int MINB, bool SPLIT>
-__global__ void __launch_bounds__(TB, MINB) k_faces_c(Tables T, const double4 *__restrict__ cur, double4 *F,
-                                                      const DevScalars *__restrict__ sc, double g, DenC gm1,
-                                                      DenC d2) {
-    const int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t nu = DIR == 0 ? T.nux : T.nuy;
-    if (f >= T.NI + nu) return;
-    int32_t a, b, c, d;
-    face_slots<DIR>(T, f, a, b, c, d);
-    const double lam = DIR == 0 ? sc->lambda_x : sc->lambda_y;
-    double out[4];
-    DivConst dv(gm1, d2);
-    if constexpr (SPLIT) {
-        face_flux_slots_d<DIR>(cur, a, b, c, d, g, dv, lam, out);
-        if (!dv.ok) face_flux_slots<DIR>(cur, a, b, c, d, g, lam, out);
-    } else {
-        const Prim p0 = load_prim(cur, a), p1 = load_prim(cur, b), p2 = load_prim(cur, c), p3 = load_prim(cur, d);
-        face_flux_ref_d<DIR>(p0, p1, p2, p3, g, dv, lam, out);
-        if (!dv.ok) face_flux<DIR, false>(p0, p1, p2, p3, g, lam, out);
-    }
-    F[f] = make_double4(out[0], out[1], out[2], out[3]);
-}
-
-// Variant 15's arithmetic with the face's characteristic basis in shared
-// memory (numerics_sm.cuh): fewer live registers, so more warps per SM.
-template <int DIR, int TB, int MINB>
-__global__ void __launch_bounds__(TB, MINB) k_faces_sm(Tables T, const double4 *__restrict__ cur, double4 *F,
-                                                       const DevScalars *__restrict__ sc, double g, DenC gm1,
-                                                       DenC d2) {
-    __shared__ EigShared<TB> S;
-    const int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t nu = DIR == 0 ? T.nux : T.nuy;
-    if (f >= T.NI + nu) return;
-    int32_t a, b, c, d;
-    face_slots<DIR>(T, f, a, b, c, d);
-    const double lam = DIR == 0 ? sc->lambda_x : sc->lambda_y;
-    double out[4];
-    DivConst dv(gm1, d2);
-    face_flux_slots_sm<DIR, TB>(cur, a, b, c, d, g, dv, lam, S, threadIdx.x, out);
-    if (!dv.ok) {   // the compiler's division, the basis again in shared memory
-        DivIEEE di(g);
-        face_flux_slots_sm<DIR, TB>(cur, a, b, c, d, g, di, lam, S, threadIdx.x, out);
-    }
-    F[f] = make_double4(out[0], out[1], out[2], out[3]);
 }
 
 // Diagnostics: the faces whose branch-free division meets an operand
@@ -151,8 +65,8 @@ __global__ void __launch_bounds__(TB, MINB) k_faces_sm(Tables T, const double4 *
 // division), counted over the current state; nothing is written to F.
 template <int DIR>
 __global__ void __launch_bounds__(128) k_faces_nr_count(Tables T, const double4 *__restrict__ cur,
-                                                        const DevScalars *__restrict__ sc, double g, Den gm1,
-                                                        Den d2, unsigned long long *count) {
+                                                        const DevScalars *__restrict__ sc, double g,
+                                                        FluxDen den, unsigned long long *count) {
     const int64_t f = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int64_t nu = DIR == 0 ? T.nux : T.nuy;
     bool fell = false;
@@ -160,8 +74,8 @@ __global__ void __launch_bounds__(128) k_faces_nr_count(Tables T, const double4 
         int32_t a, b, c, d;
         face_slots<DIR>(T, f, a, b, c, d);
         double out[4];
-        DivNR dv(gm1, d2);
-        face_flux_slots_d<DIR>(cur, a, b, c, d, g, dv, DIR == 0 ? sc->lambda_x : sc->lambda_y, out);
+        DivNR dv(den);
+        face_flux_nr<DIR>(cur, a, b, c, d, g, dv, DIR == 0 ? sc->lambda_x : sc->lambda_y, out);
         fell = !dv.ok;
     }
     const unsigned m = __ballot_sync(0xffffffffu, fell);
@@ -171,13 +85,13 @@ int count_nr_fallbacks(fdm_handle *h, int64_t out[2]) {
     const Tables T = h->tables();
     const DevScalars *sc = h->scal.as<DevScalars>();
     const double g = h->G.gama;
-    const Den gm1{g - 1.0, 1.0 / (g - 1.0)}, d2{FDM_D2_WCNS, 1.0 / FDM_D2_WCNS};
+    const FluxDen den = flux_den(g);
     FDM_CK(h, h->tmp[7].ensure(2 * sizeof(unsigned long long)));
     unsigned long long *cnt = h->tmp[7].as<unsigned long long>();
     FDM_CK(h, cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned long long), h->s));
     launch_requests(h, h->B[0].as<double4>());
-    k_faces_nr_count<0><<<nblk(h->NI + h->nux, 128), 128, 0, h->s>>>(T, h->B[0].as<double4>(), sc, g, gm1, d2, cnt);
-    k_faces_nr_count<1><<<nblk(h->NI + h->nuy, 128), 128, 0, h->s>>>(T, h->B[0].as<double4>(), sc, g, gm1, d2,
+    k_faces_nr_count<0><<<nblk(h->NI + h->nux, 128), 128, 0, h->s>>>(T, h->B[0].as<double4>(), sc, g, den, cnt);
+    k_faces_nr_count<1><<<nblk(h->NI + h->nuy, 128), 128, 0, h->s>>>(T, h->B[0].as<double4>(), sc, g, den,
                                                                        cnt + 1);
     unsigned long long hc[2];
     FDM_CK(h, cudaMemcpyAsync(hc, cnt, sizeof hc, cudaMemcpyDeviceToHost, h->s));
@@ -185,67 +99,6 @@ int count_nr_fallbacks(fdm_handle *h, int64_t out[2]) {
     out[0] = (int64_t)hc[0];
     out[1] = (int64_t)hc[1];
     return FDM_OK;
-}
-
-// Four lanes per face (see face_flux in numerics.cuh for the per-face
-// algebra).  All 32 lanes of a warp run the shuffles; lanes past the last
-// face work on a clamped face and do not store.
-template <int DIR>
-__global__ void __launch_bounds__(256) k_faces4(Tables T, const double4 *__restrict__ cur, double4 *F,
-                                                const DevScalars *__restrict__ sc, double g) {
-    const int64_t gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t nf = T.NI + (DIR == 0 ? T.nux : T.nuy);
-    const int r = (int)(gt & 3);
-    int64_t f = gt >> 2;
-    const bool store = f < nf;
-    if (!store) f = nf - 1;
-    int32_t a, b, c, d;
-    if (f < T.NI) {
-        const int32_t *s = T.ist + f * 8;
-        if (DIR == 0) { a = s[1]; b = (int32_t)f; c = s[0]; d = s[4]; }
-        else { a = s[3]; b = (int32_t)f; c = s[2]; d = s[6]; }
-    } else {
-        const int32_t i = DIR == 0 ? T.uxl[f - T.NI] : T.uyl[f - T.NI];
-        const int32_t *s = T.ist + (int64_t)i * 8;
-        if (DIR == 0) { a = s[5]; b = s[1]; c = i; d = s[0]; }
-        else { a = s[7]; b = s[3]; c = i; d = s[2]; }
-    }
-    const Prim P[4] = {load_prim(cur, a), load_prim(cur, b), load_prim(cur, c), load_prim(cur, d)};
-    const double lam = DIR == 0 ? sc->lambda_x : sc->lambda_y;
-    double Um[4];
-    {
-        double U1[4], U2[4], Fd[4];
-        cons_flux<DIR>(P[1], g, U1, Fd);
-        cons_flux<DIR>(P[2], g, U2, Fd);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) Um[k] = (U1[k] + U2[k]) / 2.0;
-    }
-    EigRow E;
-    eigen_row<DIR>(Um, g, r, E);
-    double w[4], q[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        double Uk[4], Fk[4];
-        cons_flux<DIR>(P[k], g, Uk, Fk);
-        w[k] = project_row<DIR>(E, r, Uk);
-        q[k] = project_row<DIR>(E, r, Fk);
-    }
-    const double uwL = wcns_z3(w[0], w[1], w[2]);
-    const double uwR = wcns_z3(w[3], w[2], w[1]);
-    const double ugL = wcns_z3(q[0], q[1], q[2]);
-    const double ugR = wcns_z3(q[3], q[2], q[1]);
-    double awL[4], awR[4], agL[4], agR[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        awL[k] = __shfl_sync(0xffffffffu, uwL, k, 4);
-        awR[k] = __shfl_sync(0xffffffffu, uwR, k, 4);
-        agL[k] = __shfl_sync(0xffffffffu, ugL, k, 4);
-        agR[k] = __shfl_sync(0xffffffffu, ugR, k, 4);
-    }
-    const double wL = back_row<DIR>(E, r, awL), wR = back_row<DIR>(E, r, awR);
-    const double gL = back_row<DIR>(E, r, agL), gR = back_row<DIR>(E, r, agR);
-    const double out = 0.5 * (gL + gR - lam * (wR - wL));
-    if (store) reinterpret_cast<double *>(F + f)[r] = out;
 }
 
 // Residual + forward-Euler candidate fused with updateRK, 256 leaves per
@@ -346,84 +199,22 @@ void launch_requests(fdm_handle *h, const double4 *cur) {
     if (h->n_restrict > 0)
         k_requests_restrict<<<nblk(h->n_restrict, 4), 128, 0, h->s>>>(h->tables(), (double4 *)cur);
 }
-// Launch shapes of the face kernel that the autotuner chooses from.
+// Launch shapes of the face kernel that the autotuner chooses from; shape 0
+// is what a handle starts with.  The variant numbers run on past the shapes
+// and repeat them.
 template <int TB, int MINB>
-static void faces_1lane(fdm_handle *h, const double4 *cur) {
-    const Tables T = h->tables();
-    const DevScalars *sc = h->scal.as<DevScalars>();
-    k_faces<0, TB, MINB><<<nblk(h->NI + h->nux, TB), TB, 0, h->s>>>(T, cur, h->Fx.as<double4>(), sc, h->G.gama);
-    k_faces<1, TB, MINB><<<nblk(h->NI + h->nuy, TB), TB, 0, h->s>>>(T, cur, h->Fy.as<double4>(), sc, h->G.gama);
-}
-template <int TB, int MINB>
-static void faces_nr(fdm_handle *h, const double4 *cur) {
-    const Tables T = h->tables();
-    const DevScalars *sc = h->scal.as<DevScalars>();
+static void faces(fdm_handle *h, const double4 *cur) {
     const double g = h->G.gama;
-    // constant denominators with their correctly rounded reciprocals (IEEE
-    // division on the host)
-    const Den gm1{g - 1.0, 1.0 / (g - 1.0)}, d2{FDM_D2_WCNS, 1.0 / FDM_D2_WCNS};
-    k_faces_nr<0, TB, MINB><<<nblk(h->NI + h->nux, TB), TB, 0, h->s>>>(T, cur, h->Fx.as<double4>(), sc, g, gm1, d2);
-    k_faces_nr<1, TB, MINB><<<nblk(h->NI + h->nuy, TB), TB, 0, h->s>>>(T, cur, h->Fy.as<double4>(), sc, g, gm1, d2);
+    const int nbx = nblk(h->NI + h->nux, TB), nby = nblk(h->NI + h->nuy, TB);
+    k_faces<TB, MINB><<<nbx + nby, TB, 0, h->s>>>(h->tables(), cur, h->Fx.as<double4>(), h->Fy.as<double4>(),
+                                                  h->scal.as<DevScalars>(), g, flux_den(g), nbx);
 }
-template <int TB, int MINB, bool NR>
-static void faces_ref(fdm_handle *h, const double4 *cur) {
-    const Tables T = h->tables();
-    const DevScalars *sc = h->scal.as<DevScalars>();
-    const double g = h->G.gama;
-    const Den gm1{g - 1.0, 1.0 / (g - 1.0)}, d2{FDM_D2_WCNS, 1.0 / FDM_D2_WCNS};
-    k_faces_ref<0, TB, MINB, NR><<<nblk(h->NI + h->nux, TB), TB, 0, h->s>>>(T, cur, h->Fx.as<double4>(), sc, g, gm1, d2);
-    k_faces_ref<1, TB, MINB, NR><<<nblk(h->NI + h->nuy, TB), TB, 0, h->s>>>(T, cur, h->Fy.as<double4>(), sc, g, gm1, d2);
-}
-template <int TB, int MINB, bool SPLIT>
-static void faces_c(fdm_handle *h, const double4 *cur) {
-    const Tables T = h->tables();
-    const DevScalars *sc = h->scal.as<DevScalars>();
-    const double g = h->G.gama;
-    const DenC gm1{g - 1.0, 1.0 / (g - 1.0)}, d2{FDM_D2_WCNS, 1.0 / FDM_D2_WCNS};
-    k_faces_c<0, TB, MINB, SPLIT><<<nblk(h->NI + h->nux, TB), TB, 0, h->s>>>(T, cur, h->Fx.as<double4>(), sc, g, gm1, d2);
-    k_faces_c<1, TB, MINB, SPLIT><<<nblk(h->NI + h->nuy, TB), TB, 0, h->s>>>(T, cur, h->Fy.as<double4>(), sc, g, gm1, d2);
-}
-template <int TB, int MINB>
-static void faces_sm(fdm_handle *h, const double4 *cur) {
-    const Tables T = h->tables();
-    const DevScalars *sc = h->scal.as<DevScalars>();
-    const double g = h->G.gama;
-    const DenC gm1{g - 1.0, 1.0 / (g - 1.0)}, d2{FDM_D2_WCNS, 1.0 / FDM_D2_WCNS};
-    k_faces_sm<0, TB, MINB><<<nblk(h->NI + h->nux, TB), TB, 0, h->s>>>(T, cur, h->Fx.as<double4>(), sc, g, gm1, d2);
-    k_faces_sm<1, TB, MINB><<<nblk(h->NI + h->nuy, TB), TB, 0, h->s>>>(T, cur, h->Fy.as<double4>(), sc, g, gm1, d2);
-}
-static void faces_4lane(fdm_handle *h, const double4 *cur) {
-    const Tables T = h->tables();
-    const DevScalars *sc = h->scal.as<DevScalars>();
-    k_faces4<0><<<nblk(4 * (h->NI + h->nux), 256), 256, 0, h->s>>>(T, cur, h->Fx.as<double4>(), sc, h->G.gama);
-    k_faces4<1><<<nblk(4 * (h->NI + h->nuy), 256), 256, 0, h->s>>>(T, cur, h->Fy.as<double4>(), sc, h->G.gama);
-}
-
+constexpr int N_FACE_SHAPES = 6;
 const char *face_variant_name(int v) {
-    switch (v) {
-        case 0: return "1 thread/face, 128 threads, >=3 blocks/SM";
-        case 1: return "1 thread/face, 128 threads, >=4 blocks/SM";
-        case 2: return "1 thread/face, 64 threads, >=7 blocks/SM";
-        case 3: return "1 thread/face, 256 threads, >=2 blocks/SM";
-        case 4: return "4 threads/face, 256 threads";
-        case 5: return "1 thread/face, 128 threads, >=5 blocks/SM";
-        case 6: return "1 thread/face, 64 threads, >=10 blocks/SM";
-        case 7: return "1 thread/face, branch-free division, 128 threads, >=3 blocks/SM";
-        case 8: return "1 thread/face, branch-free division, 128 threads, >=4 blocks/SM";
-        case 9: return "1 thread/face, branch-free division, 256 threads, >=2 blocks/SM";
-        case 10: return "1 thread/face, branch-free division, 64 threads, >=10 blocks/SM";
-        case 11: return "1 thread/face, reference order, 256 threads, >=2 blocks/SM";
-        case 12: return "1 thread/face, reference order, 128 threads, >=4 blocks/SM";
-        case 13: return "1 thread/face, reference order, branch-free division, 256 threads, >=2 blocks/SM";
-        case 14: return "1 thread/face, reference order, branch-free division, 128 threads, >=4 blocks/SM";
-        case 15: return "1 thread/face, constant divisors by one correction, 256 threads, >=2 blocks/SM";
-        case 16: return "1 thread/face, constant divisors by one correction, 64 threads, >=10 blocks/SM";
-        case 17: return "1 thread/face, reference order, constant divisors by one correction, 256 threads, >=2 blocks/SM";
-        case 18: return "1 thread/face, variant 15 with the basis in shared memory, 128 threads, >=4 blocks/SM";
-        case 19: return "1 thread/face, variant 15 with the basis in shared memory, 128 threads, >=5 blocks/SM";
-        case 20: return "1 thread/face, variant 15 with the basis in shared memory, 128 threads, >=6 blocks/SM";
-        default: return "?";
-    }
+    static const char *const name[N_FACE_SHAPES] = {
+        "128 threads, >=4 blocks/SM", "128 threads, >=3 blocks/SM", "64 threads, >=8 blocks/SM",
+        "256 threads, >=2 blocks/SM", "128 threads, >=5 blocks/SM", "128 threads, >=6 blocks/SM"};
+    return v >= 0 ? name[v % N_FACE_SHAPES] : "?";
 }
 
 void launch_faces(fdm_handle *h, const double4 *cur, int krk) {
@@ -435,28 +226,13 @@ void launch_faces(fdm_handle *h, const double4 *cur, int krk) {
         launch_faces_fast(h, cur);
         return;
     }
-    switch (h->face_variant) {
-        case 1: faces_1lane<128, 4>(h, cur); break;
-        case 2: faces_1lane<64, 7>(h, cur); break;
-        case 3: faces_1lane<256, 2>(h, cur); break;
-        case 4: faces_4lane(h, cur); break;
-        case 5: faces_1lane<128, 5>(h, cur); break;
-        case 6: faces_1lane<64, 10>(h, cur); break;
-        case 7: faces_nr<128, 3>(h, cur); break;
-        case 8: faces_nr<128, 4>(h, cur); break;
-        case 9: faces_nr<256, 2>(h, cur); break;
-        case 10: faces_nr<64, 10>(h, cur); break;
-        case 11: faces_ref<256, 2, false>(h, cur); break;
-        case 12: faces_ref<128, 4, false>(h, cur); break;
-        case 13: faces_ref<256, 2, true>(h, cur); break;
-        case 14: faces_ref<128, 4, true>(h, cur); break;
-        case 15: faces_c<256, 2, true>(h, cur); break;
-        case 16: faces_c<64, 10, true>(h, cur); break;
-        case 17: faces_c<256, 2, false>(h, cur); break;
-        case 18: faces_sm<128, 4>(h, cur); break;
-        case 19: faces_sm<128, 5>(h, cur); break;
-        case 20: faces_sm<128, 6>(h, cur); break;
-        default: faces_1lane<128, 3>(h, cur); break;
+    switch (h->face_variant % N_FACE_SHAPES) {
+        case 1: faces<128, 3>(h, cur); break;
+        case 2: faces<64, 8>(h, cur); break;
+        case 3: faces<256, 2>(h, cur); break;
+        case 4: faces<128, 5>(h, cur); break;
+        case 5: faces<128, 6>(h, cur); break;
+        default: faces<128, 4>(h, cur); break;
     }
 }
 

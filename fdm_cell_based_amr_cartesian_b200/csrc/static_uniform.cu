@@ -18,6 +18,7 @@
 
 #include "handle.cuh"
 #include "numerics.cuh"
+#include "numerics_nr.cuh"
 
 namespace fdm {
 namespace uniform_static {
@@ -49,37 +50,47 @@ struct Grid2 {
     __device__ __forceinline__ int64_t at(int r, int c) const { return (int64_t)r * W + c; }
 };
 
-// face i of row r in x lies between interior columns 3+i-1 and 3+i
+// face i of row r in x lies between interior columns 3+i-1 and 3+i; the x
+// faces' blocks (nbx), then the y faces'
 template <int DIR>
-__global__ void __launch_bounds__(128) k_ufaces(Grid2 G, const double4 *__restrict__ cur, double4 *F,
-                                                double g, double lam) {
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+__device__ __forceinline__ void uface(const Grid2 &G, const double4 *__restrict__ cur, double4 *F, double g,
+                                      const FluxDen &den, double lam, int t) {
     const int nfr = DIR == 0 ? G.nx + 1 : G.nx;          // faces per row
     const int nrow = DIR == 0 ? G.ny : G.ny + 1;
-    if (t >= (int64_t)nfr * nrow) return;
-    const int r = (int)(t / nfr), i = (int)(t % nfr);
-    int64_t a, b, c, d;
-    if (DIR == 0) {
-        const int row = 3 + r, col = 3 + i;
-        a = G.at(row, col - 2); b = G.at(row, col - 1); c = G.at(row, col); d = G.at(row, col + 1);
-    } else {
-        const int row = 3 + r, col = 3 + i;
-        a = G.at(row - 2, col); b = G.at(row - 1, col); c = G.at(row, col); d = G.at(row + 1, col);
-    }
-    double out[4];
-    face_flux<DIR>(load_prim(cur, a), load_prim(cur, b), load_prim(cur, c), load_prim(cur, d), g, lam, out);
-    F[t] = make_double4(out[0], out[1], out[2], out[3]);
+    if (t >= nfr * nrow) return;
+    const int r = t / nfr, i = t - r * nfr;
+    const int step = DIR == 0 ? 1 : G.W, c = (int)G.at(3 + r, 3 + i);
+    F[t] = face_flux_of<DIR>(cur, c - 2 * step, c - step, c, c + step, g, den, lam);
+}
+__global__ void __launch_bounds__(64, 8) k_ufaces(Grid2 G, const double4 *__restrict__ cur, double4 *Fx, double4 *Fy,
+                                                  double g, FluxDen den, double lam_x, double lam_y, int nbx) {
+    const int b = blockIdx.x;
+    if (b < nbx) uface<0>(G, cur, Fx, g, den, lam_x, b * 64 + threadIdx.x);
+    else uface<1>(G, cur, Fy, g, den, lam_y, (b - nbx) * 64 + threadIdx.x);
 }
 
-// LXL + updateRK for every interior cell (same operations as k_cells)
-__global__ void __launch_bounds__(256) k_ucells(Grid2 G, const double4 *__restrict__ cur,
+// LXL + updateRK for every interior cell (same operations as k_cells), and
+// its periodic images among the ghosts (BC_cyc at level 0,
+// src/solution.F90:116-136): the thread that makes a value stores its copies.
+// The corners are left alone, as the reference never refills them; at stage 3
+// the threads past the cells copy them from the input.
+__global__ void __launch_bounds__(128) k_ucells(Grid2 G, const double4 *__restrict__ cur,
                                                 const double4 *__restrict__ un, double4 *next,
                                                 const double4 *__restrict__ Fx, const double4 *__restrict__ Fy,
                                                 double g, double cxa, double cxb, double cya, double cyb,
                                                 double tstep, int krk) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t >= (int64_t)G.nx * G.ny) return;
-    const int r = (int)(t / G.nx), i = (int)(t % G.nx);
+    const int ncell = G.nx * G.ny;
+    if (t >= ncell) {
+        const int k = (int)t - ncell;   // corner record k of 36: 3 x 3 at each end of both sides
+        if (krk == 3 && k < 36) {
+            const int a = k / 6, b = k % 6;
+            const int64_t at = G.at(a < 3 ? a : G.ny + a, b < 3 ? b : G.nx + b);
+            next[at] = un[at];
+        }
+        return;
+    }
+    const int r = (int)t / G.nx, i = (int)t - r * G.nx;
     const int row = 3 + r, col = 3 + i;
     const int64_t self = G.at(row, col);
     const Prim q = load_prim(cur, self);
@@ -114,33 +125,12 @@ __global__ void __launch_bounds__(256) k_ucells(Grid2 G, const double4 *__restri
     const double4 n0 = un[self];
     const double ra = krk == 1 ? 0.0 : krk == 2 ? 3.0 / 4.0 : 1.0 / 3.0;
     const double rb = krk == 1 ? 1.0 : krk == 2 ? 1.0 / 4.0 : 2.0 / 3.0;
-    next[self] = make_double4(ra * n0.x + rb * r0, ra * n0.y + rb * u0, ra * n0.z + rb * v0, ra * n0.w + rb * p0);
-}
-
-// periodic ghost fill (BC_cyc at level 0, src/solution.F90:116-136);
-// corners are left alone, as the reference never refills them
-__global__ void k_ughosts(Grid2 G, double4 *buf) {
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int H = G.ny + 6;
-    if (t >= (int64_t)G.W * H) return;
-    const int row = (int)(t / G.W), col = (int)(t % G.W);
-    const bool gx = col < 3 || col > G.nx + 2, gy = row < 3 || row > G.ny + 2;
-    if (gx == gy) return;   // interior or corner
-    int sr = row, sc = col;
-    if (col < 3) sc = col + G.nx;
-    else if (col > G.nx + 2) sc = col - G.nx;
-    if (row < 3) sr = row + G.ny;
-    else if (row > G.ny + 2) sr = row - G.ny;
-    buf[t] = buf[G.at(sr, sc)];
-}
-
-__global__ void k_ucorners(Grid2 G, const double4 *__restrict__ in, double4 *out) {
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int H = G.ny + 6;
-    if (t >= (int64_t)G.W * H) return;
-    const int row = (int)(t / G.W), col = (int)(t % G.W);
-    const bool gx = col < 3 || col > G.nx + 2, gy = row < 3 || row > G.ny + 2;
-    if (gx && gy) out[t] = in[t];
+    const double4 o = make_double4(ra * n0.x + rb * r0, ra * n0.y + rb * u0, ra * n0.z + rb * v0, ra * n0.w + rb * p0);
+    next[self] = o;
+    if (col >= G.nx) next[G.at(row, col - G.nx)] = o;
+    if (col <= 5) next[G.at(row, col + G.nx)] = o;
+    if (row >= G.ny) next[G.at(row - G.ny, col)] = o;
+    if (row <= 5) next[G.at(row + G.ny, col)] = o;
 }
 
 static inline unsigned nb(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -180,13 +170,12 @@ extern "C" int fdm_time_advance_rk_uniform_static(const double *prim_in, double 
     double4 *out = (double4 *)prim_out;
     const double4 *cur[3] = {in, U1, U2};
     double4 *next[3] = {U1, U2, out};
+    const fdm::FluxDen den = fdm::flux_den(gama);
+    const unsigned nbx = nb((int64_t)(nx + 1) * ny, 64), nby = nb((int64_t)nx * (ny + 1), 64);
     for (int krk = 1; krk <= 3; ++krk) {
-        k_ufaces<0><<<nb((int64_t)(nx + 1) * ny, 128), 128, 0, s>>>(G, cur[krk - 1], Fx, gama, lambda_x);
-        k_ufaces<1><<<nb((int64_t)nx * (ny + 1), 128), 128, 0, s>>>(G, cur[krk - 1], Fy, gama, lambda_y);
-        k_ucells<<<nb((int64_t)nx * ny, 256), 256, 0, s>>>(G, cur[krk - 1], in, next[krk - 1], Fx, Fy, gama, cxa,
-                                                           cxb, cya, cyb, tstep, krk);
-        k_ughosts<<<nb(ngrid, 256), 256, 0, s>>>(G, next[krk - 1]);
+        k_ufaces<<<nbx + nby, 64, 0, s>>>(G, cur[krk - 1], Fx, Fy, gama, den, lambda_x, lambda_y, (int)nbx);
+        k_ucells<<<nb((int64_t)nx * ny + 36, 128), 128, 0, s>>>(G, cur[krk - 1], in, next[krk - 1], Fx, Fy, gama, cxa,
+                                                                cxb, cya, cyb, tstep, krk);
     }
-    k_ucorners<<<nb(ngrid, 256), 256, 0, s>>>(G, in, out);
     return cudaGetLastError() == cudaSuccess ? FDM_OK : FDM_ERR_CUDA;
 }

@@ -90,7 +90,7 @@ namespace fdm {
 int count_nr_fallbacks(fdm_handle *h, int64_t out[2]);
 }
 // x and y faces whose branch-free division falls back to the compiler's on
-// the current state (face variants 7-10, 13, 14)
+// the current state
 extern "C" int fdm_debug_nr_fallbacks(fdm_handle *h, int64_t *out) {
     if (!h || !out) return FDM_ERR_ARG;
     if (!h->loaded) return FDM_ERR_STATE;

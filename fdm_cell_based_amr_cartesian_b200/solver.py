@@ -600,8 +600,7 @@ class Batch:
         self._check(self.L.fdm_batch_set_blocks_per_sm(self.b, int(k)))
 
     def set_face_flux(self, branch_free: bool):
-        """Face phases of the persistent kernel in the reference's order (False)
-        or the split order with the branch-free division (True): same bits."""
+        """Kept for its callers: both values choose the same face flux."""
         self._check(self.L.fdm_batch_set_face_flux(self.b, 1 if branch_free else 0))
 
     def set_wait_limit(self, seconds: float):

@@ -318,8 +318,8 @@ int fdm_fp64_peak(double *tflops);
 int fdm_autotune(fdm_handle *h, int32_t reps, int32_t *best, double *ms);
 int fdm_set_variant(fdm_handle *h, int32_t face_variant);
 /* Diagnostics: out[0], out[1] = x and y faces of the current state whose
- * branch-free division (face variants 7-10, 13, 14) meets an operand outside
- * its exact range and is computed again with the compiler's division. */
+ * branch-free division meets an operand outside its exact range and is
+ * computed again with the compiler's division. */
 int fdm_debug_nr_fallbacks(fdm_handle *h, int64_t out[2]);
 
 /* ------------------------------------------------------------ learned gate
@@ -404,9 +404,7 @@ int fdm_batch_sync(fdm_batch *b);
  * same bits every way; which is faster depends on the members' sizes
  * (measure). */
 int fdm_batch_set_blocks_per_sm(fdm_batch *b, int32_t blocks_per_sm);
-/* Face phases of the persistent kernel: 0 the reference's operation order
- * (default), 1 the split order with the branch-free correctly rounded
- * division of face variants 7-10 (the same bits; one may be faster). */
+/* Kept for its callers: 0 and 1 are accepted and choose the same face flux. */
 int fdm_batch_set_face_flux(fdm_batch *b, int32_t branch_free);
 /* Wait limit of one grid barrier of the persistent kernel in seconds
  * (0 < seconds <= 3600; default 2), measured on the GPU's global timer. */
