@@ -243,36 +243,58 @@ __device__ __forceinline__ double4 mean4(const double4 &c0, const double4 &c1, c
 }
 
 // ---------------------------------------------------- internal node values
-__global__ void k_anc_count(int64_t NL, const uint64_t *lkey, int32_t *cnt) {
+// The internal nodes from the sorted leaves: each starts where its first
+// leaf starts, so that leaf names it: leaf k names as many of its ancestors
+// as its path ends in zero digits, in key order from the outermost one in.
+// Nodes named by successive leaves ascend, so the list is made in key order.
+__device__ __forceinline__ int named_ancestors(uint64_t k) {
+    const int lvl = (int)(k & 15u);
+    if (lvl == 0) return 0;
+    const uint64_t path = (k & KEY_PATH) >> key_digit_shift(lvl);   // digit j at bit 2 (lvl - j)
+    return path == 0 ? lvl : min(lvl, (__ffsll((long long)path) - 1) >> 1);
+}
+__global__ void k_anc_count(int64_t NL, const uint64_t *lkey, int32_t *cnt, int32_t *max_lvl) {
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k < NL) cnt[k] = (int32_t)(lkey[k] & 15u);
+    int lvl = 0;
+    if (k < NL) {
+        const uint64_t key = lkey[k];
+        cnt[k] = named_ancestors(key);
+        lvl = (int)(key & 15u);
+    }
+    lvl = __reduce_max_sync(0xffffffffu, lvl);
+    if ((threadIdx.x & 31) == 0 && lvl > 0) atomicMax(max_lvl, lvl);
 }
 __global__ void k_anc_emit(int64_t NL, const uint64_t *lkey, const int32_t *off, uint64_t *out) {
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= NL) return;
-    uint64_t a = lkey[k];
-    const int l = (int)(a & 15u);
-    for (int j = 0; j < l; ++j) {
-        a = parent_key(a);
-        out[off[k] + j] = a;
-    }
+    const uint64_t key = lkey[k];
+    const int l = (int)(key & 15u), c = named_ancestors(key);
+    for (int j = 0; j < c; ++j) out[off[k] + j] = ancestor_key(key, l - c + j);
 }
 // interpA of internal nodes at one level from their children (leaves or
 // deeper internal nodes, already done)
-__global__ void k_internal_vals(int64_t NInt, const uint64_t *ikey, double4 *ival, int lvl, const uint64_t *lkey,
-                                int64_t NL, const int32_t *lslot, const double4 *B0) {
+__global__ void k_internal_vals(int64_t NInt, const uint64_t *ikey, double4 *ival, int lvl, Tables T,
+                                const double4 *B0) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= NInt) return;
     const uint64_t k = ikey[i];
     if ((int)(k & 15u) != lvl) return;
     double4 c[4];
+    int64_t at = i;   // the sons that are internal come after this node, in key order
     for (int q = 0; q < 4; ++q) {
         const uint64_t ck = child_key(k, q);
-        const int64_t li = find_key(lkey, NL, ck);
-        if (li >= 0) c[q] = B0[lslot[li]];
-        else {
-            const int64_t ii = find_key(ikey, NInt, ck);
-            c[q] = ii >= 0 ? ival[ii] : make_double4(0, 0, 0, 0);
+        const int64_t li = find_key_t(T, ck);
+        if (li >= 0) {
+            c[q] = B0[T.lslot[li]];
+        } else {
+            int64_t lo = at + 1, hi = NInt;
+            while (lo < hi) {
+                const int64_t mid = (lo + hi) >> 1;
+                if (ikey[mid] < ck) lo = mid + 1;
+                else hi = mid;
+            }
+            at = lo;
+            c[q] = lo < NInt && ikey[lo] == ck ? ival[lo] : make_double4(0, 0, 0, 0);
         }
     }
     ival[i] = mean4(c[0], c[1], c[2], c[3]);
@@ -386,39 +408,24 @@ int init_internal(fdm_handle *h) {
     const int TB = 256;
     const int64_t NL = h->NL;
     Carve cv;
-    cv.add(NL * 4); cv.add(NL * 4);
+    cv.add(NL * 4); cv.add(NL * 4); cv.add(4);
     FDM_CK(h, h->amr[8].ensure(cv.total));
     int32_t *cnt = cv.at<int32_t>(h->amr[8], 0), *off = cv.at<int32_t>(h->amr[8], 1);
-    k_anc_count<<<nblk(NL, TB), TB, 0, h->s>>>(NL, h->lkey.as<uint64_t>(), cnt);
-    int64_t na = 0;
-    int rc = scan_total32(h, cnt, off, NL, na);
-    if (rc) return rc;
-    h->NInt = 0;
-    if (na == 0) return FDM_OK;
-    FDM_CK(h, h->amr[9].ensure(na * 8 * 2 + 64));
-    uint64_t *anc = h->amr[9].as<uint64_t>(), *srt = anc + na;
-    k_anc_emit<<<nblk(NL, TB), TB, 0, h->s>>>(NL, h->lkey.as<uint64_t>(), off, anc);
-    size_t bytes = 0;
-    const int kb = 34 + root_bits(h);   // ancestor node keys
-    FDM_CK(h, cub::DeviceRadixSort::SortKeys(nullptr, bytes, anc, srt, (int)na, 0, kb, h->s));
-    FDM_CK(h, h->cub_tmp.ensure(bytes));
-    FDM_CK(h, cub::DeviceRadixSort::SortKeys(h->cub_tmp.p, bytes, anc, srt, (int)na, 0, kb, h->s));
-    FDM_CK(h, h->ikey.ensure(na * 8));
-    FDM_CK(h, h->amr[10].ensure(16));
-    int64_t *nsel = h->amr[10].as<int64_t>();
-    bytes = 0;
-    FDM_CK(h, cub::DeviceSelect::Unique(nullptr, bytes, srt, h->ikey.as<uint64_t>(), nsel, (int)na, h->s));
-    FDM_CK(h, h->cub_tmp.ensure(bytes));
-    FDM_CK(h, cub::DeviceSelect::Unique(h->cub_tmp.p, bytes, srt, h->ikey.as<uint64_t>(), nsel, (int)na, h->s));
+    int32_t *dl = cv.at<int32_t>(h->amr[8], 2), deepest = 0;   // deepest leaf
+    FDM_CK(h, cudaMemsetAsync(dl, 0, 4, h->s));
+    k_anc_count<<<nblk(NL, TB), TB, 0, h->s>>>(NL, h->lkey.as<uint64_t>(), cnt, dl);
+    FDM_CK(h, cudaMemcpyAsync(&deepest, dl, 4, cudaMemcpyDeviceToHost, h->s));
     int64_t ni = 0;
-    FDM_CK(h, cudaMemcpyAsync(&ni, nsel, 8, cudaMemcpyDeviceToHost, h->s));
-    FDM_CK(h, cudaStreamSynchronize(h->s));
+    int rc = scan_total32(h, cnt, off, NL, ni);   // waits
+    if (rc) return rc;
     h->NInt = ni;
+    if (ni == 0) return FDM_OK;
+    FDM_CK(h, h->ikey.ensure(ni * 8));
+    k_anc_emit<<<nblk(NL, TB), TB, 0, h->s>>>(NL, h->lkey.as<uint64_t>(), off, h->ikey.as<uint64_t>());
     FDM_CK(h, h->ival.ensure(ni * 32 + 32));
-    for (int l = MAXLVL_TAB - 2; l >= 0; --l)
+    for (int l = deepest - 1; l >= 0; --l)
         k_internal_vals<<<nblk(ni, TB), TB, 0, h->s>>>(ni, h->ikey.as<uint64_t>(), h->ival.as<double4>(), l,
-                                                      h->lkey.as<uint64_t>(), NL, h->lslot.as<int32_t>(),
-                                                      h->B[0].as<double4>());
+                                                      h->tables(), h->B[0].as<double4>());
     FDM_CK(h, cudaGetLastError());
     return FDM_OK;
 }

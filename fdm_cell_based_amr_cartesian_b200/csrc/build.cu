@@ -765,6 +765,20 @@ __global__ void k_restrict_list(int64_t NR, const int32_t *__restrict__ kind, in
     if (r < NR && kind[r] == RQ_RESTRICT) list[atomicAdd(count, 1ull)] = (int32_t)r;
 }
 
+__global__ void k_descents(int64_t n, const uint64_t *__restrict__ key, int32_t *flag) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i + 1 < n && key[i] > key[i + 1]) *flag = 1;
+}
+int keys_sorted(fdm_handle *h, int64_t n, const uint64_t *keys_dev, bool *sorted) {
+    int32_t *flag = h->flag.as<int32_t>(), f = 0;
+    FDM_CK(h, cudaMemsetAsync(flag, 0, 4, h->s));
+    k_descents<<<nblk(n, 256), 256, 0, h->s>>>(n, keys_dev, flag);
+    FDM_CK(h, cudaMemcpyAsync(&f, flag, 4, cudaMemcpyDeviceToHost, h->s));
+    FDM_CK(h, cudaStreamSynchronize(h->s));
+    *sorted = f == 0;
+    return FDM_OK;
+}
+
 int build_tables(fdm_handle *h, int64_t n, const uint64_t *keys_in, const double *prim_in, int key_bits) {
     Nvtx range("fdm tables");
     const int TB = 256;

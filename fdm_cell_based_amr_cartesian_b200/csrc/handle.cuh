@@ -216,11 +216,12 @@ inline int arg_fail(fdm_handle *h, const char *msg) {
 }
 
 // table construction (build.cu)
-// key_bits: the low bits of the keys that the key sort orders (64 for keys
-// from a caller, root_bits(h) + 34 for keys the device made itself)
-// key_bits: the low bits the sort looks at; 0: the keys are already sorted
-// (the regrid emits them in key order), so they are only copied
+// key_bits: the low bits the sort looks at (64 for keys from a caller); 0: the keys are already sorted
+// (the regrid emits them in key order, a caller most often has them so), so
+// they are only copied
 int build_tables(fdm_handle *h, int64_t n, const uint64_t *keys_dev, const double *prim_dev, int key_bits = 64);
+// *sorted: the keys ascend (waits for the stream)
+int keys_sorted(fdm_handle *h, int64_t n, const uint64_t *keys_dev, bool *sorted);
 // bits of the largest background-cell (root) index m*n - 1: a leaf key
 // (root << 34 | path << 4 | lvl) made on the device has no bit set at or
 // above 34 + root_bits, so radix sorts of such keys stop there
