@@ -234,7 +234,7 @@ __device__ __forceinline__ void ph_request_tile(const BatchArgs &A, int krk, int
         stage_request_geometry(M.T, t * RQ_TILE, S.geo, BT);
         const int64_t q = t * BT + threadIdx.x;
         if ((q >> 2) < M.T.NR)
-            request_item_var(M.T, cur, q >> 2, (int)(q & 3), S.geo + (threadIdx.x >> 2) * RQ_GEO);
+            request_item<1>(M.T, cur, q >> 2, (int)(q & 3), S.geo + rq_geo_at(threadIdx.x >> 2));
         __syncthreads();   // the next tile's copy overwrites S.geo
     } else {
         const int64_t w = (t - nthr) * BW + wid;

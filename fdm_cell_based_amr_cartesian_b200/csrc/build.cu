@@ -198,59 +198,28 @@ __global__ void k_emit(int64_t n, int64_t VS0, ResolveOut O, const int32_t *ridx
 }
 
 // ---------------------------------------------------------- WLS gather
-struct Gather {
-    int32_t m1, m2;
-    int32_t n1[WLS_MAXM], n2[WLS_MAXM];  // sorted leaf indices
-    bool used[8];
-    int32_t overflow;
-};
-
-__device__ __forceinline__ void g_add(Gather &g, int32_t leaf, int dir) {
-    g.used[dir - 1] = true;
-    const bool axis = (dir == 1 || dir == 3 || dir == 5 || dir == 7);
-    if (axis) {
-        for (int t = 0; t < g.m1; ++t) if (g.n1[t] == leaf) return;
-        if (g.m1 >= WLS_MAXM) { g.overflow = 1; return; }
-        g.n1[g.m1++] = leaf;
-    } else {
-        for (int t = 0; t < g.m2; ++t) if (g.n2[t] == leaf) return;
-        if (g.m2 >= WLS_MAXM) { g.overflow = 1; return; }
-        g.n2[g.m2++] = leaf;
-    }
-}
-
-// search_cell_5 (src/XuanGua.F90:152-177) on a node: its leaves in DFS
-// order son1, son2, son3, son4; the first leaf of every still-unused
-// sector joins the stencil.  The DFS rank of a leaf is its Morton path with
-// each digit mapped 0,1,2,3 -> 0,1,3,2 (son1, son2, son4, son3).
-__device__ void g_search(const Tables &T, const NodeRef &X, double x, double y, Gather &g) {
+// search_cell_5 (src/XuanGua.F90:152-177) on a node: its leaves in traversal
+// order son1, son2, son3, son4; the first leaf of every still-unused sector
+// joins the stencil.  Which leaf that is does not depend on the sectors
+// already used, so the areas of a request are searched independently (one
+// lane each): the first leaf of every sector of the area, as traversal rank
+// (the Morton path with digits 2 and 3 exchanged) above leaf index, into
+// first[8] (shared memory).
+__device__ __forceinline__ void area_search(const Tables &T, const NodeRef &X, double x, double y,
+                                            unsigned long long *first) {
+    for (int s = 0; s < 8; ++s) first[s] = ~0ull;
     if (!X.valid) return;
-    if (X.leaf >= 0) {
-        const int dir = get_direction(T.lcx[X.leaf], T.lcy[X.leaf], x, y);
-        if (!g.used[dir - 1]) g_add(g, X.leaf, dir);
-        return;
+    int64_t lo = X.leaf, hi = X.leaf + 1;
+    if (X.leaf < 0) {
+        const uint64_t p0 = node_pos(X.n);
+        lo = lower_bound_pos_t(T, p0);
+        hi = lower_bound_pos_t(T, p0 + span_of_level(X.n.lvl));
     }
-    const uint64_t p0 = node_pos(X.n);
-    const int64_t lo = lower_bound_pos_t(T, p0);
-    const int64_t hi = lower_bound_pos_t(T, p0 + span_of_level(X.n.lvl));
-    uint64_t best_rank[8];
-    int32_t best_leaf[8];
-    for (int s = 0; s < 8; ++s) { best_rank[s] = ~0ull; best_leaf[s] = -1; }
     for (int64_t k = lo; k < hi; ++k) {
-        const int dir = get_direction(T.lcx[k], T.lcy[k], x, y);
-        if (g.used[dir - 1]) continue;
+        const int s = get_direction(T.lcx[k], T.lcy[k], x, y) - 1;
         const uint64_t path = key_pos(T.lkey[k]) & ((1ull << 30) - 1ull);
-        const uint64_t rank = path ^ ((path & 0x2AAAAAAAull) >> 1);
-        if (rank < best_rank[dir - 1]) { best_rank[dir - 1] = rank; best_leaf[dir - 1] = (int32_t)k; }
-    }
-    for (;;) {
-        int bs = -1;
-        uint64_t br = ~0ull;
-        for (int s = 0; s < 8; ++s)
-            if (best_leaf[s] >= 0 && best_rank[s] < br) { br = best_rank[s]; bs = s; }
-        if (bs < 0) break;
-        g_add(g, best_leaf[bs], bs + 1);
-        best_leaf[bs] = -1;
+        const unsigned long long v = (path ^ ((path & 0x2AAAAAAAull) >> 1)) << 32 | (unsigned long long)k;
+        if (v < first[s]) first[s] = v;
     }
 }
 
@@ -339,167 +308,181 @@ struct ReqOut {
     int32_t *mem;
     double *geo;
     uint64_t *node;
-    unsigned long long *counts;   // [0] singular, [1] wls, [2] restrict, [3] copy
+    unsigned long long *counts;   // [0] singular, [2] restrict
 };
 
-// One hanging-node request: stencil gather of parent_value_weno /
-// child_value_weno (src/XuanGua.F90:45-150), then either the WLS geometry
-// (P^T W P and its three brinv inverses, src/XuanGua.F90:206-255) or the
-// reference's fallback when fewer than 7 points were found.
-__global__ void k_gather(Tables T, Geometry G, ReqDesc D, ReqOut O, int32_t *err) {
-    const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (r >= T.NR) return;
-    Gather g;
-    g.m1 = 0; g.m2 = 0; g.overflow = 0;
-    for (int s = 0; s < 8; ++s) g.used[s] = false;
+// Stencil gather of parent_value_weno / child_value_weno
+// (src/XuanGua.F90:45-150), or the reference's fallback when fewer than 7
+// points were found.  Eight lanes per request: each finds and searches one of
+// the areas that the reference visits in turn, then the areas' finds are
+// joined in that order.  (With one thread per request, which also formed the
+// geometry below, a warp ran the longest of 32 serial searches: 613 us for 81k
+// requests, 172 us for 18k; the two kernels take 223 and 59.)
+constexpr int GATHER_RPB = 16;   // requests per block
+__global__ void __launch_bounds__(GATHER_RPB * 8) k_gather(Tables T, Geometry G, ReqDesc D, ReqOut O, int32_t *err) {
+    __shared__ unsigned long long first[GATHER_RPB][8][8];
+    __shared__ int32_t list[GATHER_RPB][2][WLS_AXIS];   // axis members, diagonal members
+    const int lane = threadIdx.x & 7, g = threadIdx.x >> 3, g0 = threadIdx.x & 24;
+    const unsigned mask = 0xFFu << g0;
+    const int64_t r = (int64_t)blockIdx.x * GATHER_RPB + g;
+    if (r >= T.NR) return;   // whole groups of eight lanes
+    const bool child = D.kind[r] != 0;
     NodeRef c;
-    double x, y, xx, yy;
-    int32_t *mem = O.mem + r * WLS_MAXM;
-    double *geo = O.geo + r * RQ_GEO;
-    if (D.kind[r] == 0) {
-        // parent_value_weno on the internal node
+    c.valid = 1;
+    double x, y;
+    if (!child) {   // parent_value_weno on the internal node: sons 1..4, then left, right, down, up
         c.n = node_of_key((uint64_t)D.ref[r]);
         c.leaf = -1;
-        c.valid = 1;
         node_center(G, c.n, x, y);
-        xx = x; yy = y;
-        O.node[r] = node_key(c.n);
-        geo[G_ORIGIN] = 0.0;
-        geo[G_XX] = xx;
-        geo[G_YY] = yy;
-        const int qs[4] = {0, 1, 3, 2};
-        for (int t = 0; t < 4; ++t) g_search(T, child_ref(T, c, qs[t]), x, y, g);
-        if (g.m1 + g.m2 < 8) {
-            g_search(T, face_nb(T, G, c, DIR_LEFT), x, y, g);
-            g_search(T, face_nb(T, G, c, DIR_RIGHT), x, y, g);
-            g_search(T, face_nb(T, G, c, DIR_DOWN), x, y, g);
-            g_search(T, face_nb(T, G, c, DIR_UP), x, y, g);
-        }
-        if (g.m1 + g.m2 < 7) {
-            const uint64_t p0 = node_pos(c.n);
-            O.kind[r] = RQ_RESTRICT;
-            O.m[2 * r] = (int32_t)lower_bound_pos_t(T, p0);
-            O.m[2 * r + 1] = (int32_t)lower_bound_pos_t(T, p0 + span_of_level(c.n.lvl));
-            geo[G_LVL] = (double)c.n.lvl;
-            atomicAdd(O.counts + 2, 1ull);
-            return;
-        }
+    } else {        // child_value_weno on the coarse leaf
+        c.leaf = (int32_t)D.ref[r];
+        c.n = node_of_key(T.lkey[c.leaf]);
+        x = T.lcx[c.leaf]; y = T.lcy[c.leaf];
+    }
+    NodeRef X;
+    if (!child && lane < 4) {
+        X = child_ref(T, c, lane ^ (lane >> 1));   // sons 1, 2, 3, 4 are digits 0, 1, 3, 2
     } else {
-        // child_value_weno on the coarse leaf at the target point
-        const int32_t L = (int32_t)D.ref[r];
-        c.n = node_of_key(T.lkey[L]);
-        c.leaf = L;
-        c.valid = 1;
-        x = T.lcx[L]; y = T.lcy[L];
-        xx = D.tx[r]; yy = D.ty[r];
-        O.node[r] = T.lkey[L];
-        geo[G_ORIGIN] = 1.0;
-        geo[G_XX] = xx;
-        geo[G_YY] = yy;
-        g.n1[g.m1++] = L;
-        const bool diag = root_cross(G, c.n.root) >= 0;
-        const NodeRef nul = null_ref();
-        g_search(T, diag ? downleft_nb(T, G, c) : nul, x, y, g);
-        g_search(T, face_nb(T, G, c, DIR_LEFT), x, y, g);
-        g_search(T, diag ? upleft_nb(T, G, c) : nul, x, y, g);
-        g_search(T, face_nb(T, G, c, DIR_DOWN), x, y, g);
-        g_search(T, face_nb(T, G, c, DIR_UP), x, y, g);
-        g_search(T, diag ? downright_nb(T, G, c) : nul, x, y, g);
-        g_search(T, face_nb(T, G, c, DIR_RIGHT), x, y, g);
-        g_search(T, diag ? upright_nb(T, G, c) : nul, x, y, g);
-        if (g.m1 + g.m2 < 7) {
-            O.kind[r] = RQ_COPY;
-            mem[0] = T.lslot[L];
-            O.m[2 * r] = 1;
-            O.m[2 * r + 1] = 0;
-            atomicAdd(O.counts + 3, 1ull);
-            return;
+        // child: down-left, left, up-left, down, up, down-right, right, up-right
+        const int dx = child ? (lane < 3 ? DIR_LEFT : DIR_RIGHT) : lane == 4 ? DIR_LEFT : DIR_RIGHT;
+        const int dy = child ? (lane == 0 || lane == 3 || lane == 5 ? DIR_DOWN : DIR_UP) : lane == 6 ? DIR_DOWN : DIR_UP;
+        const bool diag = child && (lane == 0 || lane == 2 || lane == 5 || lane == 7);
+        if (diag) X = root_cross(G, c.n.root) >= 0 ? diagonal_nb(T, G, c, dx, dy) : null_ref();
+        else X = face_nb(T, G, c, child ? (lane == 1 || lane == 6 ? dx : dy) : (lane < 6 ? dx : dy));
+    }
+    area_search(T, X, x, y, first[g][lane]);
+    __syncwarp(mask);
+    int m1 = 0, m2 = 0;
+    unsigned used = 0;
+    bool overflow = false;
+    if (child) {
+        if (lane == 0) list[g][0][0] = c.leaf;
+        m1 = 1;
+    }
+    for (int a = 0; a < 8; ++a) {
+        if (!child && a == 4 && m1 + m2 >= 8) break;
+        const unsigned long long mine = first[g][a][lane];   // sector lane + 1
+        for (;;) {
+            unsigned long long v = (used >> lane) & 1u ? ~0ull : mine;
+            unsigned long long best = v;
+            for (int o = 1; o < 8; o <<= 1) best = min(best, __shfl_xor_sync(mask, best, o));
+            if (best == ~0ull) break;
+            const int s = __ffs((__ballot_sync(mask, v == best) >> g0) & 0xFFu) - 1;
+            used |= 1u << s;
+            const int32_t leaf = (int32_t)(best & 0xffffffffull);
+            // an even sector (1, 3, 5, 7 of the reference) is an axis one; a
+            // leaf already in the list is not taken twice
+            const int which = s & 1, n = which ? m2 : m1;
+            __syncwarp(mask);
+            const bool dup = lane < n && list[g][which][lane] == leaf;
+            if (__any_sync(mask, dup)) continue;
+            if (n >= (which ? WLS_MAXM - WLS_AXIS : WLS_AXIS)) { overflow = true; continue; }
+            if (lane == 0) list[g][which][n] = leaf;
+            if (which) ++m2;
+            else ++m1;
+            __syncwarp(mask);
         }
     }
-    if (g.overflow) atomicExch(err + BE_OVERFLOW, 1);
-    // WLSI_US_WENO geometry
-    const int m1 = g.m1, m2 = g.m2, m = m1 + m2;
-    O.kind[r] = RQ_WLS;
-    O.m[2 * r] = m1;
-    O.m[2 * r + 1] = m2;
-    double *gx = geo + G_X, *gy = geo + G_Y, *gw = geo + G_W;
-    for (int i = 0; i < m; ++i) {
-        const int32_t leaf = i < m1 ? g.n1[i] : g.n2[i - m1];
-        mem[i] = T.lslot[leaf];
-        const double xi = T.lcx[leaf], yi = T.lcy[leaf];
-        gx[i] = xi;
-        gy[i] = yi;
+    __syncwarp(mask);
+    double *geo = O.geo + rq_geo_at(r);
+    int32_t *mem = O.mem + rq_mem_at(r);
+    const int m = m1 + m2;
+    const bool few = m < 7;
+    if (lane == 0) {
+        if (overflow) atomicExch(err + BE_OVERFLOW, 1);
+        const uint64_t p0 = node_pos(c.n);
+        O.node[r] = node_key(c.n);
+        geo[G_ORIGIN * RQ_T] = child ? 1.0 : 0.0;
+        geo[G_XX * RQ_T] = child ? D.tx[r] : x;
+        geo[G_YY * RQ_T] = child ? D.ty[r] : y;
+        O.kind[r] = !few ? RQ_WLS : child ? RQ_COPY : RQ_RESTRICT;
+        O.m[2 * r] = !few ? m1 : child ? 1 : (int32_t)lower_bound_pos_t(T, p0);
+        O.m[2 * r + 1] = !few ? m2 : child ? 0 : (int32_t)lower_bound_pos_t(T, p0 + span_of_level(c.n.lvl));
+        if (few && child) mem[0] = T.lslot[c.leaf];
+        if (few && !child) {
+            geo[G_LVL * RQ_T] = (double)c.n.lvl;
+            atomicAdd(O.counts + 2, 1ull);
+        }
+    }
+    if (few) return;
+    for (int i = lane; i < WLS_MAXM; i += 8) {
+        const bool axis = i < WLS_AXIS, in = axis ? i < m1 : i - WLS_AXIS < m2;
+        const int32_t leaf = !in ? -1 : axis ? list[g][0][i] : list[g][1][i - WLS_AXIS];
+        mem[i * RQ_T] = in ? T.lslot[leaf] : -1;
+        geo[(G_X + i) * RQ_T] = in ? T.lcx[leaf] : 0.0;
+        geo[(G_Y + i) * RQ_T] = in ? T.lcy[leaf] : 0.0;
+    }
+    if (lane == 7) {
+        // smoothness box of the node (compute_smoothness, src/XuanGua.F90:318-323)
+        const double hx = G.xf * G.h / ipow2d(c.n.lvl + 1);
+        const double hy = G.h / ipow2d(c.n.lvl + 1);
+        geo[(G_BOX + 0) * RQ_T] = x - hx;
+        geo[(G_BOX + 1) * RQ_T] = x + hx;
+        geo[(G_BOX + 2) * RQ_T] = y - hy;
+        geo[(G_BOX + 3) * RQ_T] = y + hy;
+    }
+}
+
+// WLSI_US_WENO geometry of a request: the weights, P^T W P over all members
+// and over the axis and the diagonal ones, and their three brinv inverses
+// (src/XuanGua.F90:206-255); one thread per request, no divergence but the
+// member count.
+__global__ void __launch_bounds__(64) k_wls_geometry(Tables T, ReqOut O) {
+    const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (r >= T.NR || O.kind[r] != RQ_WLS) return;
+    double *geo = O.geo + rq_geo_at(r);
+    const int m1 = O.m[2 * r], m2 = O.m[2 * r + 1];
+    const double xx = geo[G_XX * RQ_T], yy = geo[G_YY * RQ_T];
+    double R[6][6], RA[3][3], RB[3][3];
+#pragma unroll
+    for (int a = 0; a < 6; ++a)
+#pragma unroll
+        for (int b = 0; b < 6; ++b) R[a][b] = 0.0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = 0; b < 3; ++b) { RA[a][b] = 0.0; RB[a][b] = 0.0; }
+#pragma unroll
+    for (int i = 0; i < WLS_MAXM; ++i) {
+        if (i < WLS_AXIS ? i >= m1 : i - WLS_AXIS >= m2) {
+            geo[(G_W + i) * RQ_T] = 0.0;
+            continue;
+        }
+        const double xi = geo[(G_X + i) * RQ_T], yi = geo[(G_Y + i) * RQ_T];
         const double d = sqrt((xi - xx) * (xi - xx) + (yi - yy) * (yi - yy));
-        gw[i] = 1.0 / (d + 1.e-6);
+        const double w = 1.0 / (d + 1.e-6);
+        geo[(G_W + i) * RQ_T] = w;
+        const double P[6] = {1.0, xi, yi, xi * yi, xi * xi, yi * yi};
+        double pw[6];
+#pragma unroll
+        for (int b = 0; b < 6; ++b) pw[b] = w * P[b];
+#pragma unroll
+        for (int a = 0; a < 6; ++a)
+#pragma unroll
+            for (int b = 0; b < 6; ++b) R[a][b] = R[a][b] + P[a] * pw[b];
+        if (i < WLS_AXIS) {
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                for (int b = 0; b < 3; ++b) RA[a][b] = RA[a][b] + P[a] * pw[b];
+        } else {
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                for (int b = 0; b < 3; ++b) RB[a][b] = RB[a][b] + P[a] * pw[b];
+        }
     }
-    geo[G_XX] = xx;
-    geo[G_YY] = yy;
-    double P[WLS_MAXM][6];
-    for (int i = 0; i < m; ++i) {
-        P[i][0] = 1.0; P[i][1] = gx[i]; P[i][2] = gy[i];
-        P[i][3] = gx[i] * gy[i]; P[i][4] = gx[i] * gx[i]; P[i][5] = gy[i] * gy[i];
-    }
-    double *L = geo + G_L, *A = geo + G_A, *B = geo + G_B;
     unsigned long long ns = 0;
-    {
-        double R[6][6];
+    if (!brinv_reg<3>(RA)) ++ns;
 #pragma unroll
-        for (int a = 0; a < 6; ++a)
+    for (int k = 0; k < 9; ++k) geo[(G_A + k) * RQ_T] = RA[k / 3][k % 3];
+    if (!brinv_reg<3>(RB)) ++ns;
 #pragma unroll
-            for (int b = 0; b < 6; ++b) R[a][b] = 0.0;
-        for (int i = 0; i < m; ++i) {
-            const double pw[6] = {gw[i] * P[i][0], gw[i] * P[i][1], gw[i] * P[i][2],
-                                  gw[i] * P[i][3], gw[i] * P[i][4], gw[i] * P[i][5]};
+    for (int k = 0; k < 9; ++k) geo[(G_B + k) * RQ_T] = RB[k / 3][k % 3];
+    if (!brinv_reg<6>(R)) ++ns;
 #pragma unroll
-            for (int a = 0; a < 6; ++a)
-#pragma unroll
-                for (int b = 0; b < 6; ++b) R[a][b] = R[a][b] + P[i][a] * pw[b];
-        }
-        if (!brinv_reg<6>(R)) ++ns;
-#pragma unroll
-        for (int a = 0; a < 6; ++a)
-#pragma unroll
-            for (int b = 0; b < 6; ++b) L[a * 6 + b] = R[a][b];
-    }
-    {
-        double RA[3][3], RB[3][3];
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int b = 0; b < 3; ++b) { RA[a][b] = 0.0; RB[a][b] = 0.0; }
-        for (int i = 0; i < m1; ++i) {
-            const double pw[3] = {gw[i] * P[i][0], gw[i] * P[i][1], gw[i] * P[i][2]};
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-#pragma unroll
-                for (int b = 0; b < 3; ++b) RA[a][b] = RA[a][b] + P[i][a] * pw[b];
-        }
-        for (int i = m1; i < m; ++i) {
-            const double pw[3] = {gw[i] * P[i][0], gw[i] * P[i][1], gw[i] * P[i][2]};
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-#pragma unroll
-                for (int b = 0; b < 3; ++b) RB[a][b] = RB[a][b] + P[i][a] * pw[b];
-        }
-        if (!brinv_reg<3>(RA)) ++ns;
-        if (!brinv_reg<3>(RB)) ++ns;
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int b = 0; b < 3; ++b) { A[a * 3 + b] = RA[a][b]; B[a * 3 + b] = RB[a][b]; }
-    }
+    for (int k = 0; k < 36; ++k) geo[(G_L + k) * RQ_T] = R[k / 6][k % 6];
     if (ns) atomicAdd(O.counts + 0, ns);
-    atomicAdd(O.counts + 1, 1ull);
-    // smoothness box of the node (compute_smoothness, src/XuanGua.F90:318-323)
-    double ncx, ncy;
-    node_center(G, c.n, ncx, ncy);
-    if (c.leaf >= 0) { ncx = T.lcx[c.leaf]; ncy = T.lcy[c.leaf]; }
-    const double hx = G.xf * G.h / ipow2d(c.n.lvl + 1);
-    const double hy = G.h / ipow2d(c.n.lvl + 1);
-    geo[G_BOX + 0] = ncx - hx;
-    geo[G_BOX + 1] = ncx + hx;
-    geo[G_BOX + 2] = ncy - hy;
-    geo[G_BOX + 3] = ncy + hy;
 }
 
 // ------------------------------------------------------------- ghosts
@@ -687,11 +670,14 @@ __global__ void k_validate(Tables T, const int64_t *__restrict__ face_counts, in
     if (t < T.NR) {
         const int k = T.rq_kind[t];
         const int32_t a = T.rq_m[2 * t], b = T.rq_m[2 * t + 1];
-        const int32_t *mem = T.rq_mem + t * WLS_MAXM;
+        const int32_t *mem = T.rq_mem + rq_mem_at(t);
         if (k == RQ_WLS) {
-            bad |= a < 0 || b < 0 || a + b > WLS_MAXM;
+            bad |= a < 0 || a > WLS_AXIS || b < 0 || b > WLS_MAXM - WLS_AXIS;
             if (!bad)
-                for (int i = 0; i < a + b; ++i) bad |= mem[i] < 0 || mem[i] >= NLEAF;
+                for (int i = 0; i < WLS_MAXM; ++i) {
+                    const bool in = i < WLS_AXIS ? i < a : i - WLS_AXIS < b;
+                    bad |= in ? mem[i * RQ_T] < 0 || mem[i * RQ_T] >= NLEAF : mem[i * RQ_T] != -1;
+                }
         } else if (k == RQ_RESTRICT) {
             bad |= a < 0 || b <= a || b > T.NL;
         } else if (k == RQ_COPY) {
@@ -879,7 +865,7 @@ int build_tables(fdm_handle *h, int64_t n, const uint64_t *keys_in, const double
     h->NR = NR;
     h->NS = NI + NG + NC + NR;
     const int64_t VS0 = NI + NG + NC;
-    const int64_t nrq = NR > 0 ? NR : 1;
+    const int64_t nrq = (NR > 0 ? NR + RQ_T - 1 : RQ_T) / RQ_T * RQ_T;   // whole tiles
     Carve c4;
     c4.add(nrq * 4); c4.add(nrq * 8); c4.add(nrq * 8); c4.add(nrq * 8);
     FDM_CK(h, h->tmp[4].ensure(c4.total));
@@ -902,7 +888,8 @@ int build_tables(fdm_handle *h, int64_t n, const uint64_t *keys_in, const double
         Tables T = h->tables();
         ReqOut O{h->rq_kind.as<int32_t>(), h->rq_m.as<int32_t>(), h->rq_mem.as<int32_t>(),
                  h->rq_geo.as<double>(), h->rq_node.as<uint64_t>(), counts};
-        k_gather<<<nblk(NR, 64), 64, 0, s>>>(T, h->G, RD, O, err);
+        k_gather<<<nblk(NR, GATHER_RPB), GATHER_RPB * 8, 0, s>>>(T, h->G, RD, O, err);
+        k_wls_geometry<<<nblk(NR, 64), 64, 0, s>>>(T, O);
     }
     // the interpA fallbacks among the requests, listed (in no particular
     // order: each writes only its own value), so that their warps are

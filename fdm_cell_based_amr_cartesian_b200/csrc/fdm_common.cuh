@@ -13,7 +13,11 @@ namespace fdm {
 
 constexpr int LMAX = FDM_LMAX;
 constexpr int MAXLVL_TAB = 16;   // per-level tables
-constexpr int WLS_MAXM = 12;     // members of one WLS stencil (<= 9 in practice)
+// Members of one WLS stencil: at most one per 45-degree sector and the leaf
+// itself, the axis ones (east, north, west, south, the leaf) in slots
+// 0..WLS_AXIS-1 and the diagonal ones after them; unused slots hold no
+// member (-1) and zero coordinates and weight.
+constexpr int WLS_AXIS = 5, WLS_MAXM = 9;
 
 // Request kinds: values of the "virtual" stencil slots that a leaf cannot
 // read directly from a same-level leaf (hanging nodes).
@@ -68,8 +72,8 @@ struct Tables {
     // requests (virtual slots NI+NG+NC+r)
     const int32_t *rq_kind;           // [NR]
     const int32_t *rq_m;              // [NR][2]  (m1, m2) or (lo, hi) range
-    const int32_t *rq_mem;            // [NR][WLS_MAXM] member slots
-    const double *rq_geo;             // [NR][RQ_GEO] geometry block
+    const int32_t *rq_mem;            // member slots, in tiles (rq_mem_at)
+    const double *rq_geo;             // geometry blocks, in tiles (rq_geo_at)
     const uint64_t *rq_node;          // [NR] key of the node the value belongs to
     const int32_t *rq_rlist;          // [NRR] the requests of kind RQ_RESTRICT (interpA fallbacks)
     int64_t NRR;
@@ -92,7 +96,14 @@ constexpr int G_A = G_L + 36;                     // inverse 3x3 (axis points)
 constexpr int G_B = G_A + 9;                      // inverse 3x3 (diagonal points)
 constexpr int G_LVL = G_B + 9;                    // level (restrict) as double
 constexpr int G_ORIGIN = G_LVL + 1;               // 0 parent_value_weno, 1 child_value_weno
-constexpr int RQ_GEO = G_LVL + 2;                 // 96 doubles
+constexpr int RQ_GEO = G_LVL + 2;                 // 89 doubles
+// Geometry blocks and member lists are stored in tiles of RQ_T requests,
+// element by element: element k of request r at rq_geo_at(r) + k * RQ_T (and
+// member i at rq_mem_at(r) + i * RQ_T), so the requests of a warp read
+// neighbouring words.
+constexpr int RQ_T = 8;
+FDM_HD int64_t rq_geo_at(int64_t r) { return (r / RQ_T) * (RQ_T * RQ_GEO) + r % RQ_T; }
+FDM_HD int64_t rq_mem_at(int64_t r) { return (r / RQ_T) * (RQ_T * WLS_MAXM) + r % RQ_T; }
 
 // Device-side scalars of the time loop.
 struct DevScalars {

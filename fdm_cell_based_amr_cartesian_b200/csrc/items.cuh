@@ -147,54 +147,47 @@ __device__ __forceinline__ double4 restrict_warp(const Tables &T, const double4 
     return r;
 }
 
-// hanging-node request r of kind WLS or COPY (RESTRICT: request_restrict_warp)
-__device__ __forceinline__ void request_item(const Tables &T, double4 *cur, int64_t r) {
-    const int64_t out = T.NI + T.NG + T.NC + r;
-    const int kind = T.rq_kind[r];
-    const int32_t *mem = T.rq_mem + r * WLS_MAXM;
-    if (kind == RQ_COPY) {
-        cur[out] = cur[mem[0]];
-        return;
+// components v..v+NV-1 of hanging-node request r of kind WLS or COPY (v a
+// multiple of NV): the four components of a value are independent, so 4 / NV
+// threads share a request.  geo: element 0 of the request's geometry block
+// (global memory, or a copy of its tile in shared memory).
+template <int NV>
+__device__ __forceinline__ void load_components(const double *rec, double (&c)[NV]) {
+    if constexpr (NV == 2) {
+        const double2 q = *reinterpret_cast<const double2 *>(rec);
+        c[0] = q.x; c[1] = q.y;
+    } else {
+        c[0] = *rec;
     }
-    if (kind == RQ_RESTRICT) return;
-    const int m1 = T.rq_m[2 * r], m2 = T.rq_m[2 * r + 1];
-    const int m = m1 + m2;
-    const double *geo = T.rq_geo + r * RQ_GEO;
-    double ph[4][WLS_MAXM];
-#pragma unroll
-    for (int i = 0; i < WLS_MAXM; ++i) {
-        const double4 q = i < m ? cur[mem[i]] : make_double4(0.0, 0.0, 0.0, 0.0);
-        ph[0][i] = q.x; ph[1][i] = q.y; ph[2][i] = q.z; ph[3][i] = q.w;
-    }
-    double4 v;
-    v.x = wls_eval_var(geo, m1, m2, ph[0]);
-    v.y = wls_eval_var(geo, m1, m2, ph[1]);
-    v.z = wls_eval_var(geo, m1, m2, ph[2]);
-    v.w = wls_eval_var(geo, m1, m2, ph[3]);
-    cur[out] = v;
 }
-
-// component v (0..3) of hanging-node request r of kind WLS or COPY: the
-// four components of a value are independent, so four threads can share a
-// request.  geo: the request's geometry block (global memory, or a copy of
-// it in shared memory).
-__device__ __forceinline__ void request_item_var(const Tables &T, double4 *cur, int64_t r, int v,
-                                                 const double *geo) {
-    const int64_t out = T.NI + T.NG + T.NC + r;
+template <int NV>
+__device__ __forceinline__ void request_item(const Tables &T, double4 *cur, int64_t r, int v, const double *geo) {
+    static_assert(NV == 1 || NV == 2, "components per thread");
     const int kind = T.rq_kind[r];
-    const int32_t *mem = T.rq_mem + r * WLS_MAXM;
-    double *o = reinterpret_cast<double *>(cur + out) + v;
-    if (kind == RQ_COPY) {
-        *o = reinterpret_cast<const double *>(cur + mem[0])[v];
-        return;
-    }
     if (kind == RQ_RESTRICT) return;
-    const int m1 = T.rq_m[2 * r], m2 = T.rq_m[2 * r + 1];
-    const int m = m1 + m2;
-    double ph[WLS_MAXM];
+    const int32_t *mem = T.rq_mem + rq_mem_at(r);
+    double out[NV];
+    if (kind == RQ_COPY) {
+        load_components<NV>(reinterpret_cast<const double *>(cur + mem[0]) + v, out);
+    } else {
+        int32_t slot[WLS_MAXM];
 #pragma unroll
-    for (int i = 0; i < WLS_MAXM; ++i) ph[i] = i < m ? reinterpret_cast<const double *>(cur + mem[i])[v] : 0.0;
-    *o = wls_eval_var(geo, m1, m2, ph);
+        for (int i = 0; i < WLS_MAXM; ++i) slot[i] = mem[i * RQ_T];
+        double phi[NV][WLS_MAXM];
+#pragma unroll
+        for (int i = 0; i < WLS_MAXM; ++i) {
+            double c[NV];
+#pragma unroll
+            for (int q = 0; q < NV; ++q) c[q] = 0.0;
+            if (slot[i] >= 0) load_components<NV>(reinterpret_cast<const double *>(cur + slot[i]) + v, c);
+#pragma unroll
+            for (int q = 0; q < NV; ++q) phi[q][i] = c[q];
+        }
+        wls_eval<NV>(geo, phi, out);
+    }
+    double *o = reinterpret_cast<double *>(cur + T.NI + T.NG + T.NC + r) + v;
+    if constexpr (NV == 2) *reinterpret_cast<double2 *>(o) = make_double2(out[0], out[1]);
+    else *o = out[0];
 }
 
 // The geometry blocks of the RQ_TILE requests from r0 on (contiguous in
@@ -205,6 +198,7 @@ constexpr int RQ_TILE = 64;
 __device__ __forceinline__ void stage_request_geometry(const Tables &T, int64_t r0, double *smem_geo, int nthreads) {
     int64_t nreq = T.NR - r0;
     if (nreq > RQ_TILE) nreq = RQ_TILE;
+    nreq = (nreq + RQ_T - 1) / RQ_T * RQ_T;   // whole tiles
     const int nch = nreq > 0 ? (int)(nreq * RQ_GEO / 2) : 0;   // 16-byte chunks
     const double *src = T.rq_geo + r0 * RQ_GEO;
     for (int k = threadIdx.x; k < nch; k += nthreads) {
@@ -214,25 +208,6 @@ __device__ __forceinline__ void stage_request_geometry(const Tables &T, int64_t 
     asm volatile("cp.async.commit_group;\n" ::);
     asm volatile("cp.async.wait_group 0;\n" ::);
     __syncthreads();
-}
-
-__device__ __forceinline__ void request_item_var(const Tables &T, double4 *cur, int64_t r, int v) {
-    const int64_t out = T.NI + T.NG + T.NC + r;
-    const int kind = T.rq_kind[r];
-    const int32_t *mem = T.rq_mem + r * WLS_MAXM;
-    double *o = reinterpret_cast<double *>(cur + out) + v;
-    if (kind == RQ_COPY) {
-        *o = reinterpret_cast<const double *>(cur + mem[0])[v];
-        return;
-    }
-    if (kind == RQ_RESTRICT) return;
-    const int m1 = T.rq_m[2 * r], m2 = T.rq_m[2 * r + 1];
-    const int m = m1 + m2;
-    const double *geo = T.rq_geo + r * RQ_GEO;
-    double ph[WLS_MAXM];
-#pragma unroll
-    for (int i = 0; i < WLS_MAXM; ++i) ph[i] = i < m ? reinterpret_cast<const double *>(cur + mem[i])[v] : 0.0;
-    *o = wls_eval_var(geo, m1, m2, ph);
 }
 
 // interpA fallback of parent_value_weno for request r (whole warp)

@@ -80,10 +80,10 @@ __global__ void k_neighbors_out(Tables T, Geometry G, uint64_t *out) {
     nb[2] = face_nb(T, G, c, DIR_RIGHT);
     nb[3] = face_nb(T, G, c, DIR_LEFT);
     if (root_cross(G, c.n.root) >= 0) {
-        nb[4] = upleft_nb(T, G, c);
-        nb[5] = upright_nb(T, G, c);
-        nb[6] = downleft_nb(T, G, c);
-        nb[7] = downright_nb(T, G, c);
+        nb[4] = diagonal_nb(T, G, c, DIR_LEFT, DIR_UP);
+        nb[5] = diagonal_nb(T, G, c, DIR_RIGHT, DIR_UP);
+        nb[6] = diagonal_nb(T, G, c, DIR_LEFT, DIR_DOWN);
+        nb[7] = diagonal_nb(T, G, c, DIR_RIGHT, DIR_DOWN);
     } else {
         for (int d = 4; d < 8; ++d) nb[d] = null_ref();
     }
@@ -108,17 +108,20 @@ __global__ void k_requests_out(Tables T, int32_t *kind, uint64_t *node, double *
         return;
     }
     const int64_t r = s - VS0;
-    const double *geo = T.rq_geo + r * RQ_GEO;
+    const double *geo = T.rq_geo + rq_geo_at(r);
     const int k = T.rq_kind[r];
-    const bool child = geo[G_ORIGIN] != 0.0;
+    const bool child = geo[G_ORIGIN * RQ_T] != 0.0;
     kind[o] = child ? (k == RQ_WLS ? 3 : 4) : (k == RQ_WLS ? 1 : 2);
     node[o] = T.rq_node[r];
-    xy[2 * o] = geo[G_XX];
-    xy[2 * o + 1] = geo[G_YY];
+    xy[2 * o] = geo[G_XX * RQ_T];
+    xy[2 * o + 1] = geo[G_YY * RQ_T];
     if (k == RQ_WLS) {
         const int m1 = T.rq_m[2 * r], m2 = T.rq_m[2 * r + 1];
         m12[2 * o] = m1; m12[2 * o + 1] = m2;
-        for (int i = 0; i < m1 + m2 && i < 16; ++i) mem[o * 16 + i] = T.lkey[T.slot_leaf[T.rq_mem[r * WLS_MAXM + i]]];
+        for (int i = 0; i < m1 + m2 && i < 16; ++i) {
+            const int at = i < m1 ? i : WLS_AXIS + i - m1;
+            mem[o * 16 + i] = T.lkey[T.slot_leaf[T.rq_mem[rq_mem_at(r) + at * RQ_T]]];
+        }
     } else {
         m12[2 * o] = -1; m12[2 * o + 1] = -1;
     }

@@ -265,94 +265,96 @@ __device__ __forceinline__ double smooth1(const double b[3], const double *box) 
     return (b[1] * b[1] + b[2] * b[2]) * (box[1] - box[0]) * (box[3] - box[2]);
 }
 
-// Per-stage part of WLSI_US_WENO (src/XuanGua.F90:257-307) for one variable:
+// Per-stage part of WLSI_US_WENO (src/XuanGua.F90:257-307) for NV variables:
 // the geometry (x, y, w, the three brinv inverses) was prepared at regrid.
-__device__ __forceinline__ double wls_eval_var(const double *__restrict__ geo, int m1, int m2,
-                                               const double *phi) {
-    const int m = m1 + m2;
-    const double *x = geo + G_X, *y = geo + G_Y, *w = geo + G_W;
-    const double xx = geo[G_XX], yy = geo[G_YY];
-    const double *box = geo + G_BOX;
-    // the loops run over the fixed WLS_MAXM slots with the members' count as a
-    // predicate, so the arrays stay in registers (the sums keep their order)
-    double wphi[WLS_MAXM];
+// geo: element 0 of the request's block (elements RQ_T apart); phi: the
+// members' values, +0 in the unused slots, whose weights are zero: their
+// terms are zeros, which leave every sum as it is (none of them is -0).
+template <int NV>
+__device__ __forceinline__ void wls_eval(const double *__restrict__ geo, const double (&phi)[NV][WLS_MAXM],
+                                         double (&out)[NV]) {
+    const auto at = [&](int k) { return geo[k * RQ_T]; };
+    double pt[NV][6], p1[NV][3], p2[NV][3];
 #pragma unroll
-    for (int i = 0; i < WLS_MAXM; ++i) wphi[i] = i < m ? w[i] * phi[i] : 0.0;
-    double pt[6];
-    {
-        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0, s4 = 0.0, s5 = 0.0;
+    for (int v = 0; v < NV; ++v) {
 #pragma unroll
-        for (int i = 0; i < WLS_MAXM; ++i) {
-            if (i >= m) continue;
-            const double xi = x[i], yi = y[i], wp = wphi[i];
-            s0 = s0 + 1.0 * wp;
-            s1 = s1 + xi * wp;
-            s2 = s2 + yi * wp;
-            s3 = s3 + (xi * yi) * wp;
-            s4 = s4 + (xi * xi) * wp;
-            s5 = s5 + (yi * yi) * wp;
+        for (int k = 0; k < 6; ++k) pt[v][k] = 0.0;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) { p1[v][k] = 0.0; p2[v][k] = 0.0; }
+    }
+#pragma unroll
+    for (int i = 0; i < WLS_MAXM; ++i) {
+        const double xi = at(G_X + i), yi = at(G_Y + i), wi = at(G_W + i);
+        const double xy = xi * yi, x2 = xi * xi, y2 = yi * yi;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            const double wp = wi * phi[v][i], xw = xi * wp, yw = yi * wp;
+            pt[v][0] = pt[v][0] + wp;
+            pt[v][1] = pt[v][1] + xw;
+            pt[v][2] = pt[v][2] + yw;
+            pt[v][3] = pt[v][3] + xy * wp;
+            pt[v][4] = pt[v][4] + x2 * wp;
+            pt[v][5] = pt[v][5] + y2 * wp;
+            double *p = i < WLS_AXIS ? p1[v] : p2[v];
+            p[0] = p[0] + wp;
+            p[1] = p[1] + xw;
+            p[2] = p[2] + yw;
         }
-        pt[0] = s0; pt[1] = s1; pt[2] = s2; pt[3] = s3; pt[4] = s4; pt[5] = s5;
     }
-    double arr[6];
-    const double *L = geo + G_L;
+    double arr[NV][6], c1[NV][3], c2[NV][3];
 #pragma unroll
-    for (int a = 0; a < 6; ++a) {
-        double s = 0.0;
+    for (int v = 0; v < NV; ++v) {
 #pragma unroll
-        for (int b = 0; b < 6; ++b) s = s + L[a * 6 + b] * pt[b];
-        arr[a] = s;
-    }
-    const double var_large = arr[0] + xx * arr[1] + yy * arr[2] + xx * yy * arr[3] +
-                             xx * xx * arr[4] + yy * yy * arr[5];
-    const double sm_large = smooth2(arr, box);
-    double p1[3] = {0.0, 0.0, 0.0}, p2[3] = {0.0, 0.0, 0.0};
+        for (int a = 0; a < 6; ++a) arr[v][a] = 0.0;
 #pragma unroll
-    for (int i = 0; i < WLS_MAXM; ++i) {
-        if (i >= m1) continue;
-        p1[0] = p1[0] + 1.0 * wphi[i];
-        p1[1] = p1[1] + x[i] * wphi[i];
-        p1[2] = p1[2] + y[i] * wphi[i];
+        for (int a = 0; a < 3; ++a) { c1[v][a] = 0.0; c2[v][a] = 0.0; }
     }
 #pragma unroll
-    for (int i = 0; i < WLS_MAXM; ++i) {
-        if (i < m1 || i >= m) continue;
-        p2[0] = p2[0] + 1.0 * wphi[i];
-        p2[1] = p2[1] + x[i] * wphi[i];
-        p2[2] = p2[2] + y[i] * wphi[i];
-    }
-    double c1[3], c2[3];
-    const double *A = geo + G_A, *B = geo + G_B;
+    for (int a = 0; a < 6; ++a)
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        double s = 0.0, t = 0.0;
+        for (int b = 0; b < 6; ++b) {
+            const double l = at(G_L + a * 6 + b);
+#pragma unroll
+            for (int v = 0; v < NV; ++v) arr[v][a] = arr[v][a] + l * pt[v][b];
+        }
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
 #pragma unroll
         for (int b = 0; b < 3; ++b) {
-            s = s + A[a * 3 + b] * p1[b];
-            t = t + B[a * 3 + b] * p2[b];
+            const double l1 = at(G_A + a * 3 + b), l2 = at(G_B + a * 3 + b);
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                c1[v][a] = c1[v][a] + l1 * p1[v][b];
+                c2[v][a] = c2[v][a] + l2 * p2[v][b];
+            }
         }
-        c1[a] = s;
-        c2[a] = t;
+    const double xx = at(G_XX), yy = at(G_YY);
+    const double box[4] = {at(G_BOX), at(G_BOX + 1), at(G_BOX + 2), at(G_BOX + 3)};
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        const double var_large = arr[v][0] + xx * arr[v][1] + yy * arr[v][2] + xx * yy * arr[v][3] +
+                                 xx * xx * arr[v][4] + yy * yy * arr[v][5];
+        const double sm_large = smooth2(arr[v], box);
+        const double vs1 = c1[v][0] + xx * c1[v][1] + yy * c1[v][2];
+        const double vs2 = c2[v][0] + xx * c2[v][1] + yy * c2[v][2];
+        const double sm1 = smooth1(c1[v], box), sm2 = smooth1(c2[v], box);
+        const double eps = 1.e-6;
+        double sa = 0.0;
+        sa = sa + fabs(sm_large - sm1);
+        sa = sa + fabs(sm_large - sm2);
+        double tau = sa / 2.0;
+        tau = tau * tau;
+        const double al0 = 0.98 * (1.0 + tau / (eps + sm_large));
+        const double al1 = 0.01 * (1.0 + tau / (eps + sm1));
+        const double al2 = 0.01 * (1.0 + tau / (eps + sm2));
+        double sal = 0.0;
+        sal = sal + al0;
+        sal = sal + al1;
+        sal = sal + al2;
+        const double om0 = al0 / sal, om1 = al1 / sal, om2 = al2 / sal;
+        out[v] = om0 * (1.0 / 0.98 * var_large - (0.01 / 0.98 * vs1 + 0.01 / 0.98 * vs2)) +
+                 (om1 * vs1 + om2 * vs2);
     }
-    const double vs1 = c1[0] + xx * c1[1] + yy * c1[2];
-    const double vs2 = c2[0] + xx * c2[1] + yy * c2[2];
-    const double sm1 = smooth1(c1, box), sm2 = smooth1(c2, box);
-    const double eps = 1.e-6;
-    double sa = 0.0;
-    sa = sa + fabs(sm_large - sm1);
-    sa = sa + fabs(sm_large - sm2);
-    double tau = sa / 2.0;
-    tau = tau * tau;
-    const double al0 = 0.98 * (1.0 + tau / (eps + sm_large));
-    const double al1 = 0.01 * (1.0 + tau / (eps + sm1));
-    const double al2 = 0.01 * (1.0 + tau / (eps + sm2));
-    double sal = 0.0;
-    sal = sal + al0;
-    sal = sal + al1;
-    sal = sal + al2;
-    const double om0 = al0 / sal, om1 = al1 / sal, om2 = al2 / sal;
-    return om0 * (1.0 / 0.98 * var_large - (0.01 / 0.98 * vs1 + 0.01 / 0.98 * vs2)) +
-           (om1 * vs1 + om2 * vs2);
 }
 
 }  // namespace fdm

@@ -19,12 +19,20 @@ namespace fdm {
 
 static inline int nblk(int64_t n, int t) { return (int)((n + t - 1) / t); }
 
-// four threads per request, one per component
-__global__ void __launch_bounds__(256) k_requests4(Tables T, double4 *cur) {
+// 4 / NV threads per request, NV components each; eight neighbouring lanes
+// read one tile of the geometry, so a load of an element is 64 contiguous
+// bytes for each group of them.  The 712 bytes of geometry per value bound it
+// (58 MB for 81k values, from L2 while the mesh stays); the fixed slots let
+// the loads run ahead of the sums.  81k values 24 us cold, 57k 13 us (41 and
+// 23 with one block of geometry per request, member counts as predicates and
+// a thread per component).
+constexpr int RQ_NV = 2;
+__global__ void __launch_bounds__(128) k_requests(Tables T, double4 *cur) {
+    constexpr int PER = 32 * RQ_NV / 4;   // requests per warp
     const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t r = g >> 2;
+    const int64_t r = (g >> 5) * PER + (g & (PER - 1));
     if (r >= T.NR) return;
-    request_item_var(T, cur, r, (int)(g & 3));
+    request_item<RQ_NV>(T, cur, r, ((int)g & 31) / PER * RQ_NV, T.rq_geo + rq_geo_at(r));
 }
 
 // interpA fallbacks of parent_value_weno: one warp per listed request
@@ -195,7 +203,7 @@ __global__ void k_set_tstep(DevScalars *sc, double tstep) {
 // ------------------------------------------------------------ launchers
 void launch_requests(fdm_handle *h, const double4 *cur) {
     if (h->NR == 0) return;
-    k_requests4<<<nblk(4 * h->NR, 256), 256, 0, h->s>>>(h->tables(), (double4 *)cur);
+    k_requests<<<nblk(h->NR, 128 * RQ_NV / 4), 128, 0, h->s>>>(h->tables(), (double4 *)cur);
     if (h->n_restrict > 0)
         k_requests_restrict<<<nblk(h->n_restrict, 4), 128, 0, h->s>>>(h->tables(), (double4 *)cur);
 }

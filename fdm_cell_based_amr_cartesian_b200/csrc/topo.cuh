@@ -148,88 +148,30 @@ __device__ __forceinline__ NodeRef sibling_ref(const Tables &T, const NodeRef &x
     return resolve(T, c);
 }
 
-// Diagonal walks, src/neighbor.F90:199-396.  q codes: son1 = 0, son2 = 1,
-// son3 = 3, son4 = 2.
-__device__ __forceinline__ NodeRef descend_while(const Tables &T, NodeRef r, int lvl, int q) {
-    while (r.valid && r.n.lvl < lvl && r.leaf < 0) r = child_ref(T, r, q);
-    return r;
-}
-
-__device__ inline NodeRef upleft_nb(const Tables &T, const Geometry &G, const NodeRef &c) {
-    const NodeRef celln = face_nb(T, G, c, DIR_LEFT), cellfn = face_nb(T, G, c, DIR_UP);
+// Diagonal walks up-left, up-right, down-right and down-left
+// (src/neighbor.F90:199-396), one function of the two directions: with the
+// node's quadrant in its father, a walk that stays inside the father ends at
+// the opposite son; one that leaves it both ways goes through the neighbour
+// along x and descends along the corner that faces the node; one that leaves
+// it one way goes through that neighbour, and is null when it is coarser.
+__device__ inline NodeRef diagonal_nb(const Tables &T, const Geometry &G, const NodeRef &c, int dx, int dy) {
+    const NodeRef nx = face_nb(T, G, c, dx), ny = face_nb(T, G, c, dy);
     if (c.n.lvl == 0) {
-        if (!celln.valid || !cellfn.valid) return null_ref();
-        return face_nb(T, G, celln, DIR_UP);
+        if (!nx.valid || !ny.valid) return null_ref();
+        return face_nb(T, G, nx, dy);
     }
-    const int sp = quadrant_to_sp(node_quadrant(c.n));
-    if (sp == 2) return sibling_ref(T, c, 2);
-    if (sp == 4) {
-        if (!celln.valid || !cellfn.valid) return null_ref();
-        return descend_while(T, face_nb(T, G, celln, DIR_UP), c.n.lvl, 1);
+    const int q = node_quadrant(c.n);
+    const bool inx = (q & 1) == (dx == DIR_LEFT ? 1 : 0), iny = (q >> 1) == (dy == DIR_DOWN ? 1 : 0);
+    if (inx && iny) return sibling_ref(T, c, q ^ 3);
+    if (!inx && !iny) {
+        if (!nx.valid || !ny.valid) return null_ref();
+        NodeRef r = face_nb(T, G, nx, dy);
+        while (r.valid && r.n.lvl < c.n.lvl && r.leaf < 0) r = child_ref(T, r, q ^ 3);
+        return r;
     }
-    if (sp == 1) {
-        if (!celln.valid || celln.n.lvl < c.n.lvl) return null_ref();
-        return face_nb(T, G, celln, DIR_UP);
-    }
-    if (!cellfn.valid || cellfn.n.lvl < c.n.lvl) return null_ref();
-    return face_nb(T, G, cellfn, DIR_LEFT);
-}
-__device__ inline NodeRef upright_nb(const Tables &T, const Geometry &G, const NodeRef &c) {
-    const NodeRef celln = face_nb(T, G, c, DIR_RIGHT), cellfn = face_nb(T, G, c, DIR_UP);
-    if (c.n.lvl == 0) {
-        if (!celln.valid || !cellfn.valid) return null_ref();
-        return face_nb(T, G, celln, DIR_UP);
-    }
-    const int sp = quadrant_to_sp(node_quadrant(c.n));
-    if (sp == 1) return sibling_ref(T, c, 3);
-    if (sp == 3) {
-        if (!celln.valid || !cellfn.valid) return null_ref();
-        return descend_while(T, face_nb(T, G, celln, DIR_UP), c.n.lvl, 0);
-    }
-    if (sp == 2) {
-        if (!celln.valid || celln.n.lvl < c.n.lvl) return null_ref();
-        return face_nb(T, G, celln, DIR_UP);
-    }
-    if (!cellfn.valid || cellfn.n.lvl < c.n.lvl) return null_ref();
-    return face_nb(T, G, cellfn, DIR_RIGHT);
-}
-__device__ inline NodeRef downright_nb(const Tables &T, const Geometry &G, const NodeRef &c) {
-    const NodeRef celln = face_nb(T, G, c, DIR_RIGHT), cellfn = face_nb(T, G, c, DIR_DOWN);
-    if (c.n.lvl == 0) {
-        if (!celln.valid || !cellfn.valid) return null_ref();
-        return face_nb(T, G, celln, DIR_DOWN);
-    }
-    const int sp = quadrant_to_sp(node_quadrant(c.n));
-    if (sp == 4) return sibling_ref(T, c, 1);
-    if (sp == 2) {
-        if (!celln.valid || !cellfn.valid) return null_ref();
-        return descend_while(T, face_nb(T, G, celln, DIR_DOWN), c.n.lvl, 2);
-    }
-    if (sp == 3) {
-        if (!celln.valid || celln.n.lvl < c.n.lvl) return null_ref();
-        return face_nb(T, G, celln, DIR_DOWN);
-    }
-    if (!cellfn.valid || cellfn.n.lvl < c.n.lvl) return null_ref();
-    return face_nb(T, G, cellfn, DIR_RIGHT);
-}
-__device__ inline NodeRef downleft_nb(const Tables &T, const Geometry &G, const NodeRef &c) {
-    const NodeRef celln = face_nb(T, G, c, DIR_LEFT), cellfn = face_nb(T, G, c, DIR_DOWN);
-    if (c.n.lvl == 0) {
-        if (!celln.valid || !cellfn.valid) return null_ref();
-        return face_nb(T, G, celln, DIR_DOWN);
-    }
-    const int sp = quadrant_to_sp(node_quadrant(c.n));
-    if (sp == 3) return sibling_ref(T, c, 0);
-    if (sp == 1) {
-        if (!celln.valid || !cellfn.valid) return null_ref();
-        return descend_while(T, face_nb(T, G, celln, DIR_DOWN), c.n.lvl, 3);
-    }
-    if (sp == 4) {
-        if (!celln.valid || celln.n.lvl < c.n.lvl) return null_ref();
-        return face_nb(T, G, celln, DIR_DOWN);
-    }
-    if (!cellfn.valid || cellfn.n.lvl < c.n.lvl) return null_ref();
-    return face_nb(T, G, cellfn, DIR_LEFT);
+    const NodeRef &via = inx ? ny : nx;
+    if (!via.valid || via.n.lvl < c.n.lvl) return null_ref();
+    return face_nb(T, G, via, inx ? dx : dy);
 }
 
 // gridcross (src/mesh.F90:89-142) from the background cell of a node
