@@ -745,16 +745,18 @@ __device__ __forceinline__ uint64_t gm4_key(const NodeSet &A, const Gm4 &M, int3
 }
 // What a look from s towards the node at s's level finds at time T: the node
 // itself (same: with its level that of s) or the leaf above it.  id is the
-// node's name, or -1 for a node of A that has sons.
+// node's name, or -1 for a node of A that has sons.  at holds the node of A
+// at s where it is known already (-1: not), since it never changes.
 struct Found {
     uint64_t key;
     int32_t id;
     bool sons;
 };
-__device__ __forceinline__ Found gm4_look(const NodeSet &A, const Gm4 &M, uint64_t s, uint64_t T) {
+__device__ __forceinline__ Found gm4_look(const NodeSet &A, const Gm4 &M, uint64_t s, uint64_t T, int32_t &at) {
     Found f;
     const int ls = (int)(s & 15u);
-    int32_t id = (int32_t)holder(A, s);
+    if (at < 0) at = (int32_t)holder(A, s);
+    int32_t id = at;
     uint64_t k = __ldg(A.key + id);
     int l = (int)(k & 15u);
     if (l > ls) {
@@ -778,8 +780,13 @@ struct Looks {
     bool nonleaf;            // the neighbour's neighbour is refined and has sons
     uint64_t nnkey;
 };
+// where a look's two searches ended in an earlier sweep
+struct Seen {
+    uint64_t s2;          // start of the second one
+    int32_t at1, at2;
+};
 __device__ __forceinline__ Looks gm4_looks(const NodeSet &A, const Geometry &G, const Gm4 &M, uint64_t k, uint64_t r,
-                                           int t) {
+                                           int t, Seen &seen) {
     Looks L;
     L.nb = L.nn = -1;
     L.nonleaf = false;
@@ -787,10 +794,14 @@ __device__ __forceinline__ Looks gm4_looks(const NodeSet &A, const Geometry &G, 
     const int lc = (int)(k & 15u), d = gm4_dir(t);
     uint64_t s;
     if (!shift_key(G, k, d, s)) return L;
-    const Found b = gm4_look(A, M, s, gm4_time(r, 2 * t));
+    const Found b = gm4_look(A, M, s, gm4_time(r, 2 * t), seen.at1);
     if ((int)(b.key & 15u) <= lc - 2) L.nb = b.id;   // no node at lc: a leaf
     if (!shift_key(G, b.key, d, s)) return L;
-    const Found n = gm4_look(A, M, s, gm4_time(r, 2 * t + 1));
+    if (s != seen.s2) {
+        seen.s2 = s;
+        seen.at2 = -1;
+    }
+    const Found n = gm4_look(A, M, s, gm4_time(r, 2 * t + 1), seen.at2);
     if ((int)(n.key & 15u) <= lc - 2) {
         L.nnkey = n.key;
         if (n.sons) L.nonleaf = true;
@@ -827,7 +838,7 @@ __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-constexpr int GM4_CTAS = 8, GM4_THREADS = 512;
+constexpr int GM4_CTAS = 8, GM4_THREADS = 1024;
 
 // The fixpoint, by one cluster of blocks: a sweep is all looks (four lanes
 // per leaf, one per direction), a cluster barrier, then the comparison of
@@ -836,9 +847,10 @@ constexpr int GM4_CTAS = 8, GM4_THREADS = 512;
 // has a few thousand looks: it is bound by the latency of a look (two
 // searches in a background cell's nodes, about 20 dependent L2 reads) times
 // the sweeps, not by the number of SMs.  One B200, two regrids of a developed
-// 128^2, 4-level four-quadrant run (82k leaves, 2029 refinements): 0.94 ms in
-// 39 sweeps, against 14.0 ms for visiting the leaves in order by one block;
-// 64 x 16-cell double Mach at 4 levels, four regrids: 1.0 against 10.2 ms.
+// 128^2, 4-level four-quadrant run (82k leaves, 2029 refinements): 0.67 ms in
+// 39 sweeps (0.94 before a thread kept where its look's searches ended),
+// against 14.0 ms for visiting the leaves in order by one block; 256 x 64
+// double Mach at 4 levels, four regrids: 0.82 against 10.2 ms.
 __global__ void __cluster_dims__(GM4_CTAS, 1, 1) __launch_bounds__(GM4_THREADS)
     k_gm4_fixpoint(NodeSet A, Geometry G, Gm4 M, uint64_t t0, int max_sweeps, Gm4Result *out) {
     const int nthr = GM4_CTAS * GM4_THREADS;
@@ -847,22 +859,29 @@ __global__ void __cluster_dims__(GM4_CTAS, 1, 1) __launch_bounds__(GM4_THREADS)
     int made = 0;        // made nodes that this sweep visits
     int sweep = 0;
     bool full = false;
+    Seen mine{0, -1, -1};
     if (nlist > 0) {
         for (;; ++sweep) {
             const int par = sweep & 1;
             const int64_t looks = 4 * ((int64_t)nlist + made);
-            for (int64_t x = me; x < looks; x += nthr) {
+            const auto look = [&](int64_t x, Seen &seen) {
                 const int v = (int)(x >> 2), t = (int)(x & 3);
                 const int32_t id = v < nlist ? __ldg(M.list + v) : (int32_t)(A.n + (v - nlist));
                 const uint64_t k = gm4_key(A, M, id), r = visit_rank(k);
-                if (gm4_time(r, 7) <= t0 || !gm4_visited(A, M, id, r)) continue;
-                const Looks L = gm4_looks(A, G, M, k, r, t);
+                if (gm4_time(r, 7) <= t0 || !gm4_visited(A, M, id, r)) return;
+                const Looks L = gm4_looks(A, G, M, k, r, t, seen);
                 const uint64_t Tb = gm4_time(r, 2 * t), Tn = gm4_time(r, 2 * t + 1);
                 if (L.nb >= 0 && Tb > t0) gm4_propose(A, M, L.nb, Tb);
                 if (Tn > t0) {
                     if (L.nonleaf) atomicMin((unsigned long long *)(M.nl + par), (unsigned long long)Tn);
                     else if (L.nn >= 0) gm4_propose(A, M, L.nn, Tn);
                 }
+            };
+            // a thread's first look is the same one in every sweep
+            if (me < looks) look(me, mine);
+            for (int64_t x = me + nthr; x < looks; x += nthr) {
+                Seen once{0, -1, -1};
+                look(x, once);
             }
             cluster_barrier();
             const int nrefd = __ldcg(M.w + GW_NREFD);
@@ -911,7 +930,8 @@ __global__ void __cluster_dims__(GM4_CTAS, 1, 1) __launch_bounds__(GM4_THREADS)
         uint64_t nlkey = 0;
         if (nl != GM4_NEVER && !full) {   // the look of that time again, for its node
             const uint64_t r = (nl - 1u) >> 3;
-            nlkey = gm4_looks(A, G, M, key_of_visit_rank(r), r, (int)((nl - 1u) & 7u) >> 1).nnkey;
+            Seen once{0, -1, -1};
+            nlkey = gm4_looks(A, G, M, key_of_visit_rank(r), r, (int)((nl - 1u) & 7u) >> 1, once).nnkey;
         }
         for (int q = 0; q < GW_WORDS; ++q) out->w[q] = __ldcg(M.w + q);
         out->w[GW_FULL] = full;
