@@ -94,7 +94,7 @@ struct NodeSet {
     uint64_t *key = nullptr;
     uint8_t *leaf = nullptr;
     double4 *val = nullptr;
-    const int32_t *rf = nullptr;   // per-cell index of key (index_set), or null
+    int32_t *rf = nullptr;         // per-cell index of key
     int64_t nroots = 0;
 };
 
@@ -111,11 +111,11 @@ __device__ __forceinline__ int64_t find_key(const uint64_t *__restrict__ keys, i
     return (lo < n && keys[lo] == k) ? lo : -1;
 }
 
-// find_key within the nodes of k's background cell when the set is indexed
-// (every cell holds at least its root node, and its nodes are contiguous)
+// find_key within the nodes of k's background cell (every cell holds at
+// least its root node, and its nodes are contiguous)
 __device__ __forceinline__ int64_t find_key_set(const NodeSet &A, uint64_t k) {
     const int64_t r = (int64_t)(k >> 34);
-    if (!A.rf || r >= A.nroots) return find_key(A.key, A.n, k);
+    if (r >= A.nroots) return -1;
     int64_t lo = __ldg(A.rf + r), hi = __ldg(A.rf + r + 1);
     while (lo < hi) {
         const int64_t mid = (lo + hi) >> 1;
@@ -300,39 +300,40 @@ __global__ void k_internal_vals(int64_t NInt, const uint64_t *ikey, double4 *iva
     ival[i] = mean4(c[0], c[1], c[2], c[3]);
 }
 
+// The current and the next node set; each has its three arrays (amr[0..2],
+// amr[3..5]) and its per-cell index (amr[6], amr[7]), which the kernel that
+// writes the set fills too: a cell's first node is its root node.
 struct AmrCtx {
     fdm_handle *h;
-    NodeSet A, B;          // current / next node set
-    int a = 0;             // which buffer triple (amr[0..2] or amr[3..5]) holds A
+    NodeSet A, B;
+    int a = 0;   // which buffers hold A
 };
 
-static void bind_sets(fdm_handle *h, AmrCtx &X) {
-    const int64_t na = X.A.n, nb = X.B.n;
-    NodeSet *S[2] = {&X.A, &X.B};
-    for (int s = 0; s < 2; ++s) {
-        const int b = s == 0 ? X.a : 1 - X.a;
-        S[s]->key = h->amr[3 * b + 0].as<uint64_t>();
-        S[s]->leaf = h->amr[3 * b + 1].as<uint8_t>();
-        S[s]->val = h->amr[3 * b + 2].as<double4>();
-        S[s]->rf = nullptr;
-    }
-    X.A.n = na;
-    X.B.n = nb;
-}
-static void swap_sets(fdm_handle *h, AmrCtx &X) {
-    X.a = 1 - X.a;
-    std::swap(X.A.n, X.B.n);
-    bind_sets(h, X);
-}
 // room for n nodes in the next set; the current one stays as it is
 static int grow_next(fdm_handle *h, AmrCtx &X, int64_t n) {
     const int b = 1 - X.a;
+    const int64_t nroots = (int64_t)h->G.m * h->G.n;
     FDM_CK(h, h->amr[3 * b + 0].ensure(n * 8));
     FDM_CK(h, h->amr[3 * b + 1].ensure(n));
     FDM_CK(h, h->amr[3 * b + 2].ensure(n * 32));
-    bind_sets(h, X);
+    FDM_CK(h, h->amr[6 + b].ensure((nroots + 1) * 4));
+    X.B.key = h->amr[3 * b + 0].as<uint64_t>();
+    X.B.leaf = h->amr[3 * b + 1].as<uint8_t>();
+    X.B.val = h->amr[3 * b + 2].as<double4>();
+    X.B.rf = h->amr[6 + b].as<int32_t>();
+    X.B.nroots = nroots;
+    X.B.n = n;
     return FDM_OK;
 }
+static void swap_sets(AmrCtx &X) {
+    X.a = 1 - X.a;
+    std::swap(X.A, X.B);
+}
+// the index entry of node k stored at o (and the end of the index)
+__device__ __forceinline__ void index_node(const NodeSet &out, uint64_t k, int64_t o) {
+    if ((k & 15u) == 0) out.rf[k >> 34] = (int32_t)o;
+}
+__device__ __forceinline__ void index_end(const NodeSet &out) { out.rf[out.nroots] = (int32_t)out.n; }
 
 // Merge of two key-sorted runs (keys distinct) into the node set out: an
 // entry's place is its index in its run plus the number of keys of the
@@ -356,49 +357,32 @@ __global__ void k_merge_runs(const uint64_t *__restrict__ ka, const uint8_t *__r
     out.key[o] = k;
     out.leaf[o] = in_a ? la[j] : lb[j];
     out.val[o] = in_a ? va[j] : vb[j];
+    index_node(out, k, o);
+    if (i == 0) index_end(out);
 }
 // the runs [0, m) and [m, n) of (keys, leaf, val), each sorted, into out
 static void merge_into(fdm_handle *h, const uint64_t *keys, const uint8_t *leaf, const double4 *val, int64_t m,
-                       int64_t n, NodeSet &out) {
+                       int64_t n, const NodeSet &out) {
     if (n > 0)
         k_merge_runs<<<nblk(n, 256), 256, 0, h->s>>>(keys, leaf, val, m, keys + m, leaf + m, val + m, n - m, out);
-    out.n = n;
 }
-// per-cell index of A's keys (amr[22]) for the root-confined searches
-static int index_set(fdm_handle *h, NodeSet &A) {
-    const int64_t nroots = (int64_t)h->G.m * h->G.n;
-    FDM_CK(h, h->amr[22].ensure((nroots + 1) * 4));
-    k_root_first<<<nblk(A.n + 1, 256), 256, 0, h->s>>>(A.n, A.key, nroots, h->amr[22].as<int32_t>());
-    A.rf = h->amr[22].as<int32_t>();
-    A.nroots = nroots;
-    return FDM_OK;
-}
-
-
 // exclusive scan of n counts and their total; *at_val: the prefix at index
-// at (0 <= at < n), read back in the same round trip
+// at (0 <= at < n), read back in the same round trip (through pinned memory:
+// a copy to pageable memory is a round trip of its own).  Copies that the
+// caller queued before land with it.
 static int scan_total32(fdm_handle *h, const int32_t *in, int32_t *out, int64_t n, int64_t &total,
                         int64_t at = -1, int64_t *at_val = nullptr) {
     size_t bytes = 0;
     FDM_CK(h, cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, (int)n, h->s));
     FDM_CK(h, h->cub_tmp.ensure(bytes));
     FDM_CK(h, cub::DeviceScan::ExclusiveSum(h->cub_tmp.p, bytes, in, out, (int)n, h->s));
-    int32_t a = 0, b = 0, c = 0;
-    FDM_CK(h, cudaMemcpyAsync(&a, in + n - 1, 4, cudaMemcpyDeviceToHost, h->s));
-    FDM_CK(h, cudaMemcpyAsync(&b, out + n - 1, 4, cudaMemcpyDeviceToHost, h->s));
-    if (at_val && at >= 0 && at < n) FDM_CK(h, cudaMemcpyAsync(&c, out + at, 4, cudaMemcpyDeviceToHost, h->s));
+    int32_t *r = h->pin_scan();
+    FDM_CK(h, cudaMemcpyAsync(r, in + n - 1, 4, cudaMemcpyDeviceToHost, h->s));
+    FDM_CK(h, cudaMemcpyAsync(r + 1, out + n - 1, 4, cudaMemcpyDeviceToHost, h->s));
+    if (at_val && at >= 0 && at < n) FDM_CK(h, cudaMemcpyAsync(r + 2, out + at, 4, cudaMemcpyDeviceToHost, h->s));
     FDM_CK(h, cudaStreamSynchronize(h->s));
-    total = (int64_t)a + b;
-    if (at_val) *at_val = at >= n ? total : (int64_t)c;
-    return FDM_OK;
-}
-
-// exclusive scan without reading the total back
-static int scan_i32_only(fdm_handle *h, const int32_t *in, int32_t *out, int64_t n) {
-    size_t bytes = 0;
-    FDM_CK(h, cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, (int)n, h->s));
-    FDM_CK(h, h->cub_tmp.ensure(bytes));
-    FDM_CK(h, cub::DeviceScan::ExclusiveSum(h->cub_tmp.p, bytes, in, out, (int)n, h->s));
+    total = (int64_t)r[0] + r[1];
+    if (at_val) *at_val = at >= n ? total : (int64_t)r[2];
     return FDM_OK;
 }
 
@@ -411,10 +395,10 @@ int init_internal(fdm_handle *h) {
     cv.add(NL * 4); cv.add(NL * 4); cv.add(4);
     FDM_CK(h, h->amr[8].ensure(cv.total));
     int32_t *cnt = cv.at<int32_t>(h->amr[8], 0), *off = cv.at<int32_t>(h->amr[8], 1);
-    int32_t *dl = cv.at<int32_t>(h->amr[8], 2), deepest = 0;   // deepest leaf
+    int32_t *dl = cv.at<int32_t>(h->amr[8], 2), *deepest = h->pin;   // deepest leaf
     FDM_CK(h, cudaMemsetAsync(dl, 0, 4, h->s));
     k_anc_count<<<nblk(NL, TB), TB, 0, h->s>>>(NL, h->lkey.as<uint64_t>(), cnt, dl);
-    FDM_CK(h, cudaMemcpyAsync(&deepest, dl, 4, cudaMemcpyDeviceToHost, h->s));
+    FDM_CK(h, cudaMemcpyAsync(deepest, dl, 4, cudaMemcpyDeviceToHost, h->s));
     int64_t ni = 0;
     int rc = scan_total32(h, cnt, off, NL, ni);   // waits
     if (rc) return rc;
@@ -423,7 +407,7 @@ int init_internal(fdm_handle *h) {
     FDM_CK(h, h->ikey.ensure(ni * 8));
     k_anc_emit<<<nblk(NL, TB), TB, 0, h->s>>>(NL, h->lkey.as<uint64_t>(), off, h->ikey.as<uint64_t>());
     FDM_CK(h, h->ival.ensure(ni * 32 + 32));
-    for (int l = deepest - 1; l >= 0; --l)
+    for (int l = *deepest - 1; l >= 0; --l)
         k_internal_vals<<<nblk(ni, TB), TB, 0, h->s>>>(ni, h->ikey.as<uint64_t>(), h->ival.as<double4>(), l,
                                                       h->tables(), h->B[0].as<double4>());
     FDM_CK(h, cudaGetLastError());
@@ -528,12 +512,12 @@ struct Links {
     uint8_t *leaf0;
     int8_t *cross;
 };
-__global__ void k_gm1_links(NodeSet A, Geometry G, Links L, int32_t *max_lvl) {
+__global__ void k_gm1_links(NodeSet A, Geometry G, Links L, int8_t *d) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= A.n) return;
+    d[i] = D_NONE;
     const uint64_t k = A.key[i];
     const int lvl = (int)(k & 15u);
-    if (!A.leaf[i]) atomicMax(max_lvl, lvl);   // the deepest internal node
     L.parent[i] = lvl > 0 ? (int32_t)find_key_set(A, parent_key(k)) : -1;
     L.leaf0[i] = A.leaf[i];
     L.cross[i] = (int8_t)root_cross(G, (int64_t)(k >> 34));
@@ -561,10 +545,12 @@ __device__ __forceinline__ bool gm1_has_son(const Links &L, const int8_t *d, int
 // updated in the same sweep (never older than the last sweep's), which only
 // shortens the chains; a sweep that changes nothing wrote nothing, so every
 // decision in it read final values and the fixpoint (unique: the
-// dependencies follow the visit order) is reached.
-__global__ void k_gm1_decide(int64_t n, Links L, int8_t *d, int32_t *changed, int32_t *any) {
+// dependencies follow the visit order) is reached.  changed: one word per
+// sweep; a sweep after one that changed nothing has nothing to do, so several
+// are queued without a look from the host.
+__global__ void k_gm1_decide(int64_t n, Links L, int8_t *d, int32_t *changed, int sweep) {
     const int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (x >= n) return;
+    if (x >= n || (sweep > 0 && changed[sweep - 1] == 0)) return;
     int8_t r = D_NONE;
     if (L.cross[x] == 0) {
         const uint64_t rx = L.rank[x];
@@ -586,9 +572,8 @@ __global__ void k_gm1_decide(int64_t n, Links L, int8_t *d, int32_t *changed, in
     }
     if (r != d[x]) {
         d[x] = r;
-        atomicExch(changed, 1);
+        changed[sweep] = 1;
     }
-    if (any && r != D_NONE) atomicExch(any, 1);
 }
 // values of coarsened nodes, deepest level first (interpA of the sons as they
 // are at the node's visit)
@@ -603,30 +588,48 @@ __device__ __forceinline__ bool ancestor_coarsened(const Links &L, const int8_t 
         if (d[a] == D_COARSEN) return true;
     return false;
 }
-__global__ void k_gm1_count(int64_t n, Links L, const int8_t *d, int32_t *cnt) {
+// did[0]: a node is refined or coarsened; did[1]: the longest chain of
+// coarsened nodes, each the father of the next; did[2]: their deepest level
+__global__ void k_gm1_count(NodeSet A, Links L, const int8_t *d, int32_t *cnt, int32_t *did) {
     const int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (x >= n) return;
-    cnt[x] = ancestor_coarsened(L, d, (int32_t)x) ? 0 : (d[x] == D_REFINE ? 5 : 1);
+    if (x >= A.n) return;
+    const int8_t dx = d[x];
+    cnt[x] = ancestor_coarsened(L, d, (int32_t)x) ? 0 : (dx == D_REFINE ? 5 : 1);
+    if (dx == D_NONE) return;
+    did[0] = 1;
+    if (dx != D_COARSEN) return;
+    int chain = 1;
+    for (int32_t a = L.parent[x]; a >= 0 && d[a] == D_COARSEN; a = L.parent[a]) ++chain;
+    const int lvl = (int)(A.key[x] & 15u);
+    if (did[1] < chain) atomicMax(did + 1, chain);
+    if (did[2] < lvl) atomicMax(did + 2, lvl);
 }
-__global__ void k_gm1_emit(NodeSet A, Links L, const int8_t *d, const int32_t *off, NodeSet out) {
-    uint64_t *okey = out.key;
-    uint8_t *oleaf = out.leaf;
-    double4 *oval = out.val;
+// mean: a coarsened node's value is formed here from its sons' (no chain of
+// coarsened nodes); otherwise k_gm1_vals has formed it
+__global__ void k_gm1_emit(NodeSet A, Links L, const int8_t *d, const int32_t *off, NodeSet out, bool mean) {
     const int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (x == 0) index_end(out);
     if (x >= A.n || ancestor_coarsened(L, d, (int32_t)x)) return;
     const int64_t o = off[x];
     const uint64_t k = A.key[x];
-    const double4 v = A.val[x];
-    okey[o] = k;
-    oval[o] = v;
-    if (d[x] == D_REFINE) {
-        oleaf[o] = 0;
-        for (int q = 0; q < 4; ++q) { okey[o + 1 + q] = child_key(k, q); oleaf[o + 1 + q] = 1; oval[o + 1 + q] = v; }
-    } else if (d[x] == D_COARSEN) {
-        oleaf[o] = 1;
+    const int8_t dx = d[x];
+    double4 v;
+    if (mean && dx == D_COARSEN) {
+        const int32_t *c = L.child + 4 * x;
+        v = mean4(A.val[c[0]], A.val[c[1]], A.val[c[2]], A.val[c[3]]);
     } else {
-        oleaf[o] = A.leaf[x];
+        v = A.val[x];
     }
+    out.key[o] = k;
+    out.val[o] = v;
+    out.leaf[o] = dx == D_REFINE ? 0 : dx == D_COARSEN ? 1 : A.leaf[x];
+    index_node(out, k, o);
+    if (dx == D_REFINE)
+        for (int q = 0; q < 4; ++q) {
+            out.key[o + 1 + q] = child_key(k, q);
+            out.leaf[o + 1 + q] = 1;
+            out.val[o + 1 + q] = v;
+        }
 }
 
 // ----------------------------------------------------------- gridmodify4
@@ -959,6 +962,7 @@ __device__ __forceinline__ int gm4_nodes(const NodeSet &A, const Gm4 &M, const G
     int n = 0;
     const auto put = [&](uint64_t k, bool leaf) {
         if (WRITE) {
+            index_node(out, k, o + n);
             out.key[o + n] = k;
             out.leaf[o + n] = leaf ? 1 : 0;
             out.val[o + n] = v;
@@ -998,20 +1002,22 @@ __global__ void k_gm4_count(NodeSet A, Gm4 M, const Gm4Result *res, int32_t *cnt
 }
 __global__ void k_gm4_emit(NodeSet A, Gm4 M, const Gm4Result *res, const int32_t *off, NodeSet out) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i == 0) index_end(out);
     if (i < A.n) gm4_nodes<true>(A, M, res, i, off[i], out);
 }
 
 // ------------------------------------------------------------ extraction
-__global__ void k_split_count(int64_t n, const uint8_t *leaf, int32_t *fl, int32_t *fi) {
+__global__ void k_split_count(int64_t n, const uint8_t *leaf, int32_t *fl) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i < n) { fl[i] = leaf[i] ? 1 : 0; fi[i] = leaf[i] ? 0 : 1; }
+    if (i < n) fl[i] = leaf[i] ? 1 : 0;
 }
-__global__ void k_split_emit(NodeSet A, const int32_t *ol, const int32_t *oi, uint64_t *lk, double4 *lv, uint64_t *ik,
-                             double4 *iv) {
+// ol: leaves before each node; the internal nodes before it are the others
+__global__ void k_split_emit(NodeSet A, const int32_t *ol, uint64_t *lk, double4 *lv, uint64_t *ik, double4 *iv) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= A.n) return;
-    if (A.leaf[i]) { lk[ol[i]] = A.key[i]; lv[ol[i]] = A.val[i]; }
-    else { ik[oi[i]] = A.key[i]; iv[oi[i]] = A.val[i]; }
+    const int64_t l = ol[i];
+    if (A.leaf[i]) { lk[l] = A.key[i]; lv[l] = A.val[i]; }
+    else { ik[i - l] = A.key[i]; iv[i - l] = A.val[i]; }
 }
 
 // emission helper: count kernel already ran into cnt; scan; emit kernel fills
@@ -1037,65 +1043,52 @@ static int emit_buffers(fdm_handle *h, int64_t n, Emit &E) {
         if (rc_) return rc_; \
     } while (0)
 
-// one gridmodify1 pass over the node set A -> A
 // One gridmodify1 pass over the node set A -> A; *did: a node was refined
 // or coarsened (otherwise A is left as it is).
 static int gridmodify1_pass(fdm_handle *h, AmrCtx &X, bool *did) {
     Nvtx range("fdm regrid: gridmodify1");
     const int TB = 256;
     const int64_t n = X.A.n;
+    // Sweeps are queued GM1_SWEEPS at a time (2 to 6 settle a pass); the
+    // counts that follow are taken as settled, and taken again when the
+    // changes of the last sweep say otherwise.
+    constexpr int GM1_SWEEPS = 6;
     Carve cv;
     cv.add(n * 4); cv.add(n * 16); cv.add(n * 16); cv.add(n * 8); cv.add(n); cv.add(n);
-    cv.add(n); cv.add(n); cv.add(16); cv.add(n * 4); cv.add(n * 4);
+    cv.add(n); cv.add((GM1_SWEEPS + 3) * 4); cv.add(n * 4); cv.add(n * 4);
     FDM_CK(h, h->amr[14].ensure(cv.total));
     DevBuf &b = h->amr[14];
     Links L;
     L.parent = cv.at<int32_t>(b, 0); L.child = cv.at<int32_t>(b, 1); L.nb = cv.at<int32_t>(b, 2);
     L.rank = cv.at<uint64_t>(b, 3); L.leaf0 = cv.at<uint8_t>(b, 4); L.cross = cv.at<int8_t>(b, 5);
-    int8_t *d0 = cv.at<int8_t>(b, 6);   // the decisions (slot 7 unused)
-    int32_t *changed = cv.at<int32_t>(b, 8);
-    int32_t *cnt = cv.at<int32_t>(b, 9), *off = cv.at<int32_t>(b, 10);
-    AMR_RC(index_set(h, X.A));
-    FDM_CK(h, cudaMemsetAsync(changed, 0, 16, h->s));
-    k_gm1_links<<<nblk(n, TB), TB, 0, h->s>>>(X.A, h->G, L, changed + 2);
-    FDM_CK(h, cudaMemsetAsync(d0, 0, n, h->s));
-    int8_t *cur = d0;
-    // Sweeps are enqueued GM1_SWEEPS at a time and the change flag of the
-    // last one is read: once the decisions are settled a sweep changes
-    // nothing, so the extra sweeps leave the fixpoint as it is.
-    constexpr int GM1_SWEEPS = 4;
-    int64_t it = 0;
-    int deepest = MAXLVL_TAB - 2;   // a coarsened node is internal: no deeper than the deepest internal node
-    for (;;) {
-        if (it > n + 2 + GM1_SWEEPS) { h->err = "gridmodify1 decisions did not settle"; return FDM_ERR_UNSUPPORTED; }
-        int32_t hc[3] = {0, 0, 0};   // last sweep: changed, any decision; deepest internal node
-        for (int k = 0; k < GM1_SWEEPS; ++k) {
-            const bool last = k == GM1_SWEEPS - 1;
-            if (last) FDM_CK(h, cudaMemsetAsync(changed, 0, 8, h->s));   // the level stays
-            k_gm1_decide<<<nblk(n, TB), TB, 0, h->s>>>(n, L, cur, changed, last ? changed + 1 : nullptr);
-        }
-        it += GM1_SWEEPS;
-        FDM_CK(h, cudaMemcpyAsync(hc, changed, 12, cudaMemcpyDeviceToHost, h->s));
-        FDM_CK(h, cudaStreamSynchronize(h->s));
-        if (!hc[0]) {
-            *did = hc[1] != 0;
-            deepest = hc[2];
-            break;
-        }
-    }
-    h->gm1_iters += it;
-    if (!*did) return FDM_OK;   // every decision is "nothing": A stays
-    for (int l = deepest < MAXLVL_TAB - 2 ? deepest : MAXLVL_TAB - 2; l >= 0; --l)
-        k_gm1_vals<<<nblk(n, TB), TB, 0, h->s>>>(X.A, L, cur, l);
-    k_gm1_count<<<nblk(n, TB), TB, 0, h->s>>>(n, L, cur, cnt);
+    int8_t *d = cv.at<int8_t>(b, 6);        // the decisions
+    int32_t *changed = cv.at<int32_t>(b, 7), *ddid = changed + GM1_SWEEPS;
+    int32_t *cnt = cv.at<int32_t>(b, 8), *off = cv.at<int32_t>(b, 9);
+    k_gm1_links<<<nblk(n, TB), TB, 0, h->s>>>(X.A, h->G, L, d);
+    const int32_t *r = h->pin;              // changed words, then did words
     int64_t total = 0;
-    AMR_RC(scan_total32(h, cnt, off, n, total));
+    for (int64_t it = 0;; it += GM1_SWEEPS) {
+        if (it > n + 2 + GM1_SWEEPS) { h->err = "gridmodify1 decisions did not settle"; return FDM_ERR_UNSUPPORTED; }
+        FDM_CK(h, cudaMemsetAsync(changed, 0, (GM1_SWEEPS + 3) * 4, h->s));
+        for (int k = 0; k < GM1_SWEEPS; ++k)
+            k_gm1_decide<<<nblk(n, TB), TB, 0, h->s>>>(n, L, d, changed, k);
+        k_gm1_count<<<nblk(n, TB), TB, 0, h->s>>>(X.A, L, d, cnt, ddid);
+        FDM_CK(h, cudaMemcpyAsync(h->pin, changed, (GM1_SWEEPS + 3) * 4, cudaMemcpyDeviceToHost, h->s));
+        AMR_RC(scan_total32(h, cnt, off, n, total));   // waits
+        for (int k = 0; k < GM1_SWEEPS; ++k) h->gm1_iters += k == 0 || r[k - 1] != 0;
+        if (r[GM1_SWEEPS - 1] == 0) break;
+    }
+    *did = r[GM1_SWEEPS] != 0;
+    if (!*did) return FDM_OK;   // every decision is "nothing": A stays
+    const int chain = r[GM1_SWEEPS + 1];
+    if (chain > 1)              // sons first
+        for (int l = r[GM1_SWEEPS + 2]; l >= 0; --l)
+            k_gm1_vals<<<nblk(n, TB), TB, 0, h->s>>>(X.A, L, d, l);
     // the emit keeps key order: a refined leaf's sons follow it directly and
     // lie before every later node (they fill the leaf's own span)
     AMR_RC(grow_next(h, X, total));
-    k_gm1_emit<<<nblk(n, TB), TB, 0, h->s>>>(X.A, L, cur, off, X.B);
-    X.B.n = total;
-    swap_sets(h, X);
+    k_gm1_emit<<<nblk(n, TB), TB, 0, h->s>>>(X.A, L, d, off, X.B, chain <= 1);
+    swap_sets(X);
     return FDM_OK;
 }
 
@@ -1126,7 +1119,6 @@ static int gridmodify4_pass(fdm_handle *h, AmrCtx &X, bool *did) {
         Gm4Result *res = c.at<Gm4Result>(b, 9);
         int32_t *cnt = c.at<int32_t>(b, 10), *off = c.at<int32_t>(b, 11);
         M.cap = cap;
-        AMR_RC(index_set(h, X.A));
         FDM_CK(h, cudaMemsetAsync(M.t, 0xff, c.off[4], h->s));
         FDM_CK(h, cudaMemsetAsync(M.w, 0, GW_WORDS * 4, h->s));
         k_gm4_triggers<<<nblk(4 * n, TB), TB, 0, h->s>>>(X.A, h->G, t0, list, M.w + GW_NLIST);
@@ -1134,7 +1126,8 @@ static int gridmodify4_pass(fdm_handle *h, AmrCtx &X, bool *did) {
         k_gm4_fixpoint<<<GM4_CTAS, GM4_THREADS, 0, h->s>>>(X.A, h->G, M, t0, 1 << 16, res);
         FDM_CK(h, cudaEventRecord(h->gm4_ev[1], h->s));
         k_gm4_count<<<nblk(n, TB), TB, 0, h->s>>>(X.A, M, res, cnt);
-        Gm4Result hr;
+        Gm4Result &hr = *reinterpret_cast<Gm4Result *>(h->pin);
+        static_assert(sizeof(Gm4Result) <= fdm_handle::PIN_WORDS * 4, "the result must fit the pinned words");
         FDM_CK(h, cudaMemcpyAsync(&hr, res, sizeof hr, cudaMemcpyDeviceToHost, h->s));
         int64_t total = 0;
         AMR_RC(scan_total32(h, cnt, off, n, total));   // waits
@@ -1151,8 +1144,7 @@ static int gridmodify4_pass(fdm_handle *h, AmrCtx &X, bool *did) {
         *did = true;
         AMR_RC(grow_next(h, X, total));
         k_gm4_emit<<<nblk(n, TB), TB, 0, h->s>>>(X.A, M, res, off, X.B);
-        X.B.n = total;
-        swap_sets(h, X);
+        swap_sets(X);
         if (!hr.w[GW_NONLEAF]) return FDM_OK;
         t0 = hr.nl_time;
     }
@@ -1250,7 +1242,7 @@ static int run_amr_impl(fdm_handle *h, fdm_handle *lead) {
     X.h = h;
     AMR_RC(grow_next(h, X, total));
     merge_into(h, E.key, E.leaf, E.val, split, total, X.B);
-    swap_sets(h, X);
+    swap_sets(X);
     FDM_CK(h, cudaEventRecord(h->amr_ev[2], h->s));
     // 3. solute_gridmodify: lvlAMR rounds (src/solution.F90:537-556)
     // A round that changes nothing leaves the node set as it found it, so
@@ -1265,25 +1257,23 @@ static int run_amr_impl(fdm_handle *h, fdm_handle *lead) {
     // 4. split leaves / internal nodes, rebuild the tables (idneighbor + IDgrid)
     const int64_t n = X.A.n;
     Carve cs;
-    cs.add(n * 4); cs.add(n * 4); cs.add(n * 4); cs.add(n * 4);
+    cs.add(n * 4); cs.add(n * 4);
     FDM_CK(h, h->amr[8].ensure(cs.total));
-    int32_t *fl = cs.at<int32_t>(h->amr[8], 0), *fi = cs.at<int32_t>(h->amr[8], 1);
-    int32_t *ol = cs.at<int32_t>(h->amr[8], 2), *oi = cs.at<int32_t>(h->amr[8], 3);
-    k_split_count<<<nblk(n, TB), TB, 0, h->s>>>(n, X.A.leaf, fl, fi);
-    int64_t nleaf = 0, nint = 0;
-    AMR_RC(scan_i32_only(h, fi, oi, n));
+    int32_t *fl = cs.at<int32_t>(h->amr[8], 0), *ol = cs.at<int32_t>(h->amr[8], 1);
+    k_split_count<<<nblk(n, TB), TB, 0, h->s>>>(n, X.A.leaf, fl);
+    int64_t nleaf = 0;
     AMR_RC(scan_total32(h, fl, ol, n, nleaf));
-    nint = n - nleaf;   // every node is one or the other
-    DevBuf &lk = h->amr[20], &lv = h->amr[21];   // kept between regrids
-    FDM_CK(h, lk.ensure(nleaf * 8 + 8));
+    const int64_t nint = n - nleaf;   // every node is one or the other
+    DevBuf &lv = h->amr[21];   // kept between regrids
+    FDM_CK(h, h->lkey.ensure(nleaf * 8));   // the new leaves' keys, where the tables have them
     FDM_CK(h, lv.ensure(nleaf * 32 + 32));
     FDM_CK(h, h->ikey.ensure(nint * 8 + 8));
     FDM_CK(h, h->ival.ensure(nint * 32 + 32));
-    k_split_emit<<<nblk(n, TB), TB, 0, h->s>>>(X.A, ol, oi, lk.as<uint64_t>(), lv.as<double4>(),
+    k_split_emit<<<nblk(n, TB), TB, 0, h->s>>>(X.A, ol, h->lkey.as<uint64_t>(), lv.as<double4>(),
                                                h->ikey.as<uint64_t>(), h->ival.as<double4>());
     FDM_CK(h, cudaEventRecord(h->amr_ev[4], h->s));
     h->NInt = nint;   // the rebuild is ordered after the split on the stream
-    const int rc = build_tables(h, nleaf, lk.as<uint64_t>(), lv.as<double>(), 0);   // split keeps key order
+    const int rc = build_tables(h, nleaf, h->lkey.as<uint64_t>(), lv.as<double>(), 0);   // split keeps key order
     if (rc) return rc;
     FDM_CK(h, cudaEventRecord(h->amr_ev[5], h->s));
     FDM_CK(h, cudaEventSynchronize(h->amr_ev[5]));

@@ -47,8 +47,9 @@ __device__ __forceinline__ int get_direction(double xx, double yy, double x, dou
 }
 
 // ------------------------------------------------------------ classify
+constexpr unsigned long long LEAF_INTERIOR = 1ull, LEAF_GHOST = 1ull << 32;
 __global__ void k_classify(const uint64_t *__restrict__ lkey, int64_t NL, Geometry G,
-                           int32_t *fI, int32_t *fG, int32_t *fC, int8_t *cross, int32_t *err) {
+                           unsigned long long *kind, int8_t *cross, int32_t *err) {
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= NL) return;
     const int64_t total = (int64_t)G.m * G.n;
@@ -66,36 +67,34 @@ __global__ void k_classify(const uint64_t *__restrict__ lkey, int64_t NL, Geomet
     cross[k] = (int8_t)c;
     // halo leaves of a strip take ghost slots (not advanced, not filled)
     const bool halo = root_in_halo(G, root);
-    fI[k] = c == 0 && !halo;
-    fC[k] = c == -5 && !halo;
-    fG[k] = !fI[k] && !fC[k];
+    // interior leaf in the low word, ghost in the high one: one scan counts both
+    kind[k] = c == 0 && !halo ? LEAF_INTERIOR : c == -5 && !halo ? 0ull : LEAF_GHOST;
 }
 
-__global__ void k_slots(int64_t NL, int64_t NI, int64_t NG, const int32_t *fI, const int32_t *fG,
-                        const int32_t *sI, const int32_t *sG, const int32_t *sC, int32_t *lslot,
-                        int32_t *slot_leaf) {
+// slots (interior leaves, ghosts, corners, each in key order; before: the
+// interior leaves and ghosts before each leaf) and centres
+__global__ void k_slots(int64_t NL, int64_t NI, int64_t NG, const uint64_t *__restrict__ lkey, Geometry G,
+                        const unsigned long long *__restrict__ kind, const unsigned long long *__restrict__ before,
+                        int32_t *lslot, int32_t *slot_leaf, double *cx, double *cy) {
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= NL) return;
-    const int32_t s = fI[k] ? sI[k] : fG[k] ? (int32_t)(NI + sG[k]) : (int32_t)(NI + NG + sC[k]);
+    const unsigned long long c = kind[k], p = before[k];
+    const int64_t bi = (int64_t)(p & 0xffffffffull), bg = (int64_t)(p >> 32);
+    const int32_t s = (int32_t)(c == LEAF_INTERIOR ? bi : c == LEAF_GHOST ? NI + bg : NI + NG + (k - bi - bg));
     lslot[k] = s;
     slot_leaf[s] = (int32_t)k;
+    double x, y;
+    node_center(G, node_of_key(lkey[k]), x, y);
+    cx[k] = x;
+    cy[k] = y;
 }
 
 __global__ void k_scatter(int64_t NL, const int32_t *perm, const int32_t *lslot,
                           const double *__restrict__ prim, double4 *B0) {
     const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (k >= NL) return;
-    const int64_t src = perm[k];
+    const int64_t src = perm ? perm[k] : k;
     B0[lslot[k]] = make_double4(prim[4 * src], prim[4 * src + 1], prim[4 * src + 2], prim[4 * src + 3]);
-}
-
-__global__ void k_centers(int64_t NL, const uint64_t *lkey, Geometry G, double *cx, double *cy) {
-    const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k >= NL) return;
-    double x, y;
-    node_center(G, node_of_key(lkey[k]), x, y);
-    cx[k] = x;
-    cy[k] = y;
 }
 
 // ------------------------------------------------------- stencil resolve
@@ -105,6 +104,7 @@ __global__ void k_centers(int64_t NL, const uint64_t *lkey, Geometry G, double *
 // node, or child_value_weno on a coarser leaf at a target point.
 struct ResolveOut {
     int32_t *slot;    // >= 0 direct slot, -1 request
+    int32_t *flag;    // 1: a request
     int32_t *kind;    // 0 parent, 1 child
     int64_t *ref;     // parent: node key; child: sorted leaf index
     double *tx, *ty;  // target point
@@ -129,7 +129,8 @@ __device__ __forceinline__ void target_point(const Geometry &G, double cx, doubl
     }
 }
 
-__global__ void k_resolve(Tables T, Geometry G, ResolveOut O, uint8_t *ilvl, int32_t *err) {
+// l_max: the deepest interior level
+__global__ void k_resolve(Tables T, Geometry G, ResolveOut O, uint8_t *ilvl, int32_t *err, int32_t *l_max) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= T.NI) return;
     const int32_t k = T.slot_leaf[i];
@@ -138,6 +139,7 @@ __global__ void k_resolve(Tables T, Geometry G, ResolveOut O, uint8_t *ilvl, int
     c.leaf = k;
     c.valid = 1;
     ilvl[i] = (uint8_t)c.n.lvl;
+    if (*l_max < c.n.lvl) atomicMax(l_max, c.n.lvl);
     const double cx = T.lcx[k], cy = T.lcy[k];
     const int dirs[4] = {DIR_RIGHT, DIR_LEFT, DIR_UP, DIR_DOWN};
     for (int q = 0; q < 4; ++q) {
@@ -169,13 +171,9 @@ __global__ void k_resolve(Tables T, Geometry G, ResolveOut O, uint8_t *ilvl, int
             O.slot[e] = -1; O.kind[e] = 1; O.ref[e] = cn.leaf;
             target_point(G, cx, cy, c.n.lvl, d, 2, O.tx[e], O.ty[e]);
         }
+        O.flag[i * 8 + q] = O.slot[i * 8 + q] < 0;
+        O.flag[e] = O.slot[e] < 0;
     }
-}
-
-__global__ void k_req_flags(int64_t n, const int32_t *slot, int32_t *flag) {
-    const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (e >= n) return;
-    flag[e] = slot[e] < 0;
 }
 
 struct ReqDesc {
@@ -611,7 +609,7 @@ __global__ void k_ghosts(Tables T, Geometry G, fdm_params P, GhostOut O) {
 // face is the right face of the left neighbour j when j is an interior
 // same-level leaf whose 4-point face stencil is slot-for-slot the same;
 // otherwise the leaf owns a separate left face.
-__global__ void k_face_flags(Tables T, int32_t *ux, int32_t *uy) {
+__global__ void k_face_flags(Tables T, unsigned long long *u) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= T.NI) return;
     const int32_t *s = T.ist + i * 8;
@@ -621,38 +619,37 @@ __global__ void k_face_flags(Tables T, int32_t *ux, int32_t *uy) {
         const int32_t *t = T.ist + (int64_t)j * 8;
         shared = (t[1] == s[5]) && (t[0] == (int32_t)i) && (t[4] == s[0]);
     }
-    ux[i] = !shared;
     int shy = 0;
     const int32_t jy = s[3];
     if (jy >= 0 && jy < T.NI) {
         const int32_t *t = T.ist + (int64_t)jy * 8;
         shy = (t[3] == s[7]) && (t[2] == (int32_t)i) && (t[6] == s[2]);
     }
-    uy[i] = !shy;
+    // separate x face in the low word, y face in the high one: one scan for both
+    u[i] = (shared ? 0ull : 1ull) | (shy ? 0ull : 1ull << 32);
 }
-__global__ void k_face_assign(Tables T, const int32_t *ux, const int32_t *uy, const int32_t *sx,
-                              const int32_t *sy, int32_t *ifxl, int32_t *ifyl, int32_t *uxl, int32_t *uyl) {
+__global__ void k_face_assign(Tables T, const unsigned long long *__restrict__ u,
+                              const unsigned long long *__restrict__ before, int32_t *ifxl, int32_t *ifyl,
+                              int32_t *uxl, int32_t *uyl) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= T.NI) return;
     const int32_t *s = T.ist + i * 8;
-    if (ux[i]) { ifxl[i] = (int32_t)(T.NI + sx[i]); uxl[sx[i]] = (int32_t)i; }
+    const unsigned long long v = u[i], p = before[i];
+    const int32_t px = (int32_t)(p & 0xffffffffull), py = (int32_t)(p >> 32);
+    if (v & 1ull) { ifxl[i] = (int32_t)(T.NI + px); uxl[px] = (int32_t)i; }
     else ifxl[i] = s[1];
-    if (uy[i]) { ifyl[i] = (int32_t)(T.NI + sy[i]); uyl[sy[i]] = (int32_t)i; }
+    if (v >> 32) { ifyl[i] = (int32_t)(T.NI + py); uyl[py] = (int32_t)i; }
     else ifyl[i] = s[3];
-}
-
-__global__ void k_lmax(int64_t NI, const uint8_t *ilvl, int32_t *out) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    int v = i < NI ? (int)ilvl[i] : 0;
-    for (int o = 16; o; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(out, v);
 }
 
 // Every index a stage kernel will dereference is checked once here, so that
 // no stage kernel can read or write outside its buffers.
 // face_counts: the unshared left faces (nux, nuy) as the device counted them
-__global__ void k_validate(Tables T, const int64_t *__restrict__ face_counts, int32_t *err) {
+// (words of a packed total); l_max goes to the time loop's scalars.
+__global__ void k_validate(Tables T, const int32_t *__restrict__ face_counts, int32_t *err, const int32_t *l_max,
+                           DevScalars *sc) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (t == 0) sc->l_max = *l_max;
     T.nux = face_counts[0];
     T.nuy = face_counts[1];
     const int64_t NLEAF = T.NI + T.NG + T.NC;
@@ -698,17 +695,19 @@ __global__ void k_validate(Tables T, const int64_t *__restrict__ face_counts, in
 }
 
 // ------------------------------------------------------------ host side
-static int scan_i32(fdm_handle *h, const int32_t *in, int32_t *out, int64_t n) {
+// exclusive scan and its total, written on the device
+template <class U>
+static __global__ void k_scan_total(const U *__restrict__ in, const U *__restrict__ scan, int64_t n, U *out) {
+    if (threadIdx.x == 0) *out = n > 0 ? in[n - 1] + scan[n - 1] : U(0);
+}
+template <class U>
+static int scan_total(fdm_handle *h, const U *in, U *out, int64_t n, U *total) {
     size_t bytes = 0;
     FDM_CK(h, cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, (int)n, h->s));
     FDM_CK(h, h->cub_tmp.ensure(bytes));
     FDM_CK(h, cub::DeviceScan::ExclusiveSum(h->cub_tmp.p, bytes, in, out, (int)n, h->s));
+    k_scan_total<U><<<1, 32, 0, h->s>>>(in, out, n, total);
     return FDM_OK;
-}
-// totals of exclusive scans, written on the device (read back later in one copy)
-static __global__ void k_scan_total(const int32_t *__restrict__ flags, const int32_t *__restrict__ scan, int64_t n,
-                             int64_t *out) {
-    if (threadIdx.x == 0) *out = n > 0 ? (int64_t)flags[n - 1] + scan[n - 1] : 0;
 }
 static __global__ void k_iota_b(int64_t n, int32_t *a) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -728,14 +727,20 @@ __global__ void k_root_first(int64_t n, const uint64_t *__restrict__ lkey, int64
     const int64_t cur = i == n ? nroots : root(i);
     for (int64_t x = prev + 1; x <= cur; ++x) rf[x] = (int32_t)i;
 }
-static __global__ void k_set_lmax(const int32_t *lmax, DevScalars *sc) {
-    if (threadIdx.x == 0) sc->l_max = *lmax;
-}
-// the error flags and up to 6 totals in one read-back
-static int read_back(fdm_handle *h, int32_t he[8], int64_t *tot, int nt) {
-    FDM_CK(h, cudaMemcpyAsync(he, h->flag.p, 8 * sizeof(int32_t), cudaMemcpyDeviceToHost, h->s));
-    if (nt > 0) FDM_CK(h, cudaMemcpyAsync(tot, h->tmp[7].p, nt * sizeof(int64_t), cudaMemcpyDeviceToHost, h->s));
+// What the build counts on the device, in one block that is zeroed at the
+// start and read back whole (through pinned memory) at each wait.
+struct BuildWords {
+    int32_t err[8];                // BuildErr flags
+    int32_t l_max, nr;             // deepest interior level, requests
+    unsigned long long leaves;     // interior leaves | ghosts << 32
+    int32_t faces[2];              // separate left faces, bottom faces
+    unsigned long long counts[8];  // [0] singular, [2] restrict requests, [4] restrict ghosts, [6] listed requests
+};
+static_assert(sizeof(BuildWords) <= fdm_handle::PIN_WORDS * 4, "the build's words must fit the pinned ones");
+static int read_back(fdm_handle *h, const BuildWords *&w) {
+    FDM_CK(h, cudaMemcpyAsync(h->pin, h->tmp[7].p, sizeof(BuildWords), cudaMemcpyDeviceToHost, h->s));
     FDM_CK(h, cudaStreamSynchronize(h->s));
+    w = reinterpret_cast<const BuildWords *>(h->pin);
     return FDM_OK;
 }
 
@@ -771,31 +776,32 @@ int build_tables(fdm_handle *h, int64_t n, const uint64_t *keys_in, const double
     cudaStream_t s = h->s;
     if (n <= 0 || n >= (1ll << 31) - 1) return arg_fail(h, "leaf count out of range");
     h->NL = n;
-    int32_t *err = h->flag.as<int32_t>();
-    FDM_CK(h, cudaMemsetAsync(err, 0, 8 * sizeof(int32_t), s));
+    FDM_CK(h, h->tmp[7].ensure(sizeof(BuildWords)));
+    FDM_CK(h, cudaMemsetAsync(h->tmp[7].p, 0, sizeof(BuildWords), s));
+    FDM_CK(h, cudaMemsetAsync(h->flag.p, 0, 8 * sizeof(int32_t), s));   // a halo copy's slot error ends with its tables
+    BuildWords *dw = h->tmp[7].as<BuildWords>();   // device
+    const BuildWords *w = nullptr;                 // read back
+    int32_t *err = dw->err;
     // 1. sort keys, carrying the input index
     FDM_CK(h, h->lkey.ensure(n * 8));
-    FDM_CK(h, h->tmp[0].ensure(n * 4));   // iota
-    FDM_CK(h, h->tmp[1].ensure(n * 4));   // perm
-    FDM_CK(h, h->tmp[7].ensure(6 * sizeof(int64_t)));
-    int64_t *dtot = h->tmp[7].as<int64_t>();
-    {
-        int32_t *iota = h->tmp[0].as<int32_t>();
-        if (key_bits <= 0) {
-            k_iota_b<<<nblk(n, TB), TB, 0, s>>>(n, h->tmp[1].as<int32_t>());
+    const int32_t *perm = nullptr;
+    if (key_bits <= 0) {
+        if (keys_in != h->lkey.as<uint64_t>())
             FDM_CK(h, cudaMemcpyAsync(h->lkey.as<uint64_t>(), keys_in, n * 8, cudaMemcpyDeviceToDevice, s));
-        } else {
-            k_iota_b<<<nblk(n, TB), TB, 0, s>>>(n, iota);
-            size_t bytes = 0;
-            FDM_CK(h, cub::DeviceRadixSort::SortPairs(nullptr, bytes, keys_in, h->lkey.as<uint64_t>(), iota,
-                                                      h->tmp[1].as<int32_t>(), (int)n, 0, key_bits, s));
-            FDM_CK(h, h->cub_tmp.ensure(bytes));
-            FDM_CK(h, cub::DeviceRadixSort::SortPairs(h->cub_tmp.p, bytes, keys_in, h->lkey.as<uint64_t>(), iota,
-                                                      h->tmp[1].as<int32_t>(), (int)n, 0, key_bits, s));
-        }
+    } else {
+        FDM_CK(h, h->tmp[0].ensure(n * 4));   // iota
+        FDM_CK(h, h->tmp[1].ensure(n * 4));   // perm
+        int32_t *iota = h->tmp[0].as<int32_t>();
+        k_iota_b<<<nblk(n, TB), TB, 0, s>>>(n, iota);
+        size_t bytes = 0;
+        FDM_CK(h, cub::DeviceRadixSort::SortPairs(nullptr, bytes, keys_in, h->lkey.as<uint64_t>(), iota,
+                                                  h->tmp[1].as<int32_t>(), (int)n, 0, key_bits, s));
+        FDM_CK(h, h->cub_tmp.ensure(bytes));
+        FDM_CK(h, cub::DeviceRadixSort::SortPairs(h->cub_tmp.p, bytes, keys_in, h->lkey.as<uint64_t>(), iota,
+                                                  h->tmp[1].as<int32_t>(), (int)n, 0, key_bits, s));
+        perm = h->tmp[1].as<int32_t>();
     }
     const uint64_t *lkey = h->lkey.as<uint64_t>();
-    const int32_t *perm = h->tmp[1].as<int32_t>();
     {
         const int64_t nroots = (int64_t)h->G.m * h->G.n;
         FDM_CK(h, h->rfirst.ensure((nroots + 1) * 4));
@@ -803,37 +809,26 @@ int build_tables(fdm_handle *h, int64_t n, const uint64_t *keys_in, const double
     }
     // 2. classify + partition check
     Carve c2;
-    for (int q = 0; q < 6; ++q) c2.add(n * 4);
+    c2.add(n * 8); c2.add(n * 8);
     FDM_CK(h, h->tmp[2].ensure(c2.total));
-    int32_t *fI = c2.at<int32_t>(h->tmp[2], 0), *fG = c2.at<int32_t>(h->tmp[2], 1), *fC = c2.at<int32_t>(h->tmp[2], 2);
-    int32_t *sI = c2.at<int32_t>(h->tmp[2], 3), *sG = c2.at<int32_t>(h->tmp[2], 4), *sC = c2.at<int32_t>(h->tmp[2], 5);
+    unsigned long long *lkind = c2.at<unsigned long long>(h->tmp[2], 0), *before = c2.at<unsigned long long>(h->tmp[2], 1);
     FDM_CK(h, h->lcross.ensure(n));
-    k_classify<<<nblk(n, TB), TB, 0, s>>>(lkey, n, h->G, fI, fG, fC, h->lcross.as<int8_t>(), err);
-    FDM_RC(scan_i32(h, fI, sI, n));
-    FDM_RC(scan_i32(h, fG, sG, n));
-    FDM_RC(scan_i32(h, fC, sC, n));
-    int64_t NI, NG, NC;
-    {
-        k_scan_total<<<1, 32, 0, s>>>(fI, sI, n, dtot);
-        k_scan_total<<<1, 32, 0, s>>>(fG, sG, n, dtot + 1);
-        k_scan_total<<<1, 32, 0, s>>>(fC, sC, n, dtot + 2);
-        int32_t he[8];
-        int64_t tot[3];
-        FDM_RC(read_back(h, he, tot, 3));
-        NI = tot[0]; NG = tot[1]; NC = tot[2];
-        if (he[BE_ROOT]) return arg_fail(h, "leaf key names a background cell outside the m x n grid");
-        if (he[BE_PARTITION]) return arg_fail(h, "leaf set does not partition the background grid (gap, overlap or duplicate)");
-        if (he[BE_LEVEL]) return arg_fail(h, "leaf level above the supported maximum (14)");
-    }
+    k_classify<<<nblk(n, TB), TB, 0, s>>>(lkey, n, h->G, lkind, h->lcross.as<int8_t>(), err);
+    FDM_RC(scan_total<unsigned long long>(h, lkind, before, n, &dw->leaves));
+    FDM_RC(read_back(h, w));
+    if (w->err[BE_ROOT]) return arg_fail(h, "leaf key names a background cell outside the m x n grid");
+    if (w->err[BE_PARTITION]) return arg_fail(h, "leaf set does not partition the background grid (gap, overlap or duplicate)");
+    if (w->err[BE_LEVEL]) return arg_fail(h, "leaf level above the supported maximum (14)");
+    const int64_t NI = (int64_t)(w->leaves & 0xffffffffull), NG = (int64_t)(w->leaves >> 32), NC = n - NI - NG;
     if (NI == 0) return arg_fail(h, "no interior leaves");
     h->NI = NI; h->NG = NG; h->NC = NC;
     // 3. slots, values, centres
     FDM_CK(h, h->lslot.ensure(n * 4));
     FDM_CK(h, h->slot_leaf.ensure(n * 4));
-    k_slots<<<nblk(n, TB), TB, 0, s>>>(n, NI, NG, fI, fG, sI, sG, sC, h->lslot.as<int32_t>(), h->slot_leaf.as<int32_t>());
     FDM_CK(h, h->lcx.ensure(n * 8));
     FDM_CK(h, h->lcy.ensure(n * 8));
-    k_centers<<<nblk(n, TB), TB, 0, s>>>(n, lkey, h->G, h->lcx.as<double>(), h->lcy.as<double>());
+    k_slots<<<nblk(n, TB), TB, 0, s>>>(n, NI, NG, lkey, h->G, lkind, before, h->lslot.as<int32_t>(),
+                                       h->slot_leaf.as<int32_t>(), h->lcx.as<double>(), h->lcy.as<double>());
     // 4. stencil resolution
     const int64_t ne = NI * 8;
     FDM_CK(h, h->ist.ensure(ne * 4));
@@ -847,21 +842,16 @@ int build_tables(fdm_handle *h, int64_t n, const uint64_t *keys_in, const double
     RO.ref = c3.at<int64_t>(h->tmp[3], 2);
     RO.tx = c3.at<double>(h->tmp[3], 3);
     RO.ty = c3.at<double>(h->tmp[3], 4);
-    int32_t *rflag = c3.at<int32_t>(h->tmp[3], 5);
+    RO.flag = c3.at<int32_t>(h->tmp[3], 5);
     int32_t *ridx = c3.at<int32_t>(h->tmp[3], 6);
     {
         Tables T = h->tables();
-        k_resolve<<<nblk(NI, 128), 128, 0, s>>>(T, h->G, RO, h->ilvl.as<uint8_t>(), err);
+        k_resolve<<<nblk(NI, 128), 128, 0, s>>>(T, h->G, RO, h->ilvl.as<uint8_t>(), err, &dw->l_max);
     }
-    k_req_flags<<<nblk(ne, TB), TB, 0, s>>>(ne, RO.slot, rflag);
-    FDM_RC(scan_i32(h, rflag, ridx, ne));
-    int64_t NR;
-    {
-        k_scan_total<<<1, 32, 0, s>>>(rflag, ridx, ne, dtot);
-        int32_t he[8];
-        FDM_RC(read_back(h, he, &NR, 1));
-        if (he[BE_NULLNB]) return arg_fail(h, "an interior leaf has a null stencil neighbour (fewer than 3 ghost layers?)");
-    }
+    FDM_RC(scan_total<int32_t>(h, RO.flag, ridx, ne, &dw->nr));
+    FDM_RC(read_back(h, w));
+    if (w->err[BE_NULLNB]) return arg_fail(h, "an interior leaf has a null stencil neighbour (fewer than 3 ghost layers?)");
+    const int64_t NR = w->nr;
     h->NR = NR;
     h->NS = NI + NG + NC + NR;
     const int64_t VS0 = NI + NG + NC;
@@ -881,9 +871,7 @@ int build_tables(fdm_handle *h, int64_t n, const uint64_t *keys_in, const double
     FDM_CK(h, h->rq_mem.ensure(nrq * WLS_MAXM * 4));
     FDM_CK(h, h->rq_geo.ensure(nrq * RQ_GEO * 8));
     FDM_CK(h, h->rq_node.ensure(nrq * 8));
-    FDM_CK(h, h->tmp[5].ensure(64));
-    unsigned long long *counts = h->tmp[5].as<unsigned long long>();
-    FDM_CK(h, cudaMemsetAsync(counts, 0, 64, s));
+    unsigned long long *counts = dw->counts;
     if (NR > 0) {
         Tables T = h->tables();
         ReqOut O{h->rq_kind.as<int32_t>(), h->rq_m.as<int32_t>(), h->rq_mem.as<int32_t>(),
@@ -910,25 +898,21 @@ int build_tables(fdm_handle *h, int64_t n, const uint64_t *keys_in, const double
         Tables T = h->tables();
         GhostOut O{h->gh_kind.as<int32_t>(), h->gh_a.as<int32_t>(), h->gh_b.as<int32_t>(),
                    h->gh_flip.as<int32_t>(), h->gh_x.as<double>(),  h->gh_y.as<double>(),
-                   h->tmp[5].as<unsigned long long>() + 4};
+                   counts + 4};
         k_ghosts<<<nblk(NG, 128), 128, 0, s>>>(T, h->G, h->p, O);
     }
     // 7. faces
     Carve c6;
-    for (int q = 0; q < 4; ++q) c6.add(NI * 4);
+    c6.add(NI * 8); c6.add(NI * 8);
     FDM_CK(h, h->tmp[6].ensure(c6.total));
-    int32_t *ux = c6.at<int32_t>(h->tmp[6], 0), *uy = c6.at<int32_t>(h->tmp[6], 1);
-    int32_t *sx = c6.at<int32_t>(h->tmp[6], 2), *sy = c6.at<int32_t>(h->tmp[6], 3);
+    unsigned long long *u = c6.at<unsigned long long>(h->tmp[6], 0), *ub = c6.at<unsigned long long>(h->tmp[6], 1);
     {
         Tables T = h->tables();
-        k_face_flags<<<nblk(NI, TB), TB, 0, s>>>(T, ux, uy);
+        k_face_flags<<<nblk(NI, TB), TB, 0, s>>>(T, u);
     }
-    FDM_RC(scan_i32(h, ux, sx, NI));
-    FDM_RC(scan_i32(h, uy, sy, NI));
     // the face counts come back with the final checks; until then the
     // buffers take their bound (at most one unshared left face per leaf)
-    k_scan_total<<<1, 32, 0, s>>>(ux, sx, NI, dtot + 4);
-    k_scan_total<<<1, 32, 0, s>>>(uy, sy, NI, dtot + 5);
+    FDM_RC(scan_total<unsigned long long>(h, u, ub, NI, reinterpret_cast<unsigned long long *>(dw->faces)));
     const int64_t nux_max = NI, nuy_max = NI;
     FDM_CK(h, h->ifxl.ensure(NI * 4));
     FDM_CK(h, h->ifyl.ensure(NI * 4));
@@ -936,7 +920,7 @@ int build_tables(fdm_handle *h, int64_t n, const uint64_t *keys_in, const double
     FDM_CK(h, h->uyl.ensure(nuy_max * 4));
     {
         Tables T = h->tables();
-        k_face_assign<<<nblk(NI, TB), TB, 0, s>>>(T, ux, uy, sx, sy, h->ifxl.as<int32_t>(), h->ifyl.as<int32_t>(),
+        k_face_assign<<<nblk(NI, TB), TB, 0, s>>>(T, u, ub, h->ifxl.as<int32_t>(), h->ifyl.as<int32_t>(),
                                                   h->uxl.as<int32_t>(), h->uyl.as<int32_t>());
     }
     // 8. state buffers (corner values copied into all three)
@@ -956,30 +940,19 @@ int build_tables(fdm_handle *h, int64_t n, const uint64_t *keys_in, const double
         int64_t nv = NI * 8;
         const int64_t others[5] = {nux_max, nuy_max, NR, NG, NI};
         for (int q = 0; q < 5; ++q) nv = nv > others[q] ? nv : others[q];
-        k_validate<<<nblk(nv, TB), TB, 0, s>>>(T, dtot + 4, err);
+        k_validate<<<nblk(nv, TB), TB, 0, s>>>(T, dw->faces, err, &dw->l_max, h->scal.as<DevScalars>());
     }
-    // 10. l_max
-    int32_t *dl = err + 7;
-    FDM_CK(h, cudaMemsetAsync(dl, 0, 4, s));
-    k_lmax<<<nblk(NI, TB), TB, 0, s>>>(NI, h->ilvl.as<uint8_t>(), dl);
-    k_set_lmax<<<1, 32, 0, s>>>(dl, h->scal.as<DevScalars>());
-    int32_t he[8];
-    unsigned long long hc[7];
-    FDM_CK(h, cudaMemcpyAsync(he, err, sizeof(he), cudaMemcpyDeviceToHost, s));
-    FDM_CK(h, cudaMemcpyAsync(hc, counts, sizeof(hc), cudaMemcpyDeviceToHost, s));
-    int64_t fc[2] = {0, 0};
-    FDM_CK(h, cudaMemcpyAsync(fc, dtot + 4, sizeof(fc), cudaMemcpyDeviceToHost, s));
-    FDM_CK(h, cudaStreamSynchronize(s));
+    FDM_RC(read_back(h, w));
     FDM_CK(h, cudaGetLastError());
-    h->nux = fc[0];
-    h->nuy = fc[1];
-    if (hc[2] != hc[6]) return arg_fail(h, "internal table check failed: restrict list");
-    if (he[BE_OVERFLOW]) return arg_fail(h, "hanging-node stencil larger than supported");
-    if (he[BE_INDEX]) return arg_fail(h, "internal table check failed: an index is out of range");
-    h->l_max = he[7];
-    h->n_singular += (int64_t)hc[0];
-    h->n_restrict = (int64_t)hc[2];
-    h->n_ghost_restrict = (int64_t)hc[4];
+    h->nux = w->faces[0];
+    h->nuy = w->faces[1];
+    if (w->counts[2] != w->counts[6]) return arg_fail(h, "internal table check failed: restrict list");
+    if (w->err[BE_OVERFLOW]) return arg_fail(h, "hanging-node stencil larger than supported");
+    if (w->err[BE_INDEX]) return arg_fail(h, "internal table check failed: an index is out of range");
+    h->l_max = w->l_max;
+    h->n_singular += (int64_t)w->counts[0];
+    h->n_restrict = (int64_t)w->counts[2];
+    h->n_ghost_restrict = (int64_t)w->counts[4];
     h->table_version++;
     h->gate_stage1_valid = false;
     h->lam_fresh = false;

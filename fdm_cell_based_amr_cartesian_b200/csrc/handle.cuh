@@ -121,13 +121,18 @@ struct fdm_handle {
     fdm::DevBuf cub_tmp;
     fdm::DevBuf flag;        // device error flags (int32[8])
     fdm::DevScalars *hs = nullptr;   // pinned host mirror of the scalars
+    // pinned words for small read-backs: each is read after the wait that
+    // follows its copy, before the next copy is queued
+    static constexpr int PIN_WORDS = 64;
+    int32_t *pin = nullptr;
+    int32_t *pin_scan() const { return pin + PIN_WORDS; }   // three words of a scan's totals
 
     // internal nodes of the tree and their values (the reference keeps a
     // stale U in every refined node; gridmodify4 can copy it back)
     fdm::DevBuf ikey, ival;
     int64_t NInt = 0;
-    fdm::DevBuf amr[23];     // regrid scratch: [0..5] node sets, [6..19] work arrays, [20, 21] new leaves,
-                             // [22] per-cell index of the node set
+    fdm::DevBuf amr[22];     // regrid scratch: [0..5] node sets, [6, 7] their per-cell indices, [8..19] work
+                             // arrays, [20, 21] new leaves
     int64_t gm1_iters = 0, gm4_visits = 0, gm4_nonleaf = 0, gm4_triggers = 0, gm4_refines = 0, gm4_steps = 0;
     // device-timeline phases of the last regrid (events recorded on the stream)
     static constexpr int AMR_PHASES = 5;

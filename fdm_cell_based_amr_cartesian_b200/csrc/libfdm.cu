@@ -314,6 +314,7 @@ int fdm_create(const fdm_params *p, fdm_handle **out) {
     cudaError_t e = cudaGetDevice(&h->device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->s, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMallocHost((void **)&h->hs, sizeof(DevScalars));
+    if (e == cudaSuccess) e = cudaMallocHost((void **)&h->pin, (fdm_handle::PIN_WORDS + 4) * sizeof(int32_t));
     if (e == cudaSuccess) e = h->scal.ensure(sizeof(DevScalars));
     if (e == cudaSuccess) e = h->flag.ensure(8 * sizeof(int32_t));
     if (e != cudaSuccess) {
@@ -360,6 +361,7 @@ void fdm_destroy(fdm_handle *h) {
             cudaStreamDestroy(cs);
         }
     if (h->hs) cudaFreeHost(h->hs);
+    if (h->pin) cudaFreeHost(h->pin);
     if (h->s) cudaStreamDestroy(h->s);
     delete h;
 }
