@@ -342,7 +342,7 @@ __device__ __forceinline__ void ph_ghost_tile(const BatchArgs &A, int krk, int j
 __device__ __forceinline__ void ph_end_member(const BatchArgs &A, int m, double (*fin)[8]) {
     const Member &M = A.mem[m];
     if (!A.act[m]) return;
-    res_finalize_block(M.res_part, (int)cdiv(M.T.NI, BT), M.sc, fin);
+    res_finalize_block<BT>(M.res_part, (int)cdiv(M.T.NI, BT), M.sc, fin);
     if (threadIdx.x == 0) step_end_item(M.sc, M.T.NI);
     __syncthreads();
 }

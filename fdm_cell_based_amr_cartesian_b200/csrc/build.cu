@@ -487,7 +487,8 @@ __global__ void __launch_bounds__(64) k_wls_geometry(Tables T, ReqOut O) {
 struct GhostOut {
     int32_t *kind, *a, *b, *flip;
     double *x, *y;
-    unsigned long long *n_restrict;   // ghosts imaged by a subtree restriction
+    int32_t *rlist;                   // ghosts imaged by a subtree restriction (in no particular order)
+    unsigned long long *n_restrict;
 };
 
 __device__ __forceinline__ void ghost_from_ref(const Tables &T, const NodeRef &img, GhostOut &O, int64_t g) {
@@ -498,7 +499,7 @@ __device__ __forceinline__ void ghost_from_ref(const Tables &T, const NodeRef &i
     } else {
         const uint64_t p0 = node_pos(img.n);
         O.kind[g] = GH_RESTRICT;
-        atomicAdd(O.n_restrict, 1ull);
+        O.rlist[atomicAdd(O.n_restrict, 1ull)] = (int32_t)g;
         O.a[g] = (int32_t)lower_bound_pos_t(T, p0);
         O.b[g] = (int32_t)lower_bound_pos_t(T, p0 + span_of_level(img.n.lvl));
     }
@@ -892,13 +893,14 @@ int build_tables(fdm_handle *h, int64_t n, const uint64_t *keys_in, const double
     FDM_CK(h, h->gh_a.ensure(ngh * 4));
     FDM_CK(h, h->gh_b.ensure(ngh * 4));
     FDM_CK(h, h->gh_flip.ensure(ngh * 4));
+    FDM_CK(h, h->gh_rlist.ensure(ngh * 4));
     FDM_CK(h, h->gh_x.ensure(ngh * 8));
     FDM_CK(h, h->gh_y.ensure(ngh * 8));
     if (NG > 0) {
         Tables T = h->tables();
         GhostOut O{h->gh_kind.as<int32_t>(), h->gh_a.as<int32_t>(), h->gh_b.as<int32_t>(),
                    h->gh_flip.as<int32_t>(), h->gh_x.as<double>(),  h->gh_y.as<double>(),
-                   counts + 4};
+                   h->gh_rlist.as<int32_t>(), counts + 4};
         k_ghosts<<<nblk(NG, 128), 128, 0, s>>>(T, h->G, h->p, O);
     }
     // 7. faces

@@ -79,6 +79,8 @@ struct Tables {
     int64_t NRR;
     // ghosts (slots NI .. NI+NG)
     const int32_t *gh_kind;           // [NG]
+    const int32_t *gh_rlist;          // [NGR] the ghosts of kind GH_RESTRICT
+    int64_t NGR;
     const int32_t *gh_a;              // [NG] source slot / range lo
     const int32_t *gh_b;              // [NG] range hi / state index
     const int32_t *gh_flip;           // [NG] 0 none, 1 negate u, 2 negate v

@@ -405,7 +405,7 @@ __host__ inline GhostStates ghost_states(const fdm_params &p) {
 
 // lambda/time-step control (src/solution.F90:185-201); one thread
 __device__ __forceinline__ void step_control_item(DevScalars *sc, const fdm_params &P, int use_dt) {
-    if (sc->done) return;
+    if (sc->done) return;   // (the caller resets lam_next for a step that goes on all the same)
     sc->lambda_x = fmax(sc->lambda_x, sc->lam_next_x);
     sc->lambda_y = fmax(sc->lambda_y, sc->lam_next_y);
     sc->lam_next_x = 0.0;
@@ -417,21 +417,33 @@ __device__ __forceinline__ void step_control_item(DevScalars *sc, const fdm_para
     if (sc->tt + sc->tstep > P.t_end) sc->tstep = P.t_end - sc->tt;
 }
 
-// residual partials -> Res_max / Res_rms sums over a fixed reduction tree,
-// so the result is identical run to run; all threads of a 256-thread block
+// residual partials -> Res_max / Res_rms sums over a fixed reduction tree
+// (256 strided sums of each component, then pairwise), so the result is
+// identical run to run and for every NT (256 or 1024 threads, the components
+// of a strided sum shared by NT / 256 of them); all threads of the block
+template <int NT>
 __device__ __forceinline__ void res_finalize_block(const double *__restrict__ res_part, int nb, DevScalars *sc,
                                                    double (*sh)[8]) {
-    double v[8];
-    for (int n = 0; n < 8; ++n) v[n] = 0.0;
-    for (int b = threadIdx.x; b < nb; b += 256)
-        for (int n = 0; n < 8; ++n) v[n] = n < 4 ? fmax(v[n], res_part[b * 8 + n]) : v[n] + res_part[b * 8 + n];
-    for (int n = 0; n < 8; ++n) sh[threadIdx.x][n] = v[n];
+    constexpr int NC = 8 * 256 / NT;   // components per thread
+    const int t = threadIdx.x & 255, c0 = (threadIdx.x >> 8) * NC;
+    double v[NC];
+#pragma unroll
+    for (int n = 0; n < NC; ++n) v[n] = 0.0;
+#pragma unroll 4
+    for (int b = t; b < nb; b += 256)
+#pragma unroll
+        for (int n = 0; n < NC; ++n) {
+            const double x = res_part[b * 8 + c0 + n];
+            v[n] = c0 + n < 4 ? fmax(v[n], x) : v[n] + x;
+        }
+#pragma unroll
+    for (int n = 0; n < NC; ++n) sh[t][c0 + n] = v[n];
     __syncthreads();
     for (int w = 128; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w)
-            for (int n = 0; n < 8; ++n)
-                sh[threadIdx.x][n] = n < 4 ? fmax(sh[threadIdx.x][n], sh[threadIdx.x + w][n])
-                                           : sh[threadIdx.x][n] + sh[threadIdx.x + w][n];
+        if (t < w)
+#pragma unroll
+            for (int n = 0; n < NC; ++n)
+                sh[t][c0 + n] = c0 + n < 4 ? fmax(sh[t][c0 + n], sh[t + w][c0 + n]) : sh[t][c0 + n] + sh[t + w][c0 + n];
         __syncthreads();
     }
     if (threadIdx.x < 8) {

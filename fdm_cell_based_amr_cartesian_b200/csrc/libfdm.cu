@@ -174,13 +174,6 @@ static void enqueue_rk(fdm_handle *h) {
     launch_stage(h, 3);
 }
 
-// one solute iteration without AMR: step control, RK3, tt/residual/NaN
-static void enqueue_solute_iteration(fdm_handle *h) {
-    launch_step_control(h);
-    enqueue_rk(h);
-    launch_step_end(h);
-}
-
 static int prepare_buffers(fdm_handle *h) {
     const int64_t nb = nblk(h->NI, 256);
     FDM_CK(h, h->res_part.ensure((size_t)(nb > 0 ? nb : 1) * 8 * sizeof(double)));
@@ -214,8 +207,7 @@ static int step_graph(fdm_handle *h, cudaGraphExec_t *out, bool ghosts = false) 
     }
     cudaGraph_t g = nullptr;
     FDM_CK(h, cudaStreamBeginCapture(h->s, cudaStreamCaptureModeThreadLocal));
-    enqueue_solute_iteration(h);
-    if (ghosts) launch_ghosts(h, h->B[0].as<double4>(), 1);
+    launch_step(h, ghosts);
     cudaError_t e = cudaStreamEndCapture(h->s, &g);
     if (e != cudaSuccess) return cuda_fail(h, e, "cudaStreamEndCapture");
     if (slot) {
@@ -640,7 +632,7 @@ int fdm_solute_step(fdm_handle *h) {
     CHECK_H(h);
     CHECK_LOADED(h);
     RC(ensure_lambda(h));
-    enqueue_solute_iteration(h);
+    launch_step(h, false);
     h->lam_fresh = true;
     RC(sync_scalars_from_device(h));
     FDM_CK(h, cudaGetLastError());

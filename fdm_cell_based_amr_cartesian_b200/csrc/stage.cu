@@ -31,6 +31,7 @@ __global__ void __launch_bounds__(128) k_requests(Tables T, double4 *cur) {
     constexpr int PER = 32 * RQ_NV / 4;   // requests per warp
     const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int64_t r = (g >> 5) * PER + (g & (PER - 1));
+    dep_begin();
     if (r >= T.NR) return;
     request_item<RQ_NV>(T, cur, r, ((int)g & 31) / PER * RQ_NV, T.rq_geo + rq_geo_at(r));
 }
@@ -58,6 +59,7 @@ template <int TB, int MINB>
 __global__ void __launch_bounds__(TB, MINB) k_faces(Tables T, const double4 *__restrict__ cur, double4 *Fx,
                                                     double4 *Fy, const DevScalars *__restrict__ sc, double g,
                                                     FluxDen den, int nbx) {
+    dep_begin();
     const int64_t b = blockIdx.x;
     if (b < nbx) {
         const int64_t f = b * TB + threadIdx.x;
@@ -116,6 +118,7 @@ __global__ void __launch_bounds__(256) k_cells(Tables T, LevelTab LT, const doub
                                                 const double4 *__restrict__ Fx, const double4 *__restrict__ Fy,
                                                 DevScalars *sc, double *res_part, int krk, int mode, double g) {
     __shared__ CellsSmem S;
+    dep_begin();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     double rm[4] = {0.0, 0.0, 0.0, 0.0}, rs[4] = {0.0, 0.0, 0.0, 0.0};
     double lx = 0.0, ly = 0.0;
@@ -135,25 +138,24 @@ __global__ void k_blend(int64_t NI, const double4 *__restrict__ un, const double
     cur[i] = make_double4(ra * a.x + rb * b.x, ra * a.y + rb * b.y, ra * a.z + rb * b.z, ra * a.w + rb * b.w);
 }
 
-// ghost leaves imaged by a copy or a boundary state: one thread each
-__global__ void __launch_bounds__(256) k_ghost_simple(Tables T, double4 *buf, GhostStates GS,
-                                                      const DevScalars *__restrict__ sc, int j) {
-    const int64_t gi = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (gi >= T.NG) return;
-    const int kind = T.gh_kind[gi];
-    if (kind == GH_NONE || kind == GH_RESTRICT) return;
-    ghost_store(T, buf, gi, ghost_simple_value(T, buf, GS, sc, j, gi, kind));
-}
-
-// ghost leaves imaged by a subtree restriction (interpA images can span
-// hundreds of leaves): one warp each
+// ghost leaves: the first nbs blocks take a thread for each that is imaged by
+// a copy or a boundary state, the others a warp for each that is imaged by a
+// subtree restriction (interpA images can span hundreds of leaves)
 __global__ void __launch_bounds__(128) k_ghost(Tables T, double4 *buf, GhostStates GS,
-                                               const DevScalars *__restrict__ sc, int j) {
+                                               const DevScalars *__restrict__ sc, int j, int nbs) {
     __shared__ RestrictSmem sm[4];
-    const int64_t gi = blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (gi >= T.NG) return;
-    if (T.gh_kind[gi] != GH_RESTRICT) return;
-    ghost_warp(T, buf, GS, sc, j, gi, sm[threadIdx.x >> 5]);
+    dep_begin();
+    const int64_t b = blockIdx.x;
+    if (b < nbs) {
+        const int64_t gi = b * 128 + threadIdx.x;
+        if (gi >= T.NG) return;
+        const int kind = T.gh_kind[gi];
+        if (kind == GH_NONE || kind == GH_RESTRICT) return;
+        ghost_store(T, buf, gi, ghost_simple_value(T, buf, GS, sc, j, gi, kind));
+    } else {
+        const int64_t w = (b - nbs) * 4 + (threadIdx.x >> 5);
+        if (w < T.NGR) ghost_warp(T, buf, GS, sc, j, T.gh_rlist[w], sm[threadIdx.x >> 5]);
+    }
 }
 
 __global__ void k_lambda(int64_t NI, const double4 *__restrict__ cur, DevScalars *sc, double g) {
@@ -176,23 +178,23 @@ __global__ void k_lambda(int64_t NI, const double4 *__restrict__ cur, DevScalars
 }
 
 // lambda/time-step control (src/solution.F90:185-201)
-__global__ void k_step_control(DevScalars *sc, fdm_params P, int use_dt) {
+__global__ void k_step_control(DevScalars *sc, fdm_params P, int use_dt, bool step_follows) {
+    dep_begin();
     if (threadIdx.x || blockIdx.x) return;
     step_control_item(sc, P, use_dt);
+    // the step's stage 3 collects the next lambda from zero
+    if (step_follows) { sc->lam_next_x = 0.0; sc->lam_next_y = 0.0; }
 }
 
-// residual partials -> Res_max / Res_rms sums
-__global__ void __launch_bounds__(256) k_res_finalize(const double *__restrict__ res_part, int nb, DevScalars *sc,
-                                                      int keep_when_done) {
+// residual partials -> Res_max / Res_rms sums, and (end) the end of one
+// solute iteration: tt, rms, NaN stop, t_end (src/solution.F90:205-215)
+__global__ void __launch_bounds__(1024) k_res_finalize(const double *__restrict__ res_part, int nb, DevScalars *sc,
+                                                       int keep_when_done, bool end, int64_t NI) {
     __shared__ double sh[256][8];
+    dep_begin();
     if (keep_when_done && sc->done) return;   // a no-op iteration keeps the last residual
-    res_finalize_block(res_part, nb, sc, sh);
-}
-
-// end of one solute iteration: tt, rms, NaN stop, t_end (src/solution.F90:205-215)
-__global__ void k_step_end(DevScalars *sc, int64_t NI) {
-    if (threadIdx.x || blockIdx.x) return;
-    step_end_item(sc, NI);
+    res_finalize_block<1024>(res_part, nb, sc, sh);
+    if (end && threadIdx.x == 0) step_end_item(sc, NI);
 }
 
 __global__ void k_set_tstep(DevScalars *sc, double tstep) {
@@ -203,7 +205,7 @@ __global__ void k_set_tstep(DevScalars *sc, double tstep) {
 // ------------------------------------------------------------ launchers
 void launch_requests(fdm_handle *h, const double4 *cur) {
     if (h->NR == 0) return;
-    k_requests<<<nblk(h->NR, 128 * RQ_NV / 4), 128, 0, h->s>>>(h->tables(), (double4 *)cur);
+    launch_after(h->s, nblk(h->NR, 128 * RQ_NV / 4), 128, k_requests, h->tables(), (double4 *)cur);
     if (h->n_restrict > 0)
         k_requests_restrict<<<nblk(h->n_restrict, 4), 128, 0, h->s>>>(h->tables(), (double4 *)cur);
 }
@@ -214,8 +216,8 @@ template <int TB, int MINB>
 static void faces(fdm_handle *h, const double4 *cur) {
     const double g = h->G.gama;
     const int nbx = nblk(h->NI + h->nux, TB), nby = nblk(h->NI + h->nuy, TB);
-    k_faces<TB, MINB><<<nbx + nby, TB, 0, h->s>>>(h->tables(), cur, h->Fx.as<double4>(), h->Fy.as<double4>(),
-                                                  h->scal.as<DevScalars>(), g, flux_den(g), nbx);
+    launch_after(h->s, nbx + nby, TB, k_faces<TB, MINB>, h->tables(), cur, h->Fx.as<double4>(), h->Fy.as<double4>(),
+                 h->scal.as<DevScalars>(), g, flux_den(g), nbx);
 }
 constexpr int N_FACE_SHAPES = 6;
 const char *face_variant_name(int v) {
@@ -244,21 +246,23 @@ void launch_faces(fdm_handle *h, const double4 *cur, int krk) {
     }
 }
 
-void launch_cells(fdm_handle *h, const double4 *cur, const double4 *un, double4 *next, int krk, int mode) {
-    const int nb = nblk(h->NI, 256);
-    k_cells<<<nb, 256, 0, h->s>>>(h->tables(), h->lt, cur, un, next, h->Fx.as<double4>(), h->Fy.as<double4>(),
-                                  h->scal.as<DevScalars>(), h->res_part.as<double>(), krk, mode, h->G.gama);
+static void launch_res_finalize(fdm_handle *h, bool keep_when_done, bool end) {
+    launch_after(h->s, 1, 1024, k_res_finalize, h->res_part.as<double>(), nblk(h->NI, 256), h->scal.as<DevScalars>(),
+                 keep_when_done, end, h->NI);
+}
+void launch_cells(fdm_handle *h, const double4 *cur, const double4 *un, double4 *next, int krk, int mode,
+                  bool finalize) {
+    launch_after(h->s, nblk(h->NI, 256), 256, k_cells, h->tables(), h->lt, cur, un, next, h->Fx.as<double4>(),
+                 h->Fy.as<double4>(), h->scal.as<DevScalars>(), h->res_part.as<double>(), krk, mode, h->G.gama);
     // Res_max / Res_rms are reset every stage and read after the last one
     // (src/solution.F90:276-277, 209-210): reduce them once, after stage 3
-    if (krk == 3 || mode == 1)
-        k_res_finalize<<<1, 256, 0, h->s>>>(h->res_part.as<double>(), nb, h->scal.as<DevScalars>(), mode == 0);
+    if (finalize && (krk == 3 || mode == 1)) launch_res_finalize(h, mode == 0, false);
 }
 void launch_ghosts(fdm_handle *h, double4 *next, int j) {
     if (h->NG == 0) return;
-    const GhostStates GS = ghost_states(h->p);
-    k_ghost_simple<<<nblk(h->NG, 256), 256, 0, h->s>>>(h->tables(), next, GS, h->scal.as<DevScalars>(), j);
-    if (h->n_ghost_restrict > 0)
-        k_ghost<<<nblk(h->NG, 4), 128, 0, h->s>>>(h->tables(), next, GS, h->scal.as<DevScalars>(), j);
+    const int nbs = nblk(h->NG, 128);
+    launch_after(h->s, nbs + nblk(h->n_ghost_restrict, 4), 128, k_ghost, h->tables(), next, ghost_states(h->p),
+                 h->scal.as<DevScalars>(), j, nbs);
 }
 void launch_blend(fdm_handle *h, const double4 *un, double4 *cur, int krk) {
     k_blend<<<nblk(h->NI, 256), 256, 0, h->s>>>(h->NI, un, h->Ut.as<double4>(), cur, krk);
@@ -267,10 +271,7 @@ void launch_lambda(fdm_handle *h, const double4 *cur) {
     k_lambda<<<nblk(h->NI, 256), 256, 0, h->s>>>(h->NI, cur, h->scal.as<DevScalars>(), h->G.gama);
 }
 void launch_step_control(fdm_handle *h) {
-    k_step_control<<<1, 32, 0, h->s>>>(h->scal.as<DevScalars>(), h->p, 1);
-}
-void launch_step_end(fdm_handle *h) {
-    k_step_end<<<1, 32, 0, h->s>>>(h->scal.as<DevScalars>(), h->NI);
+    k_step_control<<<1, 32, 0, h->s>>>(h->scal.as<DevScalars>(), h->p, 1, false);
 }
 void launch_set_tstep(fdm_handle *h, double tstep) {
     k_set_tstep<<<1, 32, 0, h->s>>>(h->scal.as<DevScalars>(), tstep);
@@ -278,15 +279,30 @@ void launch_set_tstep(fdm_handle *h, double tstep) {
 
 // One RK stage on the three state buffers: B0 holds the step-start state
 // (Un); stage 1: B0 -> B1, stage 2: B1 -> B2, stage 3: B2 -> B0.
-int launch_stage(fdm_handle *h, int krk) {
-    double4 *b0 = h->B[0].as<double4>(), *b1 = h->B[1].as<double4>(), *b2 = h->B[2].as<double4>();
-    const double4 *cur = krk == 1 ? b0 : krk == 2 ? b1 : b2;
-    double4 *next = krk == 1 ? b1 : krk == 2 ? b2 : b0;
+static void stage_interior(fdm_handle *h, int krk, bool finalize) {
+    double4 *b[3] = {h->B[0].as<double4>(), h->B[1].as<double4>(), h->B[2].as<double4>()};
+    const double4 *cur = b[krk - 1];
     launch_requests(h, cur);
     launch_faces(h, cur, krk);
-    launch_cells(h, cur, b0, next, krk, 0);
-    launch_ghosts(h, next, 3);
+    launch_cells(h, cur, b[0], b[krk % 3], krk, 0, finalize);
+}
+int launch_stage(fdm_handle *h, int krk) {
+    stage_interior(h, krk, true);
+    launch_ghosts(h, h->B[krk % 3].as<double4>(), 3);
     return FDM_OK;
+}
+// One solute iteration without AMR: step control, RK3, tt/residual/NaN;
+// refresh: followed by the j = 1 ghost refresh that solute does after an
+// iteration without regrid.  That refresh writes every ghost that the stage-3
+// fill (j = 3) writes, and nothing reads them in between, so it stands for it.
+void launch_step(fdm_handle *h, bool refresh) {
+    launch_after(h->s, 1, 32, k_step_control, h->scal.as<DevScalars>(), h->p, 1, true);
+    launch_stage(h, 1);
+    launch_stage(h, 2);
+    stage_interior(h, 3, false);
+    if (!refresh) launch_ghosts(h, h->B[0].as<double4>(), 3);   // before tt moves on
+    launch_res_finalize(h, true, true);
+    if (refresh) launch_ghosts(h, h->B[0].as<double4>(), 1);
 }
 
 }  // namespace fdm
