@@ -324,8 +324,8 @@ __device__ __forceinline__ void ph_cell_tile(const BatchArgs &A, int krk, int m,
     double rm[4] = {0.0, 0.0, 0.0, 0.0}, rs[4] = {0.0, 0.0, 0.0, 0.0};
     double lx = 0.0, ly = 0.0;
     if (i < M.T.NI)
-        cell_item(M.T, M.LT, stage_cur(M, krk), M.B0, stage_next(M, krk), M.Fx, M.Fy, M.sc->tstep, krk, 0, M.gama, i,
-                  rm, rs, lx, ly);
+        cell_item(M.T, M.LT, stage_cur(M, krk), M.B0, stage_next(M, krk), M.Fx, M.Fy, M.sc->tstep, krk, 0, M.gama,
+                  M.den, i, rm, rs, lx, ly);
     cells_block_reduce(rm, rs, lx, ly, M.res_part + t * 8, M.sc, krk == 3, S);
 }
 

@@ -170,10 +170,10 @@ __device__ __forceinline__ void face_flux_f_slots(const double4 *__restrict__ cu
         back_project<DIR>(E, uwR, wR);
     }
     double F0[4], F1[4], F2[4], F3[4], Ud[4];
-    cons_flux_f<DIR>(load_prim_again(cur, ia), ig1, Ud, F0);
-    cons_flux_f<DIR>(load_prim_again(cur, ib), ig1, Ud, F1);
-    cons_flux_f<DIR>(load_prim_again(cur, ic), ig1, Ud, F2);
-    cons_flux_f<DIR>(load_prim_again(cur, id), ig1, Ud, F3);
+    cons_flux_f<DIR>(load_prim(cur, ia), ig1, Ud, F0);
+    cons_flux_f<DIR>(load_prim(cur, ib), ig1, Ud, F1);
+    cons_flux_f<DIR>(load_prim(cur, ic), ig1, Ud, F2);
+    cons_flux_f<DIR>(load_prim(cur, id), ig1, Ud, F3);
     double w0[4], w1[4], w2[4], w3[4], ugL[4], ugR[4];
     project<DIR>(E, F0, w0); project<DIR>(E, F1, w1);
     project<DIR>(E, F2, w2); project<DIR>(E, F3, w3);
@@ -196,7 +196,7 @@ __device__ __forceinline__ void face_item(const Tables &T, const double4 *__rest
     face_slots<DIR>(T, f, a, b, c, d);
     double out[4];
     face_flux_f_slots<DIR>(cur, a, b, c, d, g, ig1, lam, out);
-    F[f] = make_double4(out[0], out[1], out[2], out[3]);
+    store_record(F + f, make_double4(out[0], out[1], out[2], out[3]));
 }
 
 }  // namespace fast

@@ -453,7 +453,7 @@ __device__ __forceinline__ void gate_linear_chunk(const Tables &T, const double4
     if (lin) {
         double out[4];
         face_flux_linear<DIR>(p0, p1, p2, p3, ig1, lam, out);
-        F[f] = make_double4(out[0], out[1], out[2], out[3]);
+        store_record(F + f, make_double4(out[0], out[1], out[2], out[3]));
     }
     if (in) jump1[f] = lin ? jm : -1.0f;
     append_hard(in && !lin, f, lane, hard, count);
@@ -477,7 +477,7 @@ __device__ __forceinline__ void guard_linear_chunk(const Tables &T, const double
         if (face_jump<DIR>(p0, p1, p2, p3, g) <= GUARD_GROWTH * j1 + GUARD_ABS) {
             double out[4];
             face_flux_linear<DIR>(p0, p1, p2, p3, ig1, lam, out);
-            F[f] = make_double4(out[0], out[1], out[2], out[3]);
+            store_record(F + f, make_double4(out[0], out[1], out[2], out[3]));
         } else {
             hardf = true;
         }

@@ -240,72 +240,121 @@ __device__ __forceinline__ void face_item(const Tables &T, const double4 *__rest
                                           double g, const FluxDen &den, int64_t f) {
     int32_t a, b, c, d;
     face_slots<DIR>(T, f, a, b, c, d);
-    F[f] = face_flux_of<DIR>(cur, a, b, c, d, g, den, lam);
+    store_record(F + f, face_flux_of<DIR>(cur, a, b, c, d, g, den, lam));
 }
 
 // Residual + forward-Euler candidate (LXL) fused with updateRK for leaf i.
-// mode 0: write the blended stage value into next; mode 1: write the
-// primitive candidate Ut into next (no blend) for the split API.  rm / rs /
-// lx / ly receive the leaf's residual norms and (stage 3) wave speeds.
-__device__ __forceinline__ void cell_item(const Tables &T, const LevelTab &LT, const double4 *__restrict__ cur,
-                                          const double4 *__restrict__ un, double4 *next,
-                                          const double4 *__restrict__ Fx, const double4 *__restrict__ Fy,
-                                          double tstep, int krk, int mode, double g, int64_t i, double rm[4],
-                                          double rs[4], double &lx, double &ly) {
-    const int lvl = T.ilvl[i];
-    const int32_t *s = T.ist + i * 8;
-    const Prim q = load_prim(cur, i);
-    const Prim qp = load_prim(cur, s[0]), qm = load_prim(cur, s[1]);
-    const Prim rp = load_prim(cur, s[2]), rmn = load_prim(cur, s[3]);
-    const double4 fxr = Fx[i], fxl = Fx[T.ifxl[i]];
-    const double4 fyr = Fy[i], fyl = Fy[T.ifyl[i]];
+// mode 0: the blended stage value; mode 1: the primitive candidate Ut (no
+// blend) for the split API.  rm / rs / lx / ly are the leaf's residual norms
+// and (stage 3) wave speeds.  Divisions through D: the branch-free ones
+// (DivNR, ok false when an operand is outside their range) or the compiler's.
+struct CellValue {
+    double4 o;
+    double rm[4], rs[4], lx, ly;
+    bool ok;
+};
+// the value from the records: q the cell, qp/qm/rp/rm_ its x and y neighbours,
+// fr/fl/hr/hl its face fluxes; k the level's coefficients
+struct CellCoef {
+    double cxa, cxb, cya, cyb, dx, dy;
+};
+template <class D>
+__device__ __forceinline__ CellValue cell_update(const Prim &q, const Prim &qp, const Prim &qm, const Prim &rp,
+                                                 const Prim &rmn, const double4 &fr, const double4 &fl,
+                                                 const double4 &hr, const double4 &hl, const CellCoef &k,
+                                                 const double4 *un, double tstep, int krk, int mode, double g,
+                                                 const FluxDen &den) {
+    D dv(den);
+    dv.test_numerator(q.p);
+    dv.test_numerator(qp.p);
+    dv.test_numerator(qm.p);
+    dv.test_numerator(rp.p);
+    dv.test_numerator(rmn.p);
     double Ep[4], Em[4], Gp[4], Gm[4];
-    phys_flux<0>(qp, g, Ep);
-    phys_flux<0>(qm, g, Em);
-    phys_flux<1>(rp, g, Gp);
-    phys_flux<1>(rmn, g, Gm);
-    const double FR[4] = {fxr.x, fxr.y, fxr.z, fxr.w}, FL[4] = {fxl.x, fxl.y, fxl.z, fxl.w};
-    const double HR[4] = {fyr.x, fyr.y, fyr.z, fyr.w}, HL[4] = {fyl.x, fyl.y, fyl.z, fyl.w};
-    const double cxa = LT.cxa[lvl], cxb = LT.cxb[lvl], cya = LT.cya[lvl], cyb = LT.cyb[lvl];
-    const double dx = LT.dx[lvl], dy = LT.dy[lvl];
+    phys_flux_nr<0>(qp, dv, Ep);
+    phys_flux_nr<0>(qm, dv, Em);
+    phys_flux_nr<1>(rp, dv, Gp);
+    phys_flux_nr<1>(rmn, dv, Gm);
+    const double FR[4] = {fr.x, fr.y, fr.z, fr.w}, FL[4] = {fl.x, fl.y, fl.z, fl.w};
+    const double HR[4] = {hr.x, hr.y, hr.z, hr.w}, HL[4] = {hl.x, hl.y, hl.z, hl.w};
     double U[4];
     U[0] = q.r;
     U[1] = q.r * q.u;
     U[2] = q.r * q.v;
-    U[3] = q.p / (g - 1.0) + 0.5 * q.r * (q.u * q.u + q.v * q.v);
+    U[3] = D::q(q.p, dv.gm1) + 0.5 * q.r * (q.u * q.u + q.v * q.v);
+    CellValue c;
     double Ut[4];
 #pragma unroll
     for (int n = 0; n < 4; ++n) {
-        const double dE = cxa * (FR[n] - FL[n]) - cxb * (Ep[n] - Em[n]);
-        const double dF = cya * (HR[n] - HL[n]) - cyb * (Gp[n] - Gm[n]);
+        const double dE = k.cxa * (FR[n] - FL[n]) - k.cxb * (Ep[n] - Em[n]);
+        const double dF = k.cya * (HR[n] - HL[n]) - k.cyb * (Gp[n] - Gm[n]);
         const double fu = -dE - dF;
         Ut[n] = U[n] + fu * tstep;
-        const double fr = fu * dx * dy;
-        rm[n] = fabs(fr);
-        rs[n] = fr * fr;
+        const double f = fu * k.dx * k.dy;
+        c.rm[n] = fabs(f);
+        c.rs[n] = f * f;
     }
     const double r0 = Ut[0];
-    const double u0 = Ut[1] / Ut[0];
-    const double v0 = Ut[2] / Ut[0];
-    const double p0 = (g - 1.0) * r0 * (Ut[3] / r0 - 0.5 * (u0 * u0 + v0 * v0));
-    double4 o;
+    dv.test_bits(r0);
+    dv.template test_range<-100, 100>(r0);
+    dv.test_numerator(Ut[1]);
+    dv.test_numerator(Ut[2]);
+    dv.test_numerator(Ut[3]);
+    const Den dr = D::den(r0);
+    const double u0 = D::q(Ut[1], dr);
+    const double v0 = D::q(Ut[2], dr);
+    const double p0 = (g - 1.0) * r0 * (D::q(Ut[3], dr) - 0.5 * (u0 * u0 + v0 * v0));
+    c.lx = c.ly = 0.0;
     if (mode == 1) {
-        o = make_double4(r0, u0, v0, p0);
+        c.o = make_double4(r0, u0, v0, p0);
     } else {
-        const double4 n0 = un[i];
+        const double4 n0 = load_record(un);
         const double ra = krk == 1 ? 0.0 : krk == 2 ? 3.0 / 4.0 : 1.0 / 3.0;
         const double rb = krk == 1 ? 1.0 : krk == 2 ? 1.0 / 4.0 : 2.0 / 3.0;
-        o.x = ra * n0.x + rb * r0;
-        o.y = ra * n0.y + rb * u0;
-        o.z = ra * n0.z + rb * v0;
-        o.w = ra * n0.w + rb * p0;
+        c.o.x = ra * n0.x + rb * r0;
+        c.o.y = ra * n0.y + rb * u0;
+        c.o.z = ra * n0.z + rb * v0;
+        c.o.w = ra * n0.w + rb * p0;
         if (krk == 3) {
-            const double c = sqrt(g * o.w / o.x);
-            lx = fabs(o.y) + c;
-            ly = fabs(o.z) + c;
+            const double a = sqrt(g * c.o.w / c.o.x);
+            c.lx = fabs(c.o.y) + a;
+            c.ly = fabs(c.o.z) + a;
         }
     }
-    next[i] = o;
+    c.ok = dv.ok;
+    return c;
+}
+template <class D>
+__device__ __forceinline__ CellValue cell_value(const Tables &T, const LevelTab &LT, const double4 *__restrict__ cur,
+                                                const double4 *un, const double4 *__restrict__ Fx,
+                                                const double4 *__restrict__ Fy, double tstep, int krk, int mode,
+                                                double g, const FluxDen &den, int64_t i) {
+    const int lvl = T.ilvl[i];
+    const int4 s = *reinterpret_cast<const int4 *>(T.ist + i * 8);
+    const CellCoef k{LT.cxa[lvl], LT.cxb[lvl], LT.cya[lvl], LT.cyb[lvl], LT.dx[lvl], LT.dy[lvl]};
+    return cell_update<D>(load_prim(cur, i), load_prim(cur, s.x), load_prim(cur, s.y), load_prim(cur, s.z),
+                          load_prim(cur, s.w), load_record(Fx + i), load_record(Fx + T.ifxl[i]), load_record(Fy + i),
+                          load_record(Fy + T.ifyl[i]), k, un + i, tstep, krk, mode, g, den);
+}
+// a leaf that DivNR refuses, out of line
+__device__ __noinline__ inline CellValue cell_value_again(const Tables &T, const LevelTab &LT, const double4 *cur,
+                                                          const double4 *un, const double4 *Fx, const double4 *Fy,
+                                                          double tstep, int krk, int mode, double g,
+                                                          const FluxDen &den, int64_t i) {
+    return cell_value<DivIEEE>(T, LT, cur, un, Fx, Fy, tstep, krk, mode, g, den, i);
+}
+__device__ __forceinline__ void cell_item(const Tables &T, const LevelTab &LT, const double4 *__restrict__ cur,
+                                          const double4 *un, double4 *next, const double4 *__restrict__ Fx,
+                                          const double4 *__restrict__ Fy, double tstep, int krk, int mode, double g,
+                                          const FluxDen &den, int64_t i, double rm[4], double rs[4], double &lx,
+                                          double &ly) {
+    CellValue c = cell_value<DivNR>(T, LT, cur, un, Fx, Fy, tstep, krk, mode, g, den, i);
+    if (!c.ok) c = cell_value_again(T, LT, cur, un, Fx, Fy, tstep, krk, mode, g, den, i);
+#pragma unroll
+    for (int n = 0; n < 4; ++n) { rm[n] = c.rm[n]; rs[n] = c.rs[n]; }
+    lx = c.lx;
+    ly = c.ly;
+    store_record(next + i, c.o);
 }
 
 // Block reduction of one 256-leaf tile: residual max / sum of squares into

@@ -19,8 +19,21 @@ namespace fdm {
 
 struct Prim { double r, u, v, p; };
 
+// A record (32 bytes, 32-byte aligned) in one 256-bit access: half the load
+// instructions and L1 wavefronts of two 128-bit ones.  Volatile: a load stays
+// behind the wait at a kernel's start, and a record read twice (once for each
+// half of the face flux) is not kept in registers in between.
+__device__ __forceinline__ double4 load_record(const double4 *p) {
+    double4 q;
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(q.x), "=d"(q.y), "=d"(q.z), "=d"(q.w) : "l"(p));
+    return q;
+}
+__device__ __forceinline__ void store_record(double4 *p, const double4 &q) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(q.x), "d"(q.y), "d"(q.z), "d"(q.w)
+                 : "memory");
+}
 __device__ __forceinline__ Prim load_prim(const double4 *__restrict__ s, int64_t i) {
-    const double4 q = s[i];
+    const double4 q = load_record(s + i);
     return Prim{q.x, q.y, q.z, q.w};
 }
 
@@ -162,17 +175,6 @@ __device__ __forceinline__ double wcns_z3(double u1, double u2, double u3) {
     return w1 * p1 + w2 * p2;
 }
 
-// the record of slot i read again through the non-coherent path, as an
-// opaque load (the optimiser may not replace it by an earlier read, so the
-// earlier values need not stay in registers)
-__device__ __forceinline__ Prim load_prim_again(const double4 *s, int64_t i) {
-    const double *p = reinterpret_cast<const double *>(s + i);
-    double a, b, c, d;
-    asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%4];\n\tld.global.nc.v2.f64 {%2, %3}, [%4+16];"
-                 : "=d"(a), "=d"(b), "=d"(c), "=d"(d)
-                 : "l"(p));
-    return Prim{a, b, c, d};
-}
 // the conserved state of cons_flux alone (the same operations)
 template <int DIR>
 __device__ __forceinline__ void cons_state(const Prim &q, double g, double U[4]) {
@@ -218,10 +220,10 @@ __device__ __forceinline__ void face_flux_slots(const double4 *__restrict__ cur,
         back_project<DIR>(E, uwR, wR);
     }
     double F0[4], F1[4], F2[4], F3[4];
-    phys_flux<DIR>(load_prim_again(cur, ia), g, F0);
-    phys_flux<DIR>(load_prim_again(cur, ib), g, F1);
-    phys_flux<DIR>(load_prim_again(cur, ic), g, F2);
-    phys_flux<DIR>(load_prim_again(cur, id), g, F3);
+    phys_flux<DIR>(load_prim(cur, ia), g, F0);
+    phys_flux<DIR>(load_prim(cur, ib), g, F1);
+    phys_flux<DIR>(load_prim(cur, ic), g, F2);
+    phys_flux<DIR>(load_prim(cur, id), g, F3);
     double w0[4], w1[4], w2[4], w3[4], ugL[4], ugR[4];
     project<DIR>(E, F0, w0); project<DIR>(E, F1, w1);
     project<DIR>(E, F2, w2); project<DIR>(E, F3, w3);

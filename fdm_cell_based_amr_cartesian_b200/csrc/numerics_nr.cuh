@@ -104,6 +104,19 @@ struct DivNR {
     __device__ __forceinline__ static double q(double a, const Den &d) { return q(a, d.b, d.y); }
     __device__ __forceinline__ static double q(double a, const DenC &d) { return q(a, d.b, d.y); }
 };
+// the same interface with the compiler's division
+struct DivIEEE {
+    DenC gm1, d2;
+    static constexpr bool ok = true;
+    __device__ __forceinline__ explicit DivIEEE(const FluxDen &c) : gm1(c.gm1), d2(c.d2) {}
+    __device__ __forceinline__ void test_bits(double) {}
+    template <int LO, int HI>
+    __device__ __forceinline__ void test_range(double) {}
+    __device__ __forceinline__ void test_numerator(double) {}
+    __device__ __forceinline__ static Den den(double b) { return Den{b, 0.0}; }
+    __device__ __forceinline__ static double q(double a, const Den &d) { return a / d.b; }
+    __device__ __forceinline__ static double q(double a, const DenC &d) { return a / d.b; }
+};
 
 // The characteristic basis of a face (eigen) in the few quotients that
 // differ: with the momentum columns named by their direction (n the face's,
@@ -227,10 +240,10 @@ __device__ __forceinline__ void cons_state_nr(const Prim &q, const DivNR &dv, do
     U[2] = q.r * q.v;
     U[3] = DivNR::q(q.p, dv.gm1) + 0.5 * q.r * ke;
 }
-template <int DIR>
-__device__ __forceinline__ void phys_flux_nr(const Prim &q, const DivNR &dv, double F[4]) {
+template <int DIR, class D>
+__device__ __forceinline__ void phys_flux_nr(const Prim &q, const D &dv, double F[4]) {
     const double ke = q.u * q.u + q.v * q.v;
-    const double e = DivNR::q(q.p, dv.gm1) + 0.5 * q.r * ke;
+    const double e = D::q(q.p, dv.gm1) + 0.5 * q.r * ke;
     if (DIR == 0) {
         F[0] = q.r * q.u;
         F[1] = q.r * q.u * q.u + q.p;
@@ -276,10 +289,10 @@ __device__ __forceinline__ void face_flux_nr(const double4 *__restrict__ cur, in
         back_project_nr<DIR>(E, uwR, wR);
     }
     double F0[4], F1[4], F2[4], F3[4];
-    phys_flux_nr<DIR>(load_prim_again(cur, ia), dv, F0);
-    phys_flux_nr<DIR>(load_prim_again(cur, ib), dv, F1);
-    phys_flux_nr<DIR>(load_prim_again(cur, ic), dv, F2);
-    phys_flux_nr<DIR>(load_prim_again(cur, id), dv, F3);
+    phys_flux_nr<DIR>(load_prim(cur, ia), dv, F0);
+    phys_flux_nr<DIR>(load_prim(cur, ib), dv, F1);
+    phys_flux_nr<DIR>(load_prim(cur, ic), dv, F2);
+    phys_flux_nr<DIR>(load_prim(cur, id), dv, F3);
     double w0[4], w1[4], w2[4], w3[4], ugL[4], ugR[4];
     project_nr<DIR>(E, F0, w0); project_nr<DIR>(E, F1, w1);
     project_nr<DIR>(E, F2, w2); project_nr<DIR>(E, F3, w3);

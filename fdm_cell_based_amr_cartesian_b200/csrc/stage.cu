@@ -112,11 +112,18 @@ int count_nr_fallbacks(fdm_handle *h, int64_t out[2]) {
 }
 
 // Residual + forward-Euler candidate fused with updateRK, 256 leaves per
-// block (the residual partials are per block of 256).
-__global__ void __launch_bounds__(256) k_cells(Tables T, LevelTab LT, const double4 *__restrict__ cur,
-                                                const double4 *__restrict__ un, double4 *next,
+// block (the residual partials are per block of 256).  Bound by L1: ten
+// records a leaf, of which neighbours share most.  At 1.03 M leaves 64 us with
+// 128-bit accesses and the compiler's divisions (128 registers), 55 us with
+// 256-bit ones and branch-free quotients, 45 us at 80 registers (MINB 3).
+template <int MINB>
+__global__ void __launch_bounds__(256, MINB) k_cells(const __grid_constant__ Tables T,
+                                                const __grid_constant__ LevelTab LT,
+                                                const double4 *__restrict__ cur,
+                                                const double4 *un, double4 *next,
                                                 const double4 *__restrict__ Fx, const double4 *__restrict__ Fy,
-                                                DevScalars *sc, double *res_part, int krk, int mode, double g) {
+                                                DevScalars *sc, double *res_part, int krk, int mode, double g,
+                                                const __grid_constant__ FluxDen den) {
     __shared__ CellsSmem S;
     dep_begin();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -124,7 +131,7 @@ __global__ void __launch_bounds__(256) k_cells(Tables T, LevelTab LT, const doub
     double lx = 0.0, ly = 0.0;
     // an iteration after t_end (or after a NaN residual) leaves the state as it is
     if (i < T.NI && !(mode == 0 && sc->done))
-        cell_item(T, LT, cur, un, next, Fx, Fy, sc->tstep, krk, mode, g, i, rm, rs, lx, ly);
+        cell_item(T, LT, cur, un, next, Fx, Fy, sc->tstep, krk, mode, g, den, i, rm, rs, lx, ly);
     cells_block_reduce(rm, rs, lx, ly, res_part + blockIdx.x * 8, sc, krk == 3 && mode == 0, S);
 }
 
@@ -252,8 +259,13 @@ static void launch_res_finalize(fdm_handle *h, bool keep_when_done, bool end) {
 }
 void launch_cells(fdm_handle *h, const double4 *cur, const double4 *un, double4 *next, int krk, int mode,
                   bool finalize) {
-    launch_after(h->s, nblk(h->NI, 256), 256, k_cells, h->tables(), h->lt, cur, un, next, h->Fx.as<double4>(),
-                 h->Fy.as<double4>(), h->scal.as<DevScalars>(), h->res_part.as<double>(), krk, mode, h->G.gama);
+    // three blocks per SM where the mesh fills them more than once (1.03 M
+    // leaves: the step 0.861 ms instead of 0.890); below four blocks on each
+    // of the 148 SMs the shorter code of two wins (148 k: 0.1578 ms against 0.1591)
+    const unsigned nb = nblk(h->NI, 256);
+    launch_after(h->s, nb, 256, nb > 4u * 148u ? k_cells<3> : k_cells<2>, h->tables(), h->lt, cur, un, next,
+                 h->Fx.as<double4>(), h->Fy.as<double4>(), h->scal.as<DevScalars>(), h->res_part.as<double>(), krk, mode,
+                 h->G.gama, flux_den(h->G.gama));
     // Res_max / Res_rms are reset every stage and read after the last one
     // (src/solution.F90:276-277, 209-210): reduce them once, after stage 3
     if (finalize && (krk == 3 || mode == 1)) launch_res_finalize(h, mode == 0, false);

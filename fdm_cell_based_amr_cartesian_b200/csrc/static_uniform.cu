@@ -17,8 +17,7 @@
 #include <cstdint>
 
 #include "handle.cuh"
-#include "numerics.cuh"
-#include "numerics_nr.cuh"
+#include "items.cuh"
 
 namespace fdm {
 namespace uniform_static {
@@ -60,7 +59,7 @@ __device__ __forceinline__ void uface(const Grid2 &G, const double4 *__restrict_
     if (t >= nfr * nrow) return;
     const int r = t / nfr, i = t - r * nfr;
     const int step = DIR == 0 ? 1 : G.W, c = (int)G.at(3 + r, 3 + i);
-    F[t] = face_flux_of<DIR>(cur, c - 2 * step, c - step, c, c + step, g, den, lam);
+    store_record(F + t, face_flux_of<DIR>(cur, c - 2 * step, c - step, c, c + step, g, den, lam));
 }
 __global__ void __launch_bounds__(64, 8) k_ufaces(Grid2 G, const double4 *__restrict__ cur, double4 *Fx, double4 *Fy,
                                                   double g, FluxDen den, double lam_x, double lam_y, int nbx) {
@@ -69,22 +68,41 @@ __global__ void __launch_bounds__(64, 8) k_ufaces(Grid2 G, const double4 *__rest
     else uface<1>(G, cur, Fy, g, den, lam_y, (b - nbx) * 64 + threadIdx.x);
 }
 
-// LXL + updateRK for every interior cell (same operations as k_cells), and
-// its periodic images among the ghosts (BC_cyc at level 0,
-// src/solution.F90:116-136): the thread that makes a value stores its copies.
-// The corners are left alone, as the reference never refills them; at stage 3
-// the threads past the cells copy them from the input.
-__global__ void __launch_bounds__(128) k_ucells(Grid2 G, const double4 *__restrict__ cur,
-                                                const double4 *__restrict__ un, double4 *next,
-                                                const double4 *__restrict__ Fx, const double4 *__restrict__ Fy,
-                                                double g, double cxa, double cxb, double cya, double cyb,
-                                                double tstep, int krk) {
+// the cell's value (the operations of k_cells)
+template <class D>
+__device__ __forceinline__ CellValue ucell(const Grid2 &G, const double4 *__restrict__ cur, const double4 *un,
+                                           const double4 *__restrict__ Fx, const double4 *__restrict__ Fy, double g,
+                                           const FluxDen &den, const CellCoef &k, double tstep, int krk, int r, int i) {
+    const int row = 3 + r, col = 3 + i;
+    const int64_t self = G.at(row, col), fx = (int64_t)r * (G.nx + 1) + i, fy = (int64_t)r * G.nx + i;
+    return cell_update<D>(load_prim(cur, self), load_prim(cur, G.at(row, col + 1)), load_prim(cur, G.at(row, col - 1)),
+                          load_prim(cur, G.at(row + 1, col)), load_prim(cur, G.at(row - 1, col)), load_record(Fx + fx + 1),
+                          load_record(Fx + fx), load_record(Fy + fy + G.nx), load_record(Fy + fy), k, un + self, tstep,
+                          krk, 0, g, den);
+}
+// a cell that DivNR refuses, out of line
+__device__ __noinline__ CellValue ucell_again(const Grid2 &G, const double4 *cur, const double4 *un, const double4 *Fx,
+                                              const double4 *Fy, double g, const FluxDen &den, const CellCoef &k,
+                                              double tstep, int krk, int r, int i) {
+    return ucell<DivIEEE>(G, cur, un, Fx, Fy, g, den, k, tstep, krk, r, i);
+}
+
+// LXL + updateRK for every interior cell, and its periodic images among the
+// ghosts (BC_cyc at level 0, src/solution.F90:116-136): the thread that makes
+// a value stores its copies.  The corners are left alone, as the reference
+// never refills them; at stage 3 the threads past the cells copy them from
+// the input.
+__global__ void __launch_bounds__(128) k_ucells(const __grid_constant__ Grid2 G, const double4 *__restrict__ cur,
+                                                const double4 *un, double4 *next, const double4 *__restrict__ Fx,
+                                                const double4 *__restrict__ Fy, double g,
+                                                const __grid_constant__ FluxDen den,
+                                                const __grid_constant__ CellCoef k, double tstep, int krk) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int ncell = G.nx * G.ny;
     if (t >= ncell) {
-        const int k = (int)t - ncell;   // corner record k of 36: 3 x 3 at each end of both sides
-        if (krk == 3 && k < 36) {
-            const int a = k / 6, b = k % 6;
+        const int c = (int)t - ncell;   // corner record c of 36: 3 x 3 at each end of both sides
+        if (krk == 3 && c < 36) {
+            const int a = c / 6, b = c % 6;
             const int64_t at = G.at(a < 3 ? a : G.ny + a, b < 3 ? b : G.nx + b);
             next[at] = un[at];
         }
@@ -92,45 +110,13 @@ __global__ void __launch_bounds__(128) k_ucells(Grid2 G, const double4 *__restri
     }
     const int r = (int)t / G.nx, i = (int)t - r * G.nx;
     const int row = 3 + r, col = 3 + i;
-    const int64_t self = G.at(row, col);
-    const Prim q = load_prim(cur, self);
-    const Prim qp = load_prim(cur, G.at(row, col + 1)), qm = load_prim(cur, G.at(row, col - 1));
-    const Prim rp = load_prim(cur, G.at(row + 1, col)), rmn = load_prim(cur, G.at(row - 1, col));
-    const double4 fxr = Fx[(int64_t)r * (G.nx + 1) + i + 1], fxl = Fx[(int64_t)r * (G.nx + 1) + i];
-    const double4 fyr = Fy[(int64_t)(r + 1) * G.nx + i], fyl = Fy[(int64_t)r * G.nx + i];
-    double Ep[4], Em[4], Gp[4], Gm[4];
-    phys_flux<0>(qp, g, Ep);
-    phys_flux<0>(qm, g, Em);
-    phys_flux<1>(rp, g, Gp);
-    phys_flux<1>(rmn, g, Gm);
-    const double FR[4] = {fxr.x, fxr.y, fxr.z, fxr.w}, FL[4] = {fxl.x, fxl.y, fxl.z, fxl.w};
-    const double HR[4] = {fyr.x, fyr.y, fyr.z, fyr.w}, HL[4] = {fyl.x, fyl.y, fyl.z, fyl.w};
-    double U[4];
-    U[0] = q.r;
-    U[1] = q.r * q.u;
-    U[2] = q.r * q.v;
-    U[3] = q.p / (g - 1.0) + 0.5 * q.r * (q.u * q.u + q.v * q.v);
-    double Ut[4];
-#pragma unroll
-    for (int n = 0; n < 4; ++n) {
-        const double dE = cxa * (FR[n] - FL[n]) - cxb * (Ep[n] - Em[n]);
-        const double dF = cya * (HR[n] - HL[n]) - cyb * (Gp[n] - Gm[n]);
-        const double fu = -dE - dF;
-        Ut[n] = U[n] + fu * tstep;
-    }
-    const double r0 = Ut[0];
-    const double u0 = Ut[1] / Ut[0];
-    const double v0 = Ut[2] / Ut[0];
-    const double p0 = (g - 1.0) * r0 * (Ut[3] / r0 - 0.5 * (u0 * u0 + v0 * v0));
-    const double4 n0 = un[self];
-    const double ra = krk == 1 ? 0.0 : krk == 2 ? 3.0 / 4.0 : 1.0 / 3.0;
-    const double rb = krk == 1 ? 1.0 : krk == 2 ? 1.0 / 4.0 : 2.0 / 3.0;
-    const double4 o = make_double4(ra * n0.x + rb * r0, ra * n0.y + rb * u0, ra * n0.z + rb * v0, ra * n0.w + rb * p0);
-    next[self] = o;
-    if (col >= G.nx) next[G.at(row, col - G.nx)] = o;
-    if (col <= 5) next[G.at(row, col + G.nx)] = o;
-    if (row >= G.ny) next[G.at(row - G.ny, col)] = o;
-    if (row <= 5) next[G.at(row + G.ny, col)] = o;
+    CellValue v = ucell<DivNR>(G, cur, un, Fx, Fy, g, den, k, tstep, krk, r, i);
+    if (!v.ok) v = ucell_again(G, cur, un, Fx, Fy, g, den, k, tstep, krk, r, i);
+    store_record(next + G.at(row, col), v.o);
+    if (col >= G.nx) store_record(next + G.at(row, col - G.nx), v.o);
+    if (col <= 5) store_record(next + G.at(row, col + G.nx), v.o);
+    if (row >= G.ny) store_record(next + G.at(row - G.ny, col), v.o);
+    if (row <= 5) store_record(next + G.at(row + G.ny, col), v.o);
 }
 
 static inline unsigned nb(int64_t n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -166,6 +152,7 @@ extern "C" int fdm_time_advance_rk_uniform_static(const double *prim_in, double 
     const double dy = h, dx = x_factor * dy;
     const double cxa = 4.0 / (3.0 * dx), cxb = 1.0 / (6.0 * dx);
     const double cya = 4.0 / 3.0 / dy, cyb = 1.0 / 6.0 / dy;
+    const fdm::CellCoef k{cxa, cxb, cya, cyb, dx, dy};
     const double4 *in = (const double4 *)prim_in;
     double4 *out = (double4 *)prim_out;
     const double4 *cur[3] = {in, U1, U2};
@@ -174,8 +161,8 @@ extern "C" int fdm_time_advance_rk_uniform_static(const double *prim_in, double 
     const unsigned nbx = nb((int64_t)(nx + 1) * ny, 64), nby = nb((int64_t)nx * (ny + 1), 64);
     for (int krk = 1; krk <= 3; ++krk) {
         k_ufaces<<<nbx + nby, 64, 0, s>>>(G, cur[krk - 1], Fx, Fy, gama, den, lambda_x, lambda_y, (int)nbx);
-        k_ucells<<<nb((int64_t)nx * ny + 36, 128), 128, 0, s>>>(G, cur[krk - 1], in, next[krk - 1], Fx, Fy, gama, cxa,
-                                                                cxb, cya, cyb, tstep, krk);
+        k_ucells<<<nb((int64_t)nx * ny + 36, 128), 128, 0, s>>>(G, cur[krk - 1], in, next[krk - 1], Fx, Fy, gama,
+                                                                den, k, tstep, krk);
     }
     return cudaGetLastError() == cudaSuccess ? FDM_OK : FDM_ERR_CUDA;
 }
