@@ -738,13 +738,21 @@ int fdm_solute_paired(fdm_handle *lead, fdm_handle *follow, int64_t nsteps, int6
         follow->err = "paired handles must start at the same iteration, time and leaf count";
         return FDM_ERR_STATE;
     }
+    struct Event {   // freed on every way out
+        cudaEvent_t e = nullptr;
+        ~Event() { if (e) cudaEventDestroy(e); }
+    } taken;
+    FDM_CK(follow, cudaEventCreateWithFlags(&taken.e, cudaEventDisableTiming));
     int rc = FDM_OK;
     while (k < nsteps && lead->hs->tt < lead->p.t_end) {
         const bool regrid = amr_due(lead, lead->hs->it + 1);
         RC(ensure_lambda(lead));
         RC(ensure_lambda(follow));
         FDM_CK(follow, cudaStreamSynchronize(lead->s));
+        // lead's step resets the maxima: it waits until follow has taken them
         k_take_lambda<<<1, 32, 0, follow->s>>>(lead->scal.as<DevScalars>(), follow->scal.as<DevScalars>());
+        FDM_CK(follow, cudaEventRecord(taken.e, follow->s));
+        FDM_CK(lead, cudaStreamWaitEvent(lead->s, taken.e, 0));
         cudaGraphExec_t gl = nullptr, gf = nullptr;
         RC(step_graph(lead, &gl, lead->p.iflag_amr != 0 && !regrid));
         RC(step_graph(follow, &gf, follow->p.iflag_amr != 0 && !regrid));
