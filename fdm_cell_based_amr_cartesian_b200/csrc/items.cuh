@@ -243,6 +243,17 @@ __device__ __forceinline__ void face_item(const Tables &T, const double4 *__rest
     store_record(F + f, face_flux_of<DIR>(cur, a, b, c, d, g, den, lam));
 }
 
+// the same by two neighbouring lanes, face f of n (lanes past the last face
+// compute it again and store nothing)
+template <int DIR>
+__device__ __forceinline__ void face_item_pair(const Tables &T, const double4 *__restrict__ cur, double4 *F, double lam,
+                                               double g, const FluxDen &den, int64_t f, int64_t n) {
+    int32_t a, b, c, d;
+    face_slots<DIR>(T, f < n ? f : n - 1, a, b, c, d);
+    const double2 v = face_flux_pair<DIR>(cur, a, b, c, d, g, den, lam);
+    if (f < n) reinterpret_cast<double2 *>(F + f)[threadIdx.x & 1] = v;
+}
+
 // Residual + forward-Euler candidate (LXL) fused with updateRK for leaf i.
 // mode 0: the blended stage value; mode 1: the primitive candidate Ut (no
 // blend) for the split API.  rm / rs / lx / ly are the leaf's residual norms

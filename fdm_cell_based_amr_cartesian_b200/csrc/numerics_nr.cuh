@@ -322,4 +322,73 @@ __device__ __forceinline__ double4 face_flux_of(const double4 *__restrict__ cur,
     return dv.ok ? make_double4(out[0], out[1], out[2], out[3]) : face_flux_again<DIR>(cur, a, b, c, d, g, lam);
 }
 
+
+// one half's values of a point: the conserved state or the physical flux
+template <int DIR>
+__device__ __forceinline__ void point_half_nr(const Prim &q, const DivNR &dv, bool flux, double X[4]) {
+    const double ke = q.u * q.u + q.v * q.v;
+    const double e = DivNR::q(q.p, dv.gm1) + 0.5 * q.r * ke;
+    const double ru = q.r * q.u, rv = q.r * q.v;
+    if (DIR == 0) {
+        X[0] = flux ? ru : q.r;
+        X[1] = flux ? ru * q.u + q.p : ru;
+        X[2] = flux ? ru * q.v : rv;
+        X[3] = flux ? q.u * (e + q.p) : e;
+    } else {
+        X[0] = flux ? rv : q.r;
+        X[1] = flux ? ru * q.v : ru;
+        X[2] = flux ? rv * q.v + q.p : rv;
+        X[3] = flux ? q.v * (e + q.p) : e;
+    }
+}
+// The same flux by two neighbouring lanes: lane bit 0 takes the state half or
+// the flux half, which run one code, and ends with components 0 and 1 or 2 and
+// 3; only the face's basis is computed twice.  All lanes of the warp call it.
+template <int DIR>
+__device__ __forceinline__ double2 face_flux_pair(const double4 *__restrict__ cur, int32_t a, int32_t b, int32_t c,
+                                                  int32_t d, double g, const FluxDen &den, double lam) {
+    const bool flux = threadIdx.x & 1;
+    DivNR dv(den);
+    double T[4];
+    {
+        const Prim s0 = load_prim(cur, a), s1 = load_prim(cur, b), s2 = load_prim(cur, c), s3 = load_prim(cur, d);
+        dv.test_numerator(s0.p);
+        dv.test_numerator(s1.p);
+        dv.test_numerator(s2.p);
+        dv.test_numerator(s3.p);
+        double U1[4], U2[4], Um[4];
+        cons_state_nr<DIR>(s1, dv, U1);
+        cons_state_nr<DIR>(s2, dv, U2);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) Um[r] = (U1[r] + U2[r]) / 2.0;
+        EigNR E;
+        eigen_nr<DIR>(Um, g, dv, E);
+        double X[4], w0[4], w1[4], w2[4], w3[4], uL[4], uR[4], L[4], R[4];
+        point_half_nr<DIR>(s0, dv, flux, X); project_nr<DIR>(E, X, w0);
+        point_half_nr<DIR>(s1, dv, flux, X); project_nr<DIR>(E, X, w1);
+        point_half_nr<DIR>(s2, dv, flux, X); project_nr<DIR>(E, X, w2);
+        point_half_nr<DIR>(s3, dv, flux, X); project_nr<DIR>(E, X, w3);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) wcns_pair(w0[r], w1[r], w2[r], w3[r], dv, uL[r], uR[r]);
+        back_project_nr<DIR>(E, uL, L);
+        back_project_nr<DIR>(E, uR, R);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) T[r] = R[r] + (flux ? L[r] : -L[r]);
+    }
+    const bool ok = __shfl_xor_sync(0xffffffffu, (int)dv.ok, 1) && dv.ok;
+    double o[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const double got = __shfl_xor_sync(0xffffffffu, flux ? T[r] : T[2 + r], 1);
+        const double sum = flux ? T[2 + r] : got, dif = flux ? got : T[r];
+        o[r] = 0.5 * (sum - lam * dif);
+    }
+    if (!ok) {
+        const double4 f = face_flux_again<DIR>(cur, a, b, c, d, g, lam);
+        o[0] = flux ? f.z : f.x;
+        o[1] = flux ? f.w : f.y;
+    }
+    return make_double2(o[0], o[1]);
+}
+
 }  // namespace fdm

@@ -50,20 +50,27 @@ struct Grid2 {
 };
 
 // face i of row r in x lies between interior columns 3+i-1 and 3+i; the x
-// faces' blocks (nbx), then the y faces'
+// faces' blocks (nbx), then the y faces'.  Two lanes per face (as in
+// k_faces_pair): the faces fill the GPU a few times at most.
 template <int DIR>
 __device__ __forceinline__ void uface(const Grid2 &G, const double4 *__restrict__ cur, double4 *F, double g,
                                       const FluxDen &den, double lam, int t) {
     const int nfr = DIR == 0 ? G.nx + 1 : G.nx;          // faces per row
     const int nrow = DIR == 0 ? G.ny : G.ny + 1;
-    if (t >= nfr * nrow) return;
-    const int r = t / nfr, i = t - r * nfr;
+    const int f = min(t >> 1, nfr * nrow - 1);
+    const int r = f / nfr, i = f - r * nfr;
     const int step = DIR == 0 ? 1 : G.W, c = (int)G.at(3 + r, 3 + i);
-    store_record(F + t, face_flux_of<DIR>(cur, c - 2 * step, c - step, c, c + step, g, den, lam));
+    const double2 v = face_flux_pair<DIR>(cur, c - 2 * step, c - step, c, c + step, g, den, lam);
+    if (f == t >> 1) reinterpret_cast<double2 *>(F + f)[t & 1] = v;
 }
-__global__ void __launch_bounds__(64, 8) k_ufaces(Grid2 G, const double4 *__restrict__ cur, double4 *Fx, double4 *Fy,
+// One step (six launches), us: 45 x 38 19.4, 128 x 128 24.7, 256 x 256 57.6;
+// with one thread per face 21.6, 27.2, 58.5, and with launches that wait for
+// the end of the kernel before 30.9, 37.1, 67.8 (and the cells' divisions the
+// compiler's).
+__global__ void __launch_bounds__(64, 6) k_ufaces(Grid2 G, const double4 *__restrict__ cur, double4 *Fx, double4 *Fy,
                                                   double g, FluxDen den, double lam_x, double lam_y, int nbx) {
     const int b = blockIdx.x;
+    dep_begin();
     if (b < nbx) uface<0>(G, cur, Fx, g, den, lam_x, b * 64 + threadIdx.x);
     else uface<1>(G, cur, Fy, g, den, lam_y, (b - nbx) * 64 + threadIdx.x);
 }
@@ -99,6 +106,7 @@ __global__ void __launch_bounds__(128) k_ucells(const __grid_constant__ Grid2 G,
                                                 const __grid_constant__ CellCoef k, double tstep, int krk) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int ncell = G.nx * G.ny;
+    dep_begin();
     if (t >= ncell) {
         const int c = (int)t - ncell;   // corner record c of 36: 3 x 3 at each end of both sides
         if (krk == 3 && c < 36) {
@@ -158,11 +166,17 @@ extern "C" int fdm_time_advance_rk_uniform_static(const double *prim_in, double 
     const double4 *cur[3] = {in, U1, U2};
     double4 *next[3] = {U1, U2, out};
     const fdm::FluxDen den = fdm::flux_den(gama);
-    const unsigned nbx = nb((int64_t)(nx + 1) * ny, 64), nby = nb((int64_t)nx * (ny + 1), 64);
+    const unsigned nbx = nb((int64_t)(nx + 1) * ny, 32), nby = nb((int64_t)nx * (ny + 1), 32);
     for (int krk = 1; krk <= 3; ++krk) {
-        k_ufaces<<<nbx + nby, 64, 0, s>>>(G, cur[krk - 1], Fx, Fy, gama, den, lambda_x, lambda_y, (int)nbx);
-        k_ucells<<<nb((int64_t)nx * ny + 36, 128), 128, 0, s>>>(G, cur[krk - 1], in, next[krk - 1], Fx, Fy, gama,
-                                                                den, k, tstep, krk);
+        // the first launch waits for all of the caller's work before it, the
+        // later ones' threads for the kernel before
+        if (krk == 1)
+            k_ufaces<<<nbx + nby, 64, 0, s>>>(G, cur[0], Fx, Fy, gama, den, lambda_x, lambda_y, (int)nbx);
+        else
+            fdm::launch_after(s, nbx + nby, 64, k_ufaces, G, cur[krk - 1], Fx, Fy, gama, den, lambda_x, lambda_y,
+                              (int)nbx);
+        fdm::launch_after(s, nb((int64_t)nx * ny + 36, 128), 128, k_ucells, G, cur[krk - 1], in, next[krk - 1], Fx, Fy,
+                          gama, den, k, tstep, krk);
     }
     return cudaGetLastError() == cudaSuccess ? FDM_OK : FDM_ERR_CUDA;
 }
