@@ -326,7 +326,7 @@ __device__ __forceinline__ void ph_cell_tile(const BatchArgs &A, int krk, int m,
     if (i < M.T.NI)
         cell_item(M.T, M.LT, stage_cur(M, krk), M.B0, stage_next(M, krk), M.Fx, M.Fy, M.sc->tstep, krk, 0, M.gama,
                   M.den, i, rm, rs, lx, ly);
-    cells_block_reduce(rm, rs, lx, ly, M.res_part + t * 8, M.sc, krk == 3, S);
+    if (krk == 3) cells_block_reduce(rm, rs, lx, ly, M.res_part + t * 8, M.sc, true, S);
 }
 
 // ghosts of member m, tile t: j = 3 after a stage, j = 1 after a step

@@ -11,6 +11,8 @@
 //
 // State lives in three slot arrays of 32-byte (rho,u,v,p) records: interior
 // leaves (key order), ghost leaves, corner leaves, then the virtual slots.
+#include <algorithm>
+
 #include "handle.cuh"
 #include "items.cuh"
 #include "numerics.cuh"
@@ -149,6 +151,8 @@ __global__ void __launch_bounds__(256, MINB) k_cells(const __grid_constant__ Tab
     // an iteration after t_end (or after a NaN residual) leaves the state as it is
     if (i < T.NI && !(mode == 0 && sc->done))
         cell_item(T, LT, cur, un, next, Fx, Fy, sc->tstep, krk, mode, g, den, i, rm, rs, lx, ly);
+    // the norms and wave speeds of a step are those of its last stage
+    if (mode == 0 && krk != 3) return;
     cells_block_reduce(rm, rs, lx, ly, res_part + blockIdx.x * 8, sc, krk == 3 && mode == 0, S);
 }
 
@@ -182,23 +186,29 @@ __global__ void __launch_bounds__(128) k_ghost(Tables T, double4 *buf, GhostStat
     }
 }
 
-__global__ void k_lambda(int64_t NI, const double4 *__restrict__ cur, DevScalars *sc, double g) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+// Largest wave speeds.  One atomic per block, and only where it raises the
+// maximum: one per warp (32k of them on one word at 1.03 M leaves) took 46 us.
+__global__ void __launch_bounds__(256) k_lambda(int64_t NI, const double4 *__restrict__ cur, DevScalars *sc, double g) {
+    __shared__ double sx[8], sy[8];
     double lx = 0.0, ly = 0.0;
-    if (i < NI) {
-        const double4 o = cur[i];
+    for (int64_t i = blockIdx.x * 256ll + threadIdx.x; i < NI; i += gridDim.x * 256ll) {
+        const double4 o = load_record(cur + i);
         const double c = sqrt(g * o.w / o.x);
-        lx = fabs(o.y) + c;
-        ly = fabs(o.z) + c;
+        lx = fmax(lx, fabs(o.y) + c);
+        ly = fmax(ly, fabs(o.z) + c);
     }
     for (int o = 16; o; o >>= 1) {
         lx = fmax(lx, __shfl_xor_sync(0xffffffffu, lx, o));
         ly = fmax(ly, __shfl_xor_sync(0xffffffffu, ly, o));
     }
-    if ((threadIdx.x & 31) == 0) {
+    if ((threadIdx.x & 31) == 0) { sx[threadIdx.x >> 5] = lx; sy[threadIdx.x >> 5] = ly; }
+    __syncthreads();
+    if (threadIdx.x) return;
+    for (int k = 1; k < 8; ++k) { lx = fmax(lx, sx[k]); ly = fmax(ly, sy[k]); }
+    if (lx > __ldcg(&sc->lam_next_x))
         atomicMax((unsigned long long *)&sc->lam_next_x, (unsigned long long)__double_as_longlong(lx));
+    if (ly > __ldcg(&sc->lam_next_y))
         atomicMax((unsigned long long *)&sc->lam_next_y, (unsigned long long)__double_as_longlong(ly));
-    }
 }
 
 // lambda/time-step control (src/solution.F90:185-201)
@@ -310,7 +320,7 @@ void launch_blend(fdm_handle *h, const double4 *un, double4 *cur, int krk) {
     k_blend<<<nblk(h->NI, 256), 256, 0, h->s>>>(h->NI, un, h->Ut.as<double4>(), cur, krk);
 }
 void launch_lambda(fdm_handle *h, const double4 *cur) {
-    k_lambda<<<nblk(h->NI, 256), 256, 0, h->s>>>(h->NI, cur, h->scal.as<DevScalars>(), h->G.gama);
+    k_lambda<<<std::min(nblk(h->NI, 256), 8 * 148), 256, 0, h->s>>>(h->NI, cur, h->scal.as<DevScalars>(), h->G.gama);
 }
 void launch_step_control(fdm_handle *h) {
     k_step_control<<<1, 32, 0, h->s>>>(h->scal.as<DevScalars>(), h->p, 1, false);
