@@ -274,11 +274,12 @@ __device__ __forceinline__ void ph_face_tile(const BatchArgs &A, int krk, int m,
             __syncthreads();
         }
         if (w * 32 < nf) {
+            const GateFrag frag(S.gate.W);
             if (dir == 0)
-                gate_linear_chunk<0>(M.T, cur, M.Fx, S.gate.W, S.gate.xt[wid], M.logit_thr, M.jump_thr, lam, ig1,
+                gate_linear_chunk<0>(M.T, cur, M.Fx, frag, S.gate.xt[wid], M.logit_thr, M.jump_thr, lam, ig1,
                                      M.gama, M.GL.hx, M.GL.cnt, M.GL.jx, w);
             else
-                gate_linear_chunk<1>(M.T, cur, M.Fy, S.gate.W, S.gate.xt[wid], M.logit_thr, M.jump_thr, lam, ig1,
+                gate_linear_chunk<1>(M.T, cur, M.Fy, frag, S.gate.xt[wid], M.logit_thr, M.jump_thr, lam, ig1,
                                      M.gama, M.GL.hy, M.GL.cnt + 1, M.GL.jy, w);
         }
     } else if (w * 32 < nf) {

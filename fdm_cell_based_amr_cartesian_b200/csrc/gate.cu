@@ -28,7 +28,12 @@ struct GateDir {
     int32_t *hard;
     float *jump1;
 };
-// Stage 1, persistent: each warp takes 32 faces at a time.
+// Stage 1, persistent: each warp takes 32 faces at a time.  Bound by issue
+// slots and the XU pipe (64 tanh, 8 logarithms and 14 conversions from FP64
+// per face): the weights stay in registers, the FP32 arithmetic runs on
+// packed pairs and two values are rounded to BF16 at once.  1.03 M leaves
+// 103 us in a step of 0.472 ms; 155 in 0.528 with one value per instruction,
+// single roundings and the weights read from shared memory each time.
 __global__ void __launch_bounds__(128, 4) k_gate_linear(Tables T, const double4 *__restrict__ cur,
                                                         const float *__restrict__ P, float logit_thr,
                                                         float jump_thr, const DevScalars *__restrict__ sc, double g,
@@ -42,13 +47,14 @@ __global__ void __launch_bounds__(128, 4) k_gate_linear(Tables T, const double4 
     const double ig1 = 1.0 / (g - 1.0);
     XTile &Tt = tiles[wid];
     for (int k = GF; k < XLD; ++k) Tt.X[lane][k] = __float2bfloat16_rn(0.f);
+    const GateFrag frag(W);
     const int64_t nwarps = (int64_t)gridDim.x * 4;
     for (int64_t w = blockIdx.x * 4 + wid; w < wx + wy; w += nwarps) {
         if (w < wx)
-            gate_linear_chunk<0>(T, cur, X.F, W, Tt, logit_thr, jump_thr, sc->lambda_x, ig1, g, X.hard, count, X.jump1,
+            gate_linear_chunk<0>(T, cur, X.F, frag, Tt, logit_thr, jump_thr, sc->lambda_x, ig1, g, X.hard, count, X.jump1,
                                  w);
         else
-            gate_linear_chunk<1>(T, cur, Y.F, W, Tt, logit_thr, jump_thr, sc->lambda_y, ig1, g, Y.hard, count + 1,
+            gate_linear_chunk<1>(T, cur, Y.F, frag, Tt, logit_thr, jump_thr, sc->lambda_y, ig1, g, Y.hard, count + 1,
                                  Y.jump1, w - wx);
     }
 }
@@ -108,39 +114,162 @@ __global__ void k_face_samples(Tables T, const double4 *__restrict__ cur, double
 // -(y log g + neg_w (1-y) log(1-g)), g = sigmoid(z), for a minibatch; gradients
 // of the mean loss accumulate into grad (FP32 atomics), the loss sum into
 // loss.  Samples idx0 + k*step (mod n), k < B.
-struct TrainTile {
-    WarpTile t;
-    __nv_bfloat16 DA2[32][HLD], DA1[32][HLD];
-    float dz[32];
-};
-__global__ void __launch_bounds__(64) k_mlp_grad(const float *__restrict__ X, const float *__restrict__ Y, int64_t n,
-                                                 int64_t idx0, int64_t step, int64_t B, const float *__restrict__ P,
-                                                 float neg_w, float *grad, float *loss) {
+//
+// A warp takes 32 samples at a time and keeps everything in registers: the
+// accumulators of one product are the fragments of the next (as in
+// mlp_logits_regs), and the products over the samples take theirs transposed
+// (movmatrix).  The warps' gradients are summed in shared memory, so each
+// block adds once to the result.  Bound by the latency of that chain (two
+// groups of samples per warp at 65536) and by the call's three launches: one
+// step 16 us at 65536 samples and 29 at 262144; 66 and 84 through tiles in
+// shared memory, with an atomic per warp and gradient and two memsets before.
+// Blocks of eight warps at 255 registers; of four or twelve 4 to 6 us more.
+constexpr int TRAIN_TB = 256, TRAIN_ACC = 44;
+// 8 x 8 transpose of a fragment block
+__device__ __forceinline__ uint32_t transposed(uint32_t a) {
+    uint32_t d;
+    asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
+    return d;
+}
+__device__ __forceinline__ F2 bf16_pair(uint32_t p) {
+    return F2(__uint_as_float(p << 16), __uint_as_float(p & 0xffff0000u));
+}
+// forward GELU of a layer's accumulators: fragments h of the next layer and
+// the derivatives dg
+__device__ __forceinline__ void gelu_layer(const float c[4][4], uint32_t h[2][4], F2 dg[4][2]) {
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) h[nt >> 1][2 * (nt & 1) + i] = gelu_bf16(c[nt][2 * i], c[nt][2 * i + 1], &dg[nt][i]);
+}
+// adds the two row halves of a fragment's columns (nt, pair) to sum
+__device__ __forceinline__ void add_columns(const uint32_t h[2][4], F2 s0, F2 s1, F2 sum[4]) {
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+        sum[nt] = sum[nt] + (bf16_pair(h[nt >> 1][2 * (nt & 1)]) * s0 + bf16_pair(h[nt >> 1][2 * (nt & 1) + 1]) * s1);
+}
+// column nt*8 + 2t + i summed over the warp's rows: lane (g, t) gets the one
+// with nt = g/2, i = g%2
+__device__ __forceinline__ float lane_column(const F2 sum[4]) {
+    const int g = (threadIdx.x & 31) >> 2;
+    float out = 0.f;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        float v[2];
+        sum[c >> 1].get(v[0], v[1]);
+        float x = v[c & 1];
+        x += __shfl_xor_sync(0xffffffffu, x, 4);
+        x += __shfl_xor_sync(0xffffffffu, x, 8);
+        x += __shfl_xor_sync(0xffffffffu, x, 16);
+        if (g == c) out = x;
+    }
+    return out;
+}
+// where accumulator e = acc*32 + lane of a warp belongs: an index into grad,
+// -1 the loss, -2 nothing
+__device__ __forceinline__ int train_index(int e) {
+    const int acc = e >> 5, lane = e & 31, g = lane >> 2, t = lane & 3;
+    if (acc < 32) {
+        const int mt = acc >> 4, nt = (acc >> 2) & 3, i = acc & 3;
+        return P_W2 + (mt * 16 + g + 8 * (i >> 1)) * GH + nt * 8 + 2 * t + (i & 1);
+    }
+    if (acc < 40) {
+        const int mt = (acc - 32) >> 2, i = acc & 3;
+        return P_W1 + (mt * 16 + g + 8 * (i >> 1)) * GF + 2 * t + (i & 1);
+    }
+    const int col = (g >> 1) * 8 + 2 * t + (g & 1);
+    if (acc == 40) return P_B1 + col;
+    if (acc == 41) return P_B2 + col;
+    if (acc == 42) return P_W3 + col;
+    return lane == 0 ? P_B3 : lane == 1 ? -1 : -2;
+}
+__global__ void __launch_bounds__(TRAIN_TB) k_mlp_grad(const float *__restrict__ X, const float *__restrict__ Y,
+                                                       int64_t n, int64_t idx0, int64_t step, int64_t B,
+                                                       const float *__restrict__ P, float neg_w, float *grad,
+                                                       float *loss) {
+    constexpr int NW = TRAIN_TB / 32;
     __shared__ GateWeights W;
-    __shared__ TrainTile tiles[2];
+    __shared__ uint4 xs[NW][32];
+    __shared__ float red[NW / 2][TRAIN_ACC * 32];
     load_weights_smem(W, P);
     __syncthreads();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-    TrainTile &Tt = tiles[wid];
-    // per-warp gradient accumulators
-    float gW2[2][4][4], gW1[2][4];   // dW2: [mt over out][nt over in][i]; dW1: [mt over out][i], n = features
-    for (int a = 0; a < 2; ++a) {
-        for (int b = 0; b < 4; ++b) for (int i = 0; i < 4; ++i) gW2[a][b][i] = 0.f;
-        for (int i = 0; i < 4; ++i) gW1[a][i] = 0.f;
-    }
-    float gb1 = 0.f, gb2 = 0.f, gw3 = 0.f, gb3 = 0.f, ls = 0.f;   // lane j holds index j
+    const GateFrag fr(W);
+    uint32_t w2t[4][2][2];   // B[k = out][n = in] = W2[out][in]
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+        for (int kc = 0; kc < 2; ++kc)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) w2t[nt][kc][i] = transposed(fr.w2[2 * kc + i][nt >> 1][nt & 1]);
+    F2 w3c[4];
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) w3c[nt] = bf16_pair(*reinterpret_cast<const uint32_t *>(W.w3 + nt * 8 + 2 * t));
+    float acc[TRAIN_ACC];    // dW2 [mt over out][nt over in][i], dW1 [mt over out][i]
+#pragma unroll
+    for (int a = 0; a < TRAIN_ACC; ++a) acc[a] = 0.f;
+    F2 gb1[4], gb2[4], gw3[4];
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) gb1[nt] = gb2[nt] = gw3[nt] = F2(0.f);
+    float gb3 = 0.f, ls = 0.f;
     const float invB = 1.0f / (float)B;
+    const bool wide = ((uintptr_t)X & 15u) == 0;   // rows of 32 bytes: as two vectors where the base allows
     const int64_t ngroups = (B + 31) / 32;
-    for (int64_t grp = blockIdx.x * 2 + wid; grp < ngroups; grp += (int64_t)gridDim.x * 2) {
+    for (int64_t grp = blockIdx.x * (int64_t)NW + wid; grp < ngroups; grp += (int64_t)gridDim.x * NW) {
         const int64_t k = grp * 32 + lane;
         const bool valid = k < B;
         const int64_t s = (idx0 + k * step) % n;
-        float y = 0.f;
-        for (int q = 0; q < XLD; ++q) Tt.t.X[lane][q] = __float2bfloat16_rn(valid && q < GF ? X[s * GF + q] : 0.f);
-        if (valid) y = Y[s];
+        float y = 0.f, x[GF];
+#pragma unroll
+        for (int q = 0; q < GF; ++q) x[q] = 0.f;
+        if (valid) {
+            y = Y[s];
+            if (wide) {
+                const float4 u = *reinterpret_cast<const float4 *>(X + s * GF);
+                const float4 v = *reinterpret_cast<const float4 *>(X + s * GF + 4);
+                x[0] = u.x; x[1] = u.y; x[2] = u.z; x[3] = u.w;
+                x[4] = v.x; x[5] = v.y; x[6] = v.z; x[7] = v.w;
+            } else {
+#pragma unroll
+                for (int q = 0; q < GF; ++q) x[q] = X[s * GF + q];
+            }
+        }
         __syncwarp();
-        float a1[2][4][4], a2[2][4][4], z[2][2];
-        mlp_forward(W, Tt.t, a1, a2, z);
+        xs[wid][lane] = make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]),
+                                   pack_bf16(x[6], x[7]));
+        __syncwarp();
+        const uint32_t *xw = reinterpret_cast<const uint32_t *>(xs[wid]);
+        uint32_t xa[4];      // rows g, g+8, g+16, g+24, features 2t and 2t+1
+#pragma unroll
+        for (int q = 0; q < 4; ++q) xa[q] = xw[(g + 8 * q) * 4 + t];
+        uint32_t h1[2][2][4], h2[2][2][4];
+        F2 d1[2][4][2], d2[2][4][2];
+        float z[2][2];
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+            const uint32_t a[4] = {xa[2 * mt], xa[2 * mt + 1], 0u, 0u};
+            float c4[4][4];
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) {
+                const float c[4] = {fr.b1[nt][0], fr.b1[nt][1], fr.b1[nt][0], fr.b1[nt][1]};
+                mma16816(c4[nt], a, fr.w1[nt], c);
+            }
+            gelu_layer(c4, h1[mt], d1[mt]);
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) {
+                const float c[4] = {fr.b2[nt][0], fr.b2[nt][1], fr.b2[nt][0], fr.b2[nt][1]};
+                float d[4];
+                mma16816(d, h1[mt][0], fr.w2[nt][0], c);
+                mma16816(c4[nt], h1[mt][1], fr.w2[nt][1], d);
+            }
+            gelu_layer(c4, h2[mt], d2[mt]);
+            const float c[4] = {fr.b3, 0.f, fr.b3, 0.f};
+            float d[4], e[4];
+            mma16816(d, h2[mt][0], fr.w3[0], c);
+            mma16816(e, h2[mt][1], fr.w3[1], d);
+            z[mt][0] = e[0];
+            z[mt][1] = e[2];
+        }
         const float zl = row_logit(z, lane);
         const float gs = 1.0f / (1.0f + expf(-zl));
         if (valid) {
@@ -148,121 +277,108 @@ __global__ void __launch_bounds__(64) k_mlp_grad(const float *__restrict__ X, co
             ls += -(y * logf(gs + e) + neg_w * (1.0f - y) * logf(1.0f - gs + e));
         }
         // d/dz of -(y log g + a (1-y) log(1-g)) = g (y + a (1-y)) - y
-        Tt.dz[lane] = valid ? (gs * (y + neg_w * (1.0f - y)) - y) * invB : 0.f;
-        __syncwarp();
-        // dh2 = dz w3, da2 = dh2 gelu'(a2)
-        for (int mt = 0; mt < 2; ++mt)
+        const float dz = valid ? (gs * (y + neg_w * (1.0f - y)) - y) * invB : 0.f;
+        gb3 += dz;
+        uint32_t a2[2][2][4], a1[2][2][4];   // dA2, dA1 as fragments
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+            const F2 z0(__shfl_sync(0xffffffffu, dz, mt * 16 + g)), z1(__shfl_sync(0xffffffffu, dz, mt * 16 + g + 8));
+            // dw3[j] = sum_s h2[s][j] dz[s]
+            add_columns(h2[mt], z0, z1, gw3);
+            // dh2 = dz w3, da2 = dh2 gelu'(a2); db2[j] = sum_s da2[s][j]
+#pragma unroll
             for (int nt = 0; nt < 4; ++nt)
-                for (int i = 0; i < 4; ++i) {
-                    const int r = mt * 16 + g + 8 * (i >> 1), c = nt * 8 + 2 * t + (i & 1);
-                    const float v = Tt.dz[r] * __bfloat162float(W.w3[c]) * gelu_grad(a2[mt][nt][i]);
-                    Tt.DA2[r][c] = __float2bfloat16_rn(v);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    float lo, hi;
+                    ((i ? z1 : z0) * w3c[nt] * d2[mt][nt][i]).get(lo, hi);
+                    a2[mt][nt >> 1][2 * (nt & 1) + i] = pack_bf16(lo, hi);
                 }
-        __syncwarp();
-        // dw3[j] = sum_s h2[s][j] dz[s]; db3 = sum dz; db2[j] = sum_s da2[s][j]
-        {
-            float sw = 0.f, sb = 0.f;
-            for (int r = 0; r < 32; ++r) {
-                sw += __bfloat162float(Tt.t.H2[r][lane]) * Tt.dz[r];
-            }
-            gw3 += sw;
-            for (int r = 0; r < 32; ++r) sb += __bfloat162float(Tt.DA2[r][lane]);
-            gb2 += sb;
-            gb3 += Tt.dz[lane];
-        }
-        // dh1 = DA2 W2 (B[k=o][n=i] = W2[o][i]); da1 = dh1 gelu'(a1)
-        for (int mt = 0; mt < 2; ++mt)
+            add_columns(a2[mt], F2(1.f), F2(1.f), gb2);
+            // dh1 = dA2 W2; da1 = dh1 gelu'(a1)
+#pragma unroll
             for (int nt = 0; nt < 4; ++nt) {
-                float c[4] = {0.f, 0.f, 0.f, 0.f};
-                for (int kc = 0; kc < 2; ++kc) {
-                    uint32_t a[4], b[2];
-                    load_a<HLD>(Tt.DA2, mt * 16, kc * 16, a);
-                    const int nn = nt * 8 + g, kk = kc * 16 + 2 * t;
-                    b[0] = (uint32_t)__bfloat16_as_ushort(W.W2[kk][nn]) | ((uint32_t)__bfloat16_as_ushort(W.W2[kk + 1][nn]) << 16);
-                    b[1] = (uint32_t)__bfloat16_as_ushort(W.W2[kk + 8][nn]) | ((uint32_t)__bfloat16_as_ushort(W.W2[kk + 9][nn]) << 16);
-                    float d[4];
-                    mma16816(d, a, b, c);
+                const float c[4] = {0.f, 0.f, 0.f, 0.f};
+                float d[4], e[4];
+                mma16816(d, a2[mt][0], w2t[nt][0], c);
+                mma16816(e, a2[mt][1], w2t[nt][1], d);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    float lo, hi;
+                    (F2(e[2 * i], e[2 * i + 1]) * d1[mt][nt][i]).get(lo, hi);
+                    a1[mt][nt >> 1][2 * (nt & 1) + i] = pack_bf16(lo, hi);
+                }
+            }
+            add_columns(a1[mt], F2(1.f), F2(1.f), gb1);
+        }
+        // dW2[o][i] += sum_s dA2[s][o] H1[s][i], dW1[o][f] += sum_s dA1[s][o] X[s][f]:
+        // A[m = o][k = s] and B[k = s][n = i] are the transposed blocks
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {     // samples 16 ks .. 16 ks + 15
+            uint32_t bh[4][2];
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt) {
+                bh[nt][0] = transposed(h1[ks][nt >> 1][2 * (nt & 1)]);
+                bh[nt][1] = transposed(h1[ks][nt >> 1][2 * (nt & 1) + 1]);
+            }
+            const uint32_t bx[2] = {transposed(xa[2 * ks]), transposed(xa[2 * ks + 1])};
+#pragma unroll
+            for (int mo = 0; mo < 2; ++mo) { // outputs 16 mo .. 16 mo + 15: rows o, o+8 by samples s, s+8
+                const uint32_t at2[4] = {transposed(a2[ks][mo][0]), transposed(a2[ks][mo][2]),
+                                         transposed(a2[ks][mo][1]), transposed(a2[ks][mo][3])};
+#pragma unroll
+                for (int nt = 0; nt < 4; ++nt) {
+                    float *c = acc + mo * 16 + nt * 4, d[4];
+                    mma16816(d, at2, bh[nt], c);
                     c[0] = d[0]; c[1] = d[1]; c[2] = d[2]; c[3] = d[3];
                 }
-                for (int i = 0; i < 4; ++i) {
-                    const int r = mt * 16 + g + 8 * (i >> 1), cc = nt * 8 + 2 * t + (i & 1);
-                    Tt.DA1[r][cc] = __float2bfloat16_rn(c[i] * gelu_grad(a1[mt][nt][i]));
-                }
+                const uint32_t at1[4] = {transposed(a1[ks][mo][0]), transposed(a1[ks][mo][2]),
+                                         transposed(a1[ks][mo][1]), transposed(a1[ks][mo][3])};
+                float *c = acc + 32 + mo * 4, d[4];
+                mma16816(d, at1, bx, c);
+                c[0] = d[0]; c[1] = d[1]; c[2] = d[2]; c[3] = d[3];
             }
-        __syncwarp();
-        {
-            float sb = 0.f;
-            for (int r = 0; r < 32; ++r) sb += __bfloat162float(Tt.DA1[r][lane]);
-            gb1 += sb;
-        }
-        // dW2[o][i] += sum_s DA2[s][o] H1[s][i]: A[m=o][k=s], B[k=s][n=i]
-        for (int mt = 0; mt < 2; ++mt)
-            for (int kc = 0; kc < 2; ++kc) {
-                uint32_t a[4];
-                {
-                    const int o0 = mt * 16 + g, o1 = o0 + 8, s0 = kc * 16 + 2 * t, s1 = s0 + 8;
-                    a[0] = (uint32_t)__bfloat16_as_ushort(Tt.DA2[s0][o0]) | ((uint32_t)__bfloat16_as_ushort(Tt.DA2[s0 + 1][o0]) << 16);
-                    a[1] = (uint32_t)__bfloat16_as_ushort(Tt.DA2[s0][o1]) | ((uint32_t)__bfloat16_as_ushort(Tt.DA2[s0 + 1][o1]) << 16);
-                    a[2] = (uint32_t)__bfloat16_as_ushort(Tt.DA2[s1][o0]) | ((uint32_t)__bfloat16_as_ushort(Tt.DA2[s1 + 1][o0]) << 16);
-                    a[3] = (uint32_t)__bfloat16_as_ushort(Tt.DA2[s1][o1]) | ((uint32_t)__bfloat16_as_ushort(Tt.DA2[s1 + 1][o1]) << 16);
-                }
-                for (int nt = 0; nt < 4; ++nt) {
-                    uint32_t b[2];
-                    const int nn = nt * 8 + g, kk = kc * 16 + 2 * t;
-                    b[0] = (uint32_t)__bfloat16_as_ushort(Tt.t.H1[kk][nn]) | ((uint32_t)__bfloat16_as_ushort(Tt.t.H1[kk + 1][nn]) << 16);
-                    b[1] = (uint32_t)__bfloat16_as_ushort(Tt.t.H1[kk + 8][nn]) | ((uint32_t)__bfloat16_as_ushort(Tt.t.H1[kk + 9][nn]) << 16);
-                    float d[4];
-                    mma16816(d, a, b, gW2[mt][nt]);
-                    for (int i = 0; i < 4; ++i) gW2[mt][nt][i] = d[i];
-                }
-            }
-        // dW1[o][f] += sum_s DA1[s][o] X[s][f]: N = 8 features (one n-tile)
-        for (int mt = 0; mt < 2; ++mt)
-            for (int kc = 0; kc < 2; ++kc) {
-                uint32_t a[4], b[2];
-                const int o0 = mt * 16 + g, o1 = o0 + 8, s0 = kc * 16 + 2 * t, s1 = s0 + 8;
-                a[0] = (uint32_t)__bfloat16_as_ushort(Tt.DA1[s0][o0]) | ((uint32_t)__bfloat16_as_ushort(Tt.DA1[s0 + 1][o0]) << 16);
-                a[1] = (uint32_t)__bfloat16_as_ushort(Tt.DA1[s0][o1]) | ((uint32_t)__bfloat16_as_ushort(Tt.DA1[s0 + 1][o1]) << 16);
-                a[2] = (uint32_t)__bfloat16_as_ushort(Tt.DA1[s1][o0]) | ((uint32_t)__bfloat16_as_ushort(Tt.DA1[s1 + 1][o0]) << 16);
-                a[3] = (uint32_t)__bfloat16_as_ushort(Tt.DA1[s1][o1]) | ((uint32_t)__bfloat16_as_ushort(Tt.DA1[s1 + 1][o1]) << 16);
-                const int kk = kc * 16 + 2 * t;
-                b[0] = (uint32_t)__bfloat16_as_ushort(Tt.t.X[kk][g]) | ((uint32_t)__bfloat16_as_ushort(Tt.t.X[kk + 1][g]) << 16);
-                b[1] = (uint32_t)__bfloat16_as_ushort(Tt.t.X[kk + 8][g]) | ((uint32_t)__bfloat16_as_ushort(Tt.t.X[kk + 9][g]) << 16);
-                float d[4];
-                mma16816(d, a, b, gW1[mt]);
-                for (int i = 0; i < 4; ++i) gW1[mt][i] = d[i];
-            }
-        __syncwarp();
-    }
-    // flush the warp's accumulators
-    for (int mt = 0; mt < 2; ++mt) {
-        for (int nt = 0; nt < 4; ++nt)
-            for (int i = 0; i < 4; ++i) {
-                const int o = mt * 16 + g + 8 * (i >> 1), in = nt * 8 + 2 * t + (i & 1);
-                atomicAdd(grad + P_W2 + o * GH + in, gW2[mt][nt][i]);
-            }
-        for (int i = 0; i < 4; ++i) {
-            const int o = mt * 16 + g + 8 * (i >> 1), fi = 2 * t + (i & 1);
-            atomicAdd(grad + P_W1 + o * GF + fi, gW1[mt][i]);
         }
     }
-    atomicAdd(grad + P_B1 + lane, gb1);
-    atomicAdd(grad + P_B2 + lane, gb2);
-    atomicAdd(grad + P_W3 + lane, gw3);
+    acc[40] = lane_column(gb1);
+    acc[41] = lane_column(gb2);
+    acc[42] = lane_column(gw3);
     for (int o = 16; o; o >>= 1) {
         gb3 += __shfl_xor_sync(0xffffffffu, gb3, o);
         ls += __shfl_xor_sync(0xffffffffu, ls, o);
     }
-    if (lane == 0) {
-        atomicAdd(grad + P_B3, gb3);
-        atomicAdd(loss, ls);
+    acc[43] = lane == 0 ? gb3 : ls;
+    dep_begin();   // the results are cleared; what is read above was final before the kernel that clears them
+    // the upper half of the warps to the lower half, those to all threads
+    if (wid >= NW / 2)
+#pragma unroll
+        for (int a = 0; a < TRAIN_ACC; ++a) red[wid - NW / 2][a * 32 + lane] = acc[a];
+    __syncthreads();
+    if (wid < NW / 2)
+#pragma unroll
+        for (int a = 0; a < TRAIN_ACC; ++a) red[wid][a * 32 + lane] += acc[a];
+    __syncthreads();
+    for (int e = threadIdx.x; e < TRAIN_ACC * 32; e += TRAIN_TB) {
+        float v = red[0][e];
+#pragma unroll
+        for (int w = 1; w < NW / 2; ++w) v += red[w][e];
+        const int at = train_index(e);
+        if (at >= 0) atomicAdd(grad + at, v);
+        else if (at == -1) atomicAdd(loss, v);
     }
+}
+
+__global__ void k_train_clear(float *grad, float *loss) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < P_N) grad[i] = 0.f;
+    else if (i == P_N) *loss = 0.f;
 }
 
 // Adam (FP32 master weights)
 __global__ void k_adam(float *P, const float *grad, float *m, float *v, int64_t n, float lr, float b1, float b2,
                        float eps, float c1, float c2) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    dep_begin();
     if (i >= n) return;
     const float gi = grad[i];
     const float mi = b1 * m[i] + (1.f - b1) * gi;
@@ -285,7 +401,7 @@ __global__ void __launch_bounds__(128) k_mlp_eval(const float *__restrict__ X, i
     for (int q = 0; q < XLD; ++q) Tt.X[lane][q] = __float2bfloat16_rn(r < n && q < GF ? X[r * GF + q] : 0.f);
     __syncwarp();
     float z[2][2];
-    mlp_logits_regs(W, Tt.X, z);
+    mlp_logits_regs(GateFrag(W), Tt.X, z);
     const float zl = row_logit(z, lane);
     if (r < n) prob[r] = 1.0f / (1.0f + expf(-zl));
 }
@@ -417,16 +533,16 @@ extern "C" int fdm_gate_train_step(const float *X, const float *Y, int64_t n, in
         !(neg_weight > 0.f))
         return FDM_ERR_ARG;
     cudaStream_t s = (cudaStream_t)stream;
-    if (cudaMemsetAsync(grad, 0, P_N * sizeof(float), s) != cudaSuccess) return FDM_ERR_CUDA;
-    if (cudaMemsetAsync(loss, 0, sizeof(float), s) != cudaSuccess) return FDM_ERR_CUDA;
+    // waits for all of the caller's work before it, so the weights and samples
+    // are final for the next kernel however early that one starts
+    k_train_clear<<<(P_N + 256) / 256, 256, 0, s>>>(grad, loss);
     const int64_t ngroups = (B + 31) / 32;
-    int blocks = (int)((ngroups + 1) / 2);
-    if (blocks > 1184) blocks = 1184;
-    k_mlp_grad<<<blocks, 64, 0, s>>>(X, Y, n, idx0, step, B, params, neg_weight, grad, loss);
+    const int64_t blocks = std::min<int64_t>((ngroups + TRAIN_TB / 32 - 1) / (TRAIN_TB / 32), sm_count());
+    launch_after(s, (unsigned)blocks, TRAIN_TB, k_mlp_grad, X, Y, n, idx0, step, B, params, neg_weight, grad, loss);
     if (lr > 0.f) {
         const float b1 = 0.9f, b2 = 0.999f;
         const float c1 = 1.f - powf(b1, (float)t), c2 = 1.f - powf(b2, (float)t);
-        k_adam<<<(P_N + 255) / 256, 256, 0, s>>>(params, grad, adam_m, adam_v, P_N, lr, b1, b2, 1e-8f, c1, c2);
+        launch_after(s, (P_N + 255) / 256, 256, k_adam, params, grad, adam_m, adam_v, P_N, lr, b1, b2, 1e-8f, c1, c2);
     }
     return cudaGetLastError() == cudaSuccess ? FDM_OK : FDM_ERR_CUDA;
 }

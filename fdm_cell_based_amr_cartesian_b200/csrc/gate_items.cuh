@@ -160,15 +160,17 @@ __device__ __forceinline__ void face_flux_linear(const Prim &s0, const Prim &s1,
 }
 
 // ------------------------------------------------------- tensor-core MLP
+// both rounded to nearest in one instruction
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
-    const __nv_bfloat16 a = __float2bfloat16_rn(lo), b = __float2bfloat16_rn(hi);
-    return (uint32_t)__bfloat16_as_ushort(a) | ((uint32_t)__bfloat16_as_ushort(b) << 16);
+    uint32_t d;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+    return d;
 }
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
 // D = A(16x16 bf16, row) * B(16x8 bf16, col) + C (f32)
 __device__ __forceinline__ void mma16816(float d[4], const uint32_t a[4], const uint32_t b[2], const float c[4]) {
-    asm volatile(
+    asm(
         "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
         "{%10,%11,%12,%13};\n"
         : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
@@ -183,17 +185,40 @@ __device__ __forceinline__ float tanh_fast(float x) {
     asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ float gelu(float x) {
-    const float k = 0.7978845608028654f;
-    const float t = tanh_fast(k * (x + 0.044715f * x * x * x));
-    return 0.5f * x * (1.0f + t);
+// packed pairs of floats: two operations in one instruction
+struct F2 {
+    unsigned long long v;
+    __device__ __forceinline__ F2() = default;
+    __device__ __forceinline__ F2(float lo, float hi) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi)); }
+    __device__ __forceinline__ explicit F2(float x) : F2(x, x) {}
+    __device__ __forceinline__ void get(float &lo, float &hi) const {
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+    }
+};
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) {
+    F2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
+    return d;
 }
-__device__ __forceinline__ float gelu_grad(float x) {
-    const float k = 0.7978845608028654f;
-    const float t = tanh_fast(k * (x + 0.044715f * x * x * x));
-    return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * k * (1.0f + 3.0f * 0.044715f * x * x);
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) {
+    F2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
+    return d;
 }
-
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) {   // exact sign change, one rounding
+    return a + F2(-1.0f) * b;
+}
+// GELU (tanh form) of a pair, rounded to BF16; dx: its derivative
+__device__ __forceinline__ uint32_t gelu_bf16(float x0, float x1, F2 *dx = nullptr) {
+    const float k = 0.7978845608028654f;
+    const F2 x(x0, x1), u = F2(k) * (x + F2(0.044715f) * x * x * x);
+    float u0, u1, y0, y1;
+    u.get(u0, u1);
+    const F2 t(tanh_fast(u0), tanh_fast(u1)), one(1.0f), half(0.5f);
+    (half * x * (one + t)).get(y0, y1);
+    if (dx) *dx = half * (one + t) + half * x * (one - t * t) * F2(k) * (one + F2(3.0f * 0.044715f) * x * x);
+    return pack_bf16(y0, y1);
+}
 // Shared-memory row pitches (bf16 elements), padded so that the fragment
 // reads of a warp (rows g = lane/4, word t = lane%4) hit distinct banks.
 constexpr int XLD = 24, HLD = 40;
@@ -209,14 +234,6 @@ struct __align__(16) GateWeights {
 // Per-warp staging of the 32 feature rows for inference
 struct __align__(16) XTile {
     __nv_bfloat16 X[32][XLD];   // columns GF.. stay zero
-};
-
-// Per-warp staging of 32 samples (rows) in shared memory; rows of X are
-// written as one 16-byte vector per lane (row pitch 48 bytes)
-struct __align__(16) WarpTile {
-    __nv_bfloat16 X[32][XLD];   // columns GF.. stay zero
-    __nv_bfloat16 H1[32][HLD];
-    __nv_bfloat16 H2[32][HLD];
 };
 
 // A fragment (rows m0..m0+15, cols k0..k0+15) of a row-major bf16 tile
@@ -238,130 +255,75 @@ __device__ __forceinline__ void load_b_wt(const __nv_bfloat16 (*W)[LD], int n0, 
     b[1] = (uint32_t)__bfloat16_as_ushort(W[n][k + 8]) | ((uint32_t)__bfloat16_as_ushort(W[n][k + 9]) << 16);
 }
 
-// Forward pass of 32 samples staged in T.X; pre-activations a1, a2 and the
-// logits z (per row) are returned, h1 / h2 are left in T.H1 / T.H2.
-// Layouts: acc[mt][nt][i] is row mt*16 + g + 8*(i>>1), col nt*8 + 2t + (i&1).
-__device__ __forceinline__ void mlp_forward(const GateWeights &W, WarpTile &T, float a1[2][4][4], float a2[2][4][4],
-                                            float z[2][2]) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    for (int mt = 0; mt < 2; ++mt) {
-        uint32_t a[4];
-        load_a<XLD>(T.X, mt * 16, 0, a);
+// Accumulator layouts: acc[mt][nt][i] is row mt*16 + g + 8*(i>>1), col
+// nt*8 + 2t + (i&1), with g = lane/4, t = lane%4.
+// The weights as a warp's B fragments, read once and kept in registers.
+struct GateFrag {
+    uint32_t w1[4][2], w2[4][2][2], w3[2][2];
+    float b1[4][2], b2[4][2], b3;
+    __device__ __forceinline__ explicit GateFrag(const GateWeights &W) {
+        const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
-            uint32_t b[2];
-            load_b_wt<XLD>(W.W1, nt * 8, 0, b);
-            const float c[4] = {W.b1[nt * 8 + 2 * t], W.b1[nt * 8 + 2 * t + 1], W.b1[nt * 8 + 2 * t],
-                                W.b1[nt * 8 + 2 * t + 1]};
-            mma16816(a1[mt][nt], a, b, c);
-        }
-        for (int nt = 0; nt < 4; ++nt)
-            for (int i = 0; i < 4; ++i)
-                T.H1[mt * 16 + g + 8 * (i >> 1)][nt * 8 + 2 * t + (i & 1)] = __float2bfloat16_rn(gelu(a1[mt][nt][i]));
-    }
-    __syncwarp();
-    for (int mt = 0; mt < 2; ++mt) {
-        for (int nt = 0; nt < 4; ++nt) {
-            float c[4] = {W.b2[nt * 8 + 2 * t], W.b2[nt * 8 + 2 * t + 1], W.b2[nt * 8 + 2 * t],
-                          W.b2[nt * 8 + 2 * t + 1]};
-            for (int kc = 0; kc < 2; ++kc) {
-                uint32_t a[4], b[2];
-                load_a<HLD>(T.H1, mt * 16, kc * 16, a);
-                load_b_wt<HLD>(W.W2, nt * 8, kc * 16, b);
-                float d[4];
-                mma16816(d, a, b, c);
-                c[0] = d[0]; c[1] = d[1]; c[2] = d[2]; c[3] = d[3];
+            load_b_wt<XLD>(W.W1, nt * 8, 0, w1[nt]);
+            load_b_wt<HLD>(W.W2, nt * 8, 0, w2[nt][0]);
+            load_b_wt<HLD>(W.W2, nt * 8, 16, w2[nt][1]);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                b1[nt][i] = W.b1[nt * 8 + 2 * t + i];
+                b2[nt][i] = W.b2[nt * 8 + 2 * t + i];
             }
-            for (int i = 0; i < 4; ++i) a2[mt][nt][i] = c[i];
         }
-        for (int nt = 0; nt < 4; ++nt)
-            for (int i = 0; i < 4; ++i)
-                T.H2[mt * 16 + g + 8 * (i >> 1)][nt * 8 + 2 * t + (i & 1)] = __float2bfloat16_rn(gelu(a2[mt][nt][i]));
+#pragma unroll
+        for (int kc = 0; kc < 2; ++kc)   // N padded to 8, only column 0 is w3
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int k = kc * 16 + 2 * t + 8 * i;
+                w3[kc][i] = g == 0 ? *reinterpret_cast<const uint32_t *>(W.w3 + k) : 0u;
+            }
+        b3 = W.b3;
     }
-    __syncwarp();
-    // layer 3: N padded to 8, only column 0 is w3
-    for (int mt = 0; mt < 2; ++mt) {
-        float c[4] = {W.b3, 0.f, W.b3, 0.f};
-        for (int kc = 0; kc < 2; ++kc) {
-            uint32_t a[4], b[2];
-            load_a<HLD>(T.H2, mt * 16, kc * 16, a);
-            const int k = kc * 16 + 2 * t;
-            const __nv_bfloat16 zero = __float2bfloat16_rn(0.f);
-            const __nv_bfloat16 w0 = g == 0 ? W.w3[k] : zero, w1 = g == 0 ? W.w3[k + 1] : zero;
-            const __nv_bfloat16 w8 = g == 0 ? W.w3[k + 8] : zero, w9 = g == 0 ? W.w3[k + 9] : zero;
-            b[0] = (uint32_t)__bfloat16_as_ushort(w0) | ((uint32_t)__bfloat16_as_ushort(w1) << 16);
-            b[1] = (uint32_t)__bfloat16_as_ushort(w8) | ((uint32_t)__bfloat16_as_ushort(w9) << 16);
-            float d[4];
-            mma16816(d, a, b, c);
-            c[0] = d[0]; c[1] = d[1]; c[2] = d[2]; c[3] = d[3];
-        }
-        z[mt][0] = c[0];   // row mt*16 + g (valid in lanes with t == 0)
-        z[mt][1] = c[2];   // row mt*16 + g + 8
-    }
-}
+};
 // Inference forward of the 32 samples in T.X with the hidden activations
 // kept in registers: the m16n8 accumulators of n-tiles 2kc and 2kc+1 are,
 // after GELU and BF16 rounding, exactly the m16k16 A fragment of k-chunk kc
 // of the next layer (rows g, g+8; columns 2t, 2t+1 and 2t+8, 2t+9), so no
-// shared-memory round trip is needed.  Same values as mlp_forward.
-__device__ __forceinline__ void mlp_logits_regs(const GateWeights &W, const __nv_bfloat16 (*X)[XLD], float z[2][2]) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+// shared-memory round trip is needed.
+__device__ __forceinline__ void gelu_fragment(const float c[4][4], uint32_t h[2][4]) {
+#pragma unroll
+    for (int kc = 0; kc < 2; ++kc) {
+        h[kc][0] = gelu_bf16(c[2 * kc][0], c[2 * kc][1]);
+        h[kc][1] = gelu_bf16(c[2 * kc][2], c[2 * kc][3]);
+        h[kc][2] = gelu_bf16(c[2 * kc + 1][0], c[2 * kc + 1][1]);
+        h[kc][3] = gelu_bf16(c[2 * kc + 1][2], c[2 * kc + 1][3]);
+    }
+}
+__device__ __forceinline__ void mlp_logits_regs(const GateFrag &W, const __nv_bfloat16 (*X)[XLD], float z[2][2]) {
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt) {
-        uint32_t a[4];
+        uint32_t a[4], h[2][4];
         load_a<XLD>(X, mt * 16, 0, a);
-        float c1[4][4];
+        float acc[4][4];
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
-            uint32_t b[2];
-            load_b_wt<XLD>(W.W1, nt * 8, 0, b);
-            const float bb0 = W.b1[nt * 8 + 2 * t], bb1 = W.b1[nt * 8 + 2 * t + 1];
-            const float c[4] = {bb0, bb1, bb0, bb1};
-            mma16816(c1[nt], a, b, c);
+            const float c[4] = {W.b1[nt][0], W.b1[nt][1], W.b1[nt][0], W.b1[nt][1]};
+            mma16816(acc[nt], a, W.w1[nt], c);
         }
-        uint32_t h1[2][4];
-#pragma unroll
-        for (int kc = 0; kc < 2; ++kc) {
-            h1[kc][0] = pack_bf16(gelu(c1[2 * kc][0]), gelu(c1[2 * kc][1]));
-            h1[kc][1] = pack_bf16(gelu(c1[2 * kc][2]), gelu(c1[2 * kc][3]));
-            h1[kc][2] = pack_bf16(gelu(c1[2 * kc + 1][0]), gelu(c1[2 * kc + 1][1]));
-            h1[kc][3] = pack_bf16(gelu(c1[2 * kc + 1][2]), gelu(c1[2 * kc + 1][3]));
-        }
-        float c2[4][4];
+        gelu_fragment(acc, h);
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
-            const float bb0 = W.b2[nt * 8 + 2 * t], bb1 = W.b2[nt * 8 + 2 * t + 1];
-            float c[4] = {bb0, bb1, bb0, bb1};
-#pragma unroll
-            for (int kc = 0; kc < 2; ++kc) {
-                uint32_t b[2];
-                load_b_wt<HLD>(W.W2, nt * 8, kc * 16, b);
-                float d[4];
-                mma16816(d, h1[kc], b, c);
-                c[0] = d[0]; c[1] = d[1]; c[2] = d[2]; c[3] = d[3];
-            }
-            c2[nt][0] = c[0]; c2[nt][1] = c[1]; c2[nt][2] = c[2]; c2[nt][3] = c[3];
-        }
-        float c[4] = {W.b3, 0.f, W.b3, 0.f};
-#pragma unroll
-        for (int kc = 0; kc < 2; ++kc) {
-            uint32_t h2[4];
-            h2[0] = pack_bf16(gelu(c2[2 * kc][0]), gelu(c2[2 * kc][1]));
-            h2[1] = pack_bf16(gelu(c2[2 * kc][2]), gelu(c2[2 * kc][3]));
-            h2[2] = pack_bf16(gelu(c2[2 * kc + 1][0]), gelu(c2[2 * kc + 1][1]));
-            h2[3] = pack_bf16(gelu(c2[2 * kc + 1][2]), gelu(c2[2 * kc + 1][3]));
-            const int k = kc * 16 + 2 * t;
-            const __nv_bfloat16 zero = __float2bfloat16_rn(0.f);
-            const __nv_bfloat16 w0 = g == 0 ? W.w3[k] : zero, w1 = g == 0 ? W.w3[k + 1] : zero;
-            const __nv_bfloat16 w8 = g == 0 ? W.w3[k + 8] : zero, w9 = g == 0 ? W.w3[k + 9] : zero;
-            uint32_t b[2];
-            b[0] = (uint32_t)__bfloat16_as_ushort(w0) | ((uint32_t)__bfloat16_as_ushort(w1) << 16);
-            b[1] = (uint32_t)__bfloat16_as_ushort(w8) | ((uint32_t)__bfloat16_as_ushort(w9) << 16);
+            const float c[4] = {W.b2[nt][0], W.b2[nt][1], W.b2[nt][0], W.b2[nt][1]};
             float d[4];
-            mma16816(d, h2, b, c);
-            c[0] = d[0]; c[1] = d[1]; c[2] = d[2]; c[3] = d[3];
+            mma16816(d, h[0], W.w2[nt][0], c);
+            mma16816(acc[nt], h[1], W.w2[nt][1], d);
         }
-        z[mt][0] = c[0];
-        z[mt][1] = c[2];
+        gelu_fragment(acc, h);
+        const float c[4] = {W.b3, 0.f, W.b3, 0.f};
+        float d[4], e[4];
+        mma16816(d, h[0], W.w3[0], c);
+        mma16816(e, h[1], W.w3[1], d);
+        z[mt][0] = e[0];
+        z[mt][1] = e[2];
     }
 }
 
@@ -424,20 +386,18 @@ __device__ __forceinline__ void append_hard(bool want, int64_t f, int lane, int3
 // features (the baseline the network is measured against).
 template <int DIR>
 __device__ __forceinline__ void gate_linear_chunk(const Tables &T, const double4 *__restrict__ cur, double4 *F,
-                                                  const GateWeights &W, XTile &Tt, float logit_thr, float jump_thr,
+                                                  const GateFrag &W, XTile &Tt, float logit_thr, float jump_thr,
                                                   double lam, double ig1, double g, int32_t *hard, uint32_t *count,
                                                   float *jump1, int64_t w) {
     const int lane = threadIdx.x & 31;
     const int64_t nf = T.NI + (DIR == 0 ? T.nux : T.nuy);
     const int64_t f = w * 32 + lane;
     const bool in = f < nf;
-    Prim p0, p1, p2, p3;
+    int32_t a = 0, b = 0, c = 0, d = 0;
     float feat[GF], jm = 0.f;
     if (in) {
-        int32_t a, b, c, d;
         face_slots<DIR>(T, f, a, b, c, d);
-        p0 = load_prim(cur, a); p1 = load_prim(cur, b); p2 = load_prim(cur, c); p3 = load_prim(cur, d);
-        face_features<DIR>(p0, p1, p2, p3, g, feat, &jm);
+        face_features<DIR>(load_prim(cur, a), load_prim(cur, b), load_prim(cur, c), load_prim(cur, d), g, feat, &jm);
     } else {
         for (int k = 0; k < GF; ++k) feat[k] = 0.f;
     }
@@ -451,8 +411,8 @@ __device__ __forceinline__ void gate_linear_chunk(const Tables &T, const double4
     const float zl = row_logit(z, lane);
     const bool lin = in && (jump_thr >= 0.f ? jm <= jump_thr : zl >= logit_thr);
     if (lin) {
-        double out[4];
-        face_flux_linear<DIR>(p0, p1, p2, p3, ig1, lam, out);
+        double out[4];   // the records again: the registers hold the weights over the network
+        face_flux_linear<DIR>(load_prim(cur, a), load_prim(cur, b), load_prim(cur, c), load_prim(cur, d), ig1, lam, out);
         store_record(F + f, make_double4(out[0], out[1], out[2], out[3]));
     }
     if (in) jump1[f] = lin ? jm : -1.0f;
