@@ -530,13 +530,17 @@ __global__ void k_gm1_links(NodeSet A, Geometry G, Links L, int8_t *d) {
     L.rank[i] = post_rank(k);
 }
 // "the same-level node N exists and has sons" when x is visited: decisions
-// of earlier-visited nodes applied
+// of earlier-visited nodes applied.  N is gone when a node above it was
+// coarsened; then its father was (a node is coarsened only when its sons are
+// leaves or coarsened, and sons come first), so the father's decision tells.
 __device__ __forceinline__ bool gm1_has_son(const Links &L, const int8_t *d, int32_t N, uint64_t rx) {
     if (N < 0) return false;
-    for (int32_t a = L.parent[N]; a >= 0; a = L.parent[a])
-        if (d[a] == D_COARSEN && L.rank[a] < rx) return false;
-    if (!L.leaf0[N]) return !(d[N] == D_COARSEN && L.rank[N] < rx);
-    return d[N] == D_REFINE && L.rank[N] < rx;
+    const int32_t p = L.parent[N];
+    const int8_t dn = d[N];
+    const bool leaf = L.leaf0[N];
+    if (p >= 0 && d[p] == D_COARSEN && L.rank[p] < rx) return false;
+    if (leaf) return dn == D_REFINE && L.rank[N] < rx;
+    return !(dn == D_COARSEN && L.rank[N] < rx);
 }
 // gridmodify1 decision of one node (src/mesh.F90:305-353) given the current
 // estimate of all decisions; a decision only reads decisions of nodes that
@@ -554,10 +558,10 @@ __global__ void k_gm1_decide(int64_t n, Links L, int8_t *d, int32_t *changed, in
     int8_t r = D_NONE;
     if (L.cross[x] == 0) {
         const uint64_t rx = L.rank[x];
-        const bool up = gm1_has_son(L, d, L.nb[4 * x + DIR_UP], rx);
-        const bool down = gm1_has_son(L, d, L.nb[4 * x + DIR_DOWN], rx);
-        const bool left = gm1_has_son(L, d, L.nb[4 * x + DIR_LEFT], rx);
-        const bool right = gm1_has_son(L, d, L.nb[4 * x + DIR_RIGHT], rx);
+        const int4 v = *reinterpret_cast<const int4 *>(L.nb + 4 * x);
+        const int32_t N[4] = {v.x, v.y, v.z, v.w};
+        const bool up = gm1_has_son(L, d, N[DIR_UP], rx), down = gm1_has_son(L, d, N[DIR_DOWN], rx);
+        const bool left = gm1_has_son(L, d, N[DIR_LEFT], rx), right = gm1_has_son(L, d, N[DIR_RIGHT], rx);
         if (L.leaf0[x]) {
             if ((left && right) || (up && down)) r = D_REFINE;
         } else {
@@ -583,10 +587,10 @@ __global__ void k_gm1_vals(NodeSet A, Links L, const int8_t *d, int lvl) {
     const int32_t *c = L.child + 4 * x;
     A.val[x] = mean4(A.val[c[0]], A.val[c[1]], A.val[c[2]], A.val[c[3]]);
 }
+// the node goes: its father was coarsened, or one further up, and so the father too
 __device__ __forceinline__ bool ancestor_coarsened(const Links &L, const int8_t *d, int32_t x) {
-    for (int32_t a = L.parent[x]; a >= 0; a = L.parent[a])
-        if (d[a] == D_COARSEN) return true;
-    return false;
+    const int32_t p = L.parent[x];
+    return p >= 0 && d[p] == D_COARSEN;
 }
 // did[0]: a node is refined or coarsened; did[1]: the longest chain of
 // coarsened nodes, each the father of the next; did[2]: their deepest level
@@ -841,7 +845,7 @@ __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-constexpr int GM4_CTAS = 8, GM4_THREADS = 1024;
+constexpr int GM4_CTAS = 16, GM4_THREADS = 1024;
 
 // The fixpoint, by one cluster of blocks: a sweep is all looks (four lanes
 // per leaf, one per direction), a cluster barrier, then the comparison of
@@ -851,11 +855,12 @@ constexpr int GM4_CTAS = 8, GM4_THREADS = 1024;
 // searches in a background cell's nodes, about 20 dependent L2 reads) times
 // the sweeps, not by the number of SMs.  One B200, two regrids of a developed
 // 128^2, 4-level four-quadrant run (82k leaves, 2029 refinements): 0.67 ms in
-// 39 sweeps (0.94 before a thread kept where its look's searches ended),
-// against 14.0 ms for visiting the leaves in order by one block; 256 x 64
-// double Mach at 4 levels, four regrids: 0.82 against 10.2 ms.
-__global__ void __cluster_dims__(GM4_CTAS, 1, 1) __launch_bounds__(GM4_THREADS)
-    k_gm4_fixpoint(NodeSet A, Geometry G, Gm4 M, uint64_t t0, int max_sweeps, Gm4Result *out) {
+// 39 sweeps with 8 blocks (0.94 before a thread kept where its look's searches
+// ended), 0.51 with 16, the largest cluster: the last sweeps' looks are several
+// a thread; against 14.0 ms for visiting the leaves in order by one block.
+// 256 x 64 double Mach at 4 levels, four regrids: 0.72 ms (0.82 with 8 blocks),
+// against 10.2.
+__global__ void __launch_bounds__(GM4_THREADS) k_gm4_fixpoint(NodeSet A, Geometry G, Gm4 M, uint64_t t0, int max_sweeps, Gm4Result *out) {
     const int nthr = GM4_CTAS * GM4_THREADS;
     const int me = blockIdx.x * GM4_THREADS + threadIdx.x;
     const int nlist = __ldcg(M.w + GW_NLIST);
@@ -944,6 +949,23 @@ __global__ void __cluster_dims__(GM4_CTAS, 1, 1) __launch_bounds__(GM4_THREADS)
         out->nl_time = nl;
         out->nl_key = nlkey;
     }
+}
+
+static cudaError_t launch_gm4_fixpoint(cudaStream_t s, const NodeSet &A, const Geometry &G, const Gm4 &M, uint64_t t0,
+                                       Gm4Result *res) {
+    cudaError_t e = cudaFuncSetAttribute(k_gm4_fixpoint, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(GM4_CTAS);
+    cfg.blockDim = dim3(GM4_THREADS);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = GM4_CTAS;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_gm4_fixpoint, A, G, M, t0, 1 << 16, res);
 }
 
 // The nodes of the set after the pass that come from node i of A, in key
@@ -1123,7 +1145,7 @@ static int gridmodify4_pass(fdm_handle *h, AmrCtx &X, bool *did) {
         FDM_CK(h, cudaMemsetAsync(M.w, 0, GW_WORDS * 4, h->s));
         k_gm4_triggers<<<nblk(4 * n, TB), TB, 0, h->s>>>(X.A, h->G, t0, list, M.w + GW_NLIST);
         FDM_CK(h, cudaEventRecord(h->gm4_ev[0], h->s));
-        k_gm4_fixpoint<<<GM4_CTAS, GM4_THREADS, 0, h->s>>>(X.A, h->G, M, t0, 1 << 16, res);
+        FDM_CK(h, launch_gm4_fixpoint(h->s, X.A, h->G, M, t0, res));
         FDM_CK(h, cudaEventRecord(h->gm4_ev[1], h->s));
         k_gm4_count<<<nblk(n, TB), TB, 0, h->s>>>(X.A, M, res, cnt);
         Gm4Result &hr = *reinterpret_cast<Gm4Result *>(h->pin);
