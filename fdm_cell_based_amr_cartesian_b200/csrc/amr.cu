@@ -3,6 +3,7 @@
 
 #include "handle.cuh"
 #include "ordered_sum.cuh"
+#include "scan.cuh"
 #include "topo.cuh"
 
 namespace fdm {
@@ -367,22 +368,15 @@ static void merge_into(fdm_handle *h, const uint64_t *keys, const uint8_t *leaf,
         k_merge_runs<<<nblk(n, 256), 256, 0, h->s>>>(keys, leaf, val, m, keys + m, leaf + m, val + m, n - m, out);
 }
 // exclusive scan of n counts and their total; *at_val: the prefix at index
-// at (0 <= at < n), read back in the same round trip (through pinned memory:
-// a copy to pageable memory is a round trip of its own).  Copies that the
-// caller queued before land with it.
+// at (0 <= at < n); nwords device words come back in h->pin in the same round
+// trip
 static int scan_total32(fdm_handle *h, const int32_t *in, int32_t *out, int64_t n, int64_t &total,
-                        int64_t at = -1, int64_t *at_val = nullptr) {
-    size_t bytes = 0;
-    FDM_CK(h, cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, (int)n, h->s));
-    FDM_CK(h, h->cub_tmp.ensure(bytes));
-    FDM_CK(h, cub::DeviceScan::ExclusiveSum(h->cub_tmp.p, bytes, in, out, (int)n, h->s));
+                        int64_t at = -1, int64_t *at_val = nullptr, const int32_t *words = nullptr, int nwords = 0) {
     int32_t *r = h->pin_scan();
-    FDM_CK(h, cudaMemcpyAsync(r, in + n - 1, 4, cudaMemcpyDeviceToHost, h->s));
-    FDM_CK(h, cudaMemcpyAsync(r + 1, out + n - 1, 4, cudaMemcpyDeviceToHost, h->s));
-    if (at_val && at >= 0 && at < n) FDM_CK(h, cudaMemcpyAsync(r + 2, out + at, 4, cudaMemcpyDeviceToHost, h->s));
+    FDM_CK(h, launch_scan(h, ScanArgs<int32_t>{in, out, n, r, nullptr, at_val ? at : -1, r + 1, words, h->pin, nwords}));
     FDM_CK(h, cudaStreamSynchronize(h->s));
-    total = (int64_t)r[0] + r[1];
-    if (at_val) *at_val = at >= n ? total : (int64_t)r[2];
+    total = (int64_t)r[0];
+    if (at_val) *at_val = at >= n ? total : (int64_t)r[1];
     return FDM_OK;
 }
 
@@ -398,9 +392,8 @@ int init_internal(fdm_handle *h) {
     int32_t *dl = cv.at<int32_t>(h->amr[8], 2), *deepest = h->pin;   // deepest leaf
     FDM_CK(h, cudaMemsetAsync(dl, 0, 4, h->s));
     k_anc_count<<<nblk(NL, TB), TB, 0, h->s>>>(NL, h->lkey.as<uint64_t>(), cnt, dl);
-    FDM_CK(h, cudaMemcpyAsync(deepest, dl, 4, cudaMemcpyDeviceToHost, h->s));
     int64_t ni = 0;
-    int rc = scan_total32(h, cnt, off, NL, ni);   // waits
+    int rc = scan_total32(h, cnt, off, NL, ni, -1, nullptr, dl, 1);   // waits
     if (rc) return rc;
     h->NInt = ni;
     if (ni == 0) return FDM_OK;
@@ -1095,8 +1088,7 @@ static int gridmodify1_pass(fdm_handle *h, AmrCtx &X, bool *did) {
         for (int k = 0; k < GM1_SWEEPS; ++k)
             k_gm1_decide<<<nblk(n, TB), TB, 0, h->s>>>(n, L, d, changed, k);
         k_gm1_count<<<nblk(n, TB), TB, 0, h->s>>>(X.A, L, d, cnt, ddid);
-        FDM_CK(h, cudaMemcpyAsync(h->pin, changed, (GM1_SWEEPS + 3) * 4, cudaMemcpyDeviceToHost, h->s));
-        AMR_RC(scan_total32(h, cnt, off, n, total));   // waits
+        AMR_RC(scan_total32(h, cnt, off, n, total, -1, nullptr, changed, GM1_SWEEPS + 3));   // waits
         for (int k = 0; k < GM1_SWEEPS; ++k) h->gm1_iters += k == 0 || r[k - 1] != 0;
         if (r[GM1_SWEEPS - 1] == 0) break;
     }
@@ -1150,9 +1142,9 @@ static int gridmodify4_pass(fdm_handle *h, AmrCtx &X, bool *did) {
         k_gm4_count<<<nblk(n, TB), TB, 0, h->s>>>(X.A, M, res, cnt);
         Gm4Result &hr = *reinterpret_cast<Gm4Result *>(h->pin);
         static_assert(sizeof(Gm4Result) <= fdm_handle::PIN_WORDS * 4, "the result must fit the pinned words");
-        FDM_CK(h, cudaMemcpyAsync(&hr, res, sizeof hr, cudaMemcpyDeviceToHost, h->s));
         int64_t total = 0;
-        AMR_RC(scan_total32(h, cnt, off, n, total));   // waits
+        AMR_RC(scan_total32(h, cnt, off, n, total, -1, nullptr, reinterpret_cast<const int32_t *>(res),
+                            sizeof hr / 4));   // waits
         float ms = 0.f;
         if (cudaEventElapsedTime(&ms, h->gm4_ev[0], h->gm4_ev[1]) == cudaSuccess) h->gm4_ms += ms;
         if (hr.w[GW_FULL]) { h->err = "gridmodify4 cascade exceeded its node pool"; return FDM_ERR_UNSUPPORTED; }

@@ -10,6 +10,7 @@
 #include <cub/cub.cuh>
 
 #include "handle.cuh"
+#include "scan.cuh"
 #include "topo.cuh"
 
 namespace fdm {
@@ -696,20 +697,6 @@ __global__ void k_validate(Tables T, const int32_t *__restrict__ face_counts, in
 }
 
 // ------------------------------------------------------------ host side
-// exclusive scan and its total, written on the device
-template <class U>
-static __global__ void k_scan_total(const U *__restrict__ in, const U *__restrict__ scan, int64_t n, U *out) {
-    if (threadIdx.x == 0) *out = n > 0 ? in[n - 1] + scan[n - 1] : U(0);
-}
-template <class U>
-static int scan_total(fdm_handle *h, const U *in, U *out, int64_t n, U *total) {
-    size_t bytes = 0;
-    FDM_CK(h, cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, (int)n, h->s));
-    FDM_CK(h, h->cub_tmp.ensure(bytes));
-    FDM_CK(h, cub::DeviceScan::ExclusiveSum(h->cub_tmp.p, bytes, in, out, (int)n, h->s));
-    k_scan_total<U><<<1, 32, 0, h->s>>>(in, out, n, total);
-    return FDM_OK;
-}
 static __global__ void k_iota_b(int64_t n, int32_t *a) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i < n) a[i] = (int32_t)i;
@@ -738,6 +725,21 @@ struct BuildWords {
     unsigned long long counts[8];  // [0] singular, [2] restrict requests, [4] restrict ghosts, [6] listed requests
 };
 static_assert(sizeof(BuildWords) <= fdm_handle::PIN_WORDS * 4, "the build's words must fit the pinned ones");
+// exclusive scan; its total goes to the word `total` of dw, and (read) all
+// words to the host, to be looked at after the next wait
+template <class U>
+static int scan_total(fdm_handle *h, const U *in, U *out, int64_t n, BuildWords *dw, U *total, bool read) {
+    ScanArgs<U> a{in, out, n, total, nullptr, -1, nullptr, nullptr, nullptr, 0};
+    if (read) {
+        a.total2 = reinterpret_cast<U *>(reinterpret_cast<char *>(h->pin) +
+                                         (reinterpret_cast<char *>(total) - reinterpret_cast<char *>(dw)));
+        a.words = reinterpret_cast<const int32_t *>(dw);
+        a.words_out = h->pin;
+        a.nwords = sizeof(BuildWords) / 4;
+    }
+    FDM_CK(h, launch_scan(h, a));
+    return FDM_OK;
+}
 static int read_back(fdm_handle *h, const BuildWords *&w) {
     FDM_CK(h, cudaMemcpyAsync(h->pin, h->tmp[7].p, sizeof(BuildWords), cudaMemcpyDeviceToHost, h->s));
     FDM_CK(h, cudaStreamSynchronize(h->s));
@@ -815,8 +817,9 @@ int build_tables(fdm_handle *h, int64_t n, const uint64_t *keys_in, const double
     unsigned long long *lkind = c2.at<unsigned long long>(h->tmp[2], 0), *before = c2.at<unsigned long long>(h->tmp[2], 1);
     FDM_CK(h, h->lcross.ensure(n));
     k_classify<<<nblk(n, TB), TB, 0, s>>>(lkey, n, h->G, lkind, h->lcross.as<int8_t>(), err);
-    FDM_RC(scan_total<unsigned long long>(h, lkind, before, n, &dw->leaves));
-    FDM_RC(read_back(h, w));
+    FDM_RC(scan_total<unsigned long long>(h, lkind, before, n, dw, &dw->leaves, true));
+    FDM_CK(h, cudaStreamSynchronize(s));
+    w = reinterpret_cast<const BuildWords *>(h->pin);
     if (w->err[BE_ROOT]) return arg_fail(h, "leaf key names a background cell outside the m x n grid");
     if (w->err[BE_PARTITION]) return arg_fail(h, "leaf set does not partition the background grid (gap, overlap or duplicate)");
     if (w->err[BE_LEVEL]) return arg_fail(h, "leaf level above the supported maximum (14)");
@@ -849,8 +852,8 @@ int build_tables(fdm_handle *h, int64_t n, const uint64_t *keys_in, const double
         Tables T = h->tables();
         k_resolve<<<nblk(NI, 128), 128, 0, s>>>(T, h->G, RO, h->ilvl.as<uint8_t>(), err, &dw->l_max);
     }
-    FDM_RC(scan_total<int32_t>(h, RO.flag, ridx, ne, &dw->nr));
-    FDM_RC(read_back(h, w));
+    FDM_RC(scan_total<int32_t>(h, RO.flag, ridx, ne, dw, &dw->nr, true));
+    FDM_CK(h, cudaStreamSynchronize(s));
     if (w->err[BE_NULLNB]) return arg_fail(h, "an interior leaf has a null stencil neighbour (fewer than 3 ghost layers?)");
     const int64_t NR = w->nr;
     h->NR = NR;
@@ -914,7 +917,7 @@ int build_tables(fdm_handle *h, int64_t n, const uint64_t *keys_in, const double
     }
     // the face counts come back with the final checks; until then the
     // buffers take their bound (at most one unshared left face per leaf)
-    FDM_RC(scan_total<unsigned long long>(h, u, ub, NI, reinterpret_cast<unsigned long long *>(dw->faces)));
+    FDM_RC(scan_total<unsigned long long>(h, u, ub, NI, dw, reinterpret_cast<unsigned long long *>(dw->faces), false));
     const int64_t nux_max = NI, nuy_max = NI;
     FDM_CK(h, h->ifxl.ensure(NI * 4));
     FDM_CK(h, h->ifyl.ensure(NI * 4));

@@ -194,14 +194,17 @@ static void drop_graph(fdm_handle *h) {
 // otherwise.  A re-captured graph of the same shape (the usual case after a
 // regrid: the same kernels with new sizes and table pointers) updates the
 // executable graph in place, which costs far less than instantiating it.
-static int step_graph(fdm_handle *h, cudaGraphExec_t *out, bool ghosts = false) {
+static bool graph_is_stale(fdm_handle *h, bool ghosts) {
     if (h->graph_version != h->table_version) {
         h->graph_stale[0] = h->graph_stale[1] = true;
         h->graph_version = h->table_version;
     }
+    return !(ghosts ? h->step_graph_g : h->step_graph) || h->graph_stale[ghosts ? 1 : 0];
+}
+static int step_graph(fdm_handle *h, cudaGraphExec_t *out, bool ghosts = false) {
     cudaGraphExec_t &slot = ghosts ? h->step_graph_g : h->step_graph;
     bool &stale = h->graph_stale[ghosts ? 1 : 0];
-    if (slot && !stale) {
+    if (!graph_is_stale(h, ghosts)) {
         *out = slot;
         return FDM_OK;
     }
@@ -675,11 +678,22 @@ int fdm_solute(fdm_handle *h, int64_t nsteps, int64_t *steps_done) {
         while (k + j < nsteps && j < 64 && !amr_due(h, it0 + j)) ++j;   // at most 64 before a look at tt
         const bool regrid = amr_due(h, it0 + j);
         RC(ensure_lambda(h));
-        cudaGraphExec_t gs = nullptr, gl = nullptr;   // iterations before the last, the last
-        RC(step_graph(h, &gs, h->p.iflag_amr != 0));
-        gl = gs;
-        if (regrid) RC(step_graph(h, &gl, false));
-        for (int64_t s = 0; s < j; ++s) FDM_CK(h, cudaGraphLaunch(s + 1 < j ? gs : gl, h->s));
+        // A graph of the step is worth its capture for the iterations between
+        // the first, which runs meanwhile, and one before a regrid, which has
+        // a form of its own: those two are queued kernel by kernel.
+        const bool refresh = h->p.iflag_amr != 0;
+        int64_t s = 0;
+        if (graph_is_stale(h, refresh) || j == 1) {
+            launch_step(h, refresh && !(regrid && j == 1));
+            ++s;
+        }
+        const int64_t last = regrid ? j - 1 : j;
+        if (s < last) {
+            cudaGraphExec_t g = nullptr;
+            RC(step_graph(h, &g, refresh));
+            for (; s < last; ++s) FDM_CK(h, cudaGraphLaunch(g, h->s));
+        }
+        if (s < j) launch_step(h, false);
         h->lam_fresh = true;
         RC(sync_scalars_from_device(h));
         FDM_CK(h, cudaGetLastError());
