@@ -498,6 +498,31 @@ __global__ void k_ref_emit(Tables T, const double4 *B0, const int8_t *rflag, con
     }
 }
 
+// The largest cluster of blocks, for the kernels that iterate: the hardware's
+// cluster barrier costs a fraction of a launch or a grid-wide barrier.
+constexpr int CLUSTER_CTAS = 16, CLUSTER_TB = 1024;
+__device__ __forceinline__ void cluster_barrier() {
+    __syncwarp();   // lanes come here from divergent loops
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <class... P, class... A>
+static cudaError_t launch_cluster(cudaStream_t s, void (*kernel)(P...), A... args) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(CLUSTER_CTAS);
+    cfg.blockDim = dim3(CLUSTER_TB);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CLUSTER_CTAS;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // ----------------------------------------------------------- gridmodify1
 struct Links {
     int32_t *parent, *child, *nb;   // child[4 n], nb[4 n] (up, down, right, left)
@@ -505,9 +530,7 @@ struct Links {
     uint8_t *leaf0;
     int8_t *cross;
 };
-__global__ void k_gm1_links(NodeSet A, Geometry G, Links L, int8_t *d) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= A.n) return;
+__device__ __forceinline__ void gm1_link(const NodeSet &A, const Geometry &G, const Links &L, int8_t *d, int64_t i) {
     d[i] = D_NONE;
     const uint64_t k = A.key[i];
     const int lvl = (int)(k & 15u);
@@ -521,6 +544,10 @@ __global__ void k_gm1_links(NodeSet A, Geometry G, Links L, int8_t *d) {
         L.nb[4 * i + d] = shift_key(G, k, d, nk) ? (int32_t)find_key_set(A, nk) : -1;
     }
     L.rank[i] = post_rank(k);
+}
+__global__ void k_gm1_links(NodeSet A, Geometry G, Links L, int8_t *d) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < A.n) gm1_link(A, G, L, d, i);
 }
 // "the same-level node N exists and has sons" when x is visited: decisions
 // of earlier-visited nodes applied.  N is gone when a node above it was
@@ -545,9 +572,7 @@ __device__ __forceinline__ bool gm1_has_son(const Links &L, const int8_t *d, int
 // dependencies follow the visit order) is reached.  changed: one word per
 // sweep; a sweep after one that changed nothing has nothing to do, so several
 // are queued without a look from the host.
-__global__ void k_gm1_decide(int64_t n, Links L, int8_t *d, int32_t *changed, int sweep) {
-    const int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (x >= n || (sweep > 0 && changed[sweep - 1] == 0)) return;
+__device__ __forceinline__ bool gm1_decide(const Links &L, int8_t *d, int64_t x) {   // true: the decision changed
     int8_t r = D_NONE;
     if (L.cross[x] == 0) {
         const uint64_t rx = L.rank[x];
@@ -567,10 +592,14 @@ __global__ void k_gm1_decide(int64_t n, Links L, int8_t *d, int32_t *changed, in
             if (all_leaf && ((!left && !right) || (!up && !down))) r = D_COARSEN;
         }
     }
-    if (r != d[x]) {
-        d[x] = r;
-        changed[sweep] = 1;
-    }
+    if (r == d[x]) return false;
+    d[x] = r;
+    return true;
+}
+__global__ void k_gm1_decide(int64_t n, Links L, int8_t *d, int32_t *changed, int sweep) {
+    const int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (x >= n || (sweep > 0 && changed[sweep - 1] == 0)) return;
+    if (gm1_decide(L, d, x)) changed[sweep] = 1;
 }
 // values of coarsened nodes, deepest level first (interpA of the sons as they
 // are at the node's visit)
@@ -587,9 +616,8 @@ __device__ __forceinline__ bool ancestor_coarsened(const Links &L, const int8_t 
 }
 // did[0]: a node is refined or coarsened; did[1]: the longest chain of
 // coarsened nodes, each the father of the next; did[2]: their deepest level
-__global__ void k_gm1_count(NodeSet A, Links L, const int8_t *d, int32_t *cnt, int32_t *did) {
-    const int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (x >= A.n) return;
+__device__ __forceinline__ void gm1_count(const NodeSet &A, const Links &L, const int8_t *d, int32_t *cnt, int32_t *did,
+                                          int64_t x) {
     const int8_t dx = d[x];
     cnt[x] = ancestor_coarsened(L, d, (int32_t)x) ? 0 : (dx == D_REFINE ? 5 : 1);
     if (dx == D_NONE) return;
@@ -600,6 +628,32 @@ __global__ void k_gm1_count(NodeSet A, Links L, const int8_t *d, int32_t *cnt, i
     const int lvl = (int)(A.key[x] & 15u);
     if (did[1] < chain) atomicMax(did + 1, chain);
     if (did[2] < lvl) atomicMax(did + 2, lvl);
+}
+__global__ void k_gm1_count(NodeSet A, Links L, const int8_t *d, int32_t *cnt, int32_t *did) {
+    const int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (x < A.n) gm1_count(A, L, d, cnt, did, x);
+}
+// The pass up to the counts in one launch of a cluster, for small sets: links,
+// sweeps until one changes nothing, counts.  w: [0..2] changes by sweep modulo
+// 3, GM1_DID.. the did words, then the sweeps; -1 there: not settled.
+enum { GM1_DID = 3, GM1_NSWEEPS = 6, GM1_W = 7 };
+__global__ void __launch_bounds__(CLUSTER_TB) k_gm1_pass(NodeSet A, Geometry G, Links L, int8_t *d, int32_t *cnt,
+                                                         int32_t *w) {
+    const int nthr = CLUSTER_CTAS * CLUSTER_TB, me = blockIdx.x * CLUSTER_TB + threadIdx.x, n = (int)A.n;
+    if (me < GM1_W) w[me] = 0;
+    for (int x = me; x < n; x += nthr) gm1_link(A, G, L, d, x);
+    cluster_barrier();
+    int sweep = 0;
+    for (;; ++sweep) {
+        bool changed = false;
+        for (int x = me; x < n; x += nthr) changed |= gm1_decide(L, d, x);
+        if (__any_sync(0xffffffffu, changed) && (threadIdx.x & 31) == 0) __stcg(w + sweep % 3, 1);
+        if (me == 0) __stcg(w + (sweep + 1) % 3, 0);   // last read before the barrier of the sweep before
+        cluster_barrier();
+        if (__ldcg(w + sweep % 3) == 0 || sweep > n + 2) break;
+    }
+    for (int x = me; x < n; x += nthr) gm1_count(A, L, d, cnt, w + GM1_DID, x);
+    if (me == 0) w[GM1_NSWEEPS] = sweep > n + 2 ? -1 : sweep + 1;
 }
 // mean: a coarsened node's value is formed here from its sons' (no chain of
 // coarsened nodes); otherwise k_gm1_vals has formed it
@@ -833,12 +887,6 @@ __device__ __forceinline__ void gm4_propose(const NodeSet &A, const Gm4 &M, int3
     M.refd[atomicAdd(M.w + GW_NREFD, 1)] = id;
 }
 
-__device__ __forceinline__ void cluster_barrier() {
-    __syncwarp();   // lanes come here from divergent loops
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-constexpr int GM4_CTAS = 16, GM4_THREADS = 1024;
 
 // The fixpoint, by one cluster of blocks: a sweep is all looks (four lanes
 // per leaf, one per direction), a cluster barrier, then the comparison of
@@ -853,9 +901,9 @@ constexpr int GM4_CTAS = 16, GM4_THREADS = 1024;
 // a thread; against 14.0 ms for visiting the leaves in order by one block.
 // 256 x 64 double Mach at 4 levels, four regrids: 0.72 ms (0.82 with 8 blocks),
 // against 10.2.
-__global__ void __launch_bounds__(GM4_THREADS) k_gm4_fixpoint(NodeSet A, Geometry G, Gm4 M, uint64_t t0, int max_sweeps, Gm4Result *out) {
-    const int nthr = GM4_CTAS * GM4_THREADS;
-    const int me = blockIdx.x * GM4_THREADS + threadIdx.x;
+__global__ void __launch_bounds__(CLUSTER_TB) k_gm4_fixpoint(NodeSet A, Geometry G, Gm4 M, uint64_t t0, int max_sweeps, Gm4Result *out) {
+    const int nthr = CLUSTER_CTAS * CLUSTER_TB;
+    const int me = blockIdx.x * CLUSTER_TB + threadIdx.x;
     const int nlist = __ldcg(M.w + GW_NLIST);
     int made = 0;        // made nodes that this sweep visits
     int sweep = 0;
@@ -942,23 +990,6 @@ __global__ void __launch_bounds__(GM4_THREADS) k_gm4_fixpoint(NodeSet A, Geometr
         out->nl_time = nl;
         out->nl_key = nlkey;
     }
-}
-
-static cudaError_t launch_gm4_fixpoint(cudaStream_t s, const NodeSet &A, const Geometry &G, const Gm4 &M, uint64_t t0,
-                                       Gm4Result *res) {
-    cudaError_t e = cudaFuncSetAttribute(k_gm4_fixpoint, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(GM4_CTAS);
-    cfg.blockDim = dim3(GM4_THREADS);
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = GM4_CTAS;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_gm4_fixpoint, A, G, M, t0, 1 << 16, res);
 }
 
 // The nodes of the set after the pass that come from node i of A, in key
@@ -1058,6 +1089,10 @@ static int emit_buffers(fdm_handle *h, int64_t n, Emit &E) {
         if (rc_) return rc_; \
     } while (0)
 
+// Node sets up to this size take gridmodify1 on one cluster: 5k nodes, 20
+// regrids 0.6 ms less than twelve operations a pass, 21k, four regrids 0.06; at
+// 60k its sixteen SMs are slower than a launch per sweep on all (0.45 ms more).
+constexpr int64_t GM1_CLUSTER_MAX = 32768;
 // One gridmodify1 pass over the node set A -> A; *did: a node was refined
 // or coarsened (otherwise A is left as it is).
 static int gridmodify1_pass(fdm_handle *h, AmrCtx &X, bool *did) {
@@ -1079,24 +1114,33 @@ static int gridmodify1_pass(fdm_handle *h, AmrCtx &X, bool *did) {
     int8_t *d = cv.at<int8_t>(b, 6);        // the decisions
     int32_t *changed = cv.at<int32_t>(b, 7), *ddid = changed + GM1_SWEEPS;
     int32_t *cnt = cv.at<int32_t>(b, 8), *off = cv.at<int32_t>(b, 9);
-    k_gm1_links<<<nblk(n, TB), TB, 0, h->s>>>(X.A, h->G, L, d);
-    const int32_t *r = h->pin;              // changed words, then did words
+    const int32_t *r = h->pin, *rdid = nullptr;   // changed words, then did words
     int64_t total = 0;
-    for (int64_t it = 0;; it += GM1_SWEEPS) {
-        if (it > n + 2 + GM1_SWEEPS) { h->err = "gridmodify1 decisions did not settle"; return FDM_ERR_UNSUPPORTED; }
-        FDM_CK(h, cudaMemsetAsync(changed, 0, (GM1_SWEEPS + 3) * 4, h->s));
-        for (int k = 0; k < GM1_SWEEPS; ++k)
-            k_gm1_decide<<<nblk(n, TB), TB, 0, h->s>>>(n, L, d, changed, k);
-        k_gm1_count<<<nblk(n, TB), TB, 0, h->s>>>(X.A, L, d, cnt, ddid);
-        AMR_RC(scan_total32(h, cnt, off, n, total, -1, nullptr, changed, GM1_SWEEPS + 3));   // waits
-        for (int k = 0; k < GM1_SWEEPS; ++k) h->gm1_iters += k == 0 || r[k - 1] != 0;
-        if (r[GM1_SWEEPS - 1] == 0) break;
+    if (n <= GM1_CLUSTER_MAX) {
+        FDM_CK(h, launch_cluster(h->s, k_gm1_pass, X.A, h->G, L, d, cnt, changed));
+        AMR_RC(scan_total32(h, cnt, off, n, total, -1, nullptr, changed, GM1_W));   // waits
+        if (r[GM1_NSWEEPS] < 0) { h->err = "gridmodify1 decisions did not settle"; return FDM_ERR_UNSUPPORTED; }
+        h->gm1_iters += r[GM1_NSWEEPS];
+        rdid = r + GM1_DID;
+    } else {
+        k_gm1_links<<<nblk(n, TB), TB, 0, h->s>>>(X.A, h->G, L, d);
+        for (int64_t it = 0;; it += GM1_SWEEPS) {
+            if (it > n + 2 + GM1_SWEEPS) { h->err = "gridmodify1 decisions did not settle"; return FDM_ERR_UNSUPPORTED; }
+            FDM_CK(h, cudaMemsetAsync(changed, 0, (GM1_SWEEPS + 3) * 4, h->s));
+            for (int k = 0; k < GM1_SWEEPS; ++k)
+                k_gm1_decide<<<nblk(n, TB), TB, 0, h->s>>>(n, L, d, changed, k);
+            k_gm1_count<<<nblk(n, TB), TB, 0, h->s>>>(X.A, L, d, cnt, ddid);
+            AMR_RC(scan_total32(h, cnt, off, n, total, -1, nullptr, changed, GM1_SWEEPS + 3));   // waits
+            for (int k = 0; k < GM1_SWEEPS; ++k) h->gm1_iters += k == 0 || r[k - 1] != 0;
+            if (r[GM1_SWEEPS - 1] == 0) break;
+        }
+        rdid = r + GM1_SWEEPS;
     }
-    *did = r[GM1_SWEEPS] != 0;
+    *did = rdid[0] != 0;
     if (!*did) return FDM_OK;   // every decision is "nothing": A stays
-    const int chain = r[GM1_SWEEPS + 1];
+    const int chain = rdid[1];
     if (chain > 1)              // sons first
-        for (int l = r[GM1_SWEEPS + 2]; l >= 0; --l)
+        for (int l = rdid[2]; l >= 0; --l)
             k_gm1_vals<<<nblk(n, TB), TB, 0, h->s>>>(X.A, L, d, l);
     // the emit keeps key order: a refined leaf's sons follow it directly and
     // lie before every later node (they fill the leaf's own span)
@@ -1137,7 +1181,7 @@ static int gridmodify4_pass(fdm_handle *h, AmrCtx &X, bool *did) {
         FDM_CK(h, cudaMemsetAsync(M.w, 0, GW_WORDS * 4, h->s));
         k_gm4_triggers<<<nblk(4 * n, TB), TB, 0, h->s>>>(X.A, h->G, t0, list, M.w + GW_NLIST);
         FDM_CK(h, cudaEventRecord(h->gm4_ev[0], h->s));
-        FDM_CK(h, launch_gm4_fixpoint(h->s, X.A, h->G, M, t0, res));
+        FDM_CK(h, launch_cluster(h->s, k_gm4_fixpoint, X.A, h->G, M, t0, 1 << 16, res));
         FDM_CK(h, cudaEventRecord(h->gm4_ev[1], h->s));
         k_gm4_count<<<nblk(n, TB), TB, 0, h->s>>>(X.A, M, res, cnt);
         Gm4Result &hr = *reinterpret_cast<Gm4Result *>(h->pin);
