@@ -210,6 +210,7 @@ __global__ void __launch_bounds__(TB, MINB) k_faces_fast(Tables T, const double4
                                                          int nbx) {
     const int64_t b = blockIdx.x;
     const double ig1 = 1.0 / (g - 1.0);
+    dep_begin();
     if (b < nbx) {
         const int64_t f = b * TB + threadIdx.x;
         if (f < T.NI + T.nux) fast::face_item<0>(T, cur, Fx, sc->lambda_x, g, ig1, f);
@@ -234,8 +235,8 @@ __global__ void __launch_bounds__(256, 2) k_faces_list_fast(Tables T, const doub
 template <int TB, int MINB>
 static void faces_fast(fdm_handle *h, const double4 *cur) {
     const int nbx = nblk(h->NI + h->nux, TB), nby = nblk(h->NI + h->nuy, TB);
-    k_faces_fast<TB, MINB><<<nbx + nby, TB, 0, h->s>>>(h->tables(), cur, h->Fx.as<double4>(), h->Fy.as<double4>(),
-                                                       h->scal.as<DevScalars>(), h->G.gama, nbx);
+    launch_after(h->s, nbx + nby, TB, k_faces_fast<TB, MINB>, h->tables(), cur, h->Fx.as<double4>(),
+                 h->Fy.as<double4>(), h->scal.as<DevScalars>(), h->G.gama, nbx);
 }
 
 // the launch shapes of the autotuner (stage.cu)

@@ -37,14 +37,13 @@ struct GateDir {
 __global__ void __launch_bounds__(128, 4) k_gate_linear(Tables T, const double4 *__restrict__ cur,
                                                         const float *__restrict__ P, float logit_thr,
                                                         float jump_thr, const DevScalars *__restrict__ sc, double g,
-                                                        GateDir X, GateDir Y, uint32_t *count) {
+                                                        double ig1, GateDir X, GateDir Y, uint32_t *count) {
     __shared__ GateWeights W;
     __shared__ XTile tiles[4];
     load_weights_smem(W, P);
     __syncthreads();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int64_t wx = (T.NI + T.nux + 31) / 32, wy = (T.NI + T.nuy + 31) / 32;
-    const double ig1 = 1.0 / (g - 1.0);
     XTile &Tt = tiles[wid];
     for (int k = GF; k < XLD; ++k) Tt.X[lane][k] = __float2bfloat16_rn(0.f);
     const GateFrag frag(W);
@@ -61,10 +60,9 @@ __global__ void __launch_bounds__(128, 4) k_gate_linear(Tables T, const double4 
 
 // Stages 2 and 3: the guard on the faces that were linear at stage 1.
 __global__ void __launch_bounds__(256) k_guard_linear(Tables T, const double4 *__restrict__ cur,
-                                                      const DevScalars *__restrict__ sc, double g, GateDir X,
-                                                      GateDir Y, uint32_t *count) {
+                                                      const DevScalars *__restrict__ sc, double g, double ig1,
+                                                      GateDir X, GateDir Y, uint32_t *count) {
     const int64_t wx = (T.NI + T.nux + 31) / 32, wy = (T.NI + T.nuy + 31) / 32;
-    const double ig1 = 1.0 / (g - 1.0);
     const int64_t w = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
     if (w < wx) guard_linear_chunk<0>(T, cur, X.F, X.jump1, sc->lambda_x, ig1, g, X.hard, count, w);
     else if (w < wx + wy)
@@ -434,12 +432,12 @@ void launch_gated_faces(fdm_handle *h, const double4 *cur, int krk) {
     if (krk == 1 || !h->gate_stage1_valid) {
         cudaMemsetAsync(cnt, 0, 2 * sizeof(uint32_t), h->s);
         k_gate_linear<<<(int)std::min<int64_t>(nblk(warps, 4), 4 * sms), 128, 0, h->s>>>(
-            T, cur, P, h->gate_logit_thr, h->gate_jump_thr, sc, h->G.gama, X, Y, cnt);
+            T, cur, P, h->gate_logit_thr, h->gate_jump_thr, sc, h->G.gama, 1.0 / (h->G.gama - 1.0), X, Y, cnt);
         cudaMemcpyAsync(cnt + 2, cnt, 2 * sizeof(uint32_t), cudaMemcpyDeviceToDevice, h->s);
         h->gate_stage1_valid = true;
     } else {
         cudaMemcpyAsync(cnt, cnt + 2, 2 * sizeof(uint32_t), cudaMemcpyDeviceToDevice, h->s);
-        k_guard_linear<<<nblk(warps, 8), 256, 0, h->s>>>(T, cur, sc, h->G.gama, X, Y, cnt);
+        k_guard_linear<<<nblk(warps, 8), 256, 0, h->s>>>(T, cur, sc, h->G.gama, 1.0 / (h->G.gama - 1.0), X, Y, cnt);
     }
     if (h->p.flux_variant == 1) {
         launch_faces_list_fast(h, cur, hx, hy, cnt, lx, ly);
