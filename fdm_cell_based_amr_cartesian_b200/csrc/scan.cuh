@@ -13,9 +13,9 @@ namespace fdm {
 // exchanged through distributed shared memory, and every block scans its part
 // from there.  The total, the prefix at one index and words that earlier
 // kernels left are stored where the caller wants them, pinned host memory
-// included.  against
-// five operations (scan in two launches, three copies) and the wait: a 3.8k-leaf
-// run with 20 regrids 23.3 -> 21.1 ms, a 45k-leaf one with four 8.8 -> 8.4.
+// included.  Against five operations (a scan in two launches, three copies):
+// a 3.8k-leaf run with 20 regrids 23.3 -> 21.1 ms, a 45k-leaf one with four
+// 8.8 -> 8.4.
 template <class U>
 struct ScanArgs {
     const U *in;
