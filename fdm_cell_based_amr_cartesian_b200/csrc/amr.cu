@@ -501,10 +501,6 @@ __global__ void k_ref_emit(Tables T, const double4 *B0, const int8_t *rflag, con
 // The largest cluster of blocks, for the kernels that iterate: the hardware's
 // cluster barrier costs a fraction of a launch or a grid-wide barrier.
 constexpr int CLUSTER_CTAS = 16, CLUSTER_TB = 1024;
-__device__ __forceinline__ void cluster_barrier() {
-    __syncwarp();   // lanes come here from divergent loops
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 template <class... P, class... A>
 static cudaError_t launch_cluster(cudaStream_t s, void (*kernel)(P...), A... args) {

@@ -229,6 +229,13 @@ inline cudaError_t launch_after(cudaStream_t s, unsigned grid, unsigned block, v
 // first statement of such a kernel, for all its threads: waits for the end of
 // the kernels before this one, whose writes are visible afterwards
 __device__ __forceinline__ void dep_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// barrier of all threads of a cluster, with their writes.  The aligned form
+// wants the warp's lanes together, and they may come here from lane-dependent
+// code or loops of different lengths: without the first line that is undefined.
+__device__ __forceinline__ void cluster_barrier() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 #endif
 
 // error helpers: record a message in the handle and return a status

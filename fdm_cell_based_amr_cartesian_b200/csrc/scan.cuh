@@ -78,7 +78,7 @@ __device__ __forceinline__ void scan_load(const ScanArgs<U> &a, int64_t i, U (&v
 template <class U>
 __device__ __forceinline__ U cluster_prefix(U mine, U &part, U &base) {
     if (threadIdx.x == 0) part = mine;
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_barrier();
     if (threadIdx.x < 32) {   // a lane per block
         U x = 0;
         if (threadIdx.x < blockIdx.x) {
@@ -94,7 +94,7 @@ __device__ __forceinline__ U cluster_prefix(U mine, U &part, U &base) {
         if (threadIdx.x == 0) base = x;
     }
     // base is set, and a block's part stays until every block has read it
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_barrier();
     return base;
 }
 template <class U>
