@@ -282,6 +282,7 @@ struct GateFrag {
                 w3[kc][i] = g == 0 ? *reinterpret_cast<const uint32_t *>(W.w3 + k) : 0u;
             }
         b3 = W.b3;
+        __syncwarp();   // w3 was read by some lanes only; the matrix instructions want all together
     }
 };
 // Inference forward of the 32 samples in T.X with the hidden activations
