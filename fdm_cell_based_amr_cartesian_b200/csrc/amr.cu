@@ -1,4 +1,6 @@
 // amr.cu — device regrid (src/solution.F90:408-589, src/mesh.F90:199-408).
+#include <algorithm>
+
 #include <cub/cub.cuh>
 
 #include "handle.cuh"
@@ -1155,14 +1157,23 @@ static int gridmodify4_pass(fdm_handle *h, AmrCtx &X, bool *did) {
     for (cudaEvent_t &e : h->gm4_ev)
         if (!e) FDM_CK(h, cudaEventCreate(&e));
     uint64_t t0 = 0;   // everything up to this time is in A already
+    int64_t pool = 0;
+    bool grown = false;
     for (;;) {
-        const int64_t n = X.A.n, cap = (n + 4096 + 3) / 4 * 4;   // room for as many new nodes as the set has
+        const int64_t n = X.A.n;
+        pool = std::max(pool, h->gm4_first_pool > 0 ? h->gm4_first_pool : n + 4096);   // as many new nodes as the set has
+        const int64_t cap = (pool + 3) / 4 * 4;
         Carve c;
         c.add((n + cap) * 8); c.add((n + cap) * 8); c.add((n + cap) * 4); c.add(2 * 8);   // set to all ones
         c.add(cap * 8); c.add(cap * 4); c.add((n + cap) * 4); c.add(n * 4);
         c.add(GW_WORDS * 4); c.add(sizeof(Gm4Result)); c.add(n * 4); c.add(n * 4);
-        FDM_CK(h, h->amr[15].ensure(c.total));
         DevBuf &b = h->amr[15];
+        if (const cudaError_t e = b.ensure(c.total); e != cudaSuccess) {
+            if (!grown || e != cudaErrorMemoryAllocation) return cuda_fail(h, e, "gridmodify4 nodes");
+            cudaGetLastError();   // the set is as it was: a refusal, not a loss
+            h->err = "gridmodify4 cascade exceeded its node pool, and memory has no room for a larger one";
+            return FDM_ERR_UNSUPPORTED;
+        }
         Gm4 M;
         M.t = c.at<uint64_t>(b, 0); M.tn = c.at<uint64_t>(b, 1); M.son = c.at<int32_t>(b, 2);
         M.nl = c.at<uint64_t>(b, 3); M.mkey = c.at<uint64_t>(b, 4); M.mfather = c.at<int32_t>(b, 5);
@@ -1187,7 +1198,18 @@ static int gridmodify4_pass(fdm_handle *h, AmrCtx &X, bool *did) {
                             sizeof hr / 4));   // waits
         float ms = 0.f;
         if (cudaEventElapsedTime(&ms, h->gm4_ev[0], h->gm4_ev[1]) == cudaSuccess) h->gm4_ms += ms;
-        if (hr.w[GW_FULL]) { h->err = "gridmodify4 cascade exceeded its node pool"; return FDM_ERR_UNSUPPORTED; }
+        if (hr.w[GW_FULL]) {
+            // A is untouched: the pass again with twice the room.  A node that
+            // one sweep refines and a later one does not keeps its sons, so a
+            // rough set can need more room than it ends with.
+            if (n + 2 * cap >= (1ll << 31) - 1) {
+                h->err = "gridmodify4 cascade exceeded its node pool";
+                return FDM_ERR_UNSUPPORTED;
+            }
+            pool = 2 * cap;
+            grown = true;
+            continue;
+        }
         if (hr.w[GW_STUCK]) { h->err = "gridmodify4 times did not settle"; return FDM_ERR_UNSUPPORTED; }
         h->gm4_visits += hr.w[GW_VISITS];
         h->gm4_nonleaf += hr.w[GW_NONLEAF];

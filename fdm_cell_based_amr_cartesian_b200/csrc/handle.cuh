@@ -133,6 +133,7 @@ struct fdm_handle {
     int64_t NInt = 0;
     fdm::DevBuf amr[22];     // regrid scratch: [0..5] node sets, [6, 7] their per-cell indices, [8..19] work
                              // arrays, [20, 21] new leaves
+    int64_t gm4_first_pool = 0;   // > 0: new nodes that a gridmodify4 pass has room for at first (tests)
     int64_t gm1_iters = 0, gm4_visits = 0, gm4_nonleaf = 0, gm4_triggers = 0, gm4_refines = 0, gm4_steps = 0;
     // device-timeline phases of the last regrid (events recorded on the stream)
     static constexpr int AMR_PHASES = 5;

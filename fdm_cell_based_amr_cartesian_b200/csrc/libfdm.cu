@@ -818,6 +818,15 @@ int fdm_debug_fail_alloc(int64_t after) {
     return FDM_OK;
 }
 
+// Room for new nodes with which a gridmodify4 pass starts, for tests of its
+// growth; 0 restores the usual one.
+int fdm_debug_gm4_pool(fdm_handle *h, int64_t nodes) {
+    CHECK_H(h);
+    if (nodes < 0 || nodes >= (1ll << 30)) return arg_fail(h, "pool size out of range");
+    h->gm4_first_pool = nodes;
+    return FDM_OK;
+}
+
 int fdm_get_counters(fdm_handle *h, fdm_counters *c) {
     CHECK_H(h);
     if (!c) return FDM_ERR_ARG;

@@ -47,6 +47,7 @@ EXPORTS = [
     "fdm_download_internal", "fdm_set_internal", "fdm_set_async", "fdm_debug_barrier_timeout",
     "fdm_debug_fail_alloc", "fdm_solute_paired", "fdm_output_error", "fdm_download_keys_async",
     "fdm_readback_wait", "fdm_gate_set_jump_rule", "fdm_debug_nr_fallbacks",
+    "fdm_debug_gm4_pool",
 ]
 
 
@@ -145,6 +146,7 @@ def load_library(path: str = LIB_PATH):
     L.fdm_set_async.argtypes = [vp, i32]
     L.fdm_debug_barrier_timeout.argtypes = [dp]
     L.fdm_debug_fail_alloc.argtypes = [i64]
+    L.fdm_debug_gm4_pool.argtypes = [vp, i64]
     L.fdm_solute_paired.argtypes = [vp, vp, i64, ctypes.POINTER(i64)]
     L.fdm_output_error.argtypes = [vp, dp, ctypes.POINTER(i64)]
     L.fdm_download_keys_async.argtypes = [vp, i64, u64p]

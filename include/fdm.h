@@ -285,6 +285,10 @@ int fdm_debug_barrier_timeout(double *seconds);
  * upload or regrid failed this way is left not loaded (FDM_ERR_STATE until
  * the next successful upload). */
 int fdm_debug_fail_alloc(int64_t after);
+/* Room for new nodes with which a gridmodify4 pass of this handle starts (it
+ * takes the pass again with more when that is not enough); 0: the usual room.
+ * For testing that growth. */
+int fdm_debug_gm4_pool(fdm_handle *h, int64_t nodes);
 /* AMR indicators rot/div of the interior leaves (src/solution.F90:424-466). */
 int fdm_debug_rot_div(fdm_handle *h, int64_t cap, double *rot, double *div,
                       double *srot_sdiv_ne);
