@@ -203,10 +203,10 @@ __device__ __forceinline__ void stage_request_geometry(const Tables &T, int64_t 
     const double *src = T.rq_geo + r0 * RQ_GEO;
     for (int k = threadIdx.x; k < nch; k += nthreads) {
         const unsigned d = (unsigned)__cvta_generic_to_shared(smem_geo + 2 * k);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src + 2 * k));
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src + 2 * k) : "memory");
     }
-    asm volatile("cp.async.commit_group;\n" ::);
-    asm volatile("cp.async.wait_group 0;\n" ::);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
 }
 

@@ -22,10 +22,16 @@ struct Prim { double r, u, v, p; };
 // A record (32 bytes, 32-byte aligned) in one 256-bit access: half the load
 // instructions and L1 wavefronts of two 128-bit ones.  Volatile: a load stays
 // behind the wait at a kernel's start, and a record read twice (once for each
-// half of the face flux) is not kept in registers in between.
+// half of the face flux) is not kept in registers in between.  The memory
+// clobber orders it against ordinary stores: the persistent batch kernel reads
+// hanging-node and ghost values so that an earlier phase of it stored (steps
+// of 2k to 1.03M leaves take the same time with and without it).
 __device__ __forceinline__ double4 load_record(const double4 *p) {
     double4 q;
-    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(q.x), "=d"(q.y), "=d"(q.z), "=d"(q.w) : "l"(p));
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(q.x), "=d"(q.y), "=d"(q.z), "=d"(q.w)
+                 : "l"(p)
+                 : "memory");
     return q;
 }
 __device__ __forceinline__ void store_record(double4 *p, const double4 &q) {
