@@ -239,9 +239,12 @@ static void faces_fast(fdm_handle *h, const double4 *cur) {
                  h->Fy.as<double4>(), h->scal.as<DevScalars>(), h->G.gama, nbx);
 }
 
-// the launch shapes of the autotuner (stage.cu)
+// the launch shapes of the autotuner, as many as the exact flux has (stage.cu)
+// but not the same ones.  ms per x+y pair of shapes 0 to 5 in order: 148k leaves
+// 0.0247 0.0248 0.0249 0.0257 0.0239 0.0240, 1.03M 0.162 0.162 0.162 0.164 0.151
+// 0.151; a handle starts with 0, which below 21k leaves none beats by 1 %.
 void launch_faces_fast(fdm_handle *h, const double4 *cur) {
-    switch (h->face_variant % 6) {
+    switch (h->face_variant % N_FACE_SHAPES) {
         case 1: faces_fast<128, 3>(h, cur); break;
         case 2: faces_fast<64, 8>(h, cur); break;
         case 3: faces_fast<256, 2>(h, cur); break;

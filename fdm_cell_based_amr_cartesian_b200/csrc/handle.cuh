@@ -275,6 +275,8 @@ inline int root_bits(const fdm_handle *h) {
 }
 // per-stage pipeline (stage.cu)
 void launch_requests(fdm_handle *h, const double4 *cur);
+constexpr int N_FACE_SHAPES = 6;   // launch shapes of the face kernels; a variant number stands for itself modulo this
+static_assert(N_FACE_SHAPES <= FDM_FACE_VARIANTS, "every shape needs a number");
 void launch_faces(fdm_handle *h, const double4 *cur, int krk);
 void launch_cells(fdm_handle *h, const double4 *cur, const double4 *un, double4 *next, int krk,
                   int mode, bool finalize = true);

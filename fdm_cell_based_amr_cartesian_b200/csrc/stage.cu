@@ -277,14 +277,6 @@ static void faces_pair(fdm_handle *h, const double4 *cur) {
     launch_after(h->s, nbx + nby, TB, k_faces_pair<TB, MINB>, h->tables(), cur, h->Fx.as<double4>(),
                  h->Fy.as<double4>(), h->scal.as<DevScalars>(), g, flux_den(g), nbx);
 }
-constexpr int N_FACE_SHAPES = 6;
-const char *face_variant_name(int v) {
-    static const char *const name[N_FACE_SHAPES] = {
-        "128 threads, >=4 blocks/SM (two lanes per face on small meshes)", "128 threads, >=3 blocks/SM", "64 threads, >=8 blocks/SM",
-        "256 threads, >=2 blocks/SM", "128 threads, >=5 blocks/SM", "128 threads, >=6 blocks/SM"};
-    return v >= 0 ? name[v % N_FACE_SHAPES] : "?";
-}
-
 void launch_faces(fdm_handle *h, const double4 *cur, int krk) {
     if (h->gate_on) {
         launch_gated_faces(h, cur, krk);

@@ -47,15 +47,10 @@ extern "C" int fdm_time_kernels(fdm_handle *h, int32_t reps, double *ms) {
     return FDM_OK;
 }
 
-namespace fdm {
-const char *face_variant_name(int v);
-constexpr int N_FACE_VARIANTS = FDM_FACE_VARIANTS;
-}
-
 // Autotuner: times every launch shape of the face kernel on the current leaf
 // set (CUDA events on the handle's stream, reps launches each, after one
 // untimed launch) and keeps the fastest.  ms[v] receives the average ms per
-// (x + y) launch pair of variant v.
+// (x + y) launch pair of variant v; the numbers past the shapes repeat theirs.
 extern "C" int fdm_autotune(fdm_handle *h, int32_t reps, int32_t *best, double *ms) {
     if (!h || reps <= 0) return FDM_ERR_ARG;
     if (!h->loaded) return FDM_ERR_STATE;
@@ -65,7 +60,7 @@ extern "C" int fdm_autotune(fdm_handle *h, int32_t reps, int32_t *best, double *
     const int keep = h->face_variant;
     double bt = 1e30;
     int bv = keep;
-    for (int v = 0; v < N_FACE_VARIANTS; ++v) {
+    for (int v = 0; v < N_FACE_SHAPES; ++v) {
         h->face_variant = v;
         launch_faces(h, h->B[0].as<double4>(), 1);
         FDM_CK(h, cudaEventRecord(e[0], h->s));
@@ -75,7 +70,8 @@ extern "C" int fdm_autotune(fdm_handle *h, int32_t reps, int32_t *best, double *
         float t = 0.f;
         FDM_CK(h, cudaEventElapsedTime(&t, e[0], e[1]));
         const double avg = (double)t / reps;
-        if (ms) ms[v] = avg;
+        if (ms)
+            for (int w = v; w < FDM_FACE_VARIANTS; w += N_FACE_SHAPES) ms[w] = avg;
         if (avg < bt) { bt = avg; bv = v; }
     }
     cudaEventDestroy(e[0]);
@@ -98,7 +94,7 @@ extern "C" int fdm_debug_nr_fallbacks(fdm_handle *h, int64_t *out) {
 }
 
 extern "C" int fdm_set_variant(fdm_handle *h, int32_t face_variant) {
-    if (!h || face_variant < 0 || face_variant >= N_FACE_VARIANTS) return FDM_ERR_ARG;
+    if (!h || face_variant < 0 || face_variant >= FDM_FACE_VARIANTS) return FDM_ERR_ARG;
     h->face_variant = face_variant;
     h->graph_version = -1;
     return FDM_OK;
