@@ -1064,8 +1064,8 @@ __global__ void k_split_emit(NodeSet A, const int32_t *ol, uint64_t *lk, double4
     else { ik[i - l] = A.key[i]; iv[i - l] = A.val[i]; }
 }
 
-// emission helper: count kernel already ran into cnt; scan; emit kernel fills
-// the unsorted arrays (B's storage); sort into the other set
+// where the refined and coarsened leaves and internal nodes are emitted, two
+// runs each in key order, before their merge into a node set
 struct Emit {
     uint64_t *key;
     uint8_t *leaf;

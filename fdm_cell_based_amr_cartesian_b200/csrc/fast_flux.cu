@@ -102,44 +102,6 @@ __device__ __forceinline__ double wcns_z3_f(double u1, double u2, double u3) {
     return (a1 * p1 + a2 * p2) / (a1 + a2);
 }
 
-template <int DIR>
-__device__ __forceinline__ void face_flux_f(const Prim &s0, const Prim &s1, const Prim &s2, const Prim &s3, double g,
-                                          double ig1, double lam, double out[4]) {
-    double U0[4], U1[4], U2[4], U3[4], F0[4], F1[4], F2[4], F3[4];
-    cons_flux_f<DIR>(s0, ig1, U0, F0);
-    cons_flux_f<DIR>(s1, ig1, U1, F1);
-    cons_flux_f<DIR>(s2, ig1, U2, F2);
-    cons_flux_f<DIR>(s3, ig1, U3, F3);
-    double Um[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) Um[r] = 0.5 * (U1[r] + U2[r]);
-    Eig E;
-    eigen_f<DIR>(Um, g, ig1, E);
-    double w0[4], w1[4], w2[4], w3[4];
-    double uwL[4], uwR[4], ugL[4], ugR[4];
-    project<DIR>(E, U0, w0); project<DIR>(E, U1, w1);
-    project<DIR>(E, U2, w2); project<DIR>(E, U3, w3);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        uwL[r] = wcns_z3_f(w0[r], w1[r], w2[r]);
-        uwR[r] = wcns_z3_f(w3[r], w2[r], w1[r]);
-    }
-    project<DIR>(E, F0, w0); project<DIR>(E, F1, w1);
-    project<DIR>(E, F2, w2); project<DIR>(E, F3, w3);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        ugL[r] = wcns_z3_f(w0[r], w1[r], w2[r]);
-        ugR[r] = wcns_z3_f(w3[r], w2[r], w1[r]);
-    }
-    double wL[4], wR[4], gL[4], gR[4];
-    back_project<DIR>(E, uwL, wL);
-    back_project<DIR>(E, uwR, wR);
-    back_project<DIR>(E, ugL, gL);
-    back_project<DIR>(E, ugR, gR);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) out[r] = 0.5 * (gL[r] + gR[r] - lam * (wR[r] - wL[r]));
-}
-
 // the same flux with the state half finished before the flux half, and the
 // stencil records read again for the flux half (fewer live registers)
 template <int DIR>

@@ -167,7 +167,5 @@ FDM_HD Node node_of_key(uint64_t key) {
 }
 // child quadrant of a node inside its father: q = xbit | ybit << 1
 FDM_HD int node_quadrant(const Node &n) { return (int)((n.ix & 1u) | ((n.iy & 1u) << 1)); }
-// reference sp (src/mesh.F90:204-258): son1 SW, son2 SE, son3 NE, son4 NW
-FDM_HD int quadrant_to_sp(int q) { return q == 0 ? 1 : q == 1 ? 2 : q == 3 ? 3 : 4; }
 
 }  // namespace fdm

@@ -166,7 +166,6 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
     return d;
 }
-__device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
 // D = A(16x16 bf16, row) * B(16x8 bf16, col) + C (f32)
 __device__ __forceinline__ void mma16816(float d[4], const uint32_t a[4], const uint32_t b[2], const float c[4]) {

@@ -264,15 +264,6 @@ inline int arg_fail(fdm_handle *h, const char *msg) {
 int build_tables(fdm_handle *h, int64_t n, const uint64_t *keys_dev, const double *prim_dev, int key_bits = 64);
 // *sorted: the keys ascend (waits for the stream)
 int keys_sorted(fdm_handle *h, int64_t n, const uint64_t *keys_dev, bool *sorted);
-// bits of the largest background-cell (root) index m*n - 1: a leaf key
-// (root << 34 | path << 4 | lvl) made on the device has no bit set at or
-// above 34 + root_bits, so radix sorts of such keys stop there
-inline int root_bits(const fdm_handle *h) {
-    const uint64_t top = (uint64_t)h->p.m * (uint64_t)h->p.n;
-    int b = 1;
-    while (b < 30 && (1ull << b) < top) ++b;
-    return b;
-}
 // per-stage pipeline (stage.cu)
 void launch_requests(fdm_handle *h, const double4 *cur);
 constexpr int N_FACE_SHAPES = 6;   // launch shapes of the face kernels; a variant number stands for itself modulo this
