@@ -1087,9 +1087,11 @@ static int emit_buffers(fdm_handle *h, int64_t n, Emit &E) {
         if (rc_) return rc_; \
     } while (0)
 
-// Node sets up to this size take gridmodify1 on one cluster: 5k nodes, 20
-// regrids 0.6 ms less than twelve operations a pass, 21k, four regrids 0.06; at
-// 60k its sixteen SMs are slower than a launch per sweep on all (0.45 ms more).
+// Node sets up to this size take gridmodify1 on one cluster.  The gridmodify
+// rounds of a regrid, ms, so and with a launch per sweep: 4k nodes 0.253
+// (0.298), 21k 0.298 (0.309), 28k 0.280 (0.298), 31k 0.262 (0.278), 36k 0.296
+// (0.292), 40k 0.294 (0.283), 53k 0.356 (0.337), 63k 0.354 (0.320): beyond,
+// sixteen SMs are slower than all of them.
 constexpr int64_t GM1_CLUSTER_MAX = 32768;
 // One gridmodify1 pass over the node set A -> A; *did: a node was refined
 // or coarsened (otherwise A is left as it is).

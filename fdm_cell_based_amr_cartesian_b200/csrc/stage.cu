@@ -308,9 +308,10 @@ static void launch_res_finalize(fdm_handle *h, bool keep_when_done, bool end) {
 }
 void launch_cells(fdm_handle *h, const double4 *cur, const double4 *un, double4 *next, int krk, int mode,
                   bool finalize) {
-    // three blocks per SM where the mesh fills them more than once (1.03 M
-    // leaves: the step 0.861 ms instead of 0.890); below four blocks on each
-    // of the 148 SMs the shorter code of two wins (148 k: 0.1578 ms against 0.1591)
+    // three blocks per SM above four blocks on each of the 148 SMs.  A step with
+    // three and with two, ms: 194k leaves 0.1924 (0.1935), 260k 0.244 (0.247),
+    // 328k 0.2915 (0.303), 402k 0.354 (0.365), 628k 0.543 (0.560), 1.03M 0.834
+    // (0.859); below the line, at 148k (two full waves of two), 0.1510 (0.1495).
     const unsigned nb = nblk(h->NI, 256);
     launch_after(h->s, nb, 256, nb > 4u * 148u ? k_cells<3> : k_cells<2>, h->tables(), h->lt, cur, un, next,
                  h->Fx.as<double4>(), h->Fy.as<double4>(), h->scal.as<DevScalars>(), h->res_part.as<double>(), krk, mode,
